@@ -1890,8 +1890,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
             if (final_c && (dyn & 2)) {
                 flush();
                 View dv = cur_view();
-                for (int pass = 0; pass < kSignedInsidePasses; ++pass)
-                    timed(kKDynamic, 1, [&] { launch_dynamic_collision(dv, nV, 2, S->stream); });
+                timed(kKDynamic, 1, [&] { launch_dynamic_collision(dv, nV, 2, S->stream); });
             }
             // Final pin polish whenever a contact stage ran: analytic
             // colliders, the SDF, or any last iteration (the dynamic

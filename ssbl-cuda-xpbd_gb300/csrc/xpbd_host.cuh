@@ -159,7 +159,8 @@ struct DynHost {
     int* large = nullptr;
     int *lflag = nullptr, *lpos = nullptr;  // large flags and their scan
     int *tcount = nullptr, *tstart = nullptr, *tent = nullptr, *scan_tmp = nullptr;
-    int* small = nullptr;         // large count, max bucket occupancy
+    int* small = nullptr;         // max bucket occupancy [0], span box [4..11]
+    int* pbox = nullptr;          // box of the particles' cells
     float4 *ppos = nullptr, *pprev = nullptr;
     float* prad = nullptr;
     int4* pcell = nullptr;

@@ -104,6 +104,7 @@ struct DynSet {
     const int* tent;
     const int* large;     // triangles spanning more than 64 cells, increasing id
     int large_count;
+    const int* tri_box;   // span box of the hashed triangles: lowest cell [0..2], highest [4..6]
     // particles
     int par_count;
     int par_motion_valid;
@@ -116,6 +117,7 @@ struct DynSet {
     const int4* par_cellc;
     const int* pstart;    // [par_buckets + 1]
     const int* pent;      // first 16 members of a bucket are queried
+    const int* par_box;   // box of the particles' cells, as tri_box
     // shared scene only: source id and collision layer per primitive
     const int* tri_src;
     const int* tri_layer;
@@ -428,7 +430,7 @@ void launch_sdf_build(const View& v, int cloth, int voxels, cudaStream_t s);
 // dynamic colliders: collision passes over all vertices (cloths without
 // colliders of the kind skip); `which` 0 unsigned triangles + particles
 // (cloths in unsigned mode), 1 signed triangles + particles, 2 signed
-// triangles inside-only
+// triangles inside-only (all its passes)
 void launch_dynamic_collision(const View& v, int V, int which, cudaStream_t s);
 constexpr int kSignedInsidePasses = 6;  // inside-only passes at the final constraints (abi41.cu:80)
 // exclusive scan of bucket counts into starts (counts become cursors)
