@@ -399,6 +399,7 @@ View Solver::view() const {
     v.sp_ent = sp_ent;
     v.te_off = te_off;
     v.te_ent = te_ent;
+    v.te_free = te_free ? 1 : 0;
     v.bj_off = bj_off;
     v.bj_ent = bj_ent;
     v.bends = bends;
@@ -529,6 +530,8 @@ void free_solver(Solver* S) {
     dfree(g.guard);
     dfree(g.max_delta_bits);
     dfree(S->pcg_blk);
+    dfree(S->hard_cloths);
+    dfree(S->hard_ranges);
     dfree(S->cap_edges);
     dfree(S->cap_rest);
     dfree(S->stage_idx);
@@ -1169,6 +1172,9 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
     std::vector<int2> sp_ent, te_ent, bj_ent;
     build_pair_csr(nV, springs, spring_rest, &sp_off, &sp_ent);
     build_pair_csr(nV, tethers, tether_rest, &te_off, &te_ent);
+    S->te_free = true;
+    for (const int2& t : tethers)
+        if (t.y >= 0 && t.y < nV && !(S->h_w[t.y] > 0.0f && std::isfinite(S->h_w[t.y]))) S->te_free = false;
     if (S->jacobi_bends) build_pair_csr(nV, jbends, jbend_rest, &bj_off, &bj_ent);
     S->h_pin_weight.assign(nV, -1.0f);
     S->h_pin_target.assign(nV, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
@@ -1381,7 +1387,8 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
     // does with them.
     std::vector<int2> cap_edges;
     std::vector<float> cap_rest;
-    std::vector<int> blk_cloth;
+    std::vector<int> blk_cloth, hard_cloths;
+    std::vector<int2> hard_ranges;
     if (ok && S->pcg_on) {
         S->pcg_nnz = 0;
         S->pcg_blocks = 0;
@@ -1405,6 +1412,10 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
             P.cap_jacobi = 0;
             if (!P.pcg_hard) continue;
             S->pcg_hard = true;
+            P.cap_tiny = 0;
+            for (int e = P.estart; e < P.estart + P.E; ++e)
+                if (!(spring_rest[e] > 7.5e-4f)) P.cap_tiny = 1;
+            S->cap_tiny |= P.cap_tiny != 0;
             if (S->cl[k].edge_colors.empty()) {
                 P.cap_jacobi = 1;
                 S->cap_jacobi = true;
@@ -1416,16 +1427,19 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
             ncol = std::max(ncol, (int)col_off[k].size() - 1);
         }
         S->cap_colors.assign(1, 0);
+        hard_ranges.assign((size_t)ncol * K, make_int2(0, 0));
         for (int c = 0; c < ncol; ++c) {
             for (int k = 0; k < K; ++k) {
                 const Params& P = S->hp[k];
                 if (!P.pcg_hard || c + 1 >= (int)col_off[k].size()) continue;
+                const int first = (int)cap_edges.size();
                 const int lo = std::min(std::max(col_off[k][c], 0), P.E), hi = std::min(std::max(col_off[k][c + 1], 0), P.E);
                 for (int e = lo; e < hi; ++e) {
                     const int ge = P.estart + col_order[k][e];
                     cap_edges.push_back(springs[ge]);
                     cap_rest.push_back(spring_rest[ge]);
                 }
+                hard_ranges[(size_t)c * K + k] = make_int2(first, (int)cap_edges.size() - first);
             }
             S->cap_colors.push_back((int)cap_edges.size());
         }
@@ -1444,6 +1458,25 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
              dalloc(&S->cap_edges, std::max(S->cap_count, 1), "cap edge allocation") &&
              dalloc(&S->cap_rest, std::max(S->cap_count, 1), "cap rest allocation");
         g.blk_cloth = S->pcg_blk;
+        int max_v = 0, degree = 1;
+        for (int k = 0; k < K; ++k)
+            if (S->hp[k].pcg_on) {
+                const Params& P = S->hp[k];
+                hard_cloths.push_back(k);
+                max_v = std::max(max_v, P.V);
+                degree = std::max(degree, (sp_off[P.vstart + P.V] - sp_off[P.vstart]) / std::max(P.V, 1) + 1);
+            }
+        HardPlan& h = S->hard;
+        hard_plan(&h, max_v, degree, (int)hard_cloths.size(), S->pcg_hard);
+        h.cloth_count = (int)hard_cloths.size();
+        h.count = S->cap_count;
+        h.colors = ncol;
+        ok = ok && dalloc(&S->hard_cloths, hard_cloths.size(), "PCG cloth list allocation") &&
+             dalloc(&S->hard_ranges, std::max<size_t>(hard_ranges.size(), 1), "cap range allocation");
+        h.cloths = S->hard_cloths;
+        h.edges = S->cap_edges;
+        h.rest = S->cap_rest;
+        h.ranges = S->hard_ranges;
     }
     if (!ok) return bail(0, "");
     cudaStream_t st = S->stream;
@@ -1482,6 +1515,8 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
         ok = (S->cap_count == 0 || (dupload(S->cap_edges, cap_edges.data(), S->cap_count, st, "cap edge upload") &&
                                     dupload(S->cap_rest, cap_rest.data(), S->cap_count, st, "cap rest upload"))) &&
              dupload(S->pcg_blk, blk_cloth.data(), blk_cloth.size(), st, "PCG block map upload") &&
+             dupload(S->hard_cloths, hard_cloths.data(), hard_cloths.size(), st, "PCG cloth list upload") &&
+             dupload(S->hard_ranges, hard_ranges.data(), hard_ranges.size(), st, "cap range upload") &&
              cuda_ok(cudaMemsetAsync(S->pcg.ticket, 0, sizeof(unsigned) * K, st), "reset PCG ticket") &&
              cuda_ok(cudaMemsetAsync(S->pcg.red, 0, sizeof(float) * kRedSlots * K, st), "reset PCG reductions") &&
              cuda_ok(cudaStreamSynchronize(st), "PCG buffer upload");
@@ -1700,6 +1735,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
     };
     // colour-range caps over the colour-sorted edge arrays
     auto caps = [&](int kind, int passes, bool both_ways) {
+        if (kind == 1 && !S->cap_tiny) return;
         View cv = cur_view();
         cv.edges = S->cap_edges;
         cv.edge_rest = S->cap_rest;
@@ -1730,6 +1766,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
         });
     };
     auto averaged = [&](bool tiny) {
+        if (tiny && !S->cap_tiny) return;
         View av = cur_view();
         timed(kKStretchCaps, 2, [&] { pcg_averaged_pass(av, S->pcg, nV, tiny, S->stream); });
     };
@@ -1755,9 +1792,12 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
                 // polish with normal and tiny caps, and the extreme caps
                 // (abi41.cu:9183-9201, 7806-7857, 7974-7995)
                 View gv = cur_view();
-                timed(kKPcg, 0, [&] { pcg_solve(gv, S->pcg, S->pcg_blocks, S->stream, &st->launches); });
+                if (S->hard.cluster)
+                    timed(kKPcg, 1, [&] { hard_cluster(gv, S->pcg, S->hard, false, S->stream); });
+                else
+                    timed(kKPcg, 0, [&] { pcg_solve(gv, S->pcg, S->pcg_blocks, S->stream, &st->launches); });
                 st->pcg_solves += 1;
-                if (hard) {
+                if (hard && !S->hard.cluster) {
                     for (int polish = 0; polish < 2; ++polish) {
                         averaged(false);
                         caps(0, 2, true);
@@ -1882,9 +1922,14 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
             // final ratio caps after the contacts (abi41.cu:9346-9350, 7997-8027)
             if (pcg && final_c && hard) {
                 flush();
-                caps(0, 2, true);
-                caps(2, 3, false);
-                caps(1, 3, false);
+                if (S->hard.cluster) {
+                    View gv = cur_view();
+                    timed(kKStretchCaps, 1, [&] { hard_cluster(gv, S->pcg, S->hard, true, S->stream); });
+                } else {
+                    caps(0, 2, true);
+                    caps(2, 3, false);
+                    caps(1, 3, false);
+                }
             }
             // inside-only signed passes at the final constraints (abi41.cu:9351-9360)
             if (final_c && (dyn & 2)) {

@@ -256,6 +256,7 @@ struct Solver {
     int2* sp_ent = nullptr;
     int* te_off = nullptr;
     int2* te_ent = nullptr;
+    bool te_free = false;   // every tether's dynamic end has a positive inverse mass
     int* vt_off = nullptr;  // vertex -> incident triangles (normals for pressure / fields)
     int* vt_tri = nullptr;
     float* p_area = nullptr;  // volume pressure per vertex (any cloth with pressure)
@@ -326,6 +327,10 @@ struct Solver {
     float* cap_rest = nullptr;
     int cap_count = 0;
     std::vector<int> cap_colors; // colour offsets into cap_edges
+    bool cap_tiny = false;       // some such cloth has edges for the tiny caps
+    HardPlan hard{};             // cluster form (cluster 0: launched)
+    int* hard_cloths = nullptr;
+    int2* hard_ranges = nullptr;
     int pcg_nnz = 0;
     long long pcg_iterations = 0;
 

@@ -181,6 +181,7 @@ struct Params {
     // polish and ratio caps); its CG blocks are [pcg_block0, + pcg_nblocks)
     int pcg_on, pcg_hard, pcg_block0, pcg_nblocks;
     int cap_jacobi;  // no caller edge colouring: each cap pass is one Jacobi pass over the cloth's edges
+    int cap_tiny;    // some edge is short enough for the tiny caps (rest <= 0.75 mm): without one they change nothing
     // external accelerations of the prediction (force fields, volume pressure)
     const SsblXpbdForceField* fields;  // field_count records (device)
     int field_count;
@@ -216,6 +217,23 @@ struct PcgView {
     const int* blk_cloth;  // cloth of each block of the solve grid
     unsigned long long* guard;
     unsigned* max_delta_bits;
+};
+
+// The cluster form of the hard-stretch solve: the cloths that run it, the
+// cluster size (0: launched form) and the colour-sorted cap edges with each
+// cloth's range per colour.
+constexpr int kHardMaxCluster = 16;
+constexpr int kHardMaxVertices = 2 * kHardMaxCluster * 1024;
+struct HardPlan {
+    const int* cloths;
+    int cloth_count, cluster;
+    int chunk, threads;  // vertices of the largest cloth and threads per CTA
+    int rows;            // matrix entries per CTA kept in shared memory
+    const int2* edges;
+    const float* rest;
+    int count;
+    const int2* ranges;  // [colours x K]: first cap edge, count
+    int colors;
 };
 
 // Launch configuration of the kernel classes (block sizes and tiles), chosen
@@ -267,6 +285,7 @@ struct View {
     const int2* sp_ent;
     const int* te_off;
     const int2* te_ent;
+    int te_free;          // every tether's dynamic end has a positive inverse mass
     const int* bj_off;    // bends as a gather when no colours are given
     const int2* bj_ent;
     const int2* bends;
@@ -383,6 +402,13 @@ void pcg_averaged_pass(const View& v, const PcgView& g, int V, bool tiny, cudaSt
 // edges [start, start + count) (v.edges / v.edge_rest / v.nE point at them)
 void pcg_cap_range(const View& v, int start, int count, int kind, cudaStream_t s);
 void pcg_cap_jacobi(const View& v, const PcgView& g, int V, int kind, cudaStream_t s);
+// Shape of the cluster form for `cloths` cloths of at most max_v vertices with
+// `degree` matrix entries per vertex, `hard`: some run caps (false: the
+// launched form is used); and
+// its launch: the solve with polish and caps, or the caps after the contacts
+// of a frame's last iteration.
+bool hard_plan(HardPlan* h, int max_v, int degree, int cloths, bool hard);
+void hard_cluster(const View& v, const PcgView& g, const HardPlan& h, bool final_caps, cudaStream_t s);
 void launch_predict(const View& v, int V, cudaStream_t s);
 // pass flags for launch_vertex_pass
 enum PassFlags : unsigned {
