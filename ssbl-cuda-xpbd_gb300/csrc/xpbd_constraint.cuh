@@ -13,8 +13,12 @@ namespace xg {
 // 1927-1980): corr = (pj - pi) * 0.18 * dlambda / len, dlambda = -C / (wi +
 // wj + compliance / dt^2), C = len - rest, capped at max(2.5 mm, min(0.1
 // rest, 25 mm)).  Returns false when both endpoints are fixed.
-__device__ __forceinline__ bool stretch_correction(float4 pi, float4 pj, float rest, float compliance, float dt, F3* corr_out,
-                                                   float* c_out, bool* clamped) {
+// alpha = compliance / dt^2 is the caller's (stretch_alpha): the quotient is
+// taken once per vertex or constraint rather than once per use.
+__device__ __forceinline__ float stretch_alpha(float compliance, float dt) { return fmaxf(compliance, 0.0f) / fmaxf(dt * dt, kEps); }
+
+__device__ __forceinline__ bool stretch_correction(float4 pi, float4 pj, float rest, float alpha, F3* corr_out, float* c_out,
+                                                   bool* clamped) {
     const float wi = pi.w, wj = pj.w;
     const float weight = wi + wj;
     *clamped = false;
@@ -22,14 +26,17 @@ __device__ __forceinline__ bool stretch_correction(float4 pi, float4 pj, float r
     const F3 delta = f3(pj) - f3(pi);
     const float len = sqrtf(fmaxf(dot3(delta, delta), kEps));
     const float c = len - rest;
-    const float alpha = fmaxf(compliance, 0.0f) / fmaxf(dt * dt, kEps);
     const float dlambda = -c / (weight + alpha);
     F3 corr = delta * (0.18f * dlambda / fmaxf(len, kEps));
-    const float corr_len = sqrtf(fmaxf(dot3(corr, corr), 0.0f));
+    const float corr_sq = fmaxf(dot3(corr, corr), 0.0f);
     const float max_corr = fmaxf(0.0025f, fminf(fmaxf(rest, 0.0f) * 0.10f, 0.025f));
-    if (corr_len > max_corr) {
-        corr = corr * (max_corr / fmaxf(corr_len, kEps));
-        *clamped = true;
+    // the root decides only near the cap: its rounding is far below the margin
+    if (!(corr_sq < max_corr * max_corr * 0.99999f)) {
+        const float corr_len = sqrtf(corr_sq);
+        if (corr_len > max_corr) {
+            corr = corr * (max_corr / fmaxf(corr_len, kEps));
+            *clamped = true;
+        }
     }
     *corr_out = corr;
     *c_out = c;
@@ -74,13 +81,16 @@ __device__ __forceinline__ bool bend_correction_k(float4 pi4, float4 pj4, float 
         *guard = true;
         return false;
     }
-    const float corr_len = len3(corr);
     const float max_corr = fmaxf(2.5e-4f, fminf(fmaxf(rest, thickness) * 0.08f, 0.020f));
-    if (!isfinite(corr_len) || corr_len <= 0.0f) return false;
-    if (corr_len > max_corr) {
-        corr = corr * (max_corr / fmaxf(corr_len, kEps));
-        *guard = true;
-        *clamped = true;
+    const float corr_sq = dot3(corr, corr);
+    if (!(corr_sq > 0.0f && corr_sq < max_corr * max_corr * 0.99999f)) {
+        const float corr_len = len3(corr);
+        if (!isfinite(corr_len) || corr_len <= 0.0f) return false;
+        if (corr_len > max_corr) {
+            corr = corr * (max_corr / fmaxf(corr_len, kEps));
+            *guard = true;
+            *clamped = true;
+        }
     }
     *corr_out = corr;
     return true;
@@ -101,8 +111,10 @@ __device__ __forceinline__ F3 velocity_update(F3 p, F3 prev, F3 vel, float w, fl
     const float max_delta = fmaxf(2.0e-4f, fmaxf(thickness, 0.0f) * 0.35f);
     const float max_speed = max_delta / sdt;
     F3 fb = proj * scale;
-    const float fspeed = len3(fb);
-    if (scale < 1.0f && isfinite(fspeed) && fspeed > max_speed && fspeed > kEps) fb = fb * (max_speed / fspeed);
+    if (scale < 1.0f && !(dot3(fb, fb) < max_speed * max_speed * 0.99999f)) {
+        const float fspeed = len3(fb);
+        if (isfinite(fspeed) && fspeed > max_speed && fspeed > kEps) fb = fb * (max_speed / fspeed);
+    }
     if (!finite3(fb)) fb = F3{0.0f, 0.0f, 0.0f};
     return base + fb;
 }

@@ -28,6 +28,7 @@
 #include <cstring>
 #include <vector>
 
+#include "xpbd_cluster.cuh"
 #include "xpbd_constraint.cuh"
 #include "xpbd_host.cuh"
 
@@ -111,7 +112,7 @@ __global__ void k_d_pass(DView d, unsigned flags, DState in, DState out) {
             F3 corr;
             float c;
             bool clamped;
-            if (!stretch_correction(pi, pj, d.edge_rest[e.y], d.kst[e.y], d.dt, &corr, &c, &clamped)) continue;
+            if (!stretch_correction(pi, pj, d.edge_rest[e.y], stretch_alpha(d.kst[e.y], d.dt), &corr, &c, &clamped)) continue;
             const float wself = self_is_j ? pj.w : pi.w;
             if (wself > 0.0f) {
                 const F3 dd = self_is_j ? corr * pj.w : corr * (-pi.w);
@@ -163,7 +164,7 @@ __global__ void k_d_bend(DView d, const int* order, int start, int count, DState
 // J^T g for corr = s delta (+ cap): returns d(corr . g)/d delta and, through
 // `dk`, d(corr . g)/d compliance.
 __device__ __forceinline__ F3 corr_adjoint(F3 delta, float len, float rest, float weight, float alpha, float gain, bool clamped,
-                                           float max_corr, float dt, float compliance, F3 g, float* dk) {
+                                           float max_corr, float dt, bool compliant, F3 g, float* dk) {
     const float inv = 1.0f / (weight + alpha);
     const float s = -gain * (len - rest) * inv / len;
     if (clamped) {
@@ -175,8 +176,40 @@ __device__ __forceinline__ F3 corr_adjoint(F3 delta, float len, float rest, floa
     const float q = -gain * rest * inv / (len * len * len);
     const float dg = dot3(delta, g);
     // d corr / d a = -s delta / (W + a); d a / d k = 1 / dt^2 for k > 0
-    *dk = compliance > 0.0f ? (-s * inv * dg) / fmaxf(dt * dt, kEps) : 0.0f;
+    *dk = compliant ? (-s * inv * dg) / fmaxf(dt * dt, kEps) : 0.0f;
     return g * s + delta * (q * dg);
+}
+
+// Velocity stage of a vertex, backwards: p and prev after the pin stage,
+// `base` the velocity before the stage; adds to the adjoints of p and prev
+// and replaces that of the velocity.
+__device__ __forceinline__ void velocity_back(F3 p, F3 prev, F3 base, float w, float thickness, float dt, F3* gp, F3* gq, F3* gv) {
+    F3 np{0.0f, 0.0f, 0.0f}, nq{0.0f, 0.0f, 0.0f}, nv{0.0f, 0.0f, 0.0f};
+    if (w > 0.0f) {
+        const float sdt = fmaxf(dt, kEps);
+        const F3 measured = (p - prev) * (1.0f / sdt);
+        const F3 proj = measured - base;
+        const float pdb = dot3(proj, base);
+        const float scale = (isfinite(pdb) && pdb > 0.0f) ? 0.9f : 1.0f;
+        const float max_delta = fmaxf(2.0e-4f, fmaxf(thickness, 0.0f) * 0.35f);
+        const float max_speed = max_delta / sdt;
+        const F3 fb = proj * scale;
+        const float fspeed = len3(fb);
+        F3 gproj;
+        if (scale < 1.0f && isfinite(fspeed) && fspeed > max_speed && fspeed > kEps) {
+            const float plen = len3(proj);
+            const F3 n = proj * (1.0f / plen);
+            gproj = (*gv - n * dot3(n, *gv)) * (max_speed / plen);
+        } else {
+            gproj = *gv * scale;
+        }
+        np = gproj * (1.0f / sdt);
+        nq = gproj * (-1.0f / sdt);
+        nv = *gv - gproj;
+    }
+    *gp = *gp + np;
+    *gq = *gq + nq;
+    *gv = nv;
 }
 
 // Velocity and pin stages of a pass, backwards: adjoint at the pass output
@@ -188,37 +221,8 @@ __global__ void k_d_stage_back(DView d, unsigned flags, DState in, DState out, c
     F3 gp = f3(ap[i]), gq = f3(aq[i]), gv = f3(av[i]);
     const float w = in.p[i].w;
     if (flags & kDVelocity) {
-        F3 np{0.0f, 0.0f, 0.0f}, nq{0.0f, 0.0f, 0.0f}, nv{0.0f, 0.0f, 0.0f};
-        // velocity stage inputs: x and prev after the pin stage (= pass
-        // output), velocity after the pin stage
         const bool pinned = (flags & kDPin) && d.pinned[i];
-        if (w > 0.0f) {
-            const float sdt = fmaxf(d.dt, kEps);
-            const F3 p = f3(out.p[i]), prev = f3(out.prev[i]);
-            const F3 base = pinned ? F3{0.0f, 0.0f, 0.0f} : f3(in.vel[i]);
-            const F3 measured = (p - prev) * (1.0f / sdt);
-            const F3 proj = measured - base;
-            const float pdb = dot3(proj, base);
-            const float scale = (isfinite(pdb) && pdb > 0.0f) ? 0.9f : 1.0f;
-            const float max_delta = fmaxf(2.0e-4f, fmaxf(d.thickness, 0.0f) * 0.35f);
-            const float max_speed = max_delta / sdt;
-            const F3 fb = proj * scale;
-            const float fspeed = len3(fb);
-            F3 gproj;
-            if (scale < 1.0f && isfinite(fspeed) && fspeed > max_speed && fspeed > kEps) {
-                const float plen = len3(proj);
-                const F3 n = proj * (1.0f / plen);
-                gproj = (gv - n * dot3(n, gv)) * (max_speed / plen);
-            } else {
-                gproj = gv * scale;
-            }
-            np = gproj * (1.0f / sdt);
-            nq = gproj * (-1.0f / sdt);
-            nv = gv - gproj;
-        }
-        gp = gp + np;
-        gq = gq + nq;
-        gv = nv;
+        velocity_back(f3(out.p[i]), f3(out.prev[i]), pinned ? F3{0.0f, 0.0f, 0.0f} : f3(in.vel[i]), w, d.thickness, d.dt, &gp, &gq, &gv);
     }
     if ((flags & kDPin) && d.pinned[i]) {
         gp = F3{0.0f, 0.0f, 0.0f};
@@ -228,6 +232,25 @@ __global__ void k_d_stage_back(DView d, unsigned flags, DState in, DState out, c
     mp[i] = f4(gp, 0.0f);
     mq[i] = f4(gq, 0.0f);
     mv[i] = f4(gv, 0.0f);
+}
+
+// One edge of the stretch gather, backwards: the adjoint of delta = xj - xi
+// from the endpoints' adjoints (mp of the position, mq of the previous one).
+__device__ __forceinline__ F3 edge_adjoint(float4 pi, float4 pj, float rest, float alpha, bool compliant, float dt, F3 mpi, F3 mqi,
+                                           F3 mpj, F3 mqj, float* dk) {
+    const float wi = pi.w, wj = pj.w, weight = wi + wj;
+    const F3 delta = f3(pj) - f3(pi);
+    const float len = sqrtf(fmaxf(dot3(delta, delta), kEps));
+    const float c = len - rest;
+    F3 corr;
+    float cc;
+    bool clamped;
+    stretch_correction(pi, pj, rest, alpha, &corr, &cc, &clamped);
+    const float kp = c > 0.0f ? 0.08f : 0.0f;
+    const F3 gi = (mpi + mqi * kp) * wi, gj = (mpj + mqj * kp) * wj;
+    const F3 g = gj - gi;
+    const float max_corr = fmaxf(0.0025f, fminf(fmaxf(rest, 0.0f) * 0.10f, 0.025f));
+    return corr_adjoint(delta, len, rest, weight, alpha, 0.18f, clamped, max_corr, dt, compliant, g, dk);
 }
 
 // Stretch gather, backwards: adjoint after the gather (mid) to the adjoint of
@@ -248,27 +271,37 @@ __global__ void k_d_gather_back(DView d, DState in, const float4* mp, const floa
         const int ii = self_is_j ? o : i, jj = self_is_j ? i : o;
         const float wi = pi.w, wj = pj.w, weight = wi + wj;
         if (weight <= 0.0f) continue;
-        const float rest = d.edge_rest[e.y], kc = d.kst[e.y];
-        const F3 delta = f3(pj) - f3(pi);
-        const float len = sqrtf(fmaxf(dot3(delta, delta), kEps));
-        const float c = len - rest;
-        const float alpha = fmaxf(kc, 0.0f) / fmaxf(d.dt * d.dt, kEps);
-        F3 corr;
-        float cc;
-        bool clamped;
-        stretch_correction(pi, pj, rest, kc, d.dt, &corr, &cc, &clamped);
-        const float kp = c > 0.0f ? 0.08f : 0.0f;
-        const F3 gi = (f3(mp[ii]) + f3(mq[ii]) * kp) * wi, gj = (f3(mp[jj]) + f3(mq[jj]) * kp) * wj;
-        const F3 g = gj - gi;
-        const float max_corr = fmaxf(0.0025f, fminf(fmaxf(rest, 0.0f) * 0.10f, 0.025f));
+        const float kc = d.kst[e.y];
         float dk;
-        const F3 adelta = corr_adjoint(delta, len, rest, weight, alpha, 0.18f, clamped, max_corr, d.dt, kc, g, &dk);
+        const F3 adelta = edge_adjoint(pi, pj, d.edge_rest[e.y], stretch_alpha(kc, d.dt), kc > 0.0f, d.dt, f3(mp[ii]), f3(mq[ii]),
+                                       f3(mp[jj]), f3(mq[jj]), &dk);
         acc = self_is_j ? acc + adelta : acc - adelta;
         if (!self_is_j) gk[e.y] += dk;
     }
     ap[i] = f4(acc, 0.0f);
     aq[i] = mq[i];
     av[i] = mv[i];
+}
+
+// One bend, backwards: the adjoint of delta = xj - xi; false when the bend was
+// skipped.
+__device__ __forceinline__ bool bend_adjoint(float4 pi4, float4 pj4, float rest, float kc, float thickness, float dt, F3 api, F3 aqi,
+                                             F3 apj, F3 aqj, F3* adelta, float* dk) {
+    F3 corr;
+    bool guard, clamped;
+    if (!bend_correction_k(pi4, pj4, rest, kc, thickness, dt, &corr, &guard, &clamped)) return false;
+    const float wi = pi4.w, wj = pj4.w, weight = wi + wj;
+    const F3 delta = f3(pj4) - f3(pi4);
+    const float len_sq = len_sq_xyz(delta);
+    const float inv_len = 1.0f / sqrtf(len_sq);
+    const float len = len_sq * inv_len;
+    const float alpha = fmaxf(kc, 0.0f) / fmaxf(dt * dt, kEps);
+    const F3 gi = wi > 0.0f ? (api + aqi * 0.06f) * wi : F3{0.0f, 0.0f, 0.0f};
+    const F3 gj = wj > 0.0f ? (apj + aqj * 0.06f) * wj : F3{0.0f, 0.0f, 0.0f};
+    const F3 g = gj - gi;
+    const float max_corr = fmaxf(2.5e-4f, fminf(fmaxf(rest, thickness) * 0.08f, 0.020f));
+    *adelta = corr_adjoint(delta, len, rest, weight, alpha, 0.10f, clamped, max_corr, dt, kc > 0.0f, g, dk);
+    return true;
 }
 
 // One bend colour backwards, in place on the adjoint (positions before the
@@ -282,23 +315,11 @@ __global__ void k_d_bend_back(DView d, const int* order, int start, int count, c
     const int2 pr = d.bends[b];
     const int i = pr.x, j = pr.y;
     if (i < 0 || j < 0 || i >= d.V || j >= d.V || i == j) return;
-    const float4 pi4 = before[i], pj4 = before[j];
-    const float rest = d.bend_rest[b], kc = d.kbd[b];
-    F3 corr;
-    bool guard, clamped;
-    if (!bend_correction_k(pi4, pj4, rest, kc, d.thickness, d.dt, &corr, &guard, &clamped)) return;
-    const float wi = pi4.w, wj = pj4.w, weight = wi + wj;
-    const F3 delta = f3(pj4) - f3(pi4);
-    const float len_sq = len_sq_xyz(delta);
-    const float inv_len = 1.0f / sqrtf(len_sq);
-    const float len = len_sq * inv_len;
-    const float alpha = fmaxf(kc, 0.0f) / fmaxf(d.dt * d.dt, kEps);
-    const F3 gi = wi > 0.0f ? (f3(ap[i]) + f3(aq[i]) * 0.06f) * wi : F3{0.0f, 0.0f, 0.0f};
-    const F3 gj = wj > 0.0f ? (f3(ap[j]) + f3(aq[j]) * 0.06f) * wj : F3{0.0f, 0.0f, 0.0f};
-    const F3 g = gj - gi;
-    const float max_corr = fmaxf(2.5e-4f, fminf(fmaxf(rest, d.thickness) * 0.08f, 0.020f));
+    F3 adelta;
     float dk;
-    const F3 adelta = corr_adjoint(delta, len, rest, weight, alpha, 0.10f, clamped, max_corr, d.dt, kc, g, &dk);
+    if (!bend_adjoint(before[i], before[j], d.bend_rest[b], d.kbd[b], d.thickness, d.dt, f3(ap[i]), f3(aq[i]), f3(ap[j]), f3(aq[j]),
+                      &adelta, &dk))
+        return;
     ap[j] = f4(f3(ap[j]) + adelta, 0.0f);
     ap[i] = f4(f3(ap[i]) - adelta, 0.0f);
     gk[b] += dk;
@@ -351,6 +372,393 @@ __global__ void k_d_unpack_grad(const float* g, float4* ap, float4* aq, float4* 
     av[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
+// -------------------------------------------------------- cluster form --
+// The whole rollout, or the whole backward sweep with its replays, by one
+// thread-block cluster, a vertex per thread.  The launched form is bound by
+// its launches: 37 per frame forward and about 100 more backward, 8 us each
+// issued one by one for a 64 x 64 cloth whose steps have a microsecond of
+// work.  Here a vertex's state, its adjoint and its constraint entries stay
+// on chip over all frames; only what neighbours read goes through shared
+// memory (positions, and backward the adjoints), by turns through two
+// buffers, so one barrier per gather suffices.  The tape of the frame being
+// differentiated is written and read by the same thread.
+// Per-vertex arithmetic and sum orders are the launched form's.
+struct DiffCluster {
+    int ctas, chunk, rows;   // CTAs, vertices and constraint entries per CTA
+    int frames, substeps, iterations;
+    int colours;             // bend colours: order[colour[c] .. colour[c + 1])
+    const int* colour;
+    const int* order;
+    const float4* init;      // 3 x V: state of frame 0
+    float4* ck;              // (frames + 1) x 3 x V
+    float4* tape;            // positions before each gather, then the velocity stages' rows, then the bends'
+    float* final_positions;  // forward
+    const float* grad;       // backward: dL/d(final positions), and the results
+    float *grad_stretch, *grad_bend;
+    int* lost;               // set when a barrier gave up
+};
+
+constexpr unsigned kEntSide = 1u, kEntCompliant = 2u, kEntAddr = ~7u;  // flags below the row address and its own bit
+
+__device__ __forceinline__ float4 z4() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+
+// What a vertex's thread carries from step to step.
+struct DiffVertex {
+    int i;            // vertex, -1 past the cloth
+    int begin, end;   // its entries in shared memory
+    float w;
+    bool pinned;
+    F3 p, prev, vel;
+};
+
+template <bool kOne>
+struct DiffBlock {
+    const DView& d;
+    const DiffCluster& a;
+    ClusterMap<kOne> map;
+    ClusterBarrier& bar;
+    float4* buf;             // 6 x chunk rows
+    unsigned* code;          // per entry: the neighbour's row address, side and compliance flags
+    float* rest;
+    float* alpha;
+    int turn;                // buffer of the next exchange
+    float4 *tape_p, *tape_v, *tape_b;
+
+    __device__ __forceinline__ unsigned row(int b) const { return 16u * (unsigned)(b * map.chunk); }
+
+    __device__ __forceinline__ void predict(DiffVertex& x) const {
+        if (x.i < 0) return;
+        const F3 old = x.p;
+        if (!(x.w > 0.0f)) {
+            x.vel = F3{0.0f, 0.0f, 0.0f};
+            x.p = f3(d.rest[x.i]);
+        } else {
+            const F3 accel = F3{d.gravity[0], d.gravity[1], d.gravity[2]} + F3{0.0f, 0.0f, 0.0f};
+            x.vel = x.vel + accel * d.dt;
+            x.vel = x.vel * d.damping;
+            x.p = old + x.vel * d.dt;
+        }
+        x.prev = old;
+        pin(x);
+    }
+    __device__ __forceinline__ void pin(DiffVertex& x) const {
+        if (x.i < 0 || !x.pinned) return;
+        x.p = f3(d.target[x.i]);
+        x.prev = x.p;
+        x.vel = F3{0.0f, 0.0f, 0.0f};
+    }
+    // Stretch gather from the positions all threads publish here.
+    // With `tape` the positions go there as well, between the two halves of
+    // the barrier: the arrival would wait for the store.
+    __device__ __forceinline__ void gather(DiffVertex& x, float4* tape) {
+        const int b = turn;
+        turn ^= 1;
+        if (x.i >= 0) buf[b * map.chunk + threadIdx.x] = f4(x.p, x.w);
+        bar.arrive();
+        if (tape && x.i >= 0) tape[x.i] = f4(x.p, x.w);
+        bar.finish();
+        if (x.i < 0) return;
+        const float4 p4 = f4(x.p, x.w);
+        // three entries at a time, their loads in flight together
+        for (int k = x.begin; k < x.end; k += 3) {
+            unsigned c[3];
+            float4 q[3];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                c[u] = code[min(k + u, x.end - 1)];
+                q[u] = ld_cluster<kOne>((c[u] & kEntAddr) + row(b));
+            }
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                if (k + u >= x.end) continue;
+                const bool self_is_j = (c[u] & kEntSide) != 0;
+                const float4 pi = self_is_j ? q[u] : p4, pj = self_is_j ? p4 : q[u];
+                F3 corr;
+                float cc;
+                bool clamped;
+                if (!stretch_correction(pi, pj, rest[k + u], alpha[k + u], &corr, &cc, &clamped)) continue;
+                if (x.w > 0.0f) {
+                    const F3 dd = self_is_j ? corr * x.w : corr * (-x.w);
+                    x.p = x.p + dd;
+                    if (cc > 0.0f) x.prev = x.prev + dd * 0.08f;
+                }
+            }
+        }
+    }
+    // Bend colours in place; with `record` the positions each bend started
+    // from go to the tape (by place in the colour order).
+    __device__ __forceinline__ void bends(DiffVertex& x, bool record) {
+        const int b = turn;
+        turn ^= 1;
+        const unsigned prev_row = row(2);
+        if (x.i >= 0) {
+            buf[b * map.chunk + threadIdx.x] = f4(x.p, x.w);
+            buf[2 * map.chunk + threadIdx.x] = f4(x.prev, 0.0f);
+        }
+        bar.sync();
+        for (int c = 0; c < a.colours; ++c) {
+            const int lo = __ldg(&a.colour[c]), hi = __ldg(&a.colour[c + 1]);
+            for (int k = lo + (int)(map.rank * blockDim.x + threadIdx.x); k < hi; k += a.ctas * (int)blockDim.x) {
+                const int e = __ldg(&a.order[k]);
+                if (e < 0 || e >= d.B) continue;
+                const int2 pr = __ldg(&d.bends[e]);
+                if (pr.x < 0 || pr.y < 0 || pr.x >= d.V || pr.y >= d.V || pr.x == pr.y) continue;
+                const unsigned ai = map.addr(pr.x), aj = map.addr(pr.y);
+                const float4 pi4 = ld_cluster<kOne>(ai + row(b)), pj4 = ld_cluster<kOne>(aj + row(b));
+                if (record) {
+                    tape_b[2 * (size_t)k] = pi4;
+                    tape_b[2 * (size_t)k + 1] = pj4;
+                }
+                F3 corr;
+                bool guard, clamped;
+                if (!bend_correction_k(pi4, pj4, d.bend_rest[e], d.kbd[e], d.thickness, d.dt, &corr, &guard, &clamped)) continue;
+                if (pi4.w > 0.0f) {
+                    const F3 dd = corr * (-pi4.w);
+                    st_cluster<kOne>(ai + row(b), f4(f3(pi4) + dd, pi4.w));
+                    st_cluster<kOne>(ai + prev_row, f4(f3(ld_cluster<kOne>(ai + prev_row)) + dd * 0.06f, 0.0f));
+                }
+                if (pj4.w > 0.0f) {
+                    const F3 dd = corr * pj4.w;
+                    st_cluster<kOne>(aj + row(b), f4(f3(pj4) + dd, pj4.w));
+                    st_cluster<kOne>(aj + prev_row, f4(f3(ld_cluster<kOne>(aj + prev_row)) + dd * 0.06f, 0.0f));
+                }
+            }
+            bar.sync();
+        }
+        if (x.i >= 0) {
+            x.p = f3(buf[b * map.chunk + threadIdx.x]);
+            x.prev = f3(buf[2 * map.chunk + threadIdx.x]);
+        }
+    }
+    // One frame; with `record` the tape gets what the backward sweep needs.
+    __device__ __forceinline__ void frame(DiffVertex& x, bool record) {
+        const size_t V = (size_t)d.V;
+        int g = 0;
+        for (int s = 0; s < a.substeps; ++s) {
+            predict(x);
+            for (int it = 0; it < a.iterations; ++it, ++g) {
+                gather(x, record ? tape_p + g * V : nullptr);
+                const bool last = it + 1 == a.iterations;
+                if (last && s + 1 == a.substeps && a.colours > 0) bends(x, record);
+                const F3 vel = x.vel;
+                pin(x);
+                if (!last || x.i < 0) continue;
+                if (record) {
+                    tape_v[(3 * s + 0) * V + x.i] = f4(vel, 0.0f);
+                    tape_v[(3 * s + 1) * V + x.i] = f4(x.p, 0.0f);
+                    tape_v[(3 * s + 2) * V + x.i] = f4(x.prev, 0.0f);
+                }
+                x.vel = velocity_update(x.p, x.prev, x.vel, x.w, d.thickness, d.dt);
+            }
+        }
+    }
+    // Backward through the recorded frame: the adjoint at its end becomes the
+    // adjoint at its start.  `gk` sums the compliance gradients of the entries
+    // whose first endpoint this vertex is.
+    __device__ __forceinline__ void back(const DiffVertex& x, F3& gp, F3& gq, F3& gv, float* gk) {
+        const size_t V = (size_t)d.V;
+        int g = a.substeps * a.iterations;
+        // tape rows are read one gather ahead of their use
+        float4 np = z4(), nv = z4(), vp = z4(), vq = z4();
+        auto ahead = [&](int gn, int sn) __attribute__((always_inline)) {
+            if (x.i < 0 || gn < 0) return;
+            np = tape_p[gn * V + x.i];
+            if (sn < 0) return;
+            nv = tape_v[(3 * sn + 0) * V + x.i];
+            vp = tape_v[(3 * sn + 1) * V + x.i];
+            vq = tape_v[(3 * sn + 2) * V + x.i];
+        };
+        ahead(g - 1, a.substeps - 1);
+        for (int s = a.substeps - 1; s >= 0; --s) {
+            for (int it = a.iterations - 1; it >= 0; --it) {
+                --g;
+                const bool last = it + 1 == a.iterations;
+                if (x.i >= 0) {
+                    if (last)
+                        velocity_back(f3(vp), f3(vq), x.pinned ? F3{0.0f, 0.0f, 0.0f} : f3(nv), x.w, d.thickness, d.dt, &gp, &gq, &gv);
+                    if (x.pinned) gp = gq = gv = F3{0.0f, 0.0f, 0.0f};
+                }
+                if (last && s + 1 == a.substeps && a.colours > 0) bends_back(x, gp, gq);
+                const float4 p4 = np;
+                const int b = publish_back(x, p4, gp, gq);
+                ahead(g - 1, it == 0 ? s - 1 : -1);
+                bar.finish();
+                gather_back(x, b, p4, gp, gq, gk);
+            }
+            if (x.i < 0) continue;
+            // prediction and its pin stage
+            if (x.pinned) gp = gq = gv = F3{0.0f, 0.0f, 0.0f};
+            if (x.w > 0.0f) {
+                const F3 gvel = gv + gp * d.dt;
+                gv = gvel * d.damping;
+                gp = gp + gq;
+            } else {
+                gv = F3{0.0f, 0.0f, 0.0f};
+                gp = gq;
+            }
+            gq = F3{0.0f, 0.0f, 0.0f};
+        }
+    }
+    // The rows neighbours read in gather_back (positions, adjoints of the
+    // position and of the previous position), up to the arrival at the barrier.
+    __device__ __forceinline__ int publish_back(const DiffVertex& x, float4 p4, F3 gp, F3 gq) {
+        const int b = 3 * turn;
+        turn ^= 1;
+        if (x.i >= 0) {
+            buf[b * map.chunk + threadIdx.x] = p4;
+            buf[(b + 1) * map.chunk + threadIdx.x] = f4(gp, 0.0f);
+            buf[(b + 2) * map.chunk + threadIdx.x] = f4(gq, 0.0f);
+        }
+        bar.arrive();
+        return b;
+    }
+    __device__ __forceinline__ void gather_back(const DiffVertex& x, int b, float4 p4, F3& gp, F3 gq, float* gk) const {
+        if (x.i < 0) return;
+        F3 acc = gp;
+        for (int k = x.begin; k < x.end; k += 2) {
+            unsigned c[2];
+            float4 q[2];
+            F3 op[2], oq[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                c[u] = code[min(k + u, x.end - 1)];
+                const unsigned o = c[u] & kEntAddr;
+                q[u] = ld_cluster<kOne>(o + row(b));
+                op[u] = f3(ld_cluster<kOne>(o + row(b + 1)));
+                oq[u] = f3(ld_cluster<kOne>(o + row(b + 2)));
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (k + u >= x.end) continue;
+                const bool self_is_j = (c[u] & kEntSide) != 0;
+                const float4 pi = self_is_j ? q[u] : p4, pj = self_is_j ? p4 : q[u];
+                if (pi.w + pj.w <= 0.0f) continue;
+                float dk;
+                const F3 adelta = edge_adjoint(pi, pj, rest[k + u], alpha[k + u], (c[u] & kEntCompliant) != 0, d.dt, self_is_j ? op[u] : gp,
+                                               self_is_j ? oq[u] : gq, self_is_j ? gp : op[u], self_is_j ? gq : oq[u], &dk);
+                acc = self_is_j ? acc + adelta : acc - adelta;
+                if (!self_is_j) gk[k + u] += dk;
+            }
+        }
+        gp = acc;
+    }
+    __device__ __forceinline__ void bends_back(const DiffVertex& x, F3& gp, F3 gq) {
+        const int b = 3 * turn;
+        turn ^= 1;
+        if (x.i >= 0) {
+            buf[b * map.chunk + threadIdx.x] = f4(gp, 0.0f);
+            buf[(b + 1) * map.chunk + threadIdx.x] = f4(gq, 0.0f);
+        }
+        bar.sync();
+        for (int c = a.colours - 1; c >= 0; --c) {
+            const int lo = __ldg(&a.colour[c]), hi = __ldg(&a.colour[c + 1]);
+            for (int k = lo + (int)(map.rank * blockDim.x + threadIdx.x); k < hi; k += a.ctas * (int)blockDim.x) {
+                const int e = __ldg(&a.order[k]);
+                if (e < 0 || e >= d.B) continue;
+                const int2 pr = __ldg(&d.bends[e]);
+                if (pr.x < 0 || pr.y < 0 || pr.x >= d.V || pr.y >= d.V || pr.x == pr.y) continue;
+                const unsigned ai = map.addr(pr.x) + row(b), aj = map.addr(pr.y) + row(b), q = row(1);
+                const F3 api = f3(ld_cluster<kOne>(ai)), apj = f3(ld_cluster<kOne>(aj));
+                F3 adelta;
+                float dk;
+                if (!bend_adjoint(tape_b[2 * (size_t)k], tape_b[2 * (size_t)k + 1], d.bend_rest[e], d.kbd[e], d.thickness, d.dt, api,
+                                  f3(ld_cluster<kOne>(ai + q)), apj, f3(ld_cluster<kOne>(aj + q)), &adelta, &dk))
+                    continue;
+                st_cluster<kOne>(aj, f4(apj + adelta, 0.0f));
+                st_cluster<kOne>(ai, f4(api - adelta, 0.0f));
+                a.grad_bend[e] += dk;
+            }
+            bar.sync();
+        }
+        if (x.i >= 0) gp = f3(buf[b * map.chunk + threadIdx.x]);
+    }
+};
+
+template <int T, bool kOne, bool kBack>
+__global__ void __launch_bounds__(T) k_d_cluster(DView d, DiffCluster a) {
+    extern __shared__ float4 sm[];
+    __shared__ unsigned long long s_counter;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = kOne ? 0 : (int)cluster.block_rank();
+    if (threadIdx.x == 0) {
+        ClusterBarrier::init(&s_counter, a.ctas);
+        ClusterBarrier::init_fence();
+    }
+    __syncthreads();
+    if (!kOne) cluster.sync();  // every CTA's counter is set before the first arrival
+    ClusterBarrier bar{smem_addr(&s_counter), 0u, a.ctas, false};
+    const size_t V = (size_t)d.V;
+    float4* buf = sm;
+    unsigned* code = reinterpret_cast<unsigned*>(buf + (kBack ? 6 : 3) * a.chunk);
+    float* rest = reinterpret_cast<float*>(code + a.rows);
+    float* alpha = rest + a.rows;
+    float* gk = alpha + a.rows;
+    DiffBlock<kOne> B{d, a, ClusterMap<kOne>(smem_addr(buf), a.chunk, rank), bar, buf, code, rest, alpha, 0, a.tape, nullptr, nullptr};
+    B.tape_v = B.tape_p + (size_t)a.substeps * a.iterations * V;
+    B.tape_b = B.tape_v + (size_t)a.substeps * 3 * V;
+    DiffVertex x;
+    const int l = rank * a.chunk + (int)threadIdx.x;
+    x.i = (int)threadIdx.x < a.chunk && l < d.V ? l : -1;
+    x.begin = x.end = 0;
+    x.w = 0.0f;
+    x.pinned = false;
+    int row0 = 0;
+    if (x.i >= 0) {
+        row0 = d.off[rank * a.chunk];
+        x.begin = d.off[x.i] - row0;
+        x.end = d.off[x.i + 1] - row0;
+        x.w = d.rest[x.i].w;
+        x.pinned = d.pinned[x.i] != 0;
+        for (int k = x.begin; k < x.end; ++k) {
+            const int2 e = d.ent[row0 + k];
+            const float kc = d.kst[e.y];
+            code[k] = B.map.addr(e.x & 0x7fffffff) | ((e.x & kSideBit) ? kEntSide : 0u) | (kc > 0.0f ? kEntCompliant : 0u);
+            rest[k] = d.edge_rest[e.y];
+            alpha[k] = stretch_alpha(kc, d.dt);
+            if (kBack) gk[k] = 0.0f;
+        }
+    }
+    auto load = [&](const float4* s) __attribute__((always_inline)) {
+        if (x.i < 0) return;
+        x.p = f3(s[x.i]);
+        x.prev = f3(s[V + x.i]);
+        x.vel = f3(s[2 * V + x.i]);
+    };
+    if (!kBack) {
+        load(a.init);
+        for (int f = 0; f <= a.frames; ++f) {
+            if (f > 0) B.frame(x, false);
+            if (x.i >= 0) {
+                float4* c = a.ck + (size_t)f * 3 * V;
+                c[x.i] = f4(x.p, x.w);
+                c[V + x.i] = f == 0 ? a.init[V + x.i] : f4(x.prev, 0.0f);
+                c[2 * V + x.i] = f4(x.vel, 0.0f);
+            }
+        }
+        if (x.i >= 0) {
+            a.final_positions[3 * x.i] = x.p.x;
+            a.final_positions[3 * x.i + 1] = x.p.y;
+            a.final_positions[3 * x.i + 2] = x.p.z;
+        }
+    } else {
+        F3 gp{0.0f, 0.0f, 0.0f}, gq{0.0f, 0.0f, 0.0f}, gv{0.0f, 0.0f, 0.0f};
+        if (x.i >= 0) gp = F3{a.grad[3 * x.i], a.grad[3 * x.i + 1], a.grad[3 * x.i + 2]};
+        for (int f = a.frames - 1; f >= 0; --f) {
+            load(a.ck + (size_t)f * 3 * V);
+            B.frame(x, true);
+            // the buffers change their use: nobody reads the last positions any more
+            bar.sync();
+            B.back(x, gp, gq, gv, gk);
+            bar.sync();
+        }
+        if (x.i >= 0)
+            for (int k = x.begin; k < x.end; ++k)
+                if (!(code[k] & kEntSide)) a.grad_stretch[d.ent[row0 + k].y] = gk[k];
+    }
+    if (bar.lost) *a.lost = 1;
+    bar.sync();  // no CTA leaves while another still reads its shared memory
+}
+
 // ---------------------------------------------------------------- host --
 
 struct Op {
@@ -384,6 +792,10 @@ struct DiffSolver {
     float4* adj = nullptr;          // 6 x V adjoint rows (output + mid)
     int frames = 0, substeps = 0, iterations = 0;
     std::vector<Op> ops;
+    // cluster form (ctas 0: the launched form is used)
+    int ctas = 0, chunk = 0, rows = 0;
+    int* colour = nullptr;          // colour offsets into `order`
+    int* lost = nullptr;
 
     DView view(float dt) const {
         DView d{};
@@ -413,7 +825,7 @@ void free_diff(DiffSolver* D) {
     if (!D) return;
     if (D->stream) cudaStreamSynchronize(D->stream);
     void* ptrs[] = {D->rest, D->off, D->ent, D->edge_rest, D->bends, D->bend_rest, D->order, D->pinned,
-                    D->target, D->kst, D->kbd, D->init, D->ck, D->tape, D->adj};
+                    D->target, D->kst, D->kbd, D->init, D->ck, D->tape, D->adj, D->colour, D->lost};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (D->stream) cudaStreamDestroy(D->stream);
@@ -443,7 +855,8 @@ bool ensure_buffers(DiffSolver* D, int frames) {
     const size_t V = (size_t)D->V;
     const size_t states = D->ops.size() + 1;
     const size_t ncol = D->colors.empty() ? 0 : D->colors.size() - 1;
-    const size_t need = states * 3 * V + ncol * V;
+    const size_t cluster_need = ((size_t)D->substeps * D->iterations + 3 * (size_t)D->substeps) * V + 2 * (size_t)D->B;
+    const size_t need = std::max(states * 3 * V + ncol * V, cluster_need);
     if (need > D->tape_states) {
         if (D->tape) cudaFree(D->tape);
         D->tape = nullptr;
@@ -532,6 +945,70 @@ void back_frame_ops(DiffSolver* D, float* gst, float* gbd) {
     }
 }
 
+// Shape of the cluster form: CTAs of at least 128 vertices, up to 16 of them
+// and 768 vertices each (12,288 in all: past that the launched form's
+// whole-chip passes are long enough to hide their launches, and two vertices
+// per thread would no longer fit the registers).
+constexpr int kDiffSmem = 220 * 1024;
+
+size_t diff_smem(const DiffSolver* D, bool back) { return (back ? 6 : 3) * 16 * (size_t)D->chunk + (back ? 16 : 12) * (size_t)D->rows; }
+
+template <int T, bool kOne, bool kBack>
+bool diff_cluster_fits(const DiffSolver* D) {
+    return cluster_fit(k_d_cluster<T, kOne, kBack>, D->ctas, T, kDiffSmem) > 0;
+}
+
+void plan_cluster(DiffSolver* D, const std::vector<int>& off) {
+    const int V = D->V;
+    int c = 1;
+    while (c < 16 && c * 128 < V) c *= 2;
+    const int chunk = std::max((V + 32 * c - 1) / (32 * c), 1) * 32;
+    if (chunk > 768) return;
+    int rows = 1;
+    for (int r = 0; r < c; ++r) rows = std::max(rows, off[std::min((r + 1) * chunk, V)] - off[std::min(r * chunk, V)]);
+    D->ctas = c;
+    D->chunk = chunk;
+    D->rows = rows;
+    const bool one = c == 1, small = chunk <= 384;
+    const bool fits = diff_smem(D, true) <= (size_t)kDiffSmem &&
+                      (one ? diff_cluster_fits<384, true, false>(D) && diff_cluster_fits<384, true, true>(D)
+                       : small ? diff_cluster_fits<384, false, false>(D) && diff_cluster_fits<384, false, true>(D)
+                               : diff_cluster_fits<768, false, false>(D) && diff_cluster_fits<768, false, true>(D));
+    if (!fits) D->ctas = 0;
+}
+
+template <bool kBack>
+bool run_cluster(DiffSolver* D, DiffCluster a, const char* what) {
+    a.ctas = D->ctas;
+    a.chunk = D->chunk;
+    a.rows = D->rows;
+    a.frames = D->frames;
+    a.substeps = D->substeps;
+    a.iterations = D->iterations;
+    a.colours = D->colors.empty() ? 0 : (int)D->colors.size() - 1;
+    a.colour = D->colour;
+    a.order = D->order;
+    a.init = D->init;
+    a.ck = D->ck;
+    a.tape = D->tape;
+    a.lost = D->lost;
+    const DView d = D->view(D->cfg.dt / (float)D->substeps);
+    const size_t smem = diff_smem(D, kBack);
+    if (!cuda_ok(cudaMemsetAsync(D->lost, 0, sizeof(int), D->stream), what)) return false;
+    cudaError_t e;
+    if (D->ctas == 1)
+        e = cluster_launch(k_d_cluster<384, true, kBack>, 1, 1, D->chunk, smem, D->stream, d, a);
+    else if (D->chunk <= 384)
+        e = cluster_launch(k_d_cluster<384, false, kBack>, 1, D->ctas, D->chunk, smem, D->stream, d, a);
+    else
+        e = cluster_launch(k_d_cluster<768, false, kBack>, 1, D->ctas, D->chunk, smem, D->stream, d, a);
+    int lost = 0;
+    if (!cuda_ok(e, what) || !cuda_ok(cudaMemcpyAsync(&lost, D->lost, sizeof(int), cudaMemcpyDeviceToHost, D->stream), what) ||
+        !cuda_ok(cudaStreamSynchronize(D->stream), what))
+        return false;
+    return lost ? fail(std::string(what) + ": a cluster barrier timed out") : true;
+}
+
 DiffSolver* as_diff(void* h) { return reinterpret_cast<DiffSolver*>(h); }
 
 }  // namespace
@@ -606,7 +1083,9 @@ XG_EXPORT void* xpbd_gb300_diff_create(const SsblXpbdConfig* config, const SsblX
               dalloc(&D->order, order.size(), "rollout allocation") && dalloc(&D->pinned, V, "rollout allocation") &&
               dalloc(&D->target, V, "rollout allocation") && dalloc(&D->kst, E, "rollout allocation") &&
               dalloc(&D->kbd, B, "rollout allocation") && dalloc(&D->init, 3 * (size_t)V, "rollout allocation") &&
-              dalloc(&D->adj, 6 * (size_t)V, "rollout allocation");
+              dalloc(&D->adj, 6 * (size_t)V, "rollout allocation") && dalloc(&D->lost, 1, "rollout allocation") &&
+              dalloc(&D->colour, std::max<size_t>(D->colors.size(), 1), "rollout allocation");
+    if (ok) plan_cluster(D, off);
     if (ok)
         ok = dupload(D->rest, rest4.data(), V, D->stream, "rollout upload") &&
              dupload(D->off, off.data(), off.size(), D->stream, "rollout upload") &&
@@ -615,6 +1094,7 @@ XG_EXPORT void* xpbd_gb300_diff_create(const SsblXpbdConfig* config, const SsblX
              dupload(D->bends, bends.data(), B, D->stream, "rollout upload") &&
              dupload(D->bend_rest, mesh->bend_rest_lengths, B, D->stream, "rollout upload") &&
              dupload(D->order, order.data(), order.size(), D->stream, "rollout upload") &&
+             dupload(D->colour, D->colors.data(), D->colors.size(), D->stream, "rollout upload") &&
              dupload(D->pinned, D->h_pinned.data(), V, D->stream, "rollout upload") &&
              dupload(D->target, D->h_target.data(), V, D->stream, "rollout upload") &&
              dupload(D->kst, kst.data(), E, D->stream, "rollout upload") &&
@@ -684,6 +1164,11 @@ XG_EXPORT int xpbd_gb300_diff_rollout(void* handle, const float* stretch_complia
          !cuda_ok(cudaMemcpyAsync(D->kbd, bend_compliance, sizeof(float) * D->B, cudaMemcpyDeviceToDevice, D->stream),
                   "copy bend compliance")))
         return 0;
+    if (D->ctas > 0) {
+        DiffCluster a{};
+        a.final_positions = final_positions;
+        return run_cluster<false>(D, a, "rollout") ? 1 : 0;
+    }
     // checkpoint 0 = initial state with the pins applied by the first predict
     cudaMemcpyAsync(D->ck, D->init, sizeof(float4) * 3 * (size_t)V, cudaMemcpyDeviceToDevice, D->stream);
     for (int f = 0; f < frames; ++f)
@@ -704,6 +1189,13 @@ XG_EXPORT int xpbd_gb300_diff_backward(void* handle, const float* grad_positions
     if ((D->E > 0 && !cuda_ok(cudaMemsetAsync(grad_stretch, 0, sizeof(float) * D->E, D->stream), "clear gradient")) ||
         (D->B > 0 && !cuda_ok(cudaMemsetAsync(grad_bend, 0, sizeof(float) * D->B, D->stream), "clear gradient")))
         return 0;
+    if (D->ctas > 0) {
+        DiffCluster a{};
+        a.grad = grad_positions;
+        a.grad_stretch = grad_stretch;
+        a.grad_bend = grad_bend;
+        return run_cluster<true>(D, a, "rollout backward") ? 1 : 0;
+    }
     k_d_unpack_grad<<<dblocks(V), kDiffThreads, 0, D->stream>>>(grad_positions, D->adj, D->adj + V, D->adj + 2 * (size_t)V, V);
     for (int f = D->frames - 1; f >= 0; --f) {
         // re-run frame f from its checkpoint, recording the tape

@@ -22,10 +22,9 @@
 // (k_hard_cluster) gives a cloth one thread-block cluster for the whole
 // solve and its caps, with a cluster barrier where the launched form has a
 // kernel boundary.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 
+#include "xpbd_cluster.cuh"
 #include "xpbd_solver.cuh"
 
 namespace xg {
@@ -746,90 +745,17 @@ __global__ void __launch_bounds__(kThreads) k_cap_store(View v, const float4* po
 constexpr int kHardSmem = 216 * 1024;
 constexpr int kHardColors = 64;  // edge colours the caps keep in shared memory
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned map_rank(unsigned addr, unsigned rank) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-// Loads and stores by vertex address: bit 31 marks the own CTA's memory,
-// which is read as plain shared memory (the cluster window's path is slower
-// even for it).
-constexpr unsigned kOwnBit = 0x80000000u;
-template <bool kOne>
-__device__ __forceinline__ float4 ld_cluster(unsigned addr) {
-    float4 x;
-    if (kOne || (addr & kOwnBit))
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(addr & ~kOwnBit) : "memory");
-    else
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(addr) : "memory");
-    return x;
-}
-template <bool kOne>
-__device__ __forceinline__ void st_cluster(unsigned addr, float4 x) {
-    if (kOne || (addr & kOwnBit))
-        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr & ~kOwnBit), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
-    else
-        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
-}
-// Barrier of a cluster: one thread per CTA arrives at every CTA's counter
-// after its own CTA's barrier; every thread then waits on its own counter.
-// The wait is bounded: when it runs out the barrier gives up for good and the
-// solve reports a bad status.
-struct HardBarrier {
-    unsigned counter, parity;
-    int ctas;
-    bool lost;
-    __device__ __forceinline__ void sync() {
-        __syncthreads();
-        if (ctas == 1) return;
-        if ((int)threadIdx.x < ctas)
-            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_rank(counter, threadIdx.x)) : "memory");
-        wait(counter, parity);
-        parity ^= 1u;
-    }
-    __device__ __forceinline__ void wait(unsigned bar, unsigned phase) {
-        unsigned done = lost ? 1u : 0u;
-        for (int tries = 0; !done; ++tries) {
-            asm volatile(
-                "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 100000;\nselp.u32 %0, 1, 0, p;\n}"
-                : "=r"(done)
-                : "r"(bar), "r"(phase)
-                : "memory");
-            if (!done && tries > 20000) lost = true, done = 1u;
-        }
-    }
-    // sync that also tells every CTA whether `mark` (of the own CTA, written
-    // before) holds `epoch` in some CTA; `any` is the cluster's answer, in one
-    // of two places by turns: the next answer may be written while a slower
-    // CTA still reads this one.
-    __device__ __forceinline__ bool sync_any(const volatile int* mark, volatile int* any, int epoch) {
-        if (ctas == 1) return __syncthreads_or(*mark == epoch);
-        __syncthreads();
-        if ((int)threadIdx.x < ctas && *mark == epoch)
-            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(map_rank(smem_addr((const void*)any), threadIdx.x)), "r"(epoch) : "memory");
-        sync();
-        return *any == epoch;
-    }
-};
-
-// Vertex state in the cluster's shared memory: vertex v0 + l lives in CTA
-// l / chunk (by the multiplier ceil(2^32 / chunk): exact for l < 2^16).
-// kOne: a cluster of one CTA, plain shared memory.
+// Vertex state in the cluster's shared memory: the own CTA's positions at the
+// map's base, the previous positions after them.
 template <bool kOne>
 struct ClusterState {
-    unsigned base;  // own CTA's positions; the previous positions follow
-    int v0, chunk;
-    unsigned mult, rank;
-    __device__ __forceinline__ unsigned addr(int i) const {
-        if (kOne) return (base + ((unsigned)(i - v0) << 4)) | kOwnBit;
-        const unsigned l = (unsigned)(i - v0), r = __umulhi(l, mult), a = base + ((l - r * chunk) << 4);
-        return r == rank ? (a | kOwnBit) : map_rank(a, r);
-    }
+    ClusterMap<kOne> map;
+    int v0;
+    __device__ __forceinline__ unsigned addr(int i) const { return map.addr(i - v0); }
     __device__ __forceinline__ float4 pos(int i) const { return ld_cluster<kOne>(addr(i)); }
-    __device__ __forceinline__ float4 prev(int i) const { return ld_cluster<kOne>(addr(i) + 16u * chunk); }
+    __device__ __forceinline__ float4 prev(int i) const { return ld_cluster<kOne>(addr(i) + 16u * map.chunk); }
     __device__ __forceinline__ void set_pos(int i, float4 x) const { st_cluster<kOne>(addr(i), x); }
-    __device__ __forceinline__ void set_prev(int i, float4 x) const { st_cluster<kOne>(addr(i) + 16u * chunk, x); }
+    __device__ __forceinline__ void set_prev(int i, float4 x) const { st_cluster<kOne>(addr(i) + 16u * map.chunk, x); }
 };
 
 __device__ __forceinline__ F3 next_direction(F3 d, F3 z, float beta) {
@@ -855,16 +781,16 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
     // partials of the launched grid's warps past the cluster's stay zero
     for (int k = threadIdx.x; k < 2 * kHardMaxVertices / 32; k += S) (&part[0][0])[k] = 0.0f;
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&s_counter)), "r"(C) : "memory");
-        for (int k = 0; k < 2; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_sum[k])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        ClusterBarrier::init(&s_counter, C);
+        for (int k = 0; k < 2; ++k) ClusterBarrier::init(&s_sum[k], 1);
+        ClusterBarrier::init_fence();
         s_mark = s_any[0] = s_any[1] = 0;
     }
     __syncthreads();
     const Params& P = sP;
     if (final_caps && !P.pcg_hard) return;  // uniform over the cluster
     if (C > 1) cluster.sync();  // every CTA's counter is set before the first arrival
-    HardBarrier bar{smem_addr(&s_counter), 0u, C, false};
+    ClusterBarrier bar{smem_addr(&s_counter), 0u, C, false};
     auto barrier = [&]() __attribute__((always_inline)) { bar.sync(); };
     const int lane = threadIdx.x & 31;
     const int V = P.V, v0 = P.vstart;
@@ -874,7 +800,7 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
     float4* s_off = sm + 5 * kChunk;
     unsigned* s_col = reinterpret_cast<unsigned*>(s_off + kRows);
     const int first = rank * kChunk + (int)threadIdx.x;  // local vertices first + n * S
-    const ClusterState<kOne> st{smem_addr(s_pos), v0, kChunk, (0xffffffffu / (unsigned)kChunk) + 1u, (unsigned)rank};
+    const ClusterState<kOne> st{ClusterMap<kOne>(smem_addr(s_pos), kChunk, rank), v0};
 #pragma unroll
     for (int n = 0; n < N; ++n) {
         const int t = (int)threadIdx.x + n * S, l = rank * kChunk + t;
@@ -1191,51 +1117,14 @@ void pcg_solve(const View& v, const PcgView& g, int blocks, cudaStream_t s, long
 namespace {
 
 template <int T, int N, bool kOne>
-cudaError_t hard_attributes() {
-    const cudaError_t e = cudaFuncSetAttribute(k_hard_cluster<T, N, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHardSmem);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_hard_cluster<T, N, kOne>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+int hard_fit(int c) {
+    return cluster_fit(k_hard_cluster<T, N, kOne>, c, T, kHardSmem);
 }
 
 template <int T, int N, bool kOne>
 void hard_launch(const View& v, const PcgView& g, const HardPlan& h, bool final_caps, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(h.cloth_count * h.cluster), 1, 1);
-    cfg.blockDim = dim3((unsigned)h.threads, 1, 1);
-    cfg.dynamicSmemBytes = (size_t)5 * 16 * h.chunk + 20 * (size_t)h.rows;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)h.cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_hard_cluster<T, N, kOne>, v, g, h, final_caps ? 1 : 0);
-}
-
-}  // namespace
-
-namespace {
-
-template <int T, int N, bool kOne>
-int hard_fit(int c) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)c, 1, 1);
-    cfg.blockDim = dim3(T, 1, 1);
-    cfg.dynamicSmemBytes = kHardSmem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)c;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int fit = 0;
-    if (hard_attributes<T, N, kOne>() != cudaSuccess || cudaOccupancyMaxActiveClusters(&fit, k_hard_cluster<T, N, kOne>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return fit;
+    cluster_launch(k_hard_cluster<T, N, kOne>, h.cloth_count, h.cluster, h.threads, (size_t)5 * 16 * h.chunk + 20 * (size_t)h.rows, s, v,
+                   g, h, final_caps ? 1 : 0);
 }
 
 }  // namespace

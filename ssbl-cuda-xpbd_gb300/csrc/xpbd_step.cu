@@ -211,12 +211,12 @@ __device__ void velocity_stage(const Params& P, float dt, VState* s) {
 // Stretch constraint of edge (i, j) seen from one of its endpoints
 // (abi41.cu:1927-1980): the correction is computed in the edge's own
 // orientation so both endpoints get bit-identical values.
-__device__ __forceinline__ void spring_term(const Params& P, unsigned long long* counts, float dt, float4 pi, float4 pj,
-                                            float rest, bool self_is_j, F3* dp, F3* dprev) {
+__device__ __forceinline__ void spring_term(unsigned long long* counts, float alpha, float4 pi, float4 pj, float rest,
+                                            bool self_is_j, F3* dp, F3* dprev) {
     F3 corr;
     float c;
     bool clamped;
-    if (!stretch_correction(pi, pj, rest, P.stretch_compliance, dt, &corr, &c, &clamped)) return;
+    if (!stretch_correction(pi, pj, rest, alpha, &corr, &c, &clamped)) return;
     if (clamped && !self_is_j) count1(counts, kCntHardFallbacks);
     const float wi = pi.w, wj = pj.w;
     const float wself = self_is_j ? wj : wi;
@@ -433,6 +433,7 @@ __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned 
         // 1,000-entry walk by one thread, 0.1 ms per frame of a 32 x 32 cloth).
         const bool skip = kind == 1 && v.te_free && !(p4.w > 0.0f);
         const int begin = __ldg(&off[i]), end = skip ? begin : __ldg(&off[i + 1]);
+        const float alpha = stretch_alpha(P.stretch_compliance, dt);
         F3 dp = s.p, dprev = s.prev;
         for (int k = begin; k < end; ++k) {
             const int2 e = __ldg(&ent[k]);
@@ -442,7 +443,7 @@ __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned 
             const float4 pi = self_is_j ? q4 : p4;
             const float4 pj = self_is_j ? p4 : q4;
             if (kind == 0)
-                spring_term(P, v.counts, dt, pi, pj, rest, self_is_j, &dp, &dprev);
+                spring_term(v.counts, alpha, pi, pj, rest, self_is_j, &dp, &dprev);
             else if (kind == 1)
                 tether_term(P, v.counts, dt, pi, pj, rest, self_is_j, v.te_free != 0, &dp, &dprev);
             else
