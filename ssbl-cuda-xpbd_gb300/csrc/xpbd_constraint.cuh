@@ -17,16 +17,13 @@ namespace xg {
 // taken once per vertex or constraint rather than once per use.
 __device__ __forceinline__ float stretch_alpha(float compliance, float dt) { return fmaxf(compliance, 0.0f) / fmaxf(dt * dt, kEps); }
 
-__device__ __forceinline__ bool stretch_correction(float4 pi, float4 pj, float rest, float alpha, F3* corr_out, float* c_out,
-                                                   bool* clamped) {
-    const float wi = pi.w, wj = pj.w;
-    const float weight = wi + wj;
+// The correction of an edge with a free endpoint; denom = wi + wj + alpha.
+__device__ __forceinline__ void stretch_step(F3 pi, F3 pj, float rest, float denom, F3* corr_out, float* c_out, bool* clamped) {
     *clamped = false;
-    if (weight <= 0.0f) return false;
-    const F3 delta = f3(pj) - f3(pi);
+    const F3 delta = pj - pi;
     const float len = sqrtf(fmaxf(dot3(delta, delta), kEps));
     const float c = len - rest;
-    const float dlambda = -c / (weight + alpha);
+    const float dlambda = -c / denom;
     F3 corr = delta * (0.18f * dlambda / fmaxf(len, kEps));
     const float corr_sq = fmaxf(dot3(corr, corr), 0.0f);
     const float max_corr = fmaxf(0.0025f, fminf(fmaxf(rest, 0.0f) * 0.10f, 0.025f));
@@ -40,6 +37,14 @@ __device__ __forceinline__ bool stretch_correction(float4 pi, float4 pj, float r
     }
     *corr_out = corr;
     *c_out = c;
+}
+
+__device__ __forceinline__ bool stretch_correction(float4 pi, float4 pj, float rest, float alpha, F3* corr_out, float* c_out,
+                                                   bool* clamped) {
+    const float weight = pi.w + pj.w;
+    *clamped = false;
+    if (weight <= 0.0f) return false;
+    stretch_step(f3(pi), f3(pj), rest, weight + alpha, corr_out, c_out, clamped);
     return true;
 }
 

@@ -163,9 +163,9 @@ __global__ void k_d_bend(DView d, const int* order, int start, int count, DState
 
 // J^T g for corr = s delta (+ cap): returns d(corr . g)/d delta and, through
 // `dk`, d(corr . g)/d compliance.
-__device__ __forceinline__ F3 corr_adjoint(F3 delta, float len, float rest, float weight, float alpha, float gain, bool clamped,
-                                           float max_corr, float dt, bool compliant, F3 g, float* dk) {
-    const float inv = 1.0f / (weight + alpha);
+__device__ __forceinline__ F3 corr_adjoint(F3 delta, float len, float rest, float denom, float gain, bool clamped, float max_corr,
+                                           float dt, bool compliant, F3 g, float* dk) {
+    const float inv = 1.0f / denom;
     const float s = -gain * (len - rest) * inv / len;
     if (clamped) {
         const F3 n = delta * (1.0f / len);
@@ -236,21 +236,22 @@ __global__ void k_d_stage_back(DView d, unsigned flags, DState in, DState out, c
 
 // One edge of the stretch gather, backwards: the adjoint of delta = xj - xi
 // from the endpoints' adjoints (mp of the position, mq of the previous one).
-__device__ __forceinline__ F3 edge_adjoint(float4 pi, float4 pj, float rest, float alpha, bool compliant, float dt, F3 mpi, F3 mqi,
+// denom = wi + wj + alpha.
+__device__ __forceinline__ F3 edge_adjoint(float4 pi, float4 pj, float rest, float denom, bool compliant, float dt, F3 mpi, F3 mqi,
                                            F3 mpj, F3 mqj, float* dk) {
-    const float wi = pi.w, wj = pj.w, weight = wi + wj;
+    const float wi = pi.w, wj = pj.w;
     const F3 delta = f3(pj) - f3(pi);
     const float len = sqrtf(fmaxf(dot3(delta, delta), kEps));
     const float c = len - rest;
     F3 corr;
     float cc;
     bool clamped;
-    stretch_correction(pi, pj, rest, alpha, &corr, &cc, &clamped);
+    stretch_step(f3(pi), f3(pj), rest, denom, &corr, &cc, &clamped);
     const float kp = c > 0.0f ? 0.08f : 0.0f;
     const F3 gi = (mpi + mqi * kp) * wi, gj = (mpj + mqj * kp) * wj;
     const F3 g = gj - gi;
     const float max_corr = fmaxf(0.0025f, fminf(fmaxf(rest, 0.0f) * 0.10f, 0.025f));
-    return corr_adjoint(delta, len, rest, weight, alpha, 0.18f, clamped, max_corr, dt, compliant, g, dk);
+    return corr_adjoint(delta, len, rest, denom, 0.18f, clamped, max_corr, dt, compliant, g, dk);
 }
 
 // Stretch gather, backwards: adjoint after the gather (mid) to the adjoint of
@@ -273,7 +274,7 @@ __global__ void k_d_gather_back(DView d, DState in, const float4* mp, const floa
         if (weight <= 0.0f) continue;
         const float kc = d.kst[e.y];
         float dk;
-        const F3 adelta = edge_adjoint(pi, pj, d.edge_rest[e.y], stretch_alpha(kc, d.dt), kc > 0.0f, d.dt, f3(mp[ii]), f3(mq[ii]),
+        const F3 adelta = edge_adjoint(pi, pj, d.edge_rest[e.y], weight + stretch_alpha(kc, d.dt), kc > 0.0f, d.dt, f3(mp[ii]), f3(mq[ii]),
                                        f3(mp[jj]), f3(mq[jj]), &dk);
         acc = self_is_j ? acc + adelta : acc - adelta;
         if (!self_is_j) gk[e.y] += dk;
@@ -300,7 +301,7 @@ __device__ __forceinline__ bool bend_adjoint(float4 pi4, float4 pj4, float rest,
     const F3 gj = wj > 0.0f ? (apj + aqj * 0.06f) * wj : F3{0.0f, 0.0f, 0.0f};
     const F3 g = gj - gi;
     const float max_corr = fmaxf(2.5e-4f, fminf(fmaxf(rest, thickness) * 0.08f, 0.020f));
-    *adelta = corr_adjoint(delta, len, rest, weight, alpha, 0.10f, clamped, max_corr, dt, kc > 0.0f, g, dk);
+    *adelta = corr_adjoint(delta, len, rest, weight + alpha, 0.10f, clamped, max_corr, dt, kc > 0.0f, g, dk);
     return true;
 }
 
@@ -374,19 +375,31 @@ __global__ void k_d_unpack_grad(const float* g, float4* ap, float4* aq, float4* 
 
 // -------------------------------------------------------- cluster form --
 // The whole rollout, or the whole backward sweep with its replays, by one
-// thread-block cluster, a vertex per thread.  The launched form is bound by
-// its launches: 37 per frame forward and about 100 more backward, 8 us each
-// issued one by one for a 64 x 64 cloth whose steps have a microsecond of
-// work.  Here a vertex's state, its adjoint and its constraint entries stay
-// on chip over all frames; only what neighbours read goes through shared
-// memory (positions, and backward the adjoints), by turns through two
-// buffers, so one barrier per gather suffices.  The tape of the frame being
-// differentiated is written and read by the same thread.
-// Per-vertex arithmetic and sum orders are the launched form's.
+// thread-block cluster.  The launched form is bound by its launches: 37 per
+// frame forward and about 100 more backward, 8 us each issued one by one for a
+// 64 x 64 cloth whose steps have a microsecond of work.  Here a vertex's state
+// and adjoint stay in its thread's registers over all frames; only what
+// neighbours read goes through shared memory (positions, and backward the
+// adjoints), by turns through two buffers, so one cluster barrier per gather
+// suffices.  The tape of the frame being differentiated is written and read
+// by the same thread.
+//
+// On 16 SMs a gather is bound by instruction issue (the correction's root and
+// quotients), so each CTA computes every edge of its vertices once, an edge
+// per thread, and a vertex then adds its edges' results in its entry order:
+// half the corrections of a gather that computes an edge at both ends.  Only
+// the edges between two CTAs are computed by both.  Values and sum orders are
+// the launched form's.  64 x 64, 20 frames, forward and backward: launched
+// 19.2 ms, cluster with an edge per vertex entry 5.9 ms, as here 5.1 ms.
 struct DiffCluster {
-    int ctas, chunk, rows;   // CTAs, vertices and constraint entries per CTA
+    int ctas, chunk;         // CTAs, vertices per CTA
+    int edge_rows, ent_rows; // space for a CTA's edges and its vertices' entries
     int frames, substeps, iterations;
     int colours;             // bend colours: order[colour[c] .. colour[c + 1])
+    const int* cta_off;      // CTA's edges: cta_edge[cta_off[r] .. cta_off[r + 1])
+    const int* cta_edge;     // edge ids, increasing
+    const int2* ends;        // edge -> endpoints
+    const int* cta_ent;      // per constraint entry: its edge's place among the CTA's | side bit
     const int* colour;
     const int* order;
     const float4* init;      // 3 x V: state of frame 0
@@ -398,7 +411,9 @@ struct DiffCluster {
     int* lost;               // set when a barrier gave up
 };
 
-constexpr unsigned kEntSide = 1u, kEntCompliant = 2u, kEntAddr = ~7u;  // flags below the row address and its own bit
+// Flags of an edge's endpoint address, below the row address and its own bit:
+// both endpoints fixed, compliance above zero; the first endpoint is this CTA's.
+constexpr unsigned kEdgeFixed = 1u, kEdgeCompliant = 2u, kEdgeMine = 4u, kEdgeAddr = ~7u;
 
 __device__ __forceinline__ float4 z4() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
 
@@ -417,10 +432,11 @@ struct DiffBlock {
     const DiffCluster& a;
     ClusterMap<kOne> map;
     ClusterBarrier& bar;
-    float4* buf;             // 6 x chunk rows
-    unsigned* code;          // per entry: the neighbour's row address, side and compliance flags
-    float* rest;
-    float* alpha;
+    float4* buf;             // rows neighbours read: 3 (forward) or 6 x chunk
+    float4* result;          // per edge: correction and whether the edge is stretched, or the adjoint of its delta
+    uint4* edge;             // per edge: endpoint row addresses, rest length, denominator
+    int* ent;                // per entry: edge | side bit
+    int edges;
     int turn;                // buffer of the next exchange
     float4 *tape_p, *tape_v, *tape_b;
 
@@ -457,32 +473,24 @@ struct DiffBlock {
         bar.arrive();
         if (tape && x.i >= 0) tape[x.i] = f4(x.p, x.w);
         bar.finish();
-        if (x.i < 0) return;
-        const float4 p4 = f4(x.p, x.w);
-        // three entries at a time, their loads in flight together
-        for (int k = x.begin; k < x.end; k += 3) {
-            unsigned c[3];
-            float4 q[3];
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                c[u] = code[min(k + u, x.end - 1)];
-                q[u] = ld_cluster<kOne>((c[u] & kEntAddr) + row(b));
-            }
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                if (k + u >= x.end) continue;
-                const bool self_is_j = (c[u] & kEntSide) != 0;
-                const float4 pi = self_is_j ? q[u] : p4, pj = self_is_j ? p4 : q[u];
-                F3 corr;
-                float cc;
-                bool clamped;
-                if (!stretch_correction(pi, pj, rest[k + u], alpha[k + u], &corr, &cc, &clamped)) continue;
-                if (x.w > 0.0f) {
-                    const F3 dd = self_is_j ? corr * x.w : corr * (-x.w);
-                    x.p = x.p + dd;
-                    if (cc > 0.0f) x.prev = x.prev + dd * 0.08f;
-                }
-            }
+        for (int e = threadIdx.x; e < edges; e += blockDim.x) {
+            const uint4 c = edge[e];
+            if (c.x & kEdgeFixed) continue;  // neither end moves, nobody reads the result
+            const F3 pi = f3(ld_cluster<kOne>((c.x & kEdgeAddr) + row(b))), pj = f3(ld_cluster<kOne>(c.y + row(b)));
+            F3 corr;
+            float cc;
+            bool clamped;
+            stretch_step(pi, pj, __uint_as_float(c.z), __uint_as_float(c.w), &corr, &cc, &clamped);
+            result[e] = f4(corr, cc > 0.0f ? 1.0f : 0.0f);
+        }
+        __syncthreads();
+        if (x.i < 0 || !(x.w > 0.0f)) return;
+        for (int k = x.begin; k < x.end; ++k) {
+            const int e = ent[k];
+            const float4 r = result[e & 0x7fffffff];
+            const F3 dd = f3(r) * (e < 0 ? x.w : -x.w);
+            x.p = x.p + dd;
+            if (r.w != 0.0f) x.prev = x.prev + dd * 0.08f;
         }
     }
     // Bend colours in place; with `record` the positions each bend started
@@ -553,8 +561,8 @@ struct DiffBlock {
         }
     }
     // Backward through the recorded frame: the adjoint at its end becomes the
-    // adjoint at its start.  `gk` sums the compliance gradients of the entries
-    // whose first endpoint this vertex is.
+    // adjoint at its start.  `gk` sums the compliance gradients of the edges
+    // whose first endpoint is this CTA's.
     __device__ __forceinline__ void back(const DiffVertex& x, F3& gp, F3& gq, F3& gv, float* gk) {
         const size_t V = (size_t)d.V;
         int g = a.substeps * a.iterations;
@@ -579,11 +587,10 @@ struct DiffBlock {
                     if (x.pinned) gp = gq = gv = F3{0.0f, 0.0f, 0.0f};
                 }
                 if (last && s + 1 == a.substeps && a.colours > 0) bends_back(x, gp, gq);
-                const float4 p4 = np;
-                const int b = publish_back(x, p4, gp, gq);
+                const int b = publish_back(x, np, gp, gq);
                 ahead(g - 1, it == 0 ? s - 1 : -1);
                 bar.finish();
-                gather_back(x, b, p4, gp, gq, gk);
+                gather_back(x, b, gp, gk);
             }
             if (x.i < 0) continue;
             // prediction and its pin stage
@@ -612,35 +619,27 @@ struct DiffBlock {
         bar.arrive();
         return b;
     }
-    __device__ __forceinline__ void gather_back(const DiffVertex& x, int b, float4 p4, F3& gp, F3 gq, float* gk) const {
-        if (x.i < 0) return;
-        F3 acc = gp;
-        for (int k = x.begin; k < x.end; k += 2) {
-            unsigned c[2];
-            float4 q[2];
-            F3 op[2], oq[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                c[u] = code[min(k + u, x.end - 1)];
-                const unsigned o = c[u] & kEntAddr;
-                q[u] = ld_cluster<kOne>(o + row(b));
-                op[u] = f3(ld_cluster<kOne>(o + row(b + 1)));
-                oq[u] = f3(ld_cluster<kOne>(o + row(b + 2)));
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                if (k + u >= x.end) continue;
-                const bool self_is_j = (c[u] & kEntSide) != 0;
-                const float4 pi = self_is_j ? q[u] : p4, pj = self_is_j ? p4 : q[u];
-                if (pi.w + pj.w <= 0.0f) continue;
-                float dk;
-                const F3 adelta = edge_adjoint(pi, pj, rest[k + u], alpha[k + u], (c[u] & kEntCompliant) != 0, d.dt, self_is_j ? op[u] : gp,
-                                               self_is_j ? oq[u] : gq, self_is_j ? gp : op[u], self_is_j ? gq : oq[u], &dk);
-                acc = self_is_j ? acc + adelta : acc - adelta;
-                if (!self_is_j) gk[k + u] += dk;
-            }
+    __device__ __forceinline__ void gather_back(const DiffVertex& x, int b, F3& gp, float* gk) const {
+        for (int e = threadIdx.x; e < edges; e += blockDim.x) {
+            const uint4 c = edge[e];
+            if (c.x & kEdgeFixed) continue;
+            const unsigned ai = (c.x & kEdgeAddr) + row(b), aj = c.y + row(b);
+            float dk;
+            const F3 adelta = edge_adjoint(ld_cluster<kOne>(ai), ld_cluster<kOne>(aj), __uint_as_float(c.z), __uint_as_float(c.w),
+                                           (c.x & kEdgeCompliant) != 0, d.dt, f3(ld_cluster<kOne>(ai + row(1))),
+                                           f3(ld_cluster<kOne>(ai + row(2))), f3(ld_cluster<kOne>(aj + row(1))),
+                                           f3(ld_cluster<kOne>(aj + row(2))), &dk);
+            result[e] = f4(adelta, 0.0f);
+            if (c.x & kEdgeMine) gk[e] += dk;
         }
-        gp = acc;
+        __syncthreads();
+        if (x.i < 0) return;
+        for (int k = x.begin; k < x.end; ++k) {
+            const int e = ent[k];
+            if (edge[e & 0x7fffffff].x & kEdgeFixed) continue;
+            const F3 adelta = f3(result[e & 0x7fffffff]);
+            gp = e < 0 ? gp + adelta : gp - adelta;
+        }
     }
     __device__ __forceinline__ void bends_back(const DiffVertex& x, F3& gp, F3 gq) {
         const int b = 3 * turn;
@@ -675,7 +674,7 @@ struct DiffBlock {
 };
 
 template <int T, bool kOne, bool kBack>
-__global__ void __launch_bounds__(T) k_d_cluster(DView d, DiffCluster a) {
+__global__ void __launch_bounds__(T, 1) k_d_cluster(DView d, DiffCluster a) {
     extern __shared__ float4 sm[];
     __shared__ unsigned long long s_counter;
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -689,34 +688,37 @@ __global__ void __launch_bounds__(T) k_d_cluster(DView d, DiffCluster a) {
     ClusterBarrier bar{smem_addr(&s_counter), 0u, a.ctas, false};
     const size_t V = (size_t)d.V;
     float4* buf = sm;
-    unsigned* code = reinterpret_cast<unsigned*>(buf + (kBack ? 6 : 3) * a.chunk);
-    float* rest = reinterpret_cast<float*>(code + a.rows);
-    float* alpha = rest + a.rows;
-    float* gk = alpha + a.rows;
-    DiffBlock<kOne> B{d, a, ClusterMap<kOne>(smem_addr(buf), a.chunk, rank), bar, buf, code, rest, alpha, 0, a.tape, nullptr, nullptr};
+    float4* result = buf + (kBack ? 6 : 3) * a.chunk;
+    uint4* edge = reinterpret_cast<uint4*>(result + a.edge_rows);
+    int* ent = reinterpret_cast<int*>(edge + a.edge_rows);
+    float* gk = reinterpret_cast<float*>(ent + a.ent_rows);
+    const int edge0 = a.cta_off[rank], edges = a.cta_off[rank + 1] - edge0;
+    DiffBlock<kOne> B{d, a, ClusterMap<kOne>(smem_addr(buf), a.chunk, rank), bar, buf, result, edge, ent, edges, 0, a.tape, nullptr, nullptr};
     B.tape_v = B.tape_p + (size_t)a.substeps * a.iterations * V;
     B.tape_b = B.tape_v + (size_t)a.substeps * 3 * V;
+    for (int e = threadIdx.x; e < edges; e += blockDim.x) {
+        const int id = a.cta_edge[edge0 + e];
+        const int2 p = a.ends[id];
+        const float kc = d.kst[id], weight = d.rest[p.x].w + d.rest[p.y].w;
+        const unsigned flags = (weight <= 0.0f ? kEdgeFixed : 0u) | (kc > 0.0f ? kEdgeCompliant : 0u) |
+                               (p.x >= rank * a.chunk && p.x < (rank + 1) * a.chunk ? kEdgeMine : 0u);
+        edge[e] = make_uint4(B.map.addr(p.x) | flags, B.map.addr(p.y), __float_as_uint(d.edge_rest[id]),
+                             __float_as_uint(weight + stretch_alpha(kc, d.dt)));
+        if (kBack) gk[e] = 0.0f;
+    }
     DiffVertex x;
     const int l = rank * a.chunk + (int)threadIdx.x;
     x.i = (int)threadIdx.x < a.chunk && l < d.V ? l : -1;
     x.begin = x.end = 0;
     x.w = 0.0f;
     x.pinned = false;
-    int row0 = 0;
     if (x.i >= 0) {
-        row0 = d.off[rank * a.chunk];
+        const int row0 = d.off[rank * a.chunk];
         x.begin = d.off[x.i] - row0;
         x.end = d.off[x.i + 1] - row0;
         x.w = d.rest[x.i].w;
         x.pinned = d.pinned[x.i] != 0;
-        for (int k = x.begin; k < x.end; ++k) {
-            const int2 e = d.ent[row0 + k];
-            const float kc = d.kst[e.y];
-            code[k] = B.map.addr(e.x & 0x7fffffff) | ((e.x & kSideBit) ? kEntSide : 0u) | (kc > 0.0f ? kEntCompliant : 0u);
-            rest[k] = d.edge_rest[e.y];
-            alpha[k] = stretch_alpha(kc, d.dt);
-            if (kBack) gk[k] = 0.0f;
-        }
+        for (int k = x.begin; k < x.end; ++k) ent[k] = a.cta_ent[row0 + k];
     }
     auto load = [&](const float4* s) __attribute__((always_inline)) {
         if (x.i < 0) return;
@@ -751,9 +753,8 @@ __global__ void __launch_bounds__(T) k_d_cluster(DView d, DiffCluster a) {
             B.back(x, gp, gq, gv, gk);
             bar.sync();
         }
-        if (x.i >= 0)
-            for (int k = x.begin; k < x.end; ++k)
-                if (!(code[k] & kEntSide)) a.grad_stretch[d.ent[row0 + k].y] = gk[k];
+        for (int e = threadIdx.x; e < edges; e += blockDim.x)
+            if (edge[e].x & kEdgeMine) a.grad_stretch[a.cta_edge[edge0 + e]] = gk[e];
     }
     if (bar.lost) *a.lost = 1;
     bar.sync();  // no CTA leaves while another still reads its shared memory
@@ -793,8 +794,11 @@ struct DiffSolver {
     int frames = 0, substeps = 0, iterations = 0;
     std::vector<Op> ops;
     // cluster form (ctas 0: the launched form is used)
-    int ctas = 0, chunk = 0, rows = 0;
+    int ctas = 0, chunk = 0, edge_rows = 0, ent_rows = 0;
     int* colour = nullptr;          // colour offsets into `order`
+    int* cta_plan = nullptr;        // the cluster's tables (plan_cluster)
+    const int *cta_edge = nullptr, *cta_ent = nullptr;
+    const int2* ends = nullptr;
     int* lost = nullptr;
 
     DView view(float dt) const {
@@ -825,7 +829,7 @@ void free_diff(DiffSolver* D) {
     if (!D) return;
     if (D->stream) cudaStreamSynchronize(D->stream);
     void* ptrs[] = {D->rest, D->off, D->ent, D->edge_rest, D->bends, D->bend_rest, D->order, D->pinned,
-                    D->target, D->kst, D->kbd, D->init, D->ck, D->tape, D->adj, D->colour, D->lost};
+                    D->target, D->kst, D->kbd, D->init, D->ck, D->tape, D->adj, D->colour, D->lost, D->cta_plan};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (D->stream) cudaStreamDestroy(D->stream);
@@ -951,37 +955,92 @@ void back_frame_ops(DiffSolver* D, float* gst, float* gbd) {
 // per thread would no longer fit the registers).
 constexpr int kDiffSmem = 220 * 1024;
 
-size_t diff_smem(const DiffSolver* D, bool back) { return (back ? 6 : 3) * 16 * (size_t)D->chunk + (back ? 16 : 12) * (size_t)D->rows; }
-
-template <int T, bool kOne, bool kBack>
-bool diff_cluster_fits(const DiffSolver* D) {
-    return cluster_fit(k_d_cluster<T, kOne, kBack>, D->ctas, T, kDiffSmem) > 0;
+size_t diff_smem(const DiffSolver* D, bool back) {
+    return (back ? 6 : 3) * 16 * (size_t)D->chunk + (back ? 36 : 32) * (size_t)D->edge_rows + 4 * (size_t)D->ent_rows;
 }
 
-void plan_cluster(DiffSolver* D, const std::vector<int>& off) {
+template <bool kBack>
+auto diff_kernel(int ctas, int chunk) -> void (*)(DView, DiffCluster) {
+    if (ctas == 1) return k_d_cluster<512, true, kBack>;
+    return chunk <= 512 ? k_d_cluster<512, false, kBack> : k_d_cluster<768, false, kBack>;
+}
+int diff_threads(int chunk) { return chunk <= 512 ? 512 : 768; }
+
+// Each CTA's edges (every edge of its vertices, increasing) and the place of
+// an entry's edge among them; uploads them.
+bool plan_cluster(DiffSolver* D, const std::vector<int>& off, const std::vector<int2>& ent, const std::vector<int2>& ends) {
     const int V = D->V;
     int c = 1;
     while (c < 16 && c * 128 < V) c *= 2;
     const int chunk = std::max((V + 32 * c - 1) / (32 * c), 1) * 32;
-    if (chunk > 768) return;
-    int rows = 1;
-    for (int r = 0; r < c; ++r) rows = std::max(rows, off[std::min((r + 1) * chunk, V)] - off[std::min(r * chunk, V)]);
+    if (chunk > 768) return true;
+    // one upload: the CTAs' edge offsets, their edges, the entries' places, the edges' endpoints
+    std::vector<std::vector<int>> mine(c);
+    std::vector<int> place(2 * (size_t)D->E, 0);  // among the edges of the first and of the second endpoint's CTA
+    size_t total = 0;
+    for (int r = 0; r < c; ++r) {
+        // the edges to other CTAs first, so that few warps wait for the
+        // cluster's memory, the others by first endpoint: neighbouring lanes
+        // read neighbouring rows
+        for (const bool away : {true, false})
+            for (int i = std::min(r * chunk, V); i < std::min((r + 1) * chunk, V); ++i)
+                for (int k = off[i]; k < off[i + 1]; ++k) {
+                    const bool second = (ent[k].x & kSideBit) != 0;
+                    if (((ent[k].x & 0x7fffffff) / chunk != r) != away || (!away && second)) continue;
+                    int* at = &place[2 * (size_t)ent[k].y];
+                    if (away)
+                        at[second ? 1 : 0] = (int)mine[r].size();
+                    else
+                        at[0] = at[1] = (int)mine[r].size();
+                    mine[r].push_back(ent[k].y);
+                }
+        total += mine[r].size();
+    }
+    int ent_rows = 1, edge_rows = 1;
+    for (int r = 0; r < c; ++r) {
+        ent_rows = std::max(ent_rows, off[std::min((r + 1) * chunk, V)] - off[std::min(r * chunk, V)]);
+        edge_rows = std::max(edge_rows, (int)mine[r].size());
+    }
     D->ctas = c;
     D->chunk = chunk;
-    D->rows = rows;
-    const bool one = c == 1, small = chunk <= 384;
-    const bool fits = diff_smem(D, true) <= (size_t)kDiffSmem &&
-                      (one ? diff_cluster_fits<384, true, false>(D) && diff_cluster_fits<384, true, true>(D)
-                       : small ? diff_cluster_fits<384, false, false>(D) && diff_cluster_fits<384, false, true>(D)
-                               : diff_cluster_fits<768, false, false>(D) && diff_cluster_fits<768, false, true>(D));
-    if (!fits) D->ctas = 0;
+    D->edge_rows = edge_rows;
+    D->ent_rows = ent_rows;
+    if (diff_smem(D, true) > (size_t)kDiffSmem || cluster_fit(diff_kernel<false>(c, chunk), c, diff_threads(chunk), kDiffSmem) < 1 ||
+        cluster_fit(diff_kernel<true>(c, chunk), c, diff_threads(chunk), kDiffSmem) < 1) {
+        D->ctas = 0;
+        return true;
+    }
+    const size_t at_edge = (size_t)c + 1, at_ent = at_edge + total, at_ends = (at_ent + ent.size() + 1) / 2 * 2;
+    std::vector<int> all(at_ends + 2 * (size_t)D->E, 0);
+    for (int r = 0; r < c; ++r) {
+        std::copy(mine[r].begin(), mine[r].end(), all.begin() + at_edge + all[r]);
+        all[r + 1] = all[r] + (int)mine[r].size();
+    }
+    for (size_t k = 0; k < ent.size(); ++k) {
+        const bool second = (ent[k].x & kSideBit) != 0;
+        all[at_ent + k] = place[2 * (size_t)ent[k].y + (second ? 1 : 0)] | (second ? kSideBit : 0);
+    }
+    if (D->E > 0) std::memcpy(&all[at_ends], ends.data(), sizeof(int2) * (size_t)D->E);
+    if (!dalloc(&D->cta_plan, all.size(), "rollout allocation") ||
+        !dupload(D->cta_plan, all.data(), all.size(), D->stream, "rollout upload") ||
+        !cuda_ok(cudaStreamSynchronize(D->stream), "rollout upload"))
+        return false;
+    D->cta_edge = D->cta_plan + at_edge;
+    D->cta_ent = D->cta_plan + at_ent;
+    D->ends = reinterpret_cast<const int2*>(D->cta_plan + at_ends);
+    return true;
 }
 
 template <bool kBack>
 bool run_cluster(DiffSolver* D, DiffCluster a, const char* what) {
     a.ctas = D->ctas;
     a.chunk = D->chunk;
-    a.rows = D->rows;
+    a.edge_rows = D->edge_rows;
+    a.ent_rows = D->ent_rows;
+    a.cta_off = D->cta_plan;
+    a.cta_edge = D->cta_edge;
+    a.cta_ent = D->cta_ent;
+    a.ends = D->ends;
     a.frames = D->frames;
     a.substeps = D->substeps;
     a.iterations = D->iterations;
@@ -995,13 +1054,7 @@ bool run_cluster(DiffSolver* D, DiffCluster a, const char* what) {
     const DView d = D->view(D->cfg.dt / (float)D->substeps);
     const size_t smem = diff_smem(D, kBack);
     if (!cuda_ok(cudaMemsetAsync(D->lost, 0, sizeof(int), D->stream), what)) return false;
-    cudaError_t e;
-    if (D->ctas == 1)
-        e = cluster_launch(k_d_cluster<384, true, kBack>, 1, 1, D->chunk, smem, D->stream, d, a);
-    else if (D->chunk <= 384)
-        e = cluster_launch(k_d_cluster<384, false, kBack>, 1, D->ctas, D->chunk, smem, D->stream, d, a);
-    else
-        e = cluster_launch(k_d_cluster<768, false, kBack>, 1, D->ctas, D->chunk, smem, D->stream, d, a);
+    const cudaError_t e = cluster_launch(diff_kernel<kBack>(D->ctas, D->chunk), 1, D->ctas, diff_threads(D->chunk), smem, D->stream, d, a);
     int lost = 0;
     if (!cuda_ok(e, what) || !cuda_ok(cudaMemcpyAsync(&lost, D->lost, sizeof(int), cudaMemcpyDeviceToHost, D->stream), what) ||
         !cuda_ok(cudaStreamSynchronize(D->stream), what))
@@ -1085,7 +1138,7 @@ XG_EXPORT void* xpbd_gb300_diff_create(const SsblXpbdConfig* config, const SsblX
               dalloc(&D->kbd, B, "rollout allocation") && dalloc(&D->init, 3 * (size_t)V, "rollout allocation") &&
               dalloc(&D->adj, 6 * (size_t)V, "rollout allocation") && dalloc(&D->lost, 1, "rollout allocation") &&
               dalloc(&D->colour, std::max<size_t>(D->colors.size(), 1), "rollout allocation");
-    if (ok) plan_cluster(D, off);
+    if (ok) ok = plan_cluster(D, off, ent, edges);
     if (ok)
         ok = dupload(D->rest, rest4.data(), V, D->stream, "rollout upload") &&
              dupload(D->off, off.data(), off.size(), D->stream, "rollout upload") &&
