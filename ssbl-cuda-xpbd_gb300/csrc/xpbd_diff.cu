@@ -974,52 +974,23 @@ bool plan_cluster(DiffSolver* D, const std::vector<int>& off, const std::vector<
     while (c < 16 && c * 128 < V) c *= 2;
     const int chunk = std::max((V + 32 * c - 1) / (32 * c), 1) * 32;
     if (chunk > 768) return true;
-    // one upload: the CTAs' edge offsets, their edges, the entries' places, the edges' endpoints
-    std::vector<std::vector<int>> mine(c);
-    std::vector<int> place(2 * (size_t)D->E, 0);  // among the edges of the first and of the second endpoint's CTA
-    size_t total = 0;
-    for (int r = 0; r < c; ++r) {
-        // the edges to other CTAs first, so that few warps wait for the
-        // cluster's memory, the others by first endpoint: neighbouring lanes
-        // read neighbouring rows
-        for (const bool away : {true, false})
-            for (int i = std::min(r * chunk, V); i < std::min((r + 1) * chunk, V); ++i)
-                for (int k = off[i]; k < off[i + 1]; ++k) {
-                    const bool second = (ent[k].x & kSideBit) != 0;
-                    if (((ent[k].x & 0x7fffffff) / chunk != r) != away || (!away && second)) continue;
-                    int* at = &place[2 * (size_t)ent[k].y];
-                    if (away)
-                        at[second ? 1 : 0] = (int)mine[r].size();
-                    else
-                        at[0] = at[1] = (int)mine[r].size();
-                    mine[r].push_back(ent[k].y);
-                }
-        total += mine[r].size();
-    }
-    int ent_rows = 1, edge_rows = 1;
-    for (int r = 0; r < c; ++r) {
-        ent_rows = std::max(ent_rows, off[std::min((r + 1) * chunk, V)] - off[std::min(r * chunk, V)]);
-        edge_rows = std::max(edge_rows, (int)mine[r].size());
-    }
+    ClusterTables t;
+    cluster_tables(0, V, 0, D->E, chunk, c, off.data(), ent.data(), &t);
     D->ctas = c;
     D->chunk = chunk;
-    D->edge_rows = edge_rows;
-    D->ent_rows = ent_rows;
+    D->edge_rows = t.edge_rows;
+    D->ent_rows = t.ent_rows;
     if (diff_smem(D, true) > (size_t)kDiffSmem || cluster_fit(diff_kernel<false>(c, chunk), c, diff_threads(chunk), kDiffSmem) < 1 ||
         cluster_fit(diff_kernel<true>(c, chunk), c, diff_threads(chunk), kDiffSmem) < 1) {
         D->ctas = 0;
         return true;
     }
-    const size_t at_edge = (size_t)c + 1, at_ent = at_edge + total, at_ends = (at_ent + ent.size() + 1) / 2 * 2;
-    std::vector<int> all(at_ends + 2 * (size_t)D->E, 0);
-    for (int r = 0; r < c; ++r) {
-        std::copy(mine[r].begin(), mine[r].end(), all.begin() + at_edge + all[r]);
-        all[r + 1] = all[r] + (int)mine[r].size();
-    }
-    for (size_t k = 0; k < ent.size(); ++k) {
-        const bool second = (ent[k].x & kSideBit) != 0;
-        all[at_ent + k] = place[2 * (size_t)ent[k].y + (second ? 1 : 0)] | (second ? kSideBit : 0);
-    }
+    // one upload: the CTAs' edge offsets, their edges, the entries' places, the edges' endpoints
+    const size_t at_edge = t.off.size(), at_ent = at_edge + t.edge.size(), at_ends = (at_ent + t.ent.size() + 1) / 2 * 2;
+    std::vector<int> all(t.off);
+    all.insert(all.end(), t.edge.begin(), t.edge.end());
+    all.insert(all.end(), t.ent.begin(), t.ent.end());
+    all.resize(at_ends + 2 * (size_t)D->E, 0);
     if (D->E > 0) std::memcpy(&all[at_ends], ends.data(), sizeof(int2) * (size_t)D->E);
     if (!dalloc(&D->cta_plan, all.size(), "rollout allocation") ||
         !dupload(D->cta_plan, all.data(), all.size(), D->stream, "rollout upload") ||

@@ -373,6 +373,41 @@ void reset_triangle_hash(Solver* S, cudaStream_t s) {
 }
 
 
+void cluster_tables(int v0, int V, int e0, int E, int chunk, int c, const int* off, const int2* ent, ClusterTables* t) {
+    if (t->off.empty()) t->off.push_back(0);
+    const int v1 = v0 + V;
+    std::vector<int> place(2 * (size_t)E, 0);  // among the edges of the first and of the second endpoint's CTA
+    for (int r = 0; r < c; ++r) {
+        const int lo = std::min(v0 + r * chunk, v1), hi = std::min(v0 + (r + 1) * chunk, v1);
+        const size_t first = t->edge.size();
+        // the edges to other CTAs first, so that few warps wait for the
+        // cluster's memory, the others by first endpoint: neighbouring lanes
+        // read neighbouring rows
+        for (const bool away : {true, false})
+            for (int i = lo; i < hi; ++i)
+                for (int k = off[i]; k < off[i + 1]; ++k) {
+                    const int other = ent[k].x & 0x7fffffff;
+                    const bool second = (ent[k].x & kSideBit) != 0;
+                    if ((other < lo || other >= hi) != away || (!away && second)) continue;
+                    int* at = &place[2 * (size_t)(ent[k].y - e0)];
+                    const int n = (int)(t->edge.size() - first);
+                    if (away)
+                        at[second ? 1 : 0] = n;
+                    else
+                        at[0] = at[1] = n;
+                    t->edge.push_back(ent[k].y);
+                }
+        t->off.push_back((int)t->edge.size());
+        t->edge_rows = std::max(t->edge_rows, (int)(t->edge.size() - first));
+        t->ent_rows = std::max(t->ent_rows, off[hi] - off[lo]);
+    }
+    t->ent.resize(std::max(t->ent.size(), (size_t)off[v1]));
+    for (int k = off[v0]; k < off[v1]; ++k) {
+        const bool second = (ent[k].x & kSideBit) != 0;
+        t->ent[k] = place[2 * (size_t)(ent[k].y - e0) + (second ? 1 : 0)] | (second ? kSideBit : 0);
+    }
+}
+
 View Solver::view() const {
     View v{};
     v.tune = tune;
@@ -513,7 +548,8 @@ void free_solver(Solver* S) {
     dfree(S->trim_list);
     dfree(S->trim_count);
     dfree(S->bend_ranges);
-    for (auto& f : S->fused_ops) dfree(f.second.first);
+    for (auto& f : S->fused_ops) dfree(f.second.dev);
+    dfree(S->frame_tables);
     S->fused_ops.clear();
     PcgView& g = S->pcg;
     dfree(g.diag);
@@ -1478,6 +1514,38 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
         h.rest = S->cap_rest;
         h.ranges = S->hard_ranges;
     }
+    // the fused frame's edge-per-thread form
+    std::vector<int> frame_tables;
+    if (ok && !S->pcg_on && !S->self_any && nV > 0) {
+        int max_v = 0;
+        for (const Params& P : S->hp) max_v = std::max(max_v, P.V);
+        if (frame_shape(K, max_v, &S->frame)) {
+            std::vector<int2> ids(sp_ent.size());
+            std::vector<int> at(sp_off.begin(), sp_off.end() - 1);
+            for (int e = 0; e < nE; ++e) {  // the CSR's own order, with edge ids in place of rest lengths
+                const int2 p = springs[e];
+                if (p.x < 0 || p.y < 0 || p.x >= nV || p.y >= nV || p.x == p.y) continue;
+                ids[at[p.x]++] = make_int2(p.y, e);
+                ids[at[p.y]++] = make_int2(p.x | kSideBit, e);
+            }
+            ClusterTables t;
+            for (const Params& P : S->hp)
+                cluster_tables(P.vstart, P.V, P.estart, P.E, S->frame.chunk, S->frame.ctas, sp_off.data(), ids.data(), &t);
+            S->frame.edge_rows = t.edge_rows;
+            S->frame.ent_rows = t.ent_rows;
+            if (!frame_fits(S->frame)) {
+                S->frame.ctas = 0;
+            } else {
+                frame_tables = t.off;
+                frame_tables.insert(frame_tables.end(), t.edge.begin(), t.edge.end());
+                frame_tables.insert(frame_tables.end(), t.ent.begin(), t.ent.end());
+                ok = dalloc(&S->frame_tables, frame_tables.size(), "fused frame allocation");
+                S->frame.off = S->frame_tables;
+                S->frame.edge = S->frame_tables + t.off.size();
+                S->frame.ent = S->frame.edge + t.edge.size();
+            }
+        }
+    }
     if (!ok) return bail(0, "");
     cudaStream_t st = S->stream;
     ok = dupload(S->pos[0], rest4.data(), nV, st, "position upload") && dupload(S->pos[1], rest4.data(), nV, st, "position upload") &&
@@ -1510,6 +1578,7 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
          cuda_ok(cudaMemsetAsync(S->max_delta_bits, 0, sizeof(unsigned), st), "reset self max smoothed delta") &&
          (!S->acc || cuda_ok(cudaMemsetAsync(S->acc, 0, sizeof(Acc4) * nV, st), "reset self accumulation")) &&
          (!S->nb_count || cuda_ok(cudaMemsetAsync(S->nb_count, 0, sizeof(int) * nV, st), "reset neighbor table")) &&
+         dupload(S->frame_tables, frame_tables.data(), frame_tables.size(), st, "fused frame upload") &&
          sync_params(S) && cuda_ok(cudaStreamSynchronize(st), "solver upload");
     if (ok && S->pcg_on)
         ok = (S->cap_count == 0 || (dupload(S->cap_edges, cap_edges.data(), S->cap_count, st, "cap edge upload") &&
@@ -1632,22 +1701,36 @@ GraphKey frame_key(const Solver* S, int substeps, int iterations) {
 
 // Whether every cloth fits one block and uses only stages the fused frame
 // runs (no self collision, hard stretch or dynamic colliders).
-// Fused frame form: 1 one block per cloth (default), 8 an 8-CTA cluster per
-// cloth, 2 launched kernels.  On a 32x32 cloth the block form measured 0.174
-// ms per frame, the launched kernels 0.19 ms and the cluster 0.227 ms (its
-// per-operation exchange and cluster barrier cost more than the seven extra
-// SMs save).
+// Fused frame form: 1 an edge per thread (k_frame_edges; k_frame_fused, one
+// block per cloth, where vertex normals are gathered), the default; 8 an 8-CTA
+// cluster per cloth with a full copy of the state each; 2 launched kernels.
+// On a 32x32 cloth the block form measured 0.174 ms per frame, the launched
+// kernels 0.19 ms, the cluster of copies 0.227 ms and the default 0.08 ms.
 int fused_mode(const Solver* S) {
     const int m = S->tune.v[kTuneFusedFrame];
     return m > 0 ? m : 1;
 }
 
+// The edge-per-thread form runs the default fused frame where it was planned
+// and no vertex normals are gathered (they read other vertices' positions).
+bool frame_edges_ok(const Solver* S) {
+    if (S->frame.ctas == 0 || fused_mode(S) != 1) return false;
+    for (const Params& P : S->hp)
+        if (P.needs_normal) return false;
+    return true;
+}
+
+int fused_max_v(const Solver* S) {
+    int m = 0;
+    for (const Params& P : S->hp) m = std::max(m, P.V);
+    return m;
+}
+
 bool fused_ok(const Solver* S) {
     if (fused_mode(S) == 2 || S->pcg_on || S->nV == 0) return false;
-    for (int k = 0; k < S->K; ++k) {
-        const Params& P = S->hp[k];
-        if (P.V > 1024 || S->cl[k].self_enabled || P.dyn || P.gd_mode != 0) return false;
-    }
+    if (fused_max_v(S) > 1024 && !frame_edges_ok(S)) return false;
+    for (int k = 0; k < S->K; ++k)
+        if (S->cl[k].self_enabled || S->hp[k].dyn || S->hp[k].gd_mode != 0) return false;
     return true;
 }
 
@@ -1662,15 +1745,25 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
     const int dyn = dynamic_kinds(S);
     if (!prof && !S->rec) {
         const auto f = S->fused_ops.find(frame_key(S, substeps, iterations));
-        if (f != S->fused_ops.end() && f->second.first && fused_ok(S)) {
+        if (f != S->fused_ops.end() && f->second.dev && fused_ok(S)) {
+            const Solver::FusedOps& ops = f->second;
             View v = S->view();
             v.substeps = substeps;
             v.pass = -1;
-            if (fused_mode(S) == 8)
-                launch_frame_cluster(v, f->second.first, f->second.second, S->pos[0], S->bend_ranges, S->K, fused_block(S), 8, 128,
+            if (frame_edges_ok(S)) {
+                // cloths past one block take the last substep, with the
+                // once-per-frame constraints, as a launch of its own
+                const int split = fused_max_v(S) > 1024 && ops.last > 0 ? ops.last : ops.count;
+                launch_frame_edges(v, S->frame, ops.dev, 0, split, S->pos[0], S->bend_ranges, S->K, S->stream);
+                if (split < ops.count) {
+                    launch_frame_edges(v, S->frame, ops.dev, split, ops.count, S->pos[0], S->bend_ranges, S->K, S->stream);
+                    st->launches += 1;
+                }
+            } else if (fused_mode(S) == 8)
+                launch_frame_cluster(v, ops.dev, ops.count, S->pos[0], S->bend_ranges, S->K, fused_block(S), 8, 128,
                                      S->stream);
             else
-                launch_frame_fused(v, f->second.first, f->second.second, S->pos[0], S->pos[1], S->bend_ranges, S->K,
+                launch_frame_fused(v, ops.dev, ops.count, S->pos[0], S->pos[1], S->bend_ranges, S->K,
                                    fused_block(S), S->stream);
             st->launches += 1;
             return;
@@ -1969,7 +2062,7 @@ bool prepare_fused(Solver* S, int substeps, int iterations) {
     enqueue_frame(S, substeps, iterations, &dummy, nullptr);
     S->rec = nullptr;
     if (S->rec_unsupported || ops.empty()) {
-        S->fused_ops[key] = {nullptr, 0};
+        S->fused_ops[key] = Solver::FusedOps{};
         return true;
     }
     AllocAccount account(&S->device_bytes);
@@ -1977,7 +2070,9 @@ bool prepare_fused(Solver* S, int substeps, int iterations) {
     if (!dalloc(&dev, ops.size(), "fused frame allocation") || !dupload(dev, ops.data(), ops.size(), S->stream, "fused frame upload") ||
         !cuda_ok(cudaStreamSynchronize(S->stream), "fused frame upload"))
         return false;
-    S->fused_ops[key] = {dev, (int)ops.size()};
+    int last = 0;
+    while (last < (int)ops.size() && !(ops[last].kind == 0 && ops[last].substep == substeps - 1)) ++last;
+    S->fused_ops[key] = Solver::FusedOps{dev, (int)ops.size(), last};
     return true;
 }
 

@@ -339,7 +339,14 @@ struct Solver {
     // operations per frame schedule, and each cloth's bends per colour
     std::vector<FrameOp>* rec = nullptr;  // set while recording a frame's operations
     bool rec_unsupported = false;         // a launch without a fused form was recorded
-    std::map<GraphKey, std::pair<FrameOp*, int>> fused_ops;
+    struct FusedOps {
+        FrameOp* dev = nullptr;
+        int count = 0;
+        int last = 0;  // first operation of the last substep
+    };
+    std::map<GraphKey, FusedOps> fused_ops;
+    FramePlan frame{};                    // edge-per-thread form of the fused frame (ctas 0: not used)
+    int* frame_tables = nullptr;
     std::vector<int2> h_bend_ranges;      // [colours x K]: first bend, count
     int2* bend_ranges = nullptr;
     long long device_bytes = 0;  // sum of the solver's device allocations
@@ -384,6 +391,18 @@ bool scene_update(GlobalScene* G, const SsblXpbdGlobalDynamicSceneInputs* in);
 bool scene_attach(Solver* S, int cloth, GlobalScene* G, int source_id, int layer, int mode);
 void scene_detach(Solver* S, int cloth);
 void sdf_diagnostics(Solver* S);
+
+// Tables of a cluster form that computes each edge once per CTA: the CTAs of a
+// cloth own `chunk` consecutive vertices each.
+struct ClusterTables {
+    std::vector<int> off;   // per cloth c + 1 offsets into `edge`
+    std::vector<int> edge;  // each CTA's edge ids: those to other CTAs first, then by first endpoint
+    std::vector<int> ent;   // per constraint entry: its edge's place among its CTA's | side bit
+    int edge_rows = 1, ent_rows = 1;  // largest counts of a CTA
+};
+// Appends one cloth: vertices [v0, v0 + V), CSR `off` (indexed by vertex) with
+// entries {other vertex | side bit, edge id} of edges [e0, e0 + E).
+void cluster_tables(int v0, int V, int e0, int E, int chunk, int c, const int* off, const int2* ent, ClusterTables* t);
 
 // One frame: prepare parameters, launch (graph or direct), optionally fetch.
 bool prepare_step(Solver* S, int substeps, int iterations);

@@ -446,6 +446,21 @@ void launch_frame_fused(const View& v, const FrameOp* ops, int nops, float4* buf
 // slices through distributed shared memory after every operation.
 void launch_frame_cluster(const View& v, const FrameOp* ops, int nops, float4* buf0, const int2* bend_ranges, int K, int cap,
                           int cluster, int block, cudaStream_t s);
+// The fused frame with an edge per thread: a cluster of `ctas` CTAs per cloth,
+// `chunk` vertices per CTA of the largest cloth; tables as ClusterTables.
+struct FramePlan {
+    int ctas, chunk, edge_rows, ent_rows;
+    const int* off;
+    const int* edge;
+    const int* ent;
+};
+// Shape for K cloths of at most max_v vertices; false where the form is not
+// used.  Then, with the rows known, whether it fits the GPU.
+bool frame_shape(int K, int max_v, FramePlan* f);
+bool frame_fits(const FramePlan& f);
+// Runs operations [first, last) of the recorded frame from buffer 0 to buffer 0.
+cudaError_t launch_frame_edges(const View& v, const FramePlan& f, const FrameOp* ops, int first, int last, float4* buf0,
+                               const int2* bend_ranges, int K, cudaStream_t s);
 void launch_bend_color(const View& v, int start, int count, cudaStream_t s);
 void launch_copy_pos(float4* dst, const float4* src, int V, cudaStream_t s);
 void launch_pin_scatter(const int* idx, const float4* target, const float* weight, const float* relax, int n,

@@ -13,8 +13,9 @@
 // update as the reference's atomics, without float atomics, and therefore
 // deterministic.
 #include "xpbd_constraint.cuh"
-#include <cooperative_groups.h>
+#include <algorithm>
 
+#include "xpbd_cluster.cuh"
 #include "xpbd_contact.cuh"
 #include "xpbd_fields.cuh"
 #include "xpbd_solver.cuh"
@@ -31,23 +32,26 @@ struct VState {
 // Weighted pin projection of one vertex (abi41.cu:3466-3509).  Pins are
 // stored per vertex (weight -1 = no pin; a vertex listed twice keeps its last
 // entry) and the relaxation 1 - (1 - s)^(1/(I+1)) is precomputed on the host.
-__device__ void pin_stage(const View& v, int i, float inv_mass, float dt, VState* s) {
-    const float weight = __ldg(&v.pin_weight[i]);
+__device__ __forceinline__ void pin_apply(float weight, F3 target, float relax, float inv_mass, float dt, VState* s) {
     if (!isfinite(weight) || weight < 0.05f) return;
-    const F3 target = f3(ld4(&v.pin_target[i]));
     if (weight >= 0.75f || inv_mass <= 0.0f) {
         s->p = target;
         s->prev = target;
         s->vel = F3{0.0f, 0.0f, 0.0f};
         return;
     }
-    const float relax = __ldg(&v.pin_relax[i]);
     if (relax <= 0.0f) return;
     const F3 corrected = s->p + (target - s->p) * relax;
     const F3 damped = s->vel * fmaxf(1.0f - relax, 0.0f);
     s->p = corrected;
     s->prev = corrected - damped * fmaxf(dt, kEps);
     s->vel = damped;
+}
+
+__device__ void pin_stage(const View& v, int i, float inv_mass, float dt, VState* s) {
+    const float weight = __ldg(&v.pin_weight[i]);
+    if (!isfinite(weight) || weight < 0.05f) return;
+    pin_apply(weight, f3(ld4(&v.pin_target[i])), __ldg(&v.pin_relax[i]), inv_mass, dt, s);
 }
 
 // Ground plane (z up), sphere and wall (abi41.cu:3511-3590).
@@ -340,6 +344,15 @@ __device__ bool vertex_normal(const View& v, int i, F3* out) {
     if (!isfinite(a2) || a2 <= 1.0e-10f) return false;
     *out = acc * (1.0f / sqrtf(a2));
     return true;
+}
+
+// The prediction of a free vertex without force fields or volume pressure.
+__device__ __forceinline__ void predict_free(const Params& P, float dt, VState* s) {
+    const F3 accel = F3{P.gravity[0], P.gravity[1], P.gravity[2]} + F3{0.0f, 0.0f, 0.0f};
+    F3 vel = s->vel + accel * dt;
+    vel = vel * P.damping;
+    s->vel = vel;
+    s->p = s->p + vel * dt;
 }
 
 // Integrate (abi41.cu:1869-1925): gravity, volume pressure along the vertex
@@ -685,6 +698,258 @@ __global__ void __launch_bounds__(256) k_frame_cluster(View base, const FrameOp*
         base.prev[v0 + i] = sprev[i];
         base.vel[v0 + i] = svel[i];
     }
+}
+
+// The fused frame with an edge per thread, by a cluster of C CTAs per cloth
+// (plain shared memory for one).  k_frame_fused is bound by instruction issue:
+// its one SM computes every edge's correction at both ends (5.0 us per
+// operation of a 32 x 32 cloth, 285 issue cycles per warp of edges).  Here a
+// CTA computes each edge of its vertices once into shared memory and a vertex
+// adds its edges' corrections in its entry order, which is the launched form's
+// sum; C CTAs divide the work, and only the edges between two CTAs are
+// computed twice.  A vertex's state stays in its thread's registers, positions
+// are published by turns in two buffers, so an operation costs one cluster
+// barrier.  Counters are kept per thread and added at the end: a barrier would
+// wait for atomics in flight.  Per frame with the host calls, k_frame_fused or
+// launched kernels -> this form: 8 x 8 148 -> 84 us, 32 x 32 198 -> 119,
+// 64 x 64 246 -> 145, 110 x 110 263 -> 201; 150 cloths of 8 x 8 to 32 x 32
+// 177 -> 103.
+constexpr unsigned kEdgeFixed = 1u, kEdgeMine = 2u, kEdgeAddr = ~7u;
+
+template <int T, bool kOne>
+__global__ void __launch_bounds__(T, 1) k_frame_edges(View v, FramePlan f, const FrameOp* ops, int first, int last, float4* buf0,
+                                                      const int2* bend_ranges, int K) {
+    extern __shared__ float4 sm[];
+    __shared__ unsigned long long s_counter;
+    __shared__ Params sP;
+    const cgx::cluster_group cluster = cgx::this_cluster();
+    const int C = kOne ? 1 : (int)cluster.num_blocks(), rank = kOne ? 0 : (int)cluster.block_rank();
+    const int cloth = (int)(blockIdx.x / C);
+    for (int k = threadIdx.x; k < (int)(sizeof(Params) / 4); k += blockDim.x)
+        reinterpret_cast<unsigned*>(&sP)[k] = reinterpret_cast<const unsigned*>(&v.P[cloth])[k];
+    if (threadIdx.x == 0) {
+        ClusterBarrier::init(&s_counter, C);
+        ClusterBarrier::init_fence();
+    }
+    __syncthreads();
+    const Params& P = sP;
+    if (!P.active) return;        // uniform over the cluster: the state stays as it is
+    if (!kOne) cluster.sync();    // every CTA's counter is set before the first arrival
+    ClusterBarrier bar{smem_addr(&s_counter), 0u, C, false};
+    const int chunk = f.chunk;
+    float4* rows = sm;            // positions by turns in two buffers, previous positions
+    float4* result = rows + 3 * chunk;
+    uint4* edge = reinterpret_cast<uint4*>(result + f.edge_rows);
+    int* ent = reinterpret_cast<int*>(edge + f.edge_rows);
+    const ClusterMap<kOne> map(smem_addr(rows), chunk, rank);
+    const float dt = P.sub_dt;
+    const int v0 = P.vstart, V = P.V;
+    const int* off = f.off + (size_t)cloth * C + rank;
+    const int edge0 = off[0], edges = off[1] - edge0;
+    const float alpha = stretch_alpha(P.stretch_compliance, dt);
+    for (int e = threadIdx.x; e < edges; e += blockDim.x) {
+        const int id = __ldg(&f.edge[edge0 + e]);
+        const int2 p = __ldg(&v.edges[id]);
+        const float weight = buf0[p.x].w + buf0[p.y].w;
+        const unsigned flags = (weight <= 0.0f ? kEdgeFixed : 0u) |
+                               (p.x - v0 >= rank * chunk && p.x - v0 < (rank + 1) * chunk ? kEdgeMine : 0u);
+        edge[e] = make_uint4(map.addr(p.x - v0) | flags, map.addr(p.y - v0), __float_as_uint(__ldg(&v.edge_rest[id])),
+                             __float_as_uint(weight + alpha));
+    }
+    const int t = (int)threadIdx.x, l = rank * chunk + t;
+    const bool mine = t < chunk && l < V;
+    const int i = v0 + l;
+    VState s{F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, 0.0f};
+    int begin = 0, end = 0;
+    float inv_mass = 0.0f, pin_weight = -1.0f, pin_relax = 0.0f;
+    F3 pin_target{0.0f, 0.0f, 0.0f};
+    if (mine) {
+        const float4 p4 = buf0[i];
+        s = VState{f3(p4), f3(v.prev[i]), f3(v.vel[i]), p4.w};
+        const int row0 = __ldg(&v.sp_off[v0 + rank * chunk]);
+        begin = __ldg(&v.sp_off[i]) - row0;
+        end = __ldg(&v.sp_off[i + 1]) - row0;
+        inv_mass = __ldg(&v.inv_mass[i]);
+        pin_weight = __ldg(&v.pin_weight[i]);
+        pin_relax = __ldg(&v.pin_relax[i]);
+        pin_target = f3(ld4(&v.pin_target[i]));
+        for (int k = begin; k < end; ++k) ent[k] = __ldg(&f.ent[row0 + k]);
+    }
+    unsigned clamps = 0, wings = 0, guards = 0;
+    int turn = 0;
+    bool bending = false;  // the state is in the rows, a bend colour in progress
+    for (int o = first; o < last; ++o) {
+        const FrameOp op = ops[o];
+        if (op.kind == 2) {
+            // one bend colour in place (bend_item)
+            if (!bending) {
+                if (mine) {
+                    rows[turn * chunk + t] = f4(s.p, s.w);
+                    rows[2 * chunk + t] = f4(s.prev, 0.0f);
+                }
+                bar.sync();
+                bending = true;
+            }
+            const unsigned at = 16u * (unsigned)(turn * chunk), prev_at = 16u * (unsigned)(2 * chunk);
+            const int2 r = __ldg(&bend_ranges[op.color * K + cloth]);
+            for (int b = r.x + rank * (int)blockDim.x + t; b < r.x + r.y; b += C * (int)blockDim.x) {
+                const int2 pr = __ldg(&v.bends[b]);
+                if (pr.x < 0 || pr.y < 0 || pr.x >= v.nV || pr.y >= v.nV || pr.x == pr.y) {
+                    ++guards;
+                    continue;
+                }
+                const unsigned ai = map.addr(pr.x - v0), aj = map.addr(pr.y - v0);
+                const float4 pi4 = ld_cluster<kOne>(ai + at), pj4 = ld_cluster<kOne>(aj + at);
+                F3 corr;
+                bool guard;
+                const bool applied = bend_correction(P, dt, pi4, pj4, __ldg(&v.bend_rest[b]), &corr, &guard);
+                if (guard) ++guards;
+                if (!applied) continue;
+                if (pi4.w > 0.0f) {
+                    const F3 d = corr * (-pi4.w);
+                    st_cluster<kOne>(ai + at, f4(f3(pi4) + d, pi4.w));
+                    st_cluster<kOne>(ai + prev_at, f4(f3(ld_cluster<kOne>(ai + prev_at)) + d * 0.06f, 0.0f));
+                }
+                if (pj4.w > 0.0f) {
+                    const F3 d = corr * pj4.w;
+                    st_cluster<kOne>(aj + at, f4(f3(pj4) + d, pj4.w));
+                    st_cluster<kOne>(aj + prev_at, f4(f3(ld_cluster<kOne>(aj + prev_at)) + d * 0.06f, 0.0f));
+                }
+                ++wings;
+            }
+            bar.sync();
+            continue;
+        }
+        if (bending) {
+            if (mine) {
+                s.p = f3(rows[turn * chunk + t]);
+                s.prev = f3(rows[2 * chunk + t]);
+            }
+            turn ^= 1;
+            bending = false;
+        }
+        if (op.kind == 0) {
+            if (mine) {
+                s.prev = s.p;
+                if (!(s.w > 0.0f)) {
+                    s.vel = F3{0.0f, 0.0f, 0.0f};
+                    s.p = f3(ld4(&v.rest[i]));
+                } else {
+                    predict_free(P, dt, &s);
+                }
+                pin_apply(pin_weight, pin_target, pin_relax, inv_mass, dt, &s);
+            }
+            continue;
+        }
+        if (op.kind != 1) continue;  // a buffer copy: the state is in registers
+        const unsigned gather = op.flags & (kPassSpring | kPassTether | kPassBend);
+        if (gather) {
+            const unsigned at = 16u * (unsigned)(turn * chunk);
+            if (mine) rows[turn * chunk + t] = f4(s.p, s.w);
+            turn ^= 1;
+            bar.sync();
+            if (gather & kPassSpring) {
+                for (int e = t; e < edges; e += (int)blockDim.x) {
+                    const uint4 c = edge[e];
+                    if (c.x & kEdgeFixed) continue;  // neither end moves, nobody reads the result
+                    F3 corr;
+                    float cc;
+                    bool clamped;
+                    stretch_step(f3(ld_cluster<kOne>((c.x & kEdgeAddr) + at)), f3(ld_cluster<kOne>(c.y + at)), __uint_as_float(c.z),
+                                 __uint_as_float(c.w), &corr, &cc, &clamped);
+                    if (clamped && (c.x & kEdgeMine)) ++clamps;
+                    result[e] = f4(corr, cc > 0.0f ? 1.0f : 0.0f);
+                }
+                __syncthreads();
+                if (mine && s.w > 0.0f)
+                    for (int k = begin; k < end; ++k) {
+                        const int e = ent[k];
+                        const float4 r = result[e & 0x7fffffff];
+                        const F3 d = f3(r) * (e < 0 ? s.w : -s.w);
+                        s.p = s.p + d;
+                        if (r.w != 0.0f) s.prev = s.prev + d * 0.08f;
+                    }
+            } else if (mine) {
+                const bool tether = (gather & kPassTether) != 0;
+                const int* goff = tether ? v.te_off : v.bj_off;
+                const int2* gent = tether ? v.te_ent : v.bj_ent;
+                const float4 p4 = f4(s.p, s.w);
+                const int g0 = __ldg(&goff[i]), g1 = tether && v.te_free && !(s.w > 0.0f) ? g0 : __ldg(&goff[i + 1]);
+                for (int k = g0; k < g1; ++k) {
+                    const int2 e = __ldg(&gent[k]);
+                    const bool self_is_j = (e.x & kSideBit) != 0;
+                    const float4 q4 = ld_cluster<kOne>(map.addr((e.x & 0x7fffffff) - v0) + at);
+                    const float4 pi = self_is_j ? q4 : p4, pj = self_is_j ? p4 : q4;
+                    if (tether)
+                        tether_term(P, v.counts, dt, pi, pj, __int_as_float(e.y), self_is_j, v.te_free != 0, &s.p, &s.prev);
+                    else
+                        bend_term(P, v.counts, dt, pi, pj, __int_as_float(e.y), self_is_j, &s.p, &s.prev);
+                }
+            }
+        }
+        if (!mine) continue;
+        if (op.flags & kPassPin) pin_apply(pin_weight, pin_target, pin_relax, inv_mass, dt, &s);
+        if (op.flags & kPassAnalytic) analytic_stage(P, v.counts, inv_mass, dt, &s);
+        if (op.flags & kPassSdf) sdf_stage(v, P, inv_mass, dt, &s);
+        if ((op.flags & kPassPinPolish) && (op.last_it || P.use_ground || P.use_wall || P.use_sphere || P.sdf_ready))
+            pin_apply(pin_weight, pin_target, pin_relax, inv_mass, dt, &s);
+        if (op.flags & kPassVelocity) velocity_stage(P, dt, &s);
+    }
+    clamps = __reduce_add_sync(0xffffffffu, clamps);
+    wings = __reduce_add_sync(0xffffffffu, wings);
+    guards = __reduce_add_sync(0xffffffffu, guards);
+    if ((t & 31) == 0) {
+        count_add(v.counts, kCntHardFallbacks, clamps);
+        count_add(v.counts, kCntBendingWings, wings);
+        count_add(v.counts, kCntBendingGuards, guards);
+    }
+    if (mine) {
+        buf0[i] = f4(s.p, s.w);
+        v.prev[i] = f4(s.prev, 0.0f);
+        v.vel[i] = f4(s.vel, 0.0f);
+    }
+    bar.sync();  // no CTA leaves while another still reads its shared memory
+}
+
+namespace {
+
+using FrameKernel = void (*)(View, FramePlan, const FrameOp*, int, int, float4*, const int2*, int);
+struct FrameShape {
+    FrameKernel run;
+    int threads;
+};
+FrameShape frame_kernel(const FramePlan& f) {
+    if (f.ctas == 1) return f.chunk <= 512 ? FrameShape{k_frame_edges<512, true>, 512} : FrameShape{k_frame_edges<1024, true>, 1024};
+    return f.chunk <= 512 ? FrameShape{k_frame_edges<512, false>, 512} : FrameShape{k_frame_edges<768, false>, 768};
+}
+size_t frame_smem(const FramePlan& f) { return 3 * 16 * (size_t)f.chunk + 32 * (size_t)f.edge_rows + 4 * (size_t)f.ent_rows; }
+constexpr int kFrameSmem = 220 * 1024;
+
+}  // namespace
+
+bool frame_shape(int K, int max_v, FramePlan* f) {
+    f->ctas = 0;
+    if (K < 1 || max_v < 1) return false;
+    // as many CTAs per cloth as keep every cloth resident at once, with at
+    // least 128 vertices each; past 768 vertices per CTA the launched passes
+    // are no slower (30 cloths of up to 64 x 64: 235 us launched, 232 here)
+    int c = 1;
+    while (c < 16 && c * 128 < max_v && 2 * c * (long long)K <= 152) c *= 2;
+    f->chunk = std::max((max_v + 32 * c - 1) / (32 * c), 1) * 32;
+    if (f->chunk > (c == 1 ? 1024 : 768)) return false;
+    f->ctas = c;
+    return true;
+}
+
+bool frame_fits(const FramePlan& f) {
+    const FrameShape k = frame_kernel(f);
+    return frame_smem(f) <= (size_t)kFrameSmem && cluster_fit(k.run, f.ctas, k.threads, kFrameSmem) >= 1;
+}
+
+cudaError_t launch_frame_edges(const View& v, const FramePlan& f, const FrameOp* ops, int first, int last, float4* buf0,
+                               const int2* bend_ranges, int K, cudaStream_t s) {
+    const FrameShape k = frame_kernel(f);
+    return cluster_launch(k.run, K, f.ctas, k.threads, frame_smem(f), s, v, f, ops, first, last, buf0, bend_ranges, K);
 }
 
 // cluster > 1: one cluster of that many CTAs per cloth (block threads each)

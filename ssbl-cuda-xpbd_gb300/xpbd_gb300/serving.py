@@ -100,6 +100,8 @@ def estimate_device_bytes(req: ClothRequest) -> int:
         # CG blocks, preconditioner, r / z / d / q, cap sums, off-diagonal per
         # stretch-CSR entry (two per edge), colour-sorted cap edges, partials
         b += V * (32 + 32 + 4 * 16 + 16) + E * (2 * 16 + 12) + (V // 256 + 1) * 36 + 1024
+    if not o.self_collision and not o.stretch_optimization_enabled:
+        b += E * 16 + 256  # the fused frame's edge tables
     nst = len(req.static_triangles)
     if nst:
         res = max(o.static_sdf_max_resolution if o.static_sdf_max_resolution > 0 else 160, 16)
