@@ -1370,6 +1370,10 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
     if (ok && any_pressure)
         ok = dalloc(&S->p_area, nV, "pressure area allocation") && dalloc(&S->p_rest, nV, "pressure scale allocation");
     if (ok && S->self_any) {
+        self_set_carveout();
+        step_set_carveout();
+        cudaFuncSetAttribute(k_zero_spans, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+        cudaGetLastError();
         ok = dalloc(&S->nb_count, nV, "self collision count allocation") &&
              dalloc(&S->nb_idx, (size_t)nV * kNeighborSlots, "self collision index allocation") &&
              dalloc(&S->acc, nV, "self accumulation allocation") &&
@@ -2348,7 +2352,15 @@ bool tune_value_ok(int slot, int v) {
 
 }  // namespace
 
-int effective_tune(const Solver* S, int slot) { return slot == kTuneFusedFrame ? fused_mode(S) : tune_of(S->tune, slot); }
+int effective_tune(const Solver* S, int slot) {
+    if (slot == kTuneFusedFrame) return fused_mode(S);
+    if (slot == kTuneNeighborLanes) {
+        int n = 0;
+        for (int k = 0; k < S->K; ++k) n += S->cl[k].self_enabled && !S->cl[k].fast ? S->hp[k].V : 0;
+        return neighbor_lanes(S->tune, n);
+    }
+    return tune_of(S->tune, slot);
+}
 
 bool set_launch_config(Solver* S, const int* values, int n) {
     if (!S || (!values && n > 0) || n < 0 || n > kTuneSlots) return fail("invalid launch configuration");
@@ -2421,7 +2433,7 @@ bool autotune(Solver* S, int substeps, int iterations, int rounds, float* ms_out
     };
     const LaunchTune start = S->tune;
     LaunchTune best = start;
-    for (int k = 0; k < kTuneSlots; ++k) best.v[k] = (short)tune_of(start, k);
+    for (int k = 0; k < kTuneSlots; ++k) best.v[k] = (short)effective_tune(S, k);
     S->tune = best;
     S->drop_graphs();
     float best_ms = 0.0f, default_ms = 0.0f;

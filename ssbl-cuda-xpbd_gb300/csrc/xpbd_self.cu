@@ -21,6 +21,8 @@
 // Accumulation.  Pushes are scattered into per-vertex fixed-point int64
 // accumulators (2^-32 m units) with integer atomics, so the per-vertex sums do
 // not depend on the order of the atomics.
+#include <initializer_list>
+
 #include "xpbd_solver.cuh"
 
 namespace xg {
@@ -1706,18 +1708,18 @@ __global__ void __launch_bounds__(kThreads, 4) k_ee_warp(View v) {
 // Strict VT query for cloths whose candidate budget is at least the 32 query
 // slots: every accepted pair of an item's slots is taken, so the pairs are
 // independent and their order does not matter (pushes are summed in fixed
-// point).  One warp per 32 consecutive query vertices lays their bucket
+// point).  One warp per `per_warp` consecutive query vertices lays their bucket
 // slots end to end and evaluates 32 (vertex, slot) pairs per round, so the
 // lanes stay busy however the slot counts vary.  The same pairs, counters
 // and pushes as the 8-lane group kernel, which keeps the cloths with a
 // smaller budget.
-__global__ void __launch_bounds__(kThreads, 6) k_flat_vt(View v) {
+__global__ void __launch_bounds__(kThreads, 6) k_flat_vt(View v, int per_warp) {
     const int lane = threadIdx.x & 31;
-    const int item = v.lo + warp_global_id() * 32 + lane;
+    const int item = v.lo + warp_global_id() * per_warp + lane;
     int st = 0, lim = 0;
     float target = 0.0f, onset = 0.0f;
     bool counted = false;
-    if (item < v.hi) {
+    if (lane < per_warp && item < v.hi) {
         const Params& P = params_v(v, item);
         if (P.thash && !fast_mode(P) && self_scheduled(P, v) && neighbor_budget(P) >= kBucketSlots) {
             const F3 q = f3(v.pos[item]);
@@ -1786,16 +1788,16 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_vt(View v) {
 // ballots, so the result does not depend on the order of evaluation.
 constexpr int kEeRing = 128;
 
-__global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v) {
+__global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
     __shared__ int2 ring_s[kThreads / 32][kEeRing];
     const int lane = threadIdx.x & 31;
     int2* ring = ring_s[threadIdx.x >> 5];
-    const int item = v.lo + warp_global_id() * 32 + lane;
+    const int item = v.lo + warp_global_id() * per_warp + lane;
     long long st = 0;
     int lim = 0;
     float target = 0.0f, onset = 0.0f;
     bool counted = false;
-    if (item < v.hi) {
+    if (lane < per_warp && item < v.hi) {
         const Params& P = params_e(v, item);
         bool want = P.ehash && !fast_mode(P) && self_scheduled(P, v) && neighbor_budget(P) >= kBucketSlots;
         F3 q{0.0f, 0.0f, 0.0f};
@@ -1960,23 +1962,29 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
 }
 
 // Fast-mode EE query, flattened: the same outcome as k_ee_fast.  Phase 1
-// classifies every (item, slot) pair of a warp's 32 items past the item's
+// classifies every (item, slot) pair of a warp's items past the item's
 // own id in its ordered bucket (the earlier slots give no pair), 32 pairs per round
 // with the slots of the items laid end to end (duplicate = the same id as the
 // slot before; classify is side-effect free, so pairs past an item's budget
 // cut may be classified for nothing); classes and cluster keys go to shared
 // memory.  Phase 2 gives each lane its item and walks the slots in order:
 // visited / duplicate / rest-pose counts, the budget of passing pairs, the
-// cluster filter on up to 16 held keys, and for each taken pair the push,
-// recomputed by the same classify call, accumulated in fixed point.
-constexpr int kFastWarps = kThreads / 32;
+// cluster filter on up to 16 held keys, and marks the taken pairs.  Phase 3
+// goes over the pairs flat again and computes and accumulates (in fixed point)
+// the pushes of the taken ones, 32 lanes at a time: in the walk of phase 2
+// each lane did its own, up to 16 one after another (folded 100 x 100 cloth:
+// 76 us per launch).  A warp has `per_warp` items (flat_items); its classes
+// and keys take 160 bytes of shared memory per item.
+constexpr unsigned char kPairTaken = 5;
 
-__global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v) {
-    __shared__ unsigned char cls_s[kFastWarps][32 * kBucketSlots];
-    __shared__ unsigned key_s[kFastWarps][32 * kBucketSlots];
+__global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v, int per_warp) {
+    extern __shared__ unsigned fast_s[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int e = v.lo + warp_global_id() * 32 + lane;
-    bool run = e < v.hi;
+    unsigned* key_w = fast_s + wib * per_warp * kBucketSlots;
+    unsigned char* cls_w = reinterpret_cast<unsigned char*>(fast_s + (blockDim.x >> 5) * per_warp * kBucketSlots) +
+                           wib * per_warp * kBucketSlots;
+    const int e = v.lo + warp_global_id() * per_warp + lane;
+    bool run = lane < per_warp && e < v.hi;
     const Params* P = nullptr;
     if (run) {
         P = &params_e(v, e);
@@ -2027,8 +2035,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v) {
     }
     const int total = __shfl_sync(0xffffffffu, incl, 31);
     const int excl = incl - cnt - skip;  // so that slot = w - excl starts after the prefix
-    unsigned char* cls_w = cls_s[wib];
-    unsigned* key_w = key_s[wib];
     for (int base = 0; base < total; base += 32) {
         const int w = base + lane;
         int j = 0;
@@ -2081,17 +2087,30 @@ __global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v) {
                 if (q == nkeys) keys[q] = key;
             ++nkeys;
             ++c_acc;
-            SoftPush sp;
-            sp.apply = false;
-            unsigned k2 = 0u;
-            ee_fast_classify(v, e, v.eb_slot[st + slot], target, onset, P->key_ieee, &sp, &k2);
-            if (sp.apply) {
-                ++c_contact;
-                for (int k = 0; k < 4; ++k) {
-                    const float wk = sp.w[k];
-                    if ((k > 1 ? -wk : wk) > 0.0f) accumulate(v, sp.idx[k], sp.delta * wk);
-                }
-            }
+            cls_w[lane * kBucketSlots + slot] = kPairTaken;
+        }
+    }
+    __syncwarp();
+    for (int base = 0; base < total && __any_sync(0xffffffffu, c_acc > 0); base += 32) {
+        const int w = base + lane;
+        int j = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= w) j += step;
+        const int o_item = __shfl_sync(0xffffffffu, e, j);
+        const long long o_st = __shfl_sync(0xffffffffu, st, j);
+        const int o_excl = __shfl_sync(0xffffffffu, excl, j);
+        const float o_target = __shfl_sync(0xffffffffu, target, j), o_onset = __shfl_sync(0xffffffffu, onset, j);
+        if (w >= total || cls_w[j * kBucketSlots + w - o_excl] != kPairTaken) continue;
+        SoftPush sp;
+        sp.apply = false;
+        unsigned key = 0u;
+        ee_fast_classify(v, o_item, v.eb_slot[o_st + w - o_excl], o_target, o_onset, 0, &sp, &key);
+        if (!sp.apply) continue;
+        ++c_contact;
+        for (int k = 0; k < 4; ++k) {
+            const float wk = sp.w[k];
+            if ((k > 1 ? -wk : wk) > 0.0f) accumulate(v, sp.idx[k], sp.delta * wk);
         }
     }
     const int sums[6] = {c_seen, c_dup, c_rest, c_own, c_acc, c_contact};
@@ -2629,6 +2648,15 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
     }
 }
 
+// Items per warp of a flattened query over n items: 8 up to `few`, 16 up to
+// `some`, then 32.  The warps' rounds are a chain of dependent loads, so while
+// the chip has room for more warps fewer items each are faster.
+int flat_items(int n, int few, int some) { return n < few ? 8 : (n < some ? 16 : 32); }
+
+void flat_launch(void (*kernel)(View, int), const View& v, const ItemRange& r, int b, int per_warp, size_t smem, cudaStream_t s) {
+    kernel<<<grid((r.size() + per_warp - 1) / per_warp, 32, b), b, smem, s>>>(ranged(v, r), per_warp);
+}
+
 template <int L>
 void group_queries(const View& v, const SelfVariants& sv, int b, cudaStream_t s, bool edges) {
     if (edges)
@@ -2646,7 +2674,26 @@ void group_queries_lanes(const View& v, const SelfVariants& sv, cudaStream_t s, 
     }
 }
 
+template <class... K>
+void set_carveout(K... kernels) {
+    (void)std::initializer_list<cudaError_t>{cudaFuncSetAttribute(kernels, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout)...};
+}
+
 }  // namespace
+
+void self_set_carveout() {
+    set_carveout(k_vhash_count, k_vhash_scatter, k_tri_hash<1>, k_tri_hash<2>, k_tri_hash<4>, k_tri_hash<8>, k_tri_hash<16>,
+                 k_scan_reduce, k_scan_sums, k_scan_down, k_edge_insert<1>, k_edge_insert<2>, k_edge_insert<4>, k_edge_insert<8>,
+                 k_edge_insert<16>, k_edge_ovf_offsets, k_edge_ovf_late, k_edge_ovf_collect<1>, k_edge_ovf_collect<2>,
+                 k_edge_ovf_collect<4>, k_edge_ovf_collect<8>, k_edge_ovf_collect<16>, k_edge_ovf_select, k_edge_trim, k_bucket_sort,
+                 k_bucket_trim, k_neighbors_brute, k_vv, k_vv_warp, k_vt_hash, k_vt_brute, k_ee_brute, k_vt_warp<4>, k_vt_warp<8>,
+                 k_vt_warp<16>, k_ee_warp<4>, k_ee_warp<8>, k_ee_warp<16>, k_flat_vt, k_flat_ee, k_ee_fast_flat, k_ee_fast,
+                 k_island<kIslandLanes>, k_self_apply, k_neighbors_group<true, 1>, k_neighbors_group<true, 2>,
+                 k_neighbors_group<true, 4>, k_neighbors_group<true, 8>, k_neighbors_group<true, 16>, k_neighbors_group<true, 32>,
+                 k_neighbors_group<false, 1>, k_neighbors_group<false, 2>, k_neighbors_group<false, 4>, k_neighbors_group<false, 8>,
+                 k_neighbors_group<false, 16>, k_neighbors_group<false, 32>);
+    cudaGetLastError();  // a preference: the kernels run without it
+}
 
 void scan_bucket_counts(int* counts, int* start, int n, int* block_sums, cudaStream_t s) {
     if (n > 0) scan_counts(counts, start, n, block_sums, nullptr, s);
@@ -2697,13 +2744,18 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     if (order != 0) bucket_order(v, order == 3 ? sv.eb : sv.eb_ord, nullptr, v.eb_slot, nb, 2, 3, s);
 }
 
+int neighbor_lanes(const LaunchTune& t, int vertices) {
+    if (t.v[kTuneNeighborLanes] > 0) return t.v[kTuneNeighborLanes];
+    return vertices < (4 << 10) ? 16 : (vertices < (24 << 10) ? 8 : (vertices < (64 << 10) ? 4 : 2));
+}
+
 void self_neighbors(const View& v, int mode, const SelfVariants& sv, cudaStream_t s) {
     const ItemRange& r = mode == 1 ? sv.v_fast : (mode == 2 ? sv.v_strict : sv.v_all);
     if (r.size() == 0) return;
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     if (sv.hashed_v) {
         const bool vv = mode == 2;  // strict passes: VV responses fused
-        switch (tune_of(v.tune, kTuneNeighborLanes)) {
+        switch (neighbor_lanes(v.tune, r.size())) {
             case 1: neighbors_group<1>(v, r, vv, mode, wb, s); break;
             case 4: neighbors_group<4>(v, r, vv, mode, wb, s); break;
             case 8: neighbors_group<8>(v, r, vv, mode, wb, s); break;
@@ -2724,7 +2776,7 @@ void self_vv(const View& v, const SelfVariants& sv, cudaStream_t s) {
 void self_vt(const View& v, const SelfVariants& sv, cudaStream_t s) {
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     if (sv.hashed_t && sv.strict_wide && sv.v_strict.size() > 0)
-        k_flat_vt<<<grid(sv.v_strict.size(), 1, wb), wb, 0, s>>>(ranged(v, sv.v_strict));
+        flat_launch(k_flat_vt, v, sv.v_strict, wb, flat_items(sv.v_strict.size(), 32 << 10, 32 << 10), 0, s);
     if (sv.hashed_t && sv.strict_narrow && sv.v_strict.size() > 0) group_queries_lanes(v, sv, s, false);
     if (sv.hashed_t && sv.fast && sv.v_fast.size() > 0)
         k_vt_hash<<<grid(sv.v_fast.size(), 1, qb), qb, 0, s>>>(ranged(v, sv.v_fast));
@@ -2734,12 +2786,12 @@ void self_ee(const View& v, const SelfVariants& sv, cudaStream_t s) {
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     const int gb = tune_of(v.tune, kTuneGroupBlock);
     if (sv.hashed_e && sv.strict_wide && sv.e_strict.size() > 0)
-        k_flat_ee<<<grid(sv.e_strict.size(), 1, wb), wb, 0, s>>>(ranged(v, sv.e_strict));
+        flat_launch(k_flat_ee, v, sv.e_strict, wb, flat_items(sv.e_strict.size(), 64 << 10, 300 << 10), 0, s);
     if (sv.hashed_e && sv.strict_narrow && sv.e_strict.size() > 0) group_queries_lanes(v, sv, s, true);
     if (sv.hashed_e && sv.fast && sv.e_fast.size() > 0) {
         if (tune_of(v.tune, kTuneFastEeForm) == 32) {
-            const int fb = min(wb, kThreads);  // the shared arrays hold kThreads / 32 warps
-            k_ee_fast_flat<<<grid(sv.e_fast.size(), 1, fb), fb, 0, s>>>(ranged(v, sv.e_fast));
+            const int n = flat_items(sv.e_fast.size(), 64 << 10, 1 << 30);
+            flat_launch(k_ee_fast_flat, v, sv.e_fast, wb, n, (size_t)(wb / 32) * n * kBucketSlots * 5, s);
         } else {
             k_ee_fast<<<grid(sv.e_fast.size(), kQueryLanes, gb), gb, 0, s>>>(ranged(v, sv.e_fast));
         }

@@ -252,16 +252,22 @@ enum TuneSlot {
     kTuneFastEeForm,       // fast-mode EE query: 8 = groups of 8 lanes, 32 = one warp per 32 items, flattened (32)
     kTuneFusedFrame,       // small cloths: 1 = whole frame in one block per cloth, 8 = in an 8-CTA cluster per cloth,
                            // 2 = launched kernels (1)
-    kTuneTriLanes,         // lanes per primitive of the triangle hash: 1, 2, 4, 8, 16 (8)
-    kTuneNeighborLanes,    // lanes per vertex of the neighbour table (+ strict VV): 1, 2, 4, 8, 16, 32 (2)
+    kTuneTriLanes,         // lanes per primitive of the triangle hash: 1, 2, 4, 8, 16 (1)
+    kTuneNeighborLanes,    // lanes per vertex of the neighbour table (+ strict VV): 1, 2, 4, 8, 16, 32 (by size, neighbor_lanes)
     kTuneSlots
 };
 struct LaunchTune {
     short v[kTuneSlots];
 };
-constexpr short kTuneDefault[kTuneSlots] = {128, 256, 8, 256, 256, 8, 256, 128, 32, 0, 8, 2};
+constexpr short kTuneDefault[kTuneSlots] = {128, 256, 8, 256, 256, 8, 256, 128, 32, 0, 1, 2};
 constexpr int kMaxBlock = 256;  // the kernels' launch bounds
 inline int tune_of(const LaunchTune& t, int slot) { return t.v[slot] > 0 ? t.v[slot] : kTuneDefault[slot]; }
+// Lanes per vertex of the neighbour table over so many vertices: the walk of
+// 27 cells is a chain of dependent loads, which lanes share while the chip has
+// room for them; past that every lane repeats the vertex's set-up.  Us per
+// frame with 2 lanes and as chosen: 1,369 vertices 1,033 / 669 (16 lanes);
+// 40,000 3,073 / 2,929 (4); 202,500 10,872 / 10,872 (2; 11,724 with 8).
+int neighbor_lanes(const LaunchTune& t, int vertices);
 inline int grid_for(long long threads, int block) { return (int)((threads + block - 1) / block); }
 
 // Device pointers of one solver, passed by value to each kernel, plus the
@@ -530,5 +536,14 @@ void self_vt(const View& v, const SelfVariants& sv, cudaStream_t s);
 void self_ee(const View& v, const SelfVariants& sv, cudaStream_t s);
 void self_island(const View& v, const SelfVariants& sv, cudaStream_t s);
 void self_apply(const View& v, const SelfVariants& sv, cudaStream_t s);
+// Share of an SM's L1 that every kernel of a frame asks for as shared memory
+// (percent; 64 KB).  Kernels of different branches run on an SM at the same
+// time only when they agree on it: with each kernel's own preference the
+// neighbour table (none) and the edge-edge query (64 KB) took turns, and a
+// faster neighbour table made the frame slower (100 x 100 drop 1.49 -> 2.08 ms;
+// with one share 1.18).
+constexpr int kCarveout = 28;
+void self_set_carveout();
+void step_set_carveout();
 
 }  // namespace xg

@@ -987,6 +987,14 @@ void launch_frame_fused(const View& v, const FrameOp* ops, int nops, float4* buf
     if (K > 0) k_frame_fused<<<K, block, smem, s>>>(v, ops, nops, buf0, bend_ranges, K);
 }
 
+void step_set_carveout() {
+    cudaFuncSetAttribute(k_predict, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaFuncSetAttribute(k_vertex_pass, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaFuncSetAttribute(k_bend_color, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaFuncSetAttribute(k_copy_pos, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaGetLastError();  // a preference: the kernels run without it
+}
+
 void launch_predict(const View& v, int V, cudaStream_t s) {
     const int b = tune_of(v.tune, kTuneVertexBlock);
     if (V > 0) k_predict<<<grid_for(V, b), b, 0, s>>>(v);
