@@ -1785,6 +1785,14 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
     const bool spring = S->spring_any;
     const bool hard = S->pcg_hard;
     const bool colored_bends = !S->bend_colors.empty();
+    // Two per-vertex steps ride on a neighbouring pass instead of a launch of
+    // their own: the prediction of the next substep on the velocity stage
+    // (where no vertex normals are gathered) and the last self-collision
+    // pass's pushes on the pass after it.  A profiled frame and the recorded
+    // operations keep them apart, and so do launched kernels asked for by the
+    // launch configuration.
+    const bool merge = !prof && !S->rec && fused_mode(S) != 2;
+    const bool ride = merge && !normals;
     View base = S->view();
     base.substeps = substeps;
     if (prof) {
@@ -1874,7 +1882,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
         if (normals) pv.pos = S->pos[cur ^ 1];  // vertex normals read the snapshot
         if (S->rec)
             S->rec->push_back(FrameOp{0, 0u, buf_index(S, pv.pos_in), buf_index(S, pv.pos), s, 0, 0});
-        else
+        else if (!ride || s == 0)
             timed(kKPredict, 1, [&] { launch_predict(pv, nV, S->stream); });
         if (normals) cur ^= 1;
         for (int it = 0; it < iterations; ++it) {
@@ -2007,7 +2015,10 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
                         timed(kKIsland, 1, [&] { self_island(pv2, sp.sv, lane_stream(1)); });
                     if (sp.any_e) timed(kKEdgeEdge, 1, [&] { self_ee(pv2, sp.sv, lane_stream(2)); });
                     join();
-                    timed(kKSelfApply, 1, [&] { self_apply(pv2, sp.sv, S->stream); });
+                    if (merge && pass + 1 == sp.passes && !(dyn & 2) && !(pcg && final_c && hard))
+                        pending |= kPassApply;
+                    else
+                        timed(kKSelfApply, 1, [&] { self_apply(pv2, sp.sv, S->stream); });
                 }
             }
             // signed dynamic colliders after self collision (abi41.cu:9340-9345)
@@ -2041,6 +2052,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
             if (analytic || sdf || last_it) pending |= kPassPinPolish;
         }
         pending |= kPassVelocity;
+        if (ride && s + 1 < substeps) pending |= kPassPredict;
         flush();
     }
     if (cur != 0 && S->rec)

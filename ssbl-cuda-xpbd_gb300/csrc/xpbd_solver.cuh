@@ -426,6 +426,8 @@ enum PassFlags : unsigned {
     kPassVelocity = 32u,
     kPassTether = 64u,
     kPassBend = 128u,
+    kPassPredict = 256u,  // the next substep's prediction after the velocity stage (no vertex normals)
+    kPassApply = 512u,    // the last self-collision pass's pushes before the other stages
 };
 void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s);
 

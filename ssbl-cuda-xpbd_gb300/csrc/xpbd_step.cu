@@ -419,6 +419,54 @@ __global__ void __launch_bounds__(kThreads) k_predict(View v) {
     if (i < v.nV) predict_item(v, i);
 }
 
+// Average of a vertex's accumulated self-collision pushes, clamped to 0.35 r,
+// applied with a 0.55 prev shift; the accumulators are cleared for the next
+// pass (abi41.cu:4953-4988).
+__device__ __forceinline__ void apply_pushes(const View& v, const Params& P, int i, float inv_mass, VState* s) {
+    const Acc4 a = v.acc[i];
+    if (a.w == 0) return;  // every push adds a weight: nothing accumulated, the row is still zero
+    v.acc[i] = Acc4{0, 0, 0, 0};
+    if (!(inv_mass > 0.0f) || a.w <= 0) return;
+    F3 avg = F3{from_fix(a.x), from_fix(a.y), from_fix(a.z)} * (1.0f / (float)a.w);
+    const float max_delta = fmaxf(P.self_radius * 0.35f, 1.0e-4f);
+    const float dl = len3(avg);
+    if (dl > max_delta) avg = avg * (max_delta / dl);
+    s->p = s->p + avg;
+    s->prev = s->prev + avg * 0.55f;
+    const float al = len3(avg);
+    if (al > 0.0f) atomicMax(v.max_delta_bits, __float_as_uint(al));
+}
+
+// The stages of a pass after its gather, and the vertex's rows.
+__device__ __forceinline__ void finish_vertex(const View& v, const Params& P, int i, unsigned flags, float inv_mass, float dt, VState* st) {
+    VState& s = *st;
+    if (flags & kPassApply) apply_pushes(v, P, i, inv_mass, &s);
+    if (flags & kPassPin) pin_stage(v, i, inv_mass, dt, &s);
+    if (flags & kPassAnalytic) analytic_stage(P, v.counts, inv_mass, dt, &s);
+    if (flags & kPassSdf) sdf_stage(v, P, inv_mass, dt, &s);
+    // final pin polish when this cloth ran a contact stage in this iteration
+    // (analytic colliders, SDF, or any last iteration; abi41.cu:9360-9369)
+    if ((flags & kPassPinPolish) &&
+        (v.last_it || P.use_ground || P.use_wall || P.use_sphere || P.sdf_ready))
+        pin_stage(v, i, inv_mass, dt, &s);
+    if (flags & kPassVelocity) velocity_stage(P, dt, &s);
+    if (flags & kPassPredict) {
+        // the next substep's prediction (predict_item without vertex normals)
+        s.prev = s.p;
+        if (!(s.w > 0.0f)) {
+            s.vel = F3{0.0f, 0.0f, 0.0f};
+            s.p = f3(ld4(&v.rest[i]));
+        } else {
+            predict_free(P, dt, &s);
+        }
+        pin_stage(v, i, inv_mass, dt, &s);
+    }
+    v.pos[i] = f4(s.p, s.w);
+    v.prev[i] = f4(s.prev, 0.0f);
+    v.vel[i] = f4(s.vel, 0.0f);
+}
+
+
 __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned flags) {
     const Params& P = params_v(v, i);
     const float dt = P.sub_dt;
@@ -465,18 +513,76 @@ __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned 
         s.p = dp;
         s.prev = dprev;
     }
-    if (flags & kPassPin) pin_stage(v, i, inv_mass, dt, &s);
-    if (flags & kPassAnalytic) analytic_stage(P, v.counts, inv_mass, dt, &s);
-    if (flags & kPassSdf) sdf_stage(v, P, inv_mass, dt, &s);
-    // final pin polish when this cloth ran a contact stage in this iteration
-    // (analytic colliders, SDF, or any last iteration; abi41.cu:9360-9369)
-    if ((flags & kPassPinPolish) &&
-        (v.last_it || P.use_ground || P.use_wall || P.use_sphere || P.sdf_ready))
-        pin_stage(v, i, inv_mass, dt, &s);
-    if (flags & kPassVelocity) velocity_stage(P, dt, &s);
-    v.pos[i] = f4(s.p, s.w);
-    v.prev[i] = f4(s.prev, 0.0f);
-    v.vel[i] = f4(s.vel, 0.0f);
+    finish_vertex(v, P, i, flags, inv_mass, dt, &s);
+}
+
+// The same pass with L lanes per vertex (32 / L vertices per warp) for the
+// stretch gather: lane u takes entries u, u + L, ... and the vertex's first
+// lane adds the corrections in entry order, so the sums are those of
+// vertex_pass_item.  A thread per vertex walks its six or so entries one after
+// another, each a load and a chain of a root and two quotients, while a cloth
+// of a few ten thousand vertices leaves most of the chip's warps unused.
+template <int L>
+__global__ void __launch_bounds__(kThreads) k_vertex_pass_lanes(View v, unsigned flags) {
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(g / L), sub = (int)(g % L);
+    bool work = i < v.nV;
+    const Params* P = nullptr;
+    float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int k = 0, end = 0;
+    VState s{F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, 0.0f};
+    float dt = 0.0f, alpha = 0.0f;
+    if (work) {
+        P = &params_v(v, i);
+        p4 = v.pos_in[i];
+        if (!P->active) {
+            if (sub == 0 && v.pos != v.pos_in) v.pos[i] = p4;  // keep the ping-pong buffers in step
+            work = false;
+        }
+    }
+    if (work) {
+        s.w = p4.w;
+        s.p = f3(p4);
+        if (sub == 0) {
+            s.prev = f3(v.prev[i]);
+            s.vel = f3(v.vel[i]);
+        }
+        dt = P->sub_dt;
+        alpha = stretch_alpha(P->stretch_compliance, dt);
+        if (!P->pcg_on) {
+            k = __ldg(&v.sp_off[i]);
+            end = __ldg(&v.sp_off[i + 1]);
+        }
+    }
+    const int rounds = (__reduce_max_sync(0xffffffffu, end - k) + L - 1) / L;
+    k += sub;
+    for (int n = 0; n < rounds; ++n, k += L) {
+        F3 d{0.0f, 0.0f, 0.0f};
+        int use = 0;  // bit 0 a correction, bit 1 a stretched edge
+        if (k < end) {
+            const int2 e = __ldg(&v.sp_ent[k]);
+            const bool self_is_j = (e.x & kSideBit) != 0;
+            const float4 q4 = v.pos_in[e.x & 0x7fffffff];
+            F3 corr;
+            float c;
+            bool clamped;
+            if (stretch_correction(self_is_j ? q4 : p4, self_is_j ? p4 : q4, __int_as_float(e.y), alpha, &corr, &c, &clamped)) {
+                if (clamped && !self_is_j) count1(v.counts, kCntHardFallbacks);
+                if (p4.w > 0.0f) {
+                    d = self_is_j ? corr * p4.w : corr * (-p4.w);
+                    use = c > 0.0f ? 3 : 1;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < L; ++u) {
+            const F3 du{__shfl_sync(0xffffffffu, d.x, u, L), __shfl_sync(0xffffffffu, d.y, u, L), __shfl_sync(0xffffffffu, d.z, u, L)};
+            const int uu = __shfl_sync(0xffffffffu, use, u, L);
+            if (uu & 1) s.p = s.p + du;
+            if (uu & 2) s.prev = s.prev + du * 0.08f;
+        }
+    }
+    if (work && sub == 0) finish_vertex(v, *P, i, flags, __ldg(&v.inv_mass[i]), dt, &s);
 }
 
 // Six 256-thread blocks per SM (40 registers): the gathers are latency
@@ -990,6 +1096,9 @@ void launch_frame_fused(const View& v, const FrameOp* ops, int nops, float4* buf
 void step_set_carveout() {
     cudaFuncSetAttribute(k_predict, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
     cudaFuncSetAttribute(k_vertex_pass, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaFuncSetAttribute(k_vertex_pass_lanes<2>, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaFuncSetAttribute(k_vertex_pass_lanes<4>, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
+    cudaFuncSetAttribute(k_vertex_pass_lanes<8>, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
     cudaFuncSetAttribute(k_bend_color, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
     cudaFuncSetAttribute(k_copy_pos, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
     cudaGetLastError();  // a preference: the kernels run without it
@@ -1000,9 +1109,23 @@ void launch_predict(const View& v, int V, cudaStream_t s) {
     if (V > 0) k_predict<<<grid_for(V, b), b, 0, s>>>(v);
 }
 
+// Lanes per vertex of a stretch pass over V vertices.  Us per frame of a plain
+// cloth (with the host calls) with 1, 2, 4, 8 lanes: 10,000 vertices in a drop
+// 1,165, 1,103, 1,103, 1,099; 32,400 291, 241, 241, 276; 57,600 374, 319, 359,
+// 410; 90,000 457, 430, 479, 578; 202,500 733, 732, 866, 1,076.
+constexpr int kPassLanes8 = 16 << 10, kPassLanes4 = 32 << 10, kPassLanes2 = 128 << 10;
+
 void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s) {
     const int b = tune_of(v.tune, kTuneVertexBlock);
-    if (V > 0) k_vertex_pass<<<grid_for(V, b), b, 0, s>>>(v, flags);
+    if (V <= 0) return;
+    if ((flags & kPassSpring) && V <= kPassLanes8)
+        k_vertex_pass_lanes<8><<<grid_for(8ll * V, b), b, 0, s>>>(v, flags);
+    else if ((flags & kPassSpring) && V <= kPassLanes4)
+        k_vertex_pass_lanes<4><<<grid_for(4ll * V, b), b, 0, s>>>(v, flags);
+    else if ((flags & kPassSpring) && V <= kPassLanes2)
+        k_vertex_pass_lanes<2><<<grid_for(2ll * V, b), b, 0, s>>>(v, flags);
+    else
+        k_vertex_pass<<<grid_for(V, b), b, 0, s>>>(v, flags);
 }
 
 void launch_bend_color(const View& v, int start, int count, cudaStream_t s) {
