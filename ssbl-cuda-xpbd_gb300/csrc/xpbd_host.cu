@@ -466,6 +466,7 @@ View Solver::view() const {
     v.eb_ovf_count = eb_ovf_count;
     v.eb_ovf_start = eb_ovf_start;
     v.eb_late = eb_late;
+    v.e_order = e_order;
     v.eb_late_count = eb_late_count;
     v.eb_late_cap = eb_late_cap;
     v.nb_count = nb_count;
@@ -540,6 +541,7 @@ void free_solver(Solver* S) {
     dfree(S->eb_ovf_start);
     dfree(S->eb_ovf_count);
     dfree(S->eb_late);
+    dfree(S->e_order);
     dfree(S->eb_late_count);
     dfree(S->nb_count);
     dfree(S->nb_idx);
@@ -1369,6 +1371,20 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
              dalloc(&S->vt_tri, vt_tri.size(), "incident triangle allocation");
     if (ok && any_pressure)
         ok = dalloc(&S->p_area, nV, "pressure area allocation") && dalloc(&S->p_rest, nV, "pressure scale allocation");
+    std::vector<int> e_order;
+    if (ok && S->self_any && nE > 0) {
+        // counting sort by first endpoint within each cloth, invalid edges last
+        e_order.resize(nE);
+        std::vector<int> at;
+        for (const Params& P : S->hp) {
+            at.assign(P.V + 2, 0);
+            auto key = [&](int e) { return springs[e].x >= P.vstart && springs[e].x < P.vstart + P.V ? springs[e].x - P.vstart : P.V; };
+            for (int e = P.estart; e < P.estart + P.E; ++e) at[key(e) + 1]++;
+            for (int i = 0; i <= P.V; ++i) at[i + 1] += at[i];
+            for (int e = P.estart; e < P.estart + P.E; ++e) e_order[P.estart + at[key(e)]++] = e;
+        }
+        ok = dalloc(&S->e_order, nE, "self edge order allocation");
+    }
     if (ok && S->self_any) {
         self_set_carveout();
         step_set_carveout();
@@ -1582,6 +1598,7 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
          cuda_ok(cudaMemsetAsync(S->max_delta_bits, 0, sizeof(unsigned), st), "reset self max smoothed delta") &&
          (!S->acc || cuda_ok(cudaMemsetAsync(S->acc, 0, sizeof(Acc4) * nV, st), "reset self accumulation")) &&
          (!S->nb_count || cuda_ok(cudaMemsetAsync(S->nb_count, 0, sizeof(int) * nV, st), "reset neighbor table")) &&
+         dupload(S->e_order, e_order.data(), e_order.size(), st, "self edge order upload") &&
          dupload(S->frame_tables, frame_tables.data(), frame_tables.size(), st, "fused frame upload") &&
          sync_params(S) && cuda_ok(cudaStreamSynchronize(st), "solver upload");
     if (ok && S->pcg_on)

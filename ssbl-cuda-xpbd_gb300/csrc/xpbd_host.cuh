@@ -303,6 +303,7 @@ struct Solver {
     int *eb_slot = nullptr, *eb_ovf_list = nullptr, *eb_ovf_count = nullptr, *eb_ovf_start = nullptr;
     unsigned* eb_ovf_bits = nullptr;
     long long eb_ovf_cap = 0;  // entries of eb_ovf_list
+    int* e_order = nullptr;    // each cloth's edges by first endpoint (insertion order)
     int2* eb_late = nullptr;   // insertions past a bucket's slots, as (bucket, edge)
     unsigned long long* eb_late_count = nullptr;
     long long eb_late_cap = 0;

@@ -426,16 +426,23 @@ __device__ __forceinline__ void edge_cells_walk4(const View& v, int k, int r0, b
     }
 }
 
+// Edges are inserted in the order of their first endpoint (e_order).  A caller's
+// edges come sorted by colour, so in that order every bucket is visited once
+// per colour, each time long enough after the last for its sector of slots to
+// have left L2: 860 MB of DRAM traffic for the 16 M insertions of a
+// 450 x 450 cloth, 630 us per build, 500 us in this order (256 uneven
+// cloths 2.54 -> 2.39 ms, 100 x 100 50 -> 46 us).
 template <int L>
 __global__ void __launch_bounds__(kThreads) k_edge_insert(View v) {
     __shared__ unsigned guard_s;  // the block's guard events: one global atomic per block
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = v.lo + (int)(t / L), r0 = (int)(t % L);
+    const int at = v.lo + (int)(t / L), r0 = (int)(t % L);
     if (threadIdx.x == 0) guard_s = 0u;
     __syncthreads();
     bool collapsed = false;
     unsigned past = 0u;
-    if (k < v.hi) {
+    if (at < v.hi) {
+        const int k = __ldg(&v.e_order[at]);
         edge_cells_walk4<L>(v, k, r0, &collapsed, [&](const int (&bs)[4], int n) {
             int slots[4];
 #pragma unroll

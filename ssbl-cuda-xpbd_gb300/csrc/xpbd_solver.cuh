@@ -330,6 +330,7 @@ struct View {
     int* eb_ovf_count;
     int* eb_ovf_start;      // [eb_ovf_list index] first entry of the bucket's region
     int2* eb_late;
+    const int* e_order;     // each cloth's edges by first endpoint
     unsigned long long* eb_late_count;
     long long eb_late_cap;
     int* scan_tmp;          // block sums of the bucket scans
