@@ -287,8 +287,13 @@ def cloth_inputs_device(rest: np.ndarray, triangles: np.ndarray, density: float,
         inv.ctypes.data_as(pf), bends.ctypes.data_as(pi), bend_rest.ctypes.data_as(pf), ctypes.byref(nb))
     if n < 0:
         raise RuntimeError((lib.ssbl_last_error() or b"").decode() or "device preprocessing failed")
-    return (edges[:n].copy(), edge_rest[:n].copy(), inv[:V].copy(), bends[:nb.value].copy(),
-            bend_rest[:nb.value].copy())
+    # the unused room goes back where the arrays are, with no copy into new pages
+    edges.resize((n, 2), refcheck=False)
+    edge_rest.resize(n, refcheck=False)
+    inv.resize(V, refcheck=False)
+    bends.resize((nb.value, 2), refcheck=False)
+    bend_rest.resize(nb.value, refcheck=False)
+    return edges, edge_rest, inv, bends, bend_rest
 
 
 def vertex_inverse_mass(rest: np.ndarray, triangles: np.ndarray, density: float, pin_mask: np.ndarray) -> np.ndarray:
