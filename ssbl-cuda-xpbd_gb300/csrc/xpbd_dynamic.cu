@@ -84,12 +84,22 @@ __device__ __forceinline__ void grow_box(int* box, bool use, int4 lo, int4 hi) {
     }
 }
 
+// Clears what a hash build counts into: bucket counts, the span box (every
+// cell below the lowest and above the highest) and the host's three words.
+__global__ void k_dyn_reset(int* cnt, int nb, int* words, int* box) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nb) cnt[i] = 0;
+    if (i < 8) box[i] = i < 4 ? 0x7f7f7f7f : (int)0x80808080;
+    if (words && i < 3) words[i] = 0;
+}
+
 // Count (scatter = false) or place (scatter = true) every cell of every
 // triangle; a triangle over 64 cells is flagged for the large list instead
-// (abi41.cu:3763-3930).  `occupancy` receives the largest bucket count and
-// `box` the span box of the triangles hashed, both in the count pass.
+// (abi41.cu:3763-3930).  In the count pass `words` receives what the host
+// waits for (largest bucket count, entries, large triangles) and `box` the
+// span box of the triangles hashed.
 __global__ void k_dyn_tri_hash(int T, const int4* cmin, const int4* cmax, int nb, int* cnt, int* ent, bool scatter,
-                               int* large_flag, int* occupancy, int* box) {
+                               int* large_flag, int* words, int* box) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int4 a = t < T ? cmin[t] : make_int4(0, 0, 0, 0), b = t < T ? cmax[t] : make_int4(-1, -1, -1, 0);
     const long long cells = span_cells(a, b);
@@ -97,6 +107,12 @@ __global__ void k_dyn_tri_hash(int T, const int4* cmin, const int4* cmax, int nb
     if (!scatter) {
         if (t < T) large_flag[t] = cells > kDynMaxCells ? 1 : 0;
         grow_box(box, hashed, a, b);
+        const unsigned entries = __reduce_add_sync(0xffffffffu, hashed ? (unsigned)cells : 0u);
+        const unsigned large = __popc(__ballot_sync(0xffffffffu, cells > kDynMaxCells));
+        if ((threadIdx.x & 31) == 0) {
+            if (entries) atomicAdd(&words[1], (int)entries);
+            if (large) atomicAdd(&words[2], (int)large);
+        }
     }
     if (!hashed) return;
     for (int z = a.z; z <= b.z; ++z)
@@ -107,7 +123,7 @@ __global__ void k_dyn_tri_hash(int T, const int4* cmin, const int4* cmax, int nb
                 if (scatter)
                     ent[slot] = t;
                 else
-                    atomicMax(occupancy, slot + 1);
+                    atomicMax(&words[0], slot + 1);
             }
 }
 
@@ -721,12 +737,6 @@ float rows_max_extent(const float* tris, int count) {
     return m;
 }
 
-// An empty span box: every cell below the lowest and above the highest.
-bool reset_box(int* box, cudaStream_t st) {
-    return cuda_ok(cudaMemsetAsync(box, 0x7f, sizeof(int) * 4, st), "reset dynamic span box") &&
-           cuda_ok(cudaMemsetAsync(box + 4, 0x80, sizeof(int) * 4, st), "reset dynamic span box");
-}
-
 // Bounds, cell spans and (>= 64 triangles) the hash of the triangles whose
 // rows are in D.tris (abi41.cu:3686-3760, 6220-6392).
 bool finish_triangles(const DynCtx& c, DynHost& D, int T, bool signed_mode, bool motion_valid, float cell) {
@@ -774,31 +784,30 @@ bool finish_triangles(const DynCtx& c, DynHost& D, int T, bool signed_mode, bool
                 return false;
             D.tb_cap = nb;
         }
-        if (!cuda_ok(cudaMemsetAsync(D.tcount, 0, sizeof(int) * nb, st), "reset dynamic triangle hash") ||
-            !cuda_ok(cudaMemsetAsync(D.small, 0, sizeof(int) * 4, st), "reset dynamic triangle hash") || !reset_box(D.small + 4, st))
-            return false;
+        k_dyn_reset<<<dyn_blocks(nb), kThreadsDyn, 0, st>>>(D.tcount, nb, D.small, D.small + 4);
         k_dyn_tri_hash<<<dyn_blocks(T), kThreadsDyn, 0, st>>>(T, D.cmin, D.cmax, nb, D.tcount, nullptr, false, D.lflag, D.small,
                                                              D.small + 4);
-        scan_bucket_counts(D.tcount, D.tstart, nb, D.scan_tmp, st);
-        scan_bucket_counts(D.lflag, D.lpos, T, D.scan_tmp, st);  // T <= nb / 4: the block sums fit
         int got[3] = {0, 0, 0};
-        if (!cuda_ok(cudaMemcpyAsync(&got[0], D.tstart + nb, sizeof(int), cudaMemcpyDeviceToHost, st), "dynamic triangle hash") ||
-            !cuda_ok(cudaMemcpyAsync(&got[1], D.lpos + T, sizeof(int), cudaMemcpyDeviceToHost, st), "dynamic triangle hash") ||
-            !cuda_ok(cudaMemcpyAsync(&got[2], D.small, sizeof(int), cudaMemcpyDeviceToHost, st), "dynamic triangle hash") ||
+        if (!cuda_ok(cudaMemcpyAsync(got, D.small, sizeof(got), cudaMemcpyDeviceToHost, st), "dynamic triangle hash") ||
             !cuda_ok(cudaStreamSynchronize(st), "dynamic triangle hash"))
             return false;
-        if (got[0] > D.tent_cap) {
-            if (!realloc_dev(c, &D.tent, (size_t)D.tent_cap, (size_t)got[0], "dynamic triangle hash")) return false;
-            D.tent_cap = got[0];
+        const int occupancy = got[0], entries = got[1], large = got[2];
+        scan_bucket_counts(D.tcount, D.tstart, nb, D.scan_tmp, st);
+        if (entries > D.tent_cap) {
+            if (!realloc_dev(c, &D.tent, (size_t)D.tent_cap, (size_t)entries, "dynamic triangle hash")) return false;
+            D.tent_cap = entries;
         }
         k_dyn_tri_hash<<<dyn_blocks(T), kThreadsDyn, 0, st>>>(T, D.cmin, D.cmax, nb, D.tcount, D.tent, true, nullptr, nullptr,
                                                              nullptr);
-        k_dyn_large_list<<<dyn_blocks(T), kThreadsDyn, 0, st>>>(T, D.cmin, D.cmax, D.lpos, D.large);
+        if (large > 0) {
+            scan_bucket_counts(D.lflag, D.lpos, T, D.scan_tmp, st);  // T <= nb / 4: the block sums fit
+            k_dyn_large_list<<<dyn_blocks(T), kThreadsDyn, 0, st>>>(T, D.cmin, D.cmax, D.lpos, D.large);
+        }
         k_dyn_sort_buckets<<<dyn_blocks(nb), kThreadsDyn, 0, st>>>(D.tstart, D.tent, nb);
         h.tri_buckets = nb;
-        h.large_count = got[1];
-        D.large_count = got[1];
-        D.max_occupancy = got[2];
+        h.large_count = large;
+        D.large_count = large;
+        D.max_occupancy = occupancy;
     }
     h.tris = D.tris;
     h.amin = D.amin;
@@ -908,8 +917,7 @@ bool put_particles(const DynCtx& c, DynHost& D, const float* pos, const float* p
             D.pb_cap = nb;
         }
         if (!D.pbox && !dalloc(&D.pbox, 8, "dynamic particle hash")) return false;
-        if (!cuda_ok(cudaMemsetAsync(D.pcount, 0, sizeof(int) * nb, st), "reset dynamic particle hash") || !reset_box(D.pbox, st))
-            return false;
+        k_dyn_reset<<<dyn_blocks(nb), kThreadsDyn, 0, st>>>(D.pcount, nb, nullptr, D.pbox);
         k_dyn_par_hash<<<dyn_blocks(count), kThreadsDyn, 0, st>>>(D.ppos, count, h.par_cell, nb, c.key_ieee, D.pcell, D.pcount,
                                                                    nullptr, false, D.pbox);
         scan_bucket_counts(D.pcount, D.pstart, nb, D.pscan, st);
@@ -931,16 +939,21 @@ bool put_particles(const DynCtx& c, DynHost& D, const float* pos, const float* p
 }
 
 // Copy the descriptor to the device (allocated on first use).
-bool publish_set(const DynCtx& c, DynHost& D) {
+bool put_set(const DynCtx& c, DynHost& D) {
     if (!D.dev && !dalloc(&D.dev, 1, "dynamic collider descriptor")) return false;
-    return dupload(D.dev, &D.h, 1, c.st, "dynamic collider descriptor") && cuda_ok(cudaStreamSynchronize(c.st), "dynamic collider upload");
+    return dupload(D.dev, &D.h, 1, c.st, "dynamic collider descriptor");
+}
+
+// The same for a shared scene, whose readers run on streams of their own.
+bool publish_set(const DynCtx& c, DynHost& D) {
+    return put_set(c, D) && cuda_ok(cudaStreamSynchronize(c.st), "dynamic collider upload");
 }
 
 // Point the cloth's parameters at its descriptor (null when it has no
-// dynamic collider).
+// dynamic collider).  Frames follow on the upload's own stream.
 bool publish(Solver* S, int k) {
     DynHost& D = S->cl[k].dyn;
-    if (!publish_set(cloth_ctx(S, k), D)) return false;
+    if (!put_set(cloth_ctx(S, k), D)) return false;
     const bool any = D.h.tri_count > 0 || D.h.par_count > 0;
     S->hp[k].dyn = any ? D.dev : nullptr;
     S->params_dirty = true;

@@ -523,7 +523,6 @@ void free_solver(Solver* S) {
     dfree(S->pin_relax);
     dfree(S->counts);
     dfree(S->perf);
-    dfree(S->max_delta_bits);
     dfree(S->pack);
     dfree(S->vcell);
     dfree(S->vb_count);
@@ -562,20 +561,16 @@ void free_solver(Solver* S) {
     dfree(g.q);
     dfree(g.offdiag);
     dfree(g.avg);
-    dfree(g.red);
     dfree(g.partials);
     dfree(g.ticket);
     dfree(g.guard);
-    dfree(g.max_delta_bits);
     dfree(S->pcg_blk);
     dfree(S->hard_cloths);
     dfree(S->hard_ranges);
     dfree(S->cap_edges);
     dfree(S->cap_rest);
-    dfree(S->stage_idx);
-    dfree(S->stage_target);
-    dfree(S->stage_weight);
-    dfree(S->stage_relax);
+    dfree(S->stage);
+    if (S->io) cudaFreeHost(S->io);
     for (int k = 0; k < 3; ++k) {
         if (S->aux[k]) cudaStreamDestroy(S->aux[k]);
         if (S->ev_join[k]) cudaEventDestroy(S->ev_join[k]);
@@ -584,6 +579,9 @@ void free_solver(Solver* S) {
     if (S->stream) cudaStreamDestroy(S->stream);
     delete S;
 }
+
+// 64-bit words of the span that a step with the hard polish resets
+size_t pcg_reset_words(int K) { return 2 + (sizeof(float) * kRedSlots * (size_t)K + 7) / 8; }
 
 bool sync_params(Solver* S) {
     if (!S->params_dirty) return true;
@@ -868,38 +866,48 @@ bool upload_pins(Solver* S, int cloth, const int* indices, const float* position
     const int n = (int)mod.size();
     if (n == 0) return true;
     const float exponent = 1.0f / (float)std::max(S->pin_relax_iterations + 1, 1);
-    S->h_stage_target.resize(n);
-    S->h_stage_weight.resize(n);
-    S->h_stage_relax.resize(n);
+    auto relax_of = [&](int i) {
+        return S->h_pin_relax[i] = S->pin_relax_iterations >= 0 ? pin_soft_relaxation(S->h_pin_weight[i], exponent) : 0.0f;
+    };
+    if (n <= kPinBatch) {
+        PinBatch b;
+        for (int k = 0; k < n; ++k) {
+            const int i = mod[k];
+            b.target[k] = S->h_pin_target[i];
+            b.idx[k] = i;
+            b.weight[k] = S->h_pin_weight[i];
+            b.relax[k] = relax_of(i);
+        }
+        launch_pin_batch(b, n, S->pin_target, S->pin_weight, S->pin_relax, S->nV, S->stream);
+        return cuda_ok(cudaGetLastError(), "pin upload");
+    }
+    // one copy: n targets, then the indices, weights and relaxations
+    const int rows4 = (n + 3) / 4, rows = n + 3 * rows4;
+    S->h_stage.resize(rows);
+    int* idx = reinterpret_cast<int*>(S->h_stage.data() + n);
+    float* weight = reinterpret_cast<float*>(S->h_stage.data() + n + rows4);
+    float* relax = reinterpret_cast<float*>(S->h_stage.data() + n + 2 * rows4);
     for (int k = 0; k < n; ++k) {
         const int i = mod[k];
-        S->h_stage_target[k] = S->h_pin_target[i];
-        S->h_stage_weight[k] = S->h_pin_weight[i];
-        S->h_pin_relax[i] = S->pin_relax_iterations >= 0 ? pin_soft_relaxation(S->h_pin_weight[i], exponent) : 0.0f;
-        S->h_stage_relax[k] = S->h_pin_relax[i];
+        S->h_stage[k] = S->h_pin_target[i];
+        idx[k] = i;
+        weight[k] = S->h_pin_weight[i];
+        relax[k] = relax_of(i);
     }
     AllocAccount account(&S->device_bytes);
-    if (n > S->stage_capacity) {
+    if (rows > S->stage_capacity) {
         if (!cuda_ok(cudaStreamSynchronize(S->stream), "pin staging reallocation")) return false;
-        S->device_bytes -= (long long)(sizeof(int) + sizeof(float4) + 2 * sizeof(float)) * S->stage_capacity;
-        dfree(S->stage_idx);
-        dfree(S->stage_target);
-        dfree(S->stage_weight);
-        dfree(S->stage_relax);
+        S->device_bytes -= (long long)sizeof(float4) * S->stage_capacity;
+        dfree(S->stage);
         S->stage_capacity = 0;
-        const int cap = std::max(n, 256);
-        if (!dalloc(&S->stage_idx, cap, "pin staging allocation") || !dalloc(&S->stage_target, cap, "pin staging allocation") ||
-            !dalloc(&S->stage_weight, cap, "pin staging allocation") || !dalloc(&S->stage_relax, cap, "pin staging allocation"))
-            return false;
+        const int cap = std::max(rows, 448);
+        if (!dalloc(&S->stage, cap, "pin staging allocation")) return false;
         S->stage_capacity = cap;
     }
-    if (!dupload(S->stage_idx, mod.data(), n, S->stream, "pin index upload") ||
-        !dupload(S->stage_target, S->h_stage_target.data(), n, S->stream, "pin target upload") ||
-        !dupload(S->stage_weight, S->h_stage_weight.data(), n, S->stream, "pin weight upload") ||
-        !dupload(S->stage_relax, S->h_stage_relax.data(), n, S->stream, "pin relaxation upload"))
-        return false;
-    launch_pin_scatter(S->stage_idx, S->stage_target, S->stage_weight, S->stage_relax, n, S->pin_target, S->pin_weight,
-                       S->pin_relax, S->nV, S->stream);
+    if (!dupload(S->stage, S->h_stage.data(), rows, S->stream, "pin upload")) return false;
+    launch_pin_scatter(reinterpret_cast<const int*>(S->stage + n), S->stage, reinterpret_cast<const float*>(S->stage + n + rows4),
+                       reinterpret_cast<const float*>(S->stage + n + 2 * rows4), n, S->pin_target, S->pin_weight, S->pin_relax,
+                       S->nV, S->stream);
     return cuda_ok(cudaGetLastError(), "pin upload");
 }
 
@@ -944,20 +952,39 @@ bool upload_fields(Solver* S, int cloth, const SsblXpbdForceField* fields, int c
     return cuda_ok(cudaStreamSynchronize(S->stream), "upload force fields");
 }
 
+// Transfers of at most kSmallTransfer bytes go through page-locked memory that
+// the kernel reads or writes itself, so a call is one launch and one wait: 16
+// us for the positions of 1,024 vertices through Python, 20 with a copy.  Past
+// it the host's pass over that memory costs more than the copy engine, which
+// moves 400 KB in 3 us.
+constexpr size_t kSmallTransfer = 64 << 10;
+
+float* small_transfer(Solver* S, size_t bytes) {
+    if (bytes > kSmallTransfer) return nullptr;
+    if (!S->io && cudaHostAlloc(reinterpret_cast<void**>(&S->io), kSmallTransfer, cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();  // none to be had: copy
+        S->io = nullptr;
+    }
+    return S->io;
+}
+
 bool upload_positions(Solver* S, int cloth, const float* positions, int max_floats) {
     if (!valid_cloth(S, cloth) || !positions) return fail("invalid position upload");
     const Range r = cloth_range(S, cloth);
     const int n = r.hi - r.lo;
     if (max_floats < n * 3) return fail("invalid position upload");
-    std::vector<float4> p4(n);
-    for (int i = 0; i < n; ++i) {
-        // a whole-handle upload lists the cloths in the caller's order
-        const int src = (cloth < 0 && S->permuted) ? external_vertex(S, i) : i;
-        p4[i] = make_float4(positions[src * 3], positions[src * 3 + 1], positions[src * 3 + 2], S->h_w[r.lo + i]);
+    // a whole-handle upload lists the cloths in the caller's order
+    const bool external = cloth < 0 && S->permuted;
+    const size_t bytes = sizeof(float) * 3 * (size_t)n;
+    float* src = small_transfer(S, bytes);
+    if (src) {
+        std::memcpy(src, positions, bytes);
+    } else {
+        src = S->pack + 3ll * r.lo;
+        if (!dupload(src, positions, 3 * (size_t)n, S->stream, "upload positions")) return false;
     }
-    return dupload(S->pos[0] + r.lo, p4.data(), n, S->stream, "upload positions") &&
-           dupload(S->prev + r.lo, p4.data(), n, S->stream, "upload previous positions") &&
-           cuda_ok(cudaStreamSynchronize(S->stream), "upload positions");
+    launch_unpack_positions(S->view(), S->pos[0], S->prev, src, S->rest, r.lo, n, external, S->stream);
+    return cuda_ok(cudaGetLastError(), "upload positions") && cuda_ok(cudaStreamSynchronize(S->stream), "upload positions");
 }
 
 bool download_positions(Solver* S, int cloth, float* out, int max_floats) {
@@ -965,37 +992,24 @@ bool download_positions(Solver* S, int cloth, float* out, int max_floats) {
     const Range r = cloth_range(S, cloth);
     const int n = r.hi - r.lo;
     if (max_floats < n * 3) return fail("invalid position download");
-    launch_pack_positions(S->pack + 3ll * r.lo, S->pos[0] + r.lo, n, S->stream);
-    if (cloth < 0 && S->permuted) {
-        // whole handle: each cloth's block goes to its place in the caller's order
-        if (!cuda_ok(cudaGetLastError(), "pack positions")) return false;
-        for (int k = 0; k < S->K; ++k) {
-            const Params& P = S->hp[S->ext2int[k]];
-            if (P.V > 0 && !cuda_ok(cudaMemcpyAsync(out + 3ll * S->ext_vstart[k], S->pack + 3ll * P.vstart, sizeof(float) * 3 * P.V,
-                                                    cudaMemcpyDeviceToHost, S->stream),
-                                    "download ABI41 positions"))
-                return false;
-        }
-        return cuda_ok(cudaStreamSynchronize(S->stream), "download ABI41 positions");
-    }
-    return cuda_ok(cudaGetLastError(), "pack positions") &&
-           cuda_ok(cudaMemcpyAsync(out, S->pack + 3ll * r.lo, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost, S->stream),
-                   "download ABI41 positions") &&
-           cuda_ok(cudaStreamSynchronize(S->stream), "download ABI41 positions");
+    const bool external = cloth < 0 && S->permuted;
+    const size_t bytes = sizeof(float) * 3 * (size_t)n;
+    float* small = small_transfer(S, bytes);
+    float* dst = small ? small : S->pack + 3ll * r.lo;
+    launch_pack_positions(S->view(), dst, S->pos[0], r.lo, n, external, S->stream);
+    if (!cuda_ok(cudaGetLastError(), "pack positions") ||
+        (!small && !cuda_ok(cudaMemcpyAsync(out, dst, bytes, cudaMemcpyDeviceToHost, S->stream), "download ABI41 positions")) ||
+        !cuda_ok(cudaStreamSynchronize(S->stream), "download ABI41 positions"))
+        return false;
+    if (small) std::memcpy(out, small, bytes);
+    return true;
 }
 
 bool reset_cloths(Solver* S, int cloth) {
     if (!valid_cloth(S, cloth)) return fail("invalid solver handle");
     const Range r = cloth_range(S, cloth);
-    const size_t n = (size_t)(r.hi - r.lo);
-    if (!cuda_ok(cudaMemcpyAsync(S->pos[0] + r.lo, S->rest + r.lo, sizeof(float4) * n, cudaMemcpyDeviceToDevice, S->stream),
-                 "reset positions") ||
-        !cuda_ok(cudaMemcpyAsync(S->prev + r.lo, S->rest + r.lo, sizeof(float4) * n, cudaMemcpyDeviceToDevice, S->stream),
-                 "reset previous positions") ||
-        !cuda_ok(cudaMemsetAsync(S->vel + r.lo, 0, sizeof(float4) * n, S->stream), "reset velocities") ||
-        !cuda_ok(cudaMemsetAsync(S->counts, 0, sizeof(unsigned long long) * kCntSlots, S->stream), "reset ABI41 diagnostics") ||
-        !cuda_ok(cudaStreamSynchronize(S->stream), "reset solver"))
-        return false;
+    launch_reset_state(S->pos[0] + r.lo, S->prev + r.lo, S->vel + r.lo, S->rest + r.lo, r.hi - r.lo, S->counts, S->stream);
+    if (!cuda_ok(cudaGetLastError(), "reset solver") || !cuda_ok(cudaStreamSynchronize(S->stream), "reset solver")) return false;
     S->diag = SsblXpbdDiagnostics{};
     S->diag.finite_flag = 1;
     return true;
@@ -1088,6 +1102,7 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
         C.colliders.sphere_radius = c.sphere_radius;
         Params& P = S->hp[k];
         P.vstart = (int)tv;
+        P.ext_vstart = S->ext_vstart[S->int2ext[k]];
         P.estart = (int)te;
         P.tstart = (int)tt;
         P.V = c.vertex_count;
@@ -1356,9 +1371,10 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
               dalloc(&S->edges, nE, "edge allocation") && dalloc(&S->edge_rest, nE, "edge rest allocation") &&
               dalloc(&S->pin_target, nV, "pin target allocation") && dalloc(&S->pin_weight, nV, "pin weight allocation") &&
               dalloc(&S->pin_relax, nV, "pin relaxation allocation") &&
-              dalloc(&S->counts, kCntSlots, "ABI41 diagnostic allocation") && dalloc(&S->perf, kPerfStripes * kPerfStride, "work counter allocation") &&
-              dalloc(&S->max_delta_bits, 1, "self max smoothed delta allocation") &&
+              dalloc(&S->counts, kCntSlots + 1, "ABI41 diagnostic allocation") && dalloc(&S->perf, kPerfStripes * kPerfStride, "work counter allocation") &&
               dalloc(&S->pack, (size_t)nV * 3, "download staging allocation");
+    // one span that a step resets: the counters and the largest smoothed delta
+    if (ok) S->max_delta_bits = reinterpret_cast<unsigned*>(S->counts + kCntSlots);
     if (ok && !S->h_bend_ranges.empty())
         ok = dalloc(&S->bend_ranges, S->h_bend_ranges.size(), "bend range allocation");
     if (ok && K > 1)
@@ -1506,13 +1522,16 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
              dalloc(&g.z, nV, "PCG preconditioned residual allocation") && dalloc(&g.d, nV, "PCG search direction allocation") &&
              dalloc(&g.q, nV, "PCG A*d allocation") && dalloc(&g.offdiag, sp_ent.size(), "PCG offdiagonal allocation") &&
              dalloc(&g.avg, nV, "stretch cap accumulation allocation") &&
-             dalloc(&g.red, (size_t)K * kRedSlots, "PCG reduction allocation") &&
              dalloc(&g.partials, (size_t)S->pcg_blocks * (kThreads / 32), "PCG partial sum allocation") &&
-             dalloc(&g.ticket, K, "PCG ticket allocation") && dalloc(&g.guard, 1, "PCG guard counter allocation") &&
-             dalloc(&g.max_delta_bits, 1, "PCG max delta allocation") &&
+             dalloc(&g.ticket, K, "PCG ticket allocation") && dalloc(&g.guard, pcg_reset_words(K), "PCG reduction allocation") &&
              dalloc(&S->pcg_blk, S->pcg_blocks, "PCG block map allocation") &&
              dalloc(&S->cap_edges, std::max(S->cap_count, 1), "cap edge allocation") &&
              dalloc(&S->cap_rest, std::max(S->cap_count, 1), "cap rest allocation");
+        // one span that a step resets: guard count, largest delta, reductions
+        if (ok) {
+            g.max_delta_bits = reinterpret_cast<unsigned*>(g.guard + 1);
+            g.red = reinterpret_cast<float*>(g.guard + 2);
+        }
         g.blk_cloth = S->pcg_blk;
         int max_v = 0, degree = 1;
         for (int k = 0; k < K; ++k)
@@ -1594,8 +1613,7 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
          dupload(S->vcloth, vmap.data(), vmap.size(), st, "cloth map upload") &&
          dupload(S->ecloth, emap.data(), emap.size(), st, "cloth map upload") &&
          dupload(S->tcloth, tmap.data(), tmap.size(), st, "cloth map upload") &&
-         cuda_ok(cudaMemsetAsync(S->counts, 0, sizeof(unsigned long long) * kCntSlots, st), "reset ABI41 diagnostics") &&
-         cuda_ok(cudaMemsetAsync(S->max_delta_bits, 0, sizeof(unsigned), st), "reset self max smoothed delta") &&
+         cuda_ok(cudaMemsetAsync(S->counts, 0, sizeof(unsigned long long) * (kCntSlots + 1), st), "reset ABI41 diagnostics") &&
          (!S->acc || cuda_ok(cudaMemsetAsync(S->acc, 0, sizeof(Acc4) * nV, st), "reset self accumulation")) &&
          (!S->nb_count || cuda_ok(cudaMemsetAsync(S->nb_count, 0, sizeof(int) * nV, st), "reset neighbor table")) &&
          dupload(S->e_order, e_order.data(), e_order.size(), st, "self edge order upload") &&
@@ -1608,7 +1626,7 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
              dupload(S->hard_cloths, hard_cloths.data(), hard_cloths.size(), st, "PCG cloth list upload") &&
              dupload(S->hard_ranges, hard_ranges.data(), hard_ranges.size(), st, "cap range upload") &&
              cuda_ok(cudaMemsetAsync(S->pcg.ticket, 0, sizeof(unsigned) * K, st), "reset PCG ticket") &&
-             cuda_ok(cudaMemsetAsync(S->pcg.red, 0, sizeof(float) * kRedSlots * K, st), "reset PCG reductions") &&
+             cuda_ok(cudaMemsetAsync(S->pcg.guard, 0, sizeof(unsigned long long) * pcg_reset_words(K), st), "reset PCG reductions") &&
              cuda_ok(cudaStreamSynchronize(st), "PCG buffer upload");
     if (!ok) return bail(0, "");
     S->diag.finite_flag = 1;
@@ -2283,14 +2301,11 @@ bool prepare_step(Solver* S, int substeps, int iterations) {
             S->params_dirty = true;
         }
     }
-    if (!cuda_ok(cudaMemsetAsync(S->counts, 0, sizeof(unsigned long long) * kCntSlots, S->stream), "reset ABI41 diagnostics") ||
-        !cuda_ok(cudaMemsetAsync(S->max_delta_bits, 0, sizeof(unsigned), S->stream), "reset self max smoothed delta") ||
+    if (!cuda_ok(cudaMemsetAsync(S->counts, 0, sizeof(unsigned long long) * (kCntSlots + 1), S->stream), "reset ABI41 diagnostics") ||
         !upload_pin_relax(S, iterations) || !sync_params(S))
         return false;
-    if (S->pcg_on &&
-        (!cuda_ok(cudaMemsetAsync(S->pcg.guard, 0, sizeof(unsigned long long), S->stream), "reset PCG guard count") ||
-         !cuda_ok(cudaMemsetAsync(S->pcg.max_delta_bits, 0, sizeof(unsigned), S->stream), "reset PCG max delta") ||
-         !cuda_ok(cudaMemsetAsync(S->pcg.red, 0, sizeof(float) * kRedSlots * S->K, S->stream), "reset PCG reductions")))
+    if (S->pcg_on && !cuda_ok(cudaMemsetAsync(S->pcg.guard, 0, sizeof(unsigned long long) * pcg_reset_words(S->K), S->stream),
+                              "reset PCG reductions"))
         return false;
     return true;
 }

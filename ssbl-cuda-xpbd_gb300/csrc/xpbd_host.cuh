@@ -159,7 +159,7 @@ struct DynHost {
     int* large = nullptr;
     int *lflag = nullptr, *lpos = nullptr;  // large flags and their scan
     int *tcount = nullptr, *tstart = nullptr, *tent = nullptr, *scan_tmp = nullptr;
-    int* small = nullptr;         // max bucket occupancy [0], span box [4..11]
+    int* small = nullptr;         // max bucket occupancy, entries, large triangles [0..2], span box [4..11]
     int* pbox = nullptr;          // box of the particles' cells
     float4 *ppos = nullptr, *pprev = nullptr;
     float* prad = nullptr;
@@ -274,6 +274,7 @@ struct Solver {
     unsigned long long* counts = nullptr;
     unsigned* max_delta_bits = nullptr;
     float* pack = nullptr;
+    float* io = nullptr;         // page-locked host memory of small transfers (kSmallTransfer bytes), from the first one on
 
     std::vector<float> h_w;      // effective inverse mass per vertex
     std::vector<float> h_inv;    // inverse mass as given
@@ -284,13 +285,9 @@ struct Solver {
     // pin updates: current pinned vertices, change marks, device staging
     std::vector<int> pin_set, pin_changed, pin_mark, pin_kept;
     int pin_epoch = 0;
-    std::vector<float4> h_stage_target;
-    std::vector<float> h_stage_weight, h_stage_relax;
-    int* stage_idx = nullptr;
-    float4* stage_target = nullptr;
-    float* stage_weight = nullptr;
-    float* stage_relax = nullptr;
-    int stage_capacity = 0;
+    std::vector<float4> h_stage;  // targets, then indices, weights and relaxations in rows of four
+    float4* stage = nullptr;
+    int stage_capacity = 0;       // rows
     std::vector<int> bend_colors;   // merged colour offsets into `bends`
     bool jacobi_bends = false;      // some cloth gathers its bends
 

@@ -134,6 +134,7 @@ struct DynSet {
 struct Params {
     // this cloth's ranges in the concatenated arrays
     int vstart, V, estart, E, tstart, T, B, L;
+    int ext_vstart;  // first vertex in the caller's order of the cloths
     int active;      // 0: every kernel skips this cloth's items
     float sub_dt;    // frame dt / substeps of the current step
     float frame_dt;  // collider motion interval: cfg.dt when positive, else sub_dt
@@ -474,7 +475,21 @@ void launch_bend_color(const View& v, int start, int count, cudaStream_t s);
 void launch_copy_pos(float4* dst, const float4* src, int V, cudaStream_t s);
 void launch_pin_scatter(const int* idx, const float4* target, const float* weight, const float* relax, int n,
                         float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s);
-void launch_pack_positions(float* dst, const float4* src, int V, cudaStream_t s);
+// Positions of vertices [lo, lo + n) as rows of three floats, and back into
+// positions and previous positions (inverse masses from the rest state); with
+// `external` (the whole handle) the rows follow the caller's order of the cloths.
+void launch_pack_positions(const View& v, float* dst, const float4* src, int lo, int n, bool external, cudaStream_t s);
+void launch_unpack_positions(const View& v, float4* pos, float4* prev, const float* src, const float4* rest, int lo, int n,
+                             bool external, cudaStream_t s);
+void launch_reset_state(float4* pos, float4* prev, float4* vel, const float4* rest, int n, unsigned long long* counts, cudaStream_t s);
+// At most kPinBatch pin changes, handed over as kernel arguments.
+constexpr int kPinBatch = 128;
+struct PinBatch {
+    float4 target[kPinBatch];
+    int idx[kPinBatch];
+    float weight[kPinBatch], relax[kPinBatch];
+};
+void launch_pin_batch(const PinBatch& b, int n, float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s);
 void launch_sdf_build(const View& v, int cloth, int voxels, cudaStream_t s);
 
 // dynamic colliders: collision passes over all vertices (cloths without

@@ -638,13 +638,43 @@ __global__ void k_copy_pos(float4* dst, const float4* src, int n) {
     if (i < n) dst[i] = src[i];
 }
 
-__global__ void k_pack_positions(float* dst, const float4* src, int n) {
+// Row of vertex i in a transfer of [lo, ...): its place in the caller's order
+// of the cloths, or in the range.
+__device__ __forceinline__ size_t transfer_row(const View& v, int i, int lo, bool external) {
+    if (!external) return (size_t)(i - lo);
+    const Params& P = params_v(v, i);
+    return (size_t)(P.ext_vstart + (i - P.vstart));
+}
+
+__global__ void k_pack_positions(View v, float* dst, const float4* src, int lo, int n, bool external) {
+    // a thread per float: the rows may lie in host memory, which takes whole
+    // sectors better than three passes of strided words
+    const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (at >= 3ll * n) return;
+    const int i = lo + (int)(at / 3), c = (int)(at % 3);
+    dst[3 * transfer_row(v, i, lo, external) + c] = reinterpret_cast<const float*>(src + i)[c];
+}
+
+__global__ void k_unpack_positions(View v, float4* pos, float4* prev, const float* src, const float4* rest, int lo, int n,
+                                   bool external) {
+    const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    if (at >= n) return;
+    const float* s = src + 3 * transfer_row(v, lo + at, lo, external);
+    const float4 p = make_float4(s[0], s[1], s[2], rest[lo + at].w);
+    pos[lo + at] = p;
+    prev[lo + at] = p;
+}
+
+// Back to rest, with the diagnostic counters at zero.
+__global__ void k_reset_state(float4* pos, float4* prev, float4* vel, const float4* rest, int n, unsigned long long* counts) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0)
+        for (int k = threadIdx.x; k < kCntSlots; k += blockDim.x) counts[k] = 0;
     if (i >= n) return;
-    const float4 p = src[i];
-    dst[i * 3 + 0] = p.x;
-    dst[i * 3 + 1] = p.y;
-    dst[i * 3 + 2] = p.z;
+    const float4 p = rest[i];
+    pos[i] = p;
+    prev[i] = p;
+    vel[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
 // Scatter of changed pin entries (vertices whose pin was set or cleared).
@@ -657,6 +687,19 @@ __global__ void k_pin_scatter(const int* idx, const float4* target, const float*
     pin_target[i] = target[k];
     pin_weight[i] = weight[k];
     pin_relax[i] = relax[k];
+}
+
+// A few pin changes (an animated garment moves a handful of pins per frame):
+// as kernel arguments they need no staging copy at all.
+__global__ void __launch_bounds__(kPinBatch) k_pin_batch(const __grid_constant__ PinBatch b, int n, float4* pin_target,
+                                                         float* pin_weight, float* pin_relax, int nV) {
+    const int k = threadIdx.x;
+    if (k >= n) return;
+    const int i = b.idx[k];
+    if (i < 0 || i >= nV) return;
+    pin_target[i] = b.target[k];
+    pin_weight[i] = b.weight[k];
+    pin_relax[i] = b.relax[k];
 }
 
 inline int blocks_for(int n) { return (n + kThreads - 1) / kThreads; }
@@ -1142,8 +1185,21 @@ void launch_copy_pos(float4* dst, const float4* src, int V, cudaStream_t s) {
     if (V > 0) k_copy_pos<<<blocks_for(V), kThreads, 0, s>>>(dst, src, V);
 }
 
-void launch_pack_positions(float* dst, const float4* src, int V, cudaStream_t s) {
-    if (V > 0) k_pack_positions<<<blocks_for(V), kThreads, 0, s>>>(dst, src, V);
+void launch_pin_batch(const PinBatch& b, int n, float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s) {
+    if (n > 0) k_pin_batch<<<1, kPinBatch, 0, s>>>(b, std::min(n, kPinBatch), pin_target, pin_weight, pin_relax, nV);
+}
+
+void launch_pack_positions(const View& v, float* dst, const float4* src, int lo, int n, bool external, cudaStream_t s) {
+    if (n > 0) k_pack_positions<<<(unsigned)((3ll * n + kThreads - 1) / kThreads), kThreads, 0, s>>>(v, dst, src, lo, n, external);
+}
+
+void launch_unpack_positions(const View& v, float4* pos, float4* prev, const float* src, const float4* rest, int lo, int n,
+                             bool external, cudaStream_t s) {
+    if (n > 0) k_unpack_positions<<<blocks_for(n), kThreads, 0, s>>>(v, pos, prev, src, rest, lo, n, external);
+}
+
+void launch_reset_state(float4* pos, float4* prev, float4* vel, const float4* rest, int n, unsigned long long* counts, cudaStream_t s) {
+    k_reset_state<<<std::max(blocks_for(n), 1), kThreads, 0, s>>>(pos, prev, vel, rest, n, counts);
 }
 
 }  // namespace xg
