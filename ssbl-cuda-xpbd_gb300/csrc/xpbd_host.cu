@@ -2014,19 +2014,20 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
                 }
                 fork();
                 if (sp.vhash)
-                    timed(kKVertexHash, 6, [&] {
+                    // zeroing, count, scan, scatter, ordering
+                    timed(kKVertexHash, 4 + scan_launches(S->nVB), [&] {
                         cudaMemsetAsync(S->vb_count, 0, sizeof(int) * S->nVB, lane_stream(0));
                         self_build_vertex_hash(hv[0], sp.sv, S->nVB, lane_stream(0));
                     });
                 if (sp.thash)
-                    // zeroing, count, three scan kernels, scatter, trim (+ ordering)
-                    timed(kKTriangleHash, 7 + (order_mode(sp.t_order, sp.t_plain) != 0), [&] {
+                    // zeroing, count, scan, scatter, trim (+ ordering)
+                    timed(kKTriangleHash, 4 + scan_launches(S->nTB) + (order_mode(sp.t_order, sp.t_plain) != 0), [&] {
                         reset_triangle_hash(S, lane_stream(1));
                         self_build_triangle_hash(hv[1], sp.sv, S->nTB, order_mode(sp.t_order, sp.t_plain), lane_stream(1));
                     });
                 if (sp.ehash)
-                    // zeroing, insertion, four overflow kernels, trim (+ ordering)
-                    timed(kKEdgeHash, 7 + (order_mode(sp.e_order, sp.e_plain) != 0), [&] {
+                    // zeroing, insertion, two overflow kernels, trim (+ ordering)
+                    timed(kKEdgeHash, 5 + (order_mode(sp.e_order, sp.e_plain) != 0), [&] {
                         reset_edge_hash(S, lane_stream(2));
                         self_build_edge_hash(hv[2], sp.sv, S->nEB, order_mode(sp.e_order, sp.e_plain), lane_stream(2));
                     });

@@ -243,11 +243,16 @@ __global__ void __launch_bounds__(kThreads, 8) k_tri_hash(View v, bool scatter) 
     }
 }
 
-// Exclusive scan of counts[0..n) into start[0..n] in three launches: block
-// sums of 4096-count tiles, a scan of the block sums, then each tile's local
-// scan plus its offset.  counts is overwritten with the starts so it serves
-// as the scatter cursor.
-constexpr int kScanTile = 4096;
+// Exclusive scan of counts[0..n) into start[0..n].  counts is overwritten with
+// the starts so it serves as the scatter cursor.  Up to one tile of 4,096
+// counts one block does it in one launch (a block with two or four tiles is
+// slower than two launches: 37 x 37 strict frame 570 against 551 us);
+// beyond, block sums of the tiles and then each tile's local scan plus its
+// offset, which the tile's block adds up from the sums before it.  Past
+// kScanSums tiles that sum would read more than the counts themselves, and a
+// launch of its own scans the sums first (it did so at every size before:
+// 37 x 37 frame 563 us, 100 x 100 984 against 962).
+constexpr int kScanTile = 4096, kScanSums = 8192;
 
 __device__ __forceinline__ int block_exclusive_scan4(int (&vals)[4], int* warp_sums, int* total) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -303,19 +308,46 @@ __device__ __forceinline__ void store_quad(int* a, int base, int n, const int (&
 // overflow for every insertion that finds its bucket full, abi41.cu:4569).
 // Buckets of more than 32 members are listed in `trim` (when given) for
 // k_bucket_trim.
+__device__ __forceinline__ int scan_overflow(const int (&vals)[4], int base, int* trim, int* trim_count) {
+    int over = 0;
+    for (int k = 0; k < 4; ++k) {
+        over += vals[k] > kBucketSlots ? vals[k] - kBucketSlots : 0;
+        if (trim && vals[k] > kBucketSlots) trim[atomicAdd(trim_count, 1)] = base + k;
+    }
+    return over;
+}
+
+__device__ __forceinline__ void scan_add_overflow(int over, unsigned long long* overflow) {
+    for (int o = 16; o > 0; o >>= 1) over += __shfl_down_sync(0xffffffffu, over, o);
+    if (overflow && (threadIdx.x & 31) == 0 && over > 0) atomicAdd(overflow, (unsigned long long)over);
+}
+
+// The scan of a single tile.
+__global__ void __launch_bounds__(1024) k_scan_one(int* counts, int* start, int n, unsigned long long* overflow, int* trim,
+                                                   int* trim_count) {
+    __shared__ int ws[32];
+    int vals[4], starts[4];
+    const int base = threadIdx.x * 4;
+    load_quad(counts, base, n, vals);
+    scan_add_overflow(scan_overflow(vals, base, trim, trim_count), overflow);
+    int total;
+    int run = block_exclusive_scan4(vals, ws, &total);
+    for (int k = 0; k < 4; ++k) {
+        starts[k] = run;
+        run += vals[k];
+    }
+    store_quad(start, base, n, starts);
+    store_quad(counts, base, n, starts);
+    if (threadIdx.x == blockDim.x - 1) start[n] = run;
+}
+
 __global__ void __launch_bounds__(1024) k_scan_reduce(const int* counts, int n, int* block_sums,
                                                       unsigned long long* overflow, int* trim, int* trim_count) {
     __shared__ int ws[32];
     int vals[4];
     const int base = blockIdx.x * kScanTile + threadIdx.x * 4;
-    int over = 0;
     load_quad(counts, base, n, vals);
-    for (int k = 0; k < 4; ++k) {
-        over += vals[k] > kBucketSlots ? vals[k] - kBucketSlots : 0;
-        if (trim && vals[k] > kBucketSlots) trim[atomicAdd(trim_count, 1)] = base + k;
-    }
-    for (int o = 16; o > 0; o >>= 1) over += __shfl_down_sync(0xffffffffu, over, o);
-    if (overflow && (threadIdx.x & 31) == 0 && over > 0) atomicAdd(overflow, (unsigned long long)over);
+    scan_add_overflow(scan_overflow(vals, base, trim, trim_count), overflow);
     int total;
     block_exclusive_scan4(vals, ws, &total);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
@@ -343,13 +375,21 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int* sums, int n) {
     }
 }
 
-__global__ void __launch_bounds__(1024) k_scan_down(int* counts, int* start, int n, const int* block_offsets) {
+// `offsets`: the blocks' sums, scanned already or not.
+__global__ void __launch_bounds__(1024) k_scan_down(int* counts, int* start, int n, const int* offsets, bool scanned) {
     __shared__ int ws[32];
     int vals[4];
     const int base = blockIdx.x * kScanTile + threadIdx.x * 4;
     load_quad(counts, base, n, vals);
-    int total;
-    int run = block_offsets[blockIdx.x] + block_exclusive_scan4(vals, ws, &total);
+    int total, before = 0;
+    if (scanned) {
+        before = offsets[blockIdx.x];
+    } else {
+        int mine[4] = {0, 0, 0, 0};
+        for (int i = threadIdx.x; i < blockIdx.x; i += blockDim.x) mine[0] += offsets[i];
+        block_exclusive_scan4(mine, ws, &before);
+    }
+    int run = before + block_exclusive_scan4(vals, ws, &total);
     int starts[4];
     for (int k = 0; k < 4; ++k) {
         starts[k] = run;
@@ -362,10 +402,15 @@ __global__ void __launch_bounds__(1024) k_scan_down(int* counts, int* start, int
 
 void scan_counts(int* counts, int* start, int n, int* block_sums, unsigned long long* overflow, cudaStream_t s,
                  int* trim = nullptr, int* trim_count = nullptr) {
+    if (n <= kScanTile) {
+        k_scan_one<<<1, 1024, 0, s>>>(counts, start, n, overflow, trim, trim_count);
+        return;
+    }
     const int blocks = (n + kScanTile - 1) / kScanTile;
+    const bool sums = blocks > kScanSums;
     k_scan_reduce<<<blocks, 1024, 0, s>>>(counts, n, block_sums, overflow, trim, trim_count);
-    k_scan_sums<<<1, 1024, 0, s>>>(block_sums, blocks);
-    k_scan_down<<<blocks, 1024, 0, s>>>(counts, start, n, block_sums);
+    if (sums) k_scan_sums<<<1, 1024, 0, s>>>(block_sums, blocks);
+    k_scan_down<<<blocks, 1024, 0, s>>>(counts, start, n, block_sums, sums);
 }
 
 __device__ __forceinline__ int warp_global_id() { return (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); }
@@ -512,14 +557,8 @@ __global__ void __launch_bounds__(1024) k_edge_ovf_offsets(View v) {
 
 // Overflow regions from what the insertion kept: each listed bucket's
 // kEdgeSlots slot members, then its recorded late insertions through the
-// region's fill cursor.  A fixed grid striding over both; nothing to do
-// without overflow, or when the late insertions did not all fit (the second
-// walk below fills the regions then).
-__global__ void __launch_bounds__(kThreads) k_edge_ovf_late(View v) {
-    const int n = *v.eb_ovf_count;
-    if (n == 0 || !edge_late_complete(v)) return;
-    const long long threads = (long long)gridDim.x * blockDim.x;
-    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// region's fill cursor.
+__device__ __forceinline__ void edge_ovf_late(const View& v, int n, long long t0, long long threads) {
     for (long long t = t0; t < (long long)n * kEdgeSlots; t += threads) {
         const int w = (int)(t / kEdgeSlots), i = (int)(t % kEdgeSlots);
         v.eb_ent[v.eb_ovf_start[w] + i] = v.eb_slot[edge_bucket_base(v.eb_ovf_list[w]) + i];
@@ -531,16 +570,13 @@ __global__ void __launch_bounds__(kThreads) k_edge_ovf_late(View v) {
     }
 }
 
-// Second walk, only when some bucket overflowed and its late insertions were
-// not all recorded: every insertion into an overflowing bucket is written to
-// that bucket's region.  A fixed grid striding over the edges, so the usual
-// build pays for a few hundred blocks that exit at once.
+// The same by a second walk, when the late insertions were not all recorded:
+// every insertion into an overflowing bucket is written to that bucket's
+// region.
 template <int L>
-__global__ void __launch_bounds__(kThreads) k_edge_ovf_collect(View v) {
-    if (*v.eb_ovf_count == 0 || edge_late_complete(v)) return;
-    const long long threads = (long long)gridDim.x * blockDim.x;
+__device__ __forceinline__ void edge_ovf_collect(const View& v, long long t0, long long threads) {
     const long long items = (long long)(v.hi - v.lo) * L;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += threads) {
+    for (long long t = t0; t < items; t += threads) {
         const int k = v.lo + (int)(t / L), r0 = (int)(t % L);
         bool collapsed = false;
         edge_cells_walk<L>(v, k, r0, &collapsed, [&](int b) {
@@ -549,14 +585,27 @@ __global__ void __launch_bounds__(kThreads) k_edge_ovf_collect(View v) {
     }
 }
 
+// Fills the overflow regions, either way: a fixed grid striding over the
+// items, so the usual build, without overflow, pays for a few hundred blocks
+// that exit at once.
+template <int L>
+__global__ void __launch_bounds__(kThreads) k_edge_ovf_fill(View v) {
+    const int n = *v.eb_ovf_count;
+    if (n == 0) return;
+    const long long threads = (long long)gridDim.x * blockDim.x;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (edge_late_complete(v))
+        edge_ovf_late(v, n, t0, threads);
+    else
+        edge_ovf_collect<L>(v, t0, threads);
+}
+
 // The 32 smallest ids (with multiplicity) of each overflowing bucket's region,
 // in increasing order, into its first 32 slots: one warp per bucket, 32
 // rounds of a warp-wide minimum above the last value taken.
-__global__ void __launch_bounds__(kThreads) k_edge_ovf_select(View v) {
-    const int lane = threadIdx.x & 31;
-    const int warps = (int)((gridDim.x * (long long)blockDim.x) >> 5);
+__device__ __forceinline__ void edge_ovf_select(const View& v, int w0, int warps, int lane) {
     const int total = *v.eb_ovf_count;
-    for (int w = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); w < total; w += warps) {
+    for (int w = w0; w < total; w += warps) {
         const int b = v.eb_ovf_list[w];
         const int n = v.eb_count[b];
         const int* e = v.eb_ent + (v.eb_start[b] - n);
@@ -593,11 +642,13 @@ __global__ void __launch_bounds__(kThreads) k_edge_ovf_select(View v) {
 __global__ void __launch_bounds__(kThreads) k_edge_trim(View v) {
     const int lane = threadIdx.x & 31;
     const int warps = (int)((gridDim.x * (long long)blockDim.x) >> 5);
+    const int w0 = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+    edge_ovf_select(v, w0, warps, lane);
     const int total = *v.trim_count;
-    for (int w = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); w < total; w += warps) {
+    for (int w = w0; w < total; w += warps) {
         const int b = v.trim_list[w];
         const int n = v.eb_count[b];
-        if (n > kEdgeSlots) continue;  // ordered by k_edge_ovf_select
+        if (n > kEdgeSlots) continue;  // ordered by edge_ovf_select
         int* e = v.eb_slot + edge_bucket_base(b);
         const int k0 = lane < n ? e[lane] : 0x7fffffff, k1 = lane + 32 < n ? e[lane + 32] : 0x7fffffff;
         int r0 = 0, r1 = 0;
@@ -2690,9 +2741,9 @@ void set_carveout(K... kernels) {
 
 void self_set_carveout() {
     set_carveout(k_vhash_count, k_vhash_scatter, k_tri_hash<1>, k_tri_hash<2>, k_tri_hash<4>, k_tri_hash<8>, k_tri_hash<16>,
-                 k_scan_reduce, k_scan_sums, k_scan_down, k_edge_insert<1>, k_edge_insert<2>, k_edge_insert<4>, k_edge_insert<8>,
-                 k_edge_insert<16>, k_edge_ovf_offsets, k_edge_ovf_late, k_edge_ovf_collect<1>, k_edge_ovf_collect<2>,
-                 k_edge_ovf_collect<4>, k_edge_ovf_collect<8>, k_edge_ovf_collect<16>, k_edge_ovf_select, k_edge_trim, k_bucket_sort,
+                 k_scan_one, k_scan_reduce, k_scan_sums, k_scan_down, k_edge_insert<1>, k_edge_insert<2>, k_edge_insert<4>, k_edge_insert<8>,
+                 k_edge_insert<16>, k_edge_ovf_offsets, k_edge_ovf_fill<1>, k_edge_ovf_fill<2>,
+                 k_edge_ovf_fill<4>, k_edge_ovf_fill<8>, k_edge_ovf_fill<16>, k_edge_trim, k_bucket_sort,
                  k_bucket_trim, k_neighbors_brute, k_vv, k_vv_warp, k_vt_hash, k_vt_brute, k_ee_brute, k_vt_warp<4>, k_vt_warp<8>,
                  k_vt_warp<16>, k_ee_warp<4>, k_ee_warp<8>, k_ee_warp<16>, k_flat_vt, k_flat_ee, k_ee_fast_flat, k_ee_fast,
                  k_island<kIslandLanes>, k_self_apply, k_neighbors_group<true, 1>, k_neighbors_group<true, 2>,
@@ -2701,6 +2752,8 @@ void self_set_carveout() {
                  k_neighbors_group<false, 16>, k_neighbors_group<false, 32>);
     cudaGetLastError();  // a preference: the kernels run without it
 }
+
+int scan_launches(int n) { return n <= kScanTile ? 1 : (n <= kScanSums * kScanTile ? 2 : 3); }
 
 void scan_bucket_counts(int* counts, int* start, int n, int* block_sums, cudaStream_t s) {
     if (n > 0) scan_counts(counts, start, n, block_sums, nullptr, s);
@@ -2738,15 +2791,13 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
         default: k_edge_insert<8><<<grid(n, 8, b), b, 0, s>>>(iv); break;
     }
     k_edge_ovf_offsets<<<1, 1024, 0, s>>>(v);
-    k_edge_ovf_late<<<kTrimBlocks, kThreads, 0, s>>>(v);
     switch (lanes) {
-        case 1: k_edge_ovf_collect<1><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        case 2: k_edge_ovf_collect<2><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        case 4: k_edge_ovf_collect<4><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        case 16: k_edge_ovf_collect<16><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        default: k_edge_ovf_collect<8><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
+        case 1: k_edge_ovf_fill<1><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
+        case 2: k_edge_ovf_fill<2><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
+        case 4: k_edge_ovf_fill<4><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
+        case 16: k_edge_ovf_fill<16><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
+        default: k_edge_ovf_fill<8><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
     }
-    k_edge_ovf_select<<<kTrimBlocks, kThreads, 0, s>>>(v);
     k_edge_trim<<<kTrimBlocks, kThreads, 0, s>>>(v);
     if (order != 0) bucket_order(v, order == 3 ? sv.eb : sv.eb_ord, nullptr, v.eb_slot, nb, 2, 3, s);
 }

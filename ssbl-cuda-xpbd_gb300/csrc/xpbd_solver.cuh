@@ -500,6 +500,7 @@ void launch_dynamic_collision(const View& v, int V, int which, cudaStream_t s);
 constexpr int kSignedInsidePasses = 6;  // inside-only passes at the final constraints (abi41.cu:80)
 // exclusive scan of bucket counts into starts (counts become cursors)
 void scan_bucket_counts(int* counts, int* start, int n, int* block_sums, cudaStream_t s);
+int scan_launches(int n);  // its launches
 
 // Contiguous item range covering the cloths added to it.
 struct ItemRange {
