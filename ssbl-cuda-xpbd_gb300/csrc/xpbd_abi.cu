@@ -324,7 +324,7 @@ XG_EXPORT int xpbd_gb300_build_self_structures(void* handle) {
     }
     const View v = S->view();
     if (S->nVB > 0) {
-        cudaMemsetAsync(S->vb_count, 0, sizeof(int) * S->nVB, S->stream);
+        cudaMemsetAsync(S->vb_count, 0, 5 * (size_t)S->nVB, S->stream);
         self_build_vertex_hash(v, sv, S->nVB, S->stream);
     }
     if (S->nTB > 0) {

@@ -454,6 +454,7 @@ View Solver::view() const {
     v.vb_count = vb_count;
     v.vb_start = vb_start;
     v.vb_ent = vb_ent;
+    v.vb_bits = vb_bits;
     v.tb_count = tb_count;
     v.tb_start = tb_start;
     v.tb_ent = tb_ent;
@@ -1413,9 +1414,11 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
         S->scan_seg = std::max(std::max(S->nVB, S->nTB), S->nEB) / 4096 + 2;
         if (ok && S->nVB > 0)
             ok = dalloc(&S->vcell, nV, "self collision cell allocation") &&
-                 dalloc(&S->vb_count, S->nVB, "self collision hash count allocation") &&
+                 dalloc(&S->vb_count, (size_t)S->nVB + S->nVB / 4, "self collision hash count allocation") &&
                  dalloc(&S->vb_start, S->nVB + 1, "self collision hash start allocation") &&
                  dalloc(&S->vb_ent, nV, "self collision hash index allocation");
+        // the counts and the cells' bytes are zeroed as one span
+        if (ok && S->nVB > 0) S->vb_bits = reinterpret_cast<unsigned*>(S->vb_count + S->nVB);
         // overflowing buckets (more than 32 members) listed by the scans
         if (ok)
             ok = dalloc(&S->trim_list, (size_t)std::max(std::max(S->nVB, S->nTB), S->nEB) * 3, "bucket trim list allocation") &&
@@ -2016,7 +2019,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
                 if (sp.vhash)
                     // zeroing, count, scan, scatter, ordering
                     timed(kKVertexHash, 4 + scan_launches(S->nVB), [&] {
-                        cudaMemsetAsync(S->vb_count, 0, sizeof(int) * S->nVB, lane_stream(0));
+                        cudaMemsetAsync(S->vb_count, 0, 5 * (size_t)S->nVB, lane_stream(0));
                         self_build_vertex_hash(hv[0], sp.sv, S->nVB, lane_stream(0));
                     });
                 if (sp.thash)

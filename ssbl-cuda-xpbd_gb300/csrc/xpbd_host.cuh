@@ -295,6 +295,7 @@ struct Solver {
     bool self_any = false;
     int4* vcell = nullptr;
     int *vb_count = nullptr, *vb_start = nullptr, *vb_ent = nullptr;
+    unsigned* vb_bits = nullptr;
     int *tb_count = nullptr, *tb_start = nullptr, *tb_ent = nullptr;
     int *eb_count = nullptr, *eb_start = nullptr, *eb_ent = nullptr;
     int *eb_slot = nullptr, *eb_ovf_list = nullptr, *eb_ovf_count = nullptr, *eb_ovf_start = nullptr;

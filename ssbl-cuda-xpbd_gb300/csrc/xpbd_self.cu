@@ -175,6 +175,14 @@ __device__ CellRange edge_cells(const View& v, const Params& P, int e, bool* ok,
     return primitive_cells(lo, hi, mid, P.ecell, P.key_ieee, collapsed);
 }
 
+// A byte per vertex bucket tells which of eight further hash values its
+// members' cells have: a cell without members is passed over without a look at
+// the bucket, also where the bucket holds other cells.
+__device__ __forceinline__ unsigned cell_bit(int x, int y, int z, int buckets) {
+    const unsigned h = (unsigned)x * 73856093u ^ (unsigned)y * 19349663u ^ (unsigned)z * 83492791u;
+    return 1u << ((h >> __popc((unsigned)(buckets - 1))) & 7u);
+}
+
 __global__ void k_vhash_count(View v) {
     const int i = v.lo + (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= v.hi) return;
@@ -184,6 +192,8 @@ __global__ void k_vhash_count(View v) {
     const int cx = cell_of(p.x, P.vcell, P.key_ieee), cy = cell_of(p.y, P.vcell, P.key_ieee), cz = cell_of(p.z, P.vcell, P.key_ieee);
     const int b = P.vbase + (int)bucket_of(cx, cy, cz, P.vbuckets);
     v.vcell[i] = make_int4(cx, cy, cz, b);
+    const unsigned bit = cell_bit(cx, cy, cz, P.vbuckets);
+    atomicOr(&v.vb_bits[b >> 2], bit << (8 * (b & 3)));
     atomicAdd(&v.vb_count[b], 1);  // overflow past 32 slots is counted from the totals in the scan
 }
 
@@ -1369,7 +1379,7 @@ __device__ __forceinline__ void vv_strict_warp(const View& v, const Params& P, i
 
 
 // VV responses of strict cloths whose table k_neighbors_brute built (the
-// hashed ones run fused into k_neighbors_group); `all` = 1 covers every
+// hashed ones run fused into k_neighbors); `all` = 1 covers every
 // strict cloth.
 __global__ void __launch_bounds__(kThreads, 8) k_vv_warp(View v, int all) {
     const int src = v.lo + warp_global_id();
@@ -1382,21 +1392,61 @@ __global__ void __launch_bounds__(kThreads, 8) k_vv_warp(View v, int all) {
 }
 
 
+// The r-th (from 0) set bit of m.
+__device__ __forceinline__ int select_bit(unsigned m, int r) {
+    int at = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const int low = __popc((m >> at) & ((1u << step) - 1u));
+        if (r >= low) {
+            r -= low;
+            at += step;
+        }
+    }
+    return at;
+}
+
+__device__ __forceinline__ int warp_inclusive_sum(int x, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += t;
+    }
+    return x;
+}
+
+// The first lane whose inclusive sum exceeds w.
+__device__ __forceinline__ int warp_owner(int incl, int w) {
+    int j = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= w) j += step;
+    return j;
+}
+
 // VV neighbour table (abi41.cu:4756-4781) and, with kVv (strict passes), the
-// VV responses computed from it at once (the next operation on that branch;
-// positions do not change in between).  G lanes per vertex (a tile choice of
-// the autotuner; 32 / G vertices per warp): lane l scans cells c = l, G + l,
-// ... in rounds, cell c = (dz, dy, dx) = (c/9-1, c/3%3-1, c%3-1), the
-// reference's nested-loop order; each round's hits are placed after the
-// earlier cells' by a prefix sum over the vertex's lanes, so the table lists
-// neighbours in walk order.  The VV responses take neighbours l, G + l, ...
-// and sum their fixed-point pushes.  With few lanes per vertex the
-// per-vertex set-up and response arithmetic of several vertices share one
-// instruction stream (the table walk is issue-bound).
+// VV responses of its entries at once (the next operation on that branch;
+// positions do not change in between).  A warp takes 32 / G vertices (G lanes
+// per vertex, a tile choice of the autotuner).  Of a vertex's 27 cells, in the
+// reference's nested-loop order c = (dz, dy, dx) = (c/9-1, c/3%3-1, c%3-1),
+// most have no members: the bytes beside the bucket counts tell, and only the
+// others are looked at.  The warp lays first its vertices' cells with members
+// end to end, then those cells' members, and tests 32 members per round, so
+// that a round's chain of dependent loads (bucket, member, its cell, its
+// positions) is paid once for 32 members: with a lane per cell, a warp waited
+// through as many chains as its fullest lane had members (49 cycles per
+// instruction issued; 215 -> 79 us per pass for 256 uneven cloths, 59 -> 37 us
+// for 450 x 450 vertices, 37 x 37 strict frame 551 -> 518 us).  A vertex's members stay in walk order, so the table
+// lists neighbours in walk order: an entry's place is the count of accepted
+// members of its vertex before it.  The counts stay in registers: with a
+// shared-memory word per vertex the kernel alone took the same time, but the
+// triangle and edge queries no longer ran beside it (100 x 100 frame 885
+// against 1,066 us).
 template <bool kVv, int G>
-__global__ void __launch_bounds__(kThreads, 8) k_neighbors_group(View v, int mode) {
+__global__ void __launch_bounds__(kThreads, 6) k_neighbors(View v, int mode) {
+    constexpr int W = 32 / G;
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-    const int src = v.lo + warp_global_id() * (32 / G) + lane / G;
+    const int src0 = v.lo + warp_global_id() * W, src = src0 + lane / G;
     bool run = src < v.hi;
     const Params* P = nullptr;
     if (run) {
@@ -1407,101 +1457,115 @@ __global__ void __launch_bounds__(kThreads, 8) k_neighbors_group(View v, int mod
     if (run) {
         target = contact_radius(*P);
         if (target <= 0.0f) {
-            if (gl == 0) v.nb_count[src] = 0;
             run = false;
+            if (gl == 0) v.nb_count[src] = 0;
         }
     }
-    const float onset = fmaxf(target * 1.8f, target + kEps);
-    int cx = 0, cy = 0, cz = 0;
+    if (run && gl == 0) v.nb_count[src] = 0;
+    int cx = 0, cy = 0, cz = 0, vbase = 0, buckets = 0;
     if (run) {
         const float4 p = v.pos[src];
         cx = cell_of(p.x, P->vcell, P->key_ieee);
         cy = cell_of(p.y, P->vcell, P->key_ieee);
         cz = cell_of(p.z, P->vcell, P->key_ieee);
+        vbase = P->vbase;
+        buckets = P->vbuckets;
     }
-    int total = 0;  // neighbours of the earlier rounds (the same in the vertex's lanes)
-    if (G == 1) {
-        // one lane per vertex: the cells in walk order, each neighbour
-        // written to the table as it is found
-        for (int c = 0; c < 27 && run; ++c) {
-            const int qx = cx + c % 3 - 1, qy = cy + (c / 3) % 3 - 1, qz = cz + c / 9 - 1;
-            const int b = P->vbase + (int)bucket_of(qx, qy, qz, P->vbuckets);
-            const int st = v.vb_start[b];
-            const int lim = min(v.vb_start[b + 1] - st, kBucketSlots);
-            for (int k = 0; k < lim; ++k) {
-                const int other = v.vb_ent[st + k];
-                const int4 oc = v.vcell[other];
-                if (oc.x != qx || oc.y != qy || oc.z != qz || !vv_valid(v, src, other, target, onset)) continue;
-                if (total < kNeighborSlots) v.nb_idx[src * kNeighborSlots + total] = other;
-                ++total;
-            }
-        }
-    }
-    for (int c0 = 0; G > 1 && c0 < 27; c0 += G) {
+    unsigned occupied = 0u;  // the vertex's cells that may have members
+#pragma unroll
+    for (int c0 = 0; c0 < 27; c0 += G) {
         const int c = c0 + gl;
-        int found[kNeighborSlots];
-        int nfound = 0;
+        bool some = false;
         if (run && c < 27) {
             const int qx = cx + c % 3 - 1, qy = cy + (c / 3) % 3 - 1, qz = cz + c / 9 - 1;
-            const int b = P->vbase + (int)bucket_of(qx, qy, qz, P->vbuckets);
-            const int st = v.vb_start[b];
-            const int lim = min(v.vb_start[b + 1] - st, kBucketSlots);
-            for (int k = 0; k < lim; ++k) {
-                const int other = v.vb_ent[st + k];
+            const int b = vbase + (int)bucket_of(qx, qy, qz, buckets);
+            some = reinterpret_cast<const unsigned char*>(v.vb_bits)[b] & cell_bit(qx, qy, qz, buckets);
+        }
+        if (G == 1) {
+            occupied |= (some ? 1u : 0u) << c;
+        } else {
+            const unsigned m = __ballot_sync(0xffffffffu, some) >> (lane - gl);
+            occupied |= (G == 32 ? m : m & ((1u << (G & 31)) - 1u)) << c0;
+        }
+    }
+    __syncwarp();
+    // lane j < W: the cells of vertex j
+    unsigned cells = __shfl_sync(0xffffffffu, occupied, (lane * G) & 31);
+    if (lane >= W) cells = 0u;
+    const int cell_incl = warp_inclusive_sum(__popc(cells), lane), cell_count = __shfl_sync(0xffffffffu, cell_incl, 31);
+    unsigned candidates = 0u, contacts = 0u;
+    // accepted so far, and of them before the vertex that the last round ended in
+    int done = 0, open_j = -1, open_start = 0;
+    for (int base = 0; base < cell_count; base += 32) {
+        const int at = base + lane, j = warp_owner(cell_incl, at);
+        const unsigned of = __shfl_sync(0xffffffffu, cells, j);
+        const int c = select_bit(of, at - __shfl_sync(0xffffffffu, cell_incl, j) + __popc(of)), holder = (j * G) & 31;
+        const int qx = __shfl_sync(0xffffffffu, cx, holder) + c % 3 - 1;
+        const int qy = __shfl_sync(0xffffffffu, cy, holder) + (c / 3) % 3 - 1;
+        const int qz = __shfl_sync(0xffffffffu, cz, holder) + c / 9 - 1;
+        const int bb = __shfl_sync(0xffffffffu, vbase, holder), bn = __shfl_sync(0xffffffffu, buckets, holder);
+        int st = 0, lim = 0;
+        if (at < cell_count) {
+            const int b = bb + (int)bucket_of(qx, qy, qz, bn);
+            st = v.vb_start[b];
+            lim = min(v.vb_start[b + 1] - st, kBucketSlots);
+        }
+        const int incl = warp_inclusive_sum(lim, lane), members = __shfl_sync(0xffffffffu, incl, 31);
+        const int first = st - (incl - lim);
+        for (int mb = 0; mb < members; mb += 32) {
+            const int w = mb + lane, q = warp_owner(incl, w);
+            const int o_first = __shfl_sync(0xffffffffu, first, q), o_j = __shfl_sync(0xffffffffu, j, q);
+            const int ox = __shfl_sync(0xffffffffu, qx, q), oy = __shfl_sync(0xffffffffu, qy, q), oz = __shfl_sync(0xffffffffu, qz, q);
+            const float o_target = __shfl_sync(0xffffffffu, target, (o_j * G) & 31);
+            int other = -1;
+            bool accepted = false;
+            if (w < members) {
+                other = v.vb_ent[o_first + w];
                 const int4 oc = v.vcell[other];
-                if (oc.x != qx || oc.y != qy || oc.z != qz || !vv_valid(v, src, other, target, onset)) continue;
-                found[nfound++] = other;
+                accepted = oc.x == ox && oc.y == oy && oc.z == oz &&
+                           vv_valid(v, src0 + o_j, other, o_target, fmaxf(o_target * 1.8f, o_target + kEps));
             }
+            const unsigned m = __ballot_sync(0xffffffffu, accepted);
+            // accepted before the vertex's first member: the vertex a round
+            // starts in may have begun in an earlier one
+            const unsigned same = __match_any_sync(0xffffffffu, w < members ? o_j : -1);
+            const int start = o_j == open_j ? open_start : done + __popc(m & ((same & (0u - same)) - 1u));
+            const int rank = done + __popc(m & ((1u << lane) - 1u)) - start;
+            const int last = min(members - mb, 32) - 1;
+            open_j = __shfl_sync(0xffffffffu, o_j, last);
+            open_start = __shfl_sync(0xffffffffu, start, last);
+            done += __popc(m);
+            accepted = accepted && rank < kNeighborSlots;
+            if (accepted) v.nb_idx[(src0 + o_j) * kNeighborSlots + rank] = other;
+            // the vertex's last member of the round knows its count so far; a
+            // later round's overwrites it
+            const int found = rank + (int)((m >> lane) & 1u);
+            if (w < members && (same >> lane) == 1u && found > 0) v.nb_count[src0 + o_j] = min(found, kNeighborSlots);
+            if (accepted && rank == kNeighborSlots - 1) count1(v.counts, kCntSelfOverflow);
+            __syncwarp();
+            if (m == 0u) continue;
+            if (!kVv) continue;
+            bool contact = false, candidate = false;
+            if (accepted) {
+                long long px, py, pz;
+                int cand = 0;
+                contact = vv_pair(v, params_v(v, src0 + o_j), src0 + o_j, other, &px, &py, &pz, &cand);
+                candidate = cand != 0;
+                if (contact) {
+                    unsigned long long* acc = reinterpret_cast<unsigned long long*>(&v.acc[src0 + o_j]);
+                    atomicAdd(acc + 0, (unsigned long long)px);
+                    atomicAdd(acc + 1, (unsigned long long)py);
+                    atomicAdd(acc + 2, (unsigned long long)pz);
+                    atomicAdd(acc + 3, 1ull);
+                }
+            }
+            candidates += __popc(__ballot_sync(0xffffffffu, candidate));
+            contacts += __popc(__ballot_sync(0xffffffffu, contact));
         }
-        int incl = nfound;
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o, G);
-            if (gl >= o) incl += t;
-        }
-        const int offset = total + incl - nfound;
-        for (int k = 0; k < nfound && offset + k < kNeighborSlots; ++k) v.nb_idx[src * kNeighborSlots + offset + k] = found[k];
-        total += __shfl_sync(0xffffffffu, incl, G - 1, G);
     }
-    if (run && gl == 0) {
-        if (total >= kNeighborSlots) count1(v.counts, kCntSelfOverflow);
-        v.nb_count[src] = min(total, kNeighborSlots);
-    }
-    if (!kVv) return;
-    __syncwarp();  // the table's writes are visible to the whole warp
-    const bool vv = run && __ldg(&v.inv_mass[src]) > 0.0f;
-    const int count = vv ? min(total, kNeighborSlots) : 0;
-    long long ax = 0, ay = 0, az = 0;
-    int candidates = 0, contacts = 0;
-    for (int n = gl; n < count; n += G) {
-        long long px, py, pz;
-        int cand = 0;
-        if (vv_pair(v, *P, src, v.nb_idx[src * kNeighborSlots + n], &px, &py, &pz, &cand)) {
-            ax += px;
-            ay += py;
-            az += pz;
-            ++contacts;
-        }
-        candidates += cand;
-    }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-        ax += __shfl_down_sync(0xffffffffu, ax, o, G);
-        ay += __shfl_down_sync(0xffffffffu, ay, o, G);
-        az += __shfl_down_sync(0xffffffffu, az, o, G);
-        candidates += __shfl_down_sync(0xffffffffu, candidates, o, G);
-        contacts += __shfl_down_sync(0xffffffffu, contacts, o, G);
-    }
-    if (vv && gl == 0) {
+    if (kVv && lane == 0) {
         if (candidates) count_add(v.counts, kCntSelfCandidates, (unsigned long long)candidates);
-        if (contacts) {
-            count_add(v.counts, kCntExactImpulseContacts, (unsigned long long)contacts);
-            unsigned long long* acc = reinterpret_cast<unsigned long long*>(&v.acc[src]);
-            atomicAdd(acc + 0, (unsigned long long)ax);
-            atomicAdd(acc + 1, (unsigned long long)ay);
-            atomicAdd(acc + 2, (unsigned long long)az);
-            atomicAdd(acc + 3, (unsigned long long)contacts);
-        }
+        if (contacts) count_add(v.counts, kCntExactImpulseContacts, (unsigned long long)contacts);
     }
 }
 
@@ -2671,9 +2735,9 @@ void tri_pass_lanes(const View& iv, long long items, int lanes, int b, bool scat
 template <int G>
 void neighbors_group(const View& v, const ItemRange& r, bool vv, int mode, int b, cudaStream_t s) {
     if (vv)
-        k_neighbors_group<true, G><<<grid(r.size(), G, b), b, 0, s>>>(ranged(v, r), mode);
+        k_neighbors<true, G><<<grid(r.size(), G, b), b, 0, s>>>(ranged(v, r), mode);
     else
-        k_neighbors_group<false, G><<<grid(r.size(), G, b), b, 0, s>>>(ranged(v, r), mode);
+        k_neighbors<false, G><<<grid(r.size(), G, b), b, 0, s>>>(ranged(v, r), mode);
 }
 
 void bucket_order(const View& v, const ItemRange& buckets, const int* start, int* ent, int nb, int kind, int mode,
@@ -2746,10 +2810,10 @@ void self_set_carveout() {
                  k_edge_ovf_fill<4>, k_edge_ovf_fill<8>, k_edge_ovf_fill<16>, k_edge_trim, k_bucket_sort,
                  k_bucket_trim, k_neighbors_brute, k_vv, k_vv_warp, k_vt_hash, k_vt_brute, k_ee_brute, k_vt_warp<4>, k_vt_warp<8>,
                  k_vt_warp<16>, k_ee_warp<4>, k_ee_warp<8>, k_ee_warp<16>, k_flat_vt, k_flat_ee, k_ee_fast_flat, k_ee_fast,
-                 k_island<kIslandLanes>, k_self_apply, k_neighbors_group<true, 1>, k_neighbors_group<true, 2>,
-                 k_neighbors_group<true, 4>, k_neighbors_group<true, 8>, k_neighbors_group<true, 16>, k_neighbors_group<true, 32>,
-                 k_neighbors_group<false, 1>, k_neighbors_group<false, 2>, k_neighbors_group<false, 4>, k_neighbors_group<false, 8>,
-                 k_neighbors_group<false, 16>, k_neighbors_group<false, 32>);
+                 k_island<kIslandLanes>, k_self_apply, k_neighbors<true, 1>, k_neighbors<true, 2>,
+                 k_neighbors<true, 4>, k_neighbors<true, 8>, k_neighbors<true, 16>, k_neighbors<true, 32>,
+                 k_neighbors<false, 1>, k_neighbors<false, 2>, k_neighbors<false, 4>, k_neighbors<false, 8>,
+                 k_neighbors<false, 16>, k_neighbors<false, 32>);
     cudaGetLastError();  // a preference: the kernels run without it
 }
 
@@ -2804,7 +2868,7 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
 
 int neighbor_lanes(const LaunchTune& t, int vertices) {
     if (t.v[kTuneNeighborLanes] > 0) return t.v[kTuneNeighborLanes];
-    return vertices < (4 << 10) ? 16 : (vertices < (24 << 10) ? 8 : (vertices < (64 << 10) ? 4 : 2));
+    return vertices < (6 << 10) ? 8 : (vertices < (20 << 10) ? 4 : (vertices < (48 << 10) ? 2 : 1));
 }
 
 void self_neighbors(const View& v, int mode, const SelfVariants& sv, cudaStream_t s) {

@@ -263,11 +263,11 @@ struct LaunchTune {
 constexpr short kTuneDefault[kTuneSlots] = {128, 256, 8, 256, 256, 8, 256, 128, 32, 0, 1, 2};
 constexpr int kMaxBlock = 256;  // the kernels' launch bounds
 inline int tune_of(const LaunchTune& t, int slot) { return t.v[slot] > 0 ? t.v[slot] : kTuneDefault[slot]; }
-// Lanes per vertex of the neighbour table over so many vertices: the walk of
-// 27 cells is a chain of dependent loads, which lanes share while the chip has
-// room for them; past that every lane repeats the vertex's set-up.  Us per
-// frame with 2 lanes and as chosen: 1,369 vertices 1,033 / 669 (16 lanes);
-// 40,000 3,073 / 2,929 (4); 202,500 10,872 / 10,872 (2; 11,724 with 8).
+// Lanes per vertex of the neighbour table over so many vertices: fewer lanes
+// give a warp more vertices and so fuller rounds, more lanes more warps while
+// the chip has room for them.  Us per frame with 8, 4, 2 and 1 lanes: 4,096
+// vertices 616, 629, 739, 766; 10,000 901, 888, 923, 960; 40,000 1,961, 1,876,
+// 1,877, 1,885; 202,500 7,601, 7,262, 7,109, 7,023.
 int neighbor_lanes(const LaunchTune& t, int vertices);
 inline int grid_for(long long threads, int block) { return (int)((threads + block - 1) / block); }
 
@@ -313,6 +313,7 @@ struct View {
     int* vb_count;          // [all cloths' vertex buckets]
     int* vb_start;          // [+1]
     int* vb_ent;            // [nV]
+    unsigned* vb_bits;      // a byte per vertex bucket: which cells its members lie in (cell_bit)
     int* tb_count;
     int* tb_start;
     int* tb_ent;

@@ -90,7 +90,7 @@ def estimate_device_bytes(req: ClothRequest) -> int:
         tb = pow2(max(1024, 4 * T)) if T >= 64 else 0
         eb = pow2(max(1024, 4 * E)) if E >= 64 else 0
         b += V * (4 + 4 * 32 + 32 + 16 + 4) + (vb + tb + eb) * 8 + T * 64 * 4 + E * 64 * 4 + 3 * (max(vb, tb, eb) // 4096 + 2) * 4
-        b += E * 4  # insertion order of the edges
+        b += E * 4 + vb  # insertion order of the edges, a byte per vertex bucket
         b += 3 * max(vb, tb, eb) * 4 + 3 * 4  # lists of buckets of more than 32 members
         # edge hash: 64 member slots per bucket, overflow bits, list and region
         # starts, the record of insertions past the slots (8 B each)

@@ -1,5 +1,5 @@
 """The self-collision queries give a warp 8, 16 or 32 items and a vertex of the
-neighbour table 16, 8, 4 or 2 lanes, by the number of items.  On both sides of
+neighbour table 8, 4, 2 or 1 lanes, by the number of items.  On both sides of
 each change positions and all counters must equal the oracle's, for a cloth
 folded onto itself (every query finds contacts)."""
 import numpy as np
@@ -11,10 +11,10 @@ from xpbd_gb300.native import NativeXpbdSolver
 pytestmark = pytest.mark.gpu
 
 
-# vertices 3,969 / 4,096 (neighbour lanes 16 / 8), 24,336 / 24,649 (8 / 4),
-# 64,009 / 65,536 (4 / 2); edges 64,237 / 65,121 (8 / 16 items per warp),
+# vertices 6,084 / 6,241 (neighbour lanes 8 / 4), 20,449 / 20,736 (4 / 2),
+# 48,841 / 49,284 (2 / 1); edges 64,237 / 65,121 (8 / 16 items per warp),
 # 305,921 / 307,840 (16 / 32); 32,761 / 33,124 vertices (8 / 32)
-@pytest.mark.parametrize("n", [63, 64, 147, 148, 156, 157, 181, 182, 253, 256, 320, 321])
+@pytest.mark.parametrize("n", [63, 64, 78, 79, 143, 144, 147, 148, 156, 157, 181, 182, 221, 222, 253, 256, 320, 321])
 @pytest.mark.parametrize("mode", [2, 1], ids=["strict", "fast"])
 def test_folded(n, mode, gpu_lib, oracle_lib):
     sc = scene.drop_scene(12, 1, seed=1, self_mode=mode)
