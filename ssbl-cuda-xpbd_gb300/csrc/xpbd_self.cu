@@ -2083,28 +2083,23 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
     return __ffs(m) - 1;
 }
 
-// Fast-mode EE query, flattened: the same outcome as k_ee_fast.  Phase 1
-// classifies every (item, slot) pair of a warp's items past the item's
-// own id in its ordered bucket (the earlier slots give no pair), 32 pairs per round
-// with the slots of the items laid end to end (duplicate = the same id as the
-// slot before; classify is side-effect free, so pairs past an item's budget
-// cut may be classified for nothing); classes and cluster keys go to shared
-// memory.  Phase 2 gives each lane its item and walks the slots in order:
-// visited / duplicate / rest-pose counts, the budget of passing pairs, the
-// cluster filter on up to 16 held keys, and marks the taken pairs.  Phase 3
-// goes over the pairs flat again and computes and accumulates (in fixed point)
-// the pushes of the taken ones, 32 lanes at a time: in the walk of phase 2
-// each lane did its own, up to 16 one after another (folded 100 x 100 cloth:
-// 76 us per launch).  A warp has `per_warp` items (flat_items); its classes
-// and keys take 160 bytes of shared memory per item.
-constexpr unsigned char kPairTaken = 5;
-
+// Fast-mode EE query, flattened: the same outcome as k_ee_fast.  The pairs of
+// a warp's items past the item's own id in its ordered bucket (the earlier
+// slots give no pair) are laid end to end and taken 32 per round, in slot
+// order: classified (duplicate = the same id as the slot before it), ranked
+// against the item's passing pairs for its budget, and its cluster filter's
+// keys compared among the round's pairs by warp matches.  Only the item that a
+// round ends in carries anything into the next: its passing pairs and up to 16
+// held keys, a key per lane.  So the warp needs no memory of its own, and the
+// registers alone decide how many warps an SM holds: with classes and keys of
+// all pairs in shared memory, walked by a lane per item, it held 24 (a quarter
+// of the launch's time was the walk): folded 100 x 100 cloth 1,114 -> 1,045 us
+// per frame, 256 uneven cloths 50.3 -> 45.8 ms.  A warp has `per_warp` items
+// (flat_items): with 8, 16 and 32 the 29,601 edges of the former take 1,045,
+// 1,250 and 1,830 us, the 119,401 of a 200 x 200 cloth 2,542, 2,208 and 2,525,
+// the 2.3 M of the latter 53.5, 48.4 and 45.8 ms.
 __global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v, int per_warp) {
-    extern __shared__ unsigned fast_s[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned* key_w = fast_s + wib * per_warp * kBucketSlots;
-    unsigned char* cls_w = reinterpret_cast<unsigned char*>(fast_s + (blockDim.x >> 5) * per_warp * kBucketSlots) +
-                           wib * per_warp * kBucketSlots;
+    const int lane = threadIdx.x & 31;
     const int e = v.lo + warp_global_id() * per_warp + lane;
     bool run = lane < per_warp && e < v.hi;
     const Params* P = nullptr;
@@ -2134,129 +2129,118 @@ __global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v, int per_wa
     // pair is taken from its lower edge: the members up to this edge's own
     // id form a prefix whose slots are each visited (seen) and give no pair,
     // an id equal to the one before being a duplicate.  Only the slots after
-    // the prefix are classified.
+    // the prefix are classified.  A bucket's slots are whole int4 quads.
     int skip = 0, skip_dup = 0;
-    if (run) {
-        int lo = 0, hi = lim;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (v.eb_slot[st + mid] > e)
-                hi = mid;
-            else
-                lo = mid + 1;
+    {
+        const int4* row = reinterpret_cast<const int4*>(v.eb_slot + st);
+        int before = -1;
+#pragma unroll
+        for (int q = 0; q < kBucketSlots / 4; ++q) {
+            const int4 t = 4 * q < lim ? row[q] : make_int4(0, 0, 0, 0);
+            const int ids[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (4 * q + k < lim && ids[k] <= e) {
+                    ++skip;
+                    skip_dup += ids[k] == before ? 1 : 0;
+                }
+                before = ids[k];
+            }
         }
-        skip = lo;
-        for (int j = 1; j < skip; ++j) skip_dup += v.eb_slot[st + j] == v.eb_slot[st + j - 1] ? 1 : 0;
     }
     const int cnt = lim - skip;
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += n;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int incl = warp_inclusive_sum(cnt, lane), total = __shfl_sync(0xffffffffu, incl, 31);
     const int excl = incl - cnt - skip;  // so that slot = w - excl starts after the prefix
+    const unsigned lower = (1u << lane) - 1u;
+    int n_seen = __reduce_add_sync(0xffffffffu, skip), n_dup = __reduce_add_sync(0xffffffffu, skip_dup);
+    int n_rest = 0, n_own = 0, n_taken = 0, n_contact = 0;
+    int open_j = -1, open_passed = 0, open_keys = 0;  // the item the last round ended in
+    unsigned open_key = 0u;                           // lane k: its k-th key
     for (int base = 0; base < total; base += 32) {
-        const int w = base + lane;
-        int j = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= w) j += step;
+        const int w = base + lane, j = warp_owner(incl, w);
         const int o_item = __shfl_sync(0xffffffffu, e, j);
         const long long o_st = __shfl_sync(0xffffffffu, st, j);
-        const int o_excl = __shfl_sync(0xffffffffu, excl, j);
+        const int slot = w - __shfl_sync(0xffffffffu, excl, j), o_budget = __shfl_sync(0xffffffffu, budget, j);
         const float o_target = __shfl_sync(0xffffffffu, target, j), o_onset = __shfl_sync(0xffffffffu, onset, j);
         const int o_ieee = __shfl_sync(0xffffffffu, run ? P->key_ieee : 0, j);
-        if (w < total) {
-            const int slot = w - o_excl;
-            const int id = v.eb_slot[o_st + slot];
-            const bool dup = slot > 0 && id == v.eb_slot[o_st + slot - 1];
+        const bool live = w < total;
+        int cls = 0, id = -1;
+        unsigned key = 0u;
+        if (live) {
+            id = v.eb_slot[o_st + slot];
+            SoftPush sp;
+            cls = slot > 0 && id == v.eb_slot[o_st + slot - 1]
+                      ? 4
+                      : ee_fast_classify<false>(v, o_item, id, o_target, o_onset, o_ieee, &sp, &key);
+        }
+        const unsigned item = __match_any_sync(0xffffffffu, live ? j : -1);
+        const bool carried = live && j == open_j;
+        const unsigned passing = __ballot_sync(0xffffffffu, cls == 3);
+        // a slot is visited while fewer than `budget` pairs before it passed
+        const bool visited = live && __popc(passing & item & lower) + (carried ? open_passed : 0) < o_budget;
+        const bool candidate = visited && cls == 3;
+        n_seen += __popc(__ballot_sync(0xffffffffu, visited));
+        n_dup += __popc(__ballot_sync(0xffffffffu, visited && cls == 4));
+        n_rest += __popc(__ballot_sync(0xffffffffu, visited && cls == 1));
+        const unsigned candidates = __ballot_sync(0xffffffffu, candidate);
+        unsigned taken = 0u;
+        if (candidates) {
+            const unsigned alike = __match_any_sync(0xffffffffu, key);
+            bool first = candidate && !(alike & candidates & item & lower);
+            for (int q = 0; q < open_keys; ++q) {
+                const unsigned held = __shfl_sync(0xffffffffu, open_key, q);
+                if (carried && held == key) first = false;
+            }
+            const unsigned firsts = __ballot_sync(0xffffffffu, first);
+            const bool take = first && __popc(firsts & item & lower) + (carried ? open_keys : 0) < 16;
+            taken = __ballot_sync(0xffffffffu, take);
+            n_taken += __popc(taken);
+            n_own += __popc(candidates & ~taken);
             SoftPush sp;
             sp.apply = false;
-            unsigned key = 0u;
-            const int cls = dup ? 4 : ee_fast_classify<false>(v, o_item, id, o_target, o_onset, o_ieee, &sp, &key);
-            cls_w[j * kBucketSlots + slot] = (unsigned char)cls;
-            key_w[j * kBucketSlots + slot] = key;
-        }
-    }
-    __syncwarp();
-    int c_seen = skip, c_dup = skip_dup, c_rest = 0, c_own = 0, c_acc = 0, c_contact = 0, visited = skip;
-    if (run) {
-        unsigned keys[16];
-        int nkeys = 0, passed = 0;
-        for (int slot = skip; slot < lim && passed < budget; ++slot) {
-            ++visited;
-            ++c_seen;
-            const int cls = cls_w[lane * kBucketSlots + slot];
-            if (cls == 4) {
-                ++c_dup;
-                continue;
+            if (take) {
+                unsigned same_key;
+                ee_fast_classify(v, o_item, id, o_target, o_onset, o_ieee, &sp, &same_key);
+                if (sp.apply) {
+                    for (int k = 0; k < 4; ++k) {
+                        const float wk = sp.w[k];
+                        if ((k > 1 ? -wk : wk) > 0.0f) accumulate(v, sp.idx[k], sp.delta * wk);
+                    }
+                }
             }
-            if (cls == 1) ++c_rest;
-            if (cls != 3) continue;
-            ++passed;
-            const unsigned key = key_w[lane * kBucketSlots + slot];
-            bool first = true;
-#pragma unroll
-            for (int q = 0; q < 16; ++q) first = first && !(q < nkeys && keys[q] == key);
-            if (!(first && nkeys < 16)) {
-                ++c_own;
-                continue;
-            }
-#pragma unroll
-            for (int q = 0; q < 16; ++q)
-                if (q == nkeys) keys[q] = key;
-            ++nkeys;
-            ++c_acc;
-            cls_w[lane * kBucketSlots + slot] = kPairTaken;
+            n_contact += __popc(__ballot_sync(0xffffffffu, sp.apply));
+        }
+        const int last = min(total - base, 32) - 1;
+        const unsigned last_item = __shfl_sync(0xffffffffu, item, last);
+        const int last_j = __shfl_sync(0xffffffffu, j, last);
+        if (last_j != open_j) open_passed = open_keys = 0;
+        open_j = last_j;
+        open_passed += __popc(passing & last_item);
+        for (unsigned m = taken & last_item; m; m &= m - 1u, ++open_keys) {
+            const unsigned k = __shfl_sync(0xffffffffu, key, __ffs(m) - 1);
+            if (lane == open_keys) open_key = k;
         }
     }
-    __syncwarp();
-    for (int base = 0; base < total && __any_sync(0xffffffffu, c_acc > 0); base += 32) {
-        const int w = base + lane;
-        int j = 0;
+    if (lane == 0) {
+        const int sums[6] = {n_seen, n_dup, n_rest, n_own, n_taken, n_contact};
+        const int slots[6] = {kCntFilterSeen, kCntFilterRejectedDuplicate, kCntFilterRejectedRest, kCntFilterRejectedOwnership,
+                              kCntFilterAcceptedEe, kCntEdgeEdgeContacts};
 #pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= w) j += step;
-        const int o_item = __shfl_sync(0xffffffffu, e, j);
-        const long long o_st = __shfl_sync(0xffffffffu, st, j);
-        const int o_excl = __shfl_sync(0xffffffffu, excl, j);
-        const float o_target = __shfl_sync(0xffffffffu, target, j), o_onset = __shfl_sync(0xffffffffu, onset, j);
-        if (w >= total || cls_w[j * kBucketSlots + w - o_excl] != kPairTaken) continue;
-        SoftPush sp;
-        sp.apply = false;
-        unsigned key = 0u;
-        ee_fast_classify(v, o_item, v.eb_slot[o_st + w - o_excl], o_target, o_onset, 0, &sp, &key);
-        if (!sp.apply) continue;
-        ++c_contact;
-        for (int k = 0; k < 4; ++k) {
-            const float wk = sp.w[k];
-            if ((k > 1 ? -wk : wk) > 0.0f) accumulate(v, sp.idx[k], sp.delta * wk);
+        for (int q = 0; q < 6; ++q)
+            if (sums[q] > 0) count_add(v.counts, slots[q], (unsigned long long)sums[q]);
+        if (n_taken > 0) {
+            count_add(v.counts, kCntClusterCount, (unsigned long long)n_taken);
+            count_add(v.counts, kCntClusterOwnedContacts, (unsigned long long)n_taken);
+            count_add(v.counts, kCntSelfCandidates, (unsigned long long)n_taken);
         }
-    }
-    const int sums[6] = {c_seen, c_dup, c_rest, c_own, c_acc, c_contact};
-    const int slots[6] = {kCntFilterSeen, kCntFilterRejectedDuplicate, kCntFilterRejectedRest, kCntFilterRejectedOwnership,
-                          kCntFilterAcceptedEe, kCntEdgeEdgeContacts};
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const int t = __reduce_add_sync(0xffffffffu, sums[q]);
-        if (lane == 0 && t > 0) count_add(v.counts, slots[q], (unsigned long long)t);
     }
     if (v.perf) {
         const int items = __reduce_add_sync(0xffffffffu, run ? 1 : 0);
-        const int slots_total = __reduce_add_sync(0xffffffffu, visited);
         if (lane == 0) {
             perf_add(v.perf, kPerfEeItems, (unsigned long long)items);
-            perf_add(v.perf, kPerfEeSlots, (unsigned long long)slots_total);
+            perf_add(v.perf, kPerfEeSlots, (unsigned long long)n_seen);
             perf_add(v.perf, kPerfEeGathers, (unsigned long long)total);
         }
-    }
-    const int acc_total = __reduce_add_sync(0xffffffffu, c_acc);
-    if (lane == 0 && acc_total > 0) {
-        count_add(v.counts, kCntClusterCount, (unsigned long long)acc_total);
-        count_add(v.counts, kCntClusterOwnedContacts, (unsigned long long)acc_total);
-        count_add(v.counts, kCntSelfCandidates, (unsigned long long)acc_total);
     }
 }
 
@@ -2775,8 +2759,8 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
 // the chip has room for more warps fewer items each are faster.
 int flat_items(int n, int few, int some) { return n < few ? 8 : (n < some ? 16 : 32); }
 
-void flat_launch(void (*kernel)(View, int), const View& v, const ItemRange& r, int b, int per_warp, size_t smem, cudaStream_t s) {
-    kernel<<<grid((r.size() + per_warp - 1) / per_warp, 32, b), b, smem, s>>>(ranged(v, r), per_warp);
+void flat_launch(void (*kernel)(View, int), const View& v, const ItemRange& r, int b, int per_warp, cudaStream_t s) {
+    kernel<<<grid((r.size() + per_warp - 1) / per_warp, 32, b), b, 0, s>>>(ranged(v, r), per_warp);
 }
 
 template <int L>
@@ -2898,7 +2882,7 @@ void self_vv(const View& v, const SelfVariants& sv, cudaStream_t s) {
 void self_vt(const View& v, const SelfVariants& sv, cudaStream_t s) {
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     if (sv.hashed_t && sv.strict_wide && sv.v_strict.size() > 0)
-        flat_launch(k_flat_vt, v, sv.v_strict, wb, flat_items(sv.v_strict.size(), 32 << 10, 32 << 10), 0, s);
+        flat_launch(k_flat_vt, v, sv.v_strict, wb, flat_items(sv.v_strict.size(), 32 << 10, 32 << 10), s);
     if (sv.hashed_t && sv.strict_narrow && sv.v_strict.size() > 0) group_queries_lanes(v, sv, s, false);
     if (sv.hashed_t && sv.fast && sv.v_fast.size() > 0)
         k_vt_hash<<<grid(sv.v_fast.size(), 1, qb), qb, 0, s>>>(ranged(v, sv.v_fast));
@@ -2908,12 +2892,12 @@ void self_ee(const View& v, const SelfVariants& sv, cudaStream_t s) {
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     const int gb = tune_of(v.tune, kTuneGroupBlock);
     if (sv.hashed_e && sv.strict_wide && sv.e_strict.size() > 0)
-        flat_launch(k_flat_ee, v, sv.e_strict, wb, flat_items(sv.e_strict.size(), 64 << 10, 300 << 10), 0, s);
+        flat_launch(k_flat_ee, v, sv.e_strict, wb, flat_items(sv.e_strict.size(), 64 << 10, 300 << 10), s);
     if (sv.hashed_e && sv.strict_narrow && sv.e_strict.size() > 0) group_queries_lanes(v, sv, s, true);
     if (sv.hashed_e && sv.fast && sv.e_fast.size() > 0) {
         if (tune_of(v.tune, kTuneFastEeForm) == 32) {
-            const int n = flat_items(sv.e_fast.size(), 64 << 10, 1 << 30);
-            flat_launch(k_ee_fast_flat, v, sv.e_fast, wb, n, (size_t)(wb / 32) * n * kBucketSlots * 5, s);
+            const int n = flat_items(sv.e_fast.size(), 64 << 10, 300 << 10);
+            flat_launch(k_ee_fast_flat, v, sv.e_fast, wb, n, s);
         } else {
             k_ee_fast<<<grid(sv.e_fast.size(), kQueryLanes, gb), gb, 0, s>>>(ranged(v, sv.e_fast));
         }
