@@ -1639,16 +1639,27 @@ __device__ bool vt_eval(const View& v, int vertex, int tri, float target, float 
     return true;
 }
 
-// Strict-mode edge-edge pair up to the accept decision (abi41.cu:5595-5722
-// without the fast-mode filter; current distance tested before the rest
-// pose, as above).
-__device__ bool ee_eval(const View& v, int ia, int ib, float target, float onset, SoftPush* out) {
+// Whether an edge-edge pair may be taken: two edges without a common vertex
+// whose boxes do not prove them too far apart.
+__device__ __forceinline__ bool ee_possible(const View& v, int ia, int ib, float onset) {
     if (ib <= ia || ia < 0 || ib < 0 || ia >= v.nE || ib >= v.nE) return false;
     const int2 ea = __ldg(&v.edges[ia]), eb = __ldg(&v.edges[ib]);
     if (!edge_valid(v.nV, ea) || !edge_valid(v.nV, eb)) return false;
     if (ea.x == eb.x || ea.x == eb.y || ea.y == eb.x || ea.y == eb.y) return false;
+    return !segments_far(f3(v.pos[ea.x]), f3(v.pos[ea.y]), f3(v.pos[eb.x]), f3(v.pos[eb.y]), onset);
+}
+
+// Strict-mode edge-edge pair up to the accept decision (abi41.cu:5595-5722
+// without the fast-mode filter; current distance tested before the rest
+// pose, as above).  kPossible: for a pair that ee_possible has let through.
+template <bool kPossible = false>
+__device__ bool ee_eval(const View& v, int ia, int ib, float target, float onset, SoftPush* out) {
+    if (!kPossible && (ib <= ia || ia < 0 || ib < 0 || ia >= v.nE || ib >= v.nE)) return false;
+    const int2 ea = __ldg(&v.edges[ia]), eb = __ldg(&v.edges[ib]);
+    if (!kPossible && (!edge_valid(v.nV, ea) || !edge_valid(v.nV, eb))) return false;
+    if (!kPossible && (ea.x == eb.x || ea.x == eb.y || ea.y == eb.x || ea.y == eb.y)) return false;
     const F3 a0 = f3(v.pos[ea.x]), a1 = f3(v.pos[ea.y]), b0 = f3(v.pos[eb.x]), b1 = f3(v.pos[eb.y]);
-    if (segments_far(a0, a1, b0, b1, onset)) return false;
+    if (!kPossible && segments_far(a0, a1, b0, b1, onset)) return false;
     float s, t;
     segment_params(a0, a1, b0, b1, &s, &t);
     const F3 pa = a0 + (a1 - a0) * s;
@@ -1908,12 +1919,47 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_vt(View v, int per_warp) {
 // waiting, so the evaluation rounds carry only pairs that can be taken.
 // Pushes go through the integer accumulators and the counters through warp
 // ballots, so the result does not depend on the order of evaluation.
+// Of the pairs read nine in ten share a vertex or lie apart by their boxes
+// (six in ten in a folded cloth), which a few instructions tell; only the
+// others go on, with kNear by way of a second ring, to the closest-point
+// arithmetic of either pose, again 32 at a time.  A warp of 8 items has too few
+// pairs for that: they go on at once (64 x 64 frame 617 against 621 us; folded
+// 160 x 160 with 16 items per warp 4.17 ms against 3.93 with the second ring,
+// 256 uneven cloths with 32 45.4 against 44.3).
 constexpr int kEeRing = 128;
 
+// Pairs waiting in shared memory: owner lane and candidate id.  kSplit: five
+// bytes a pair, for the two rings of kNear (at eight they cost occupancy: 256
+// uneven cloths 46.3 against 44.7 ms); else one word pair (a 100 x 100 frame
+// 885 against 898 us split).
+template <int N, bool kSplit>
+struct EePairs {
+    int2 pair[kSplit ? 1 : N];
+    int id[kSplit ? N : 1];
+    unsigned char owner[kSplit ? N : 1];
+    __device__ __forceinline__ void put(int at, int lane, int other) {
+        if (kSplit) {
+            id[at & (N - 1)] = other;
+            owner[at & (N - 1)] = (unsigned char)lane;
+        } else {
+            pair[at & (N - 1)] = make_int2(lane, other);
+        }
+    }
+    // lane l's of the next n pairs (owner 0 and no candidate past them)
+    __device__ __forceinline__ int2 take(int head, int l, int n) const {
+        if (l >= n) return make_int2(0, -1);
+        const int at = (head + l) & (N - 1);
+        return kSplit ? make_int2(owner[at], id[at]) : pair[at];
+    }
+};
+
+template <bool kNear>
 __global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
-    __shared__ int2 ring_s[kThreads / 32][kEeRing];
+    __shared__ EePairs<kEeRing, kNear> ring_s[kThreads / 32];
+    __shared__ EePairs<kNear ? 64 : 1, true> near_s[kThreads / 32];
     const int lane = threadIdx.x & 31;
-    int2* ring = ring_s[threadIdx.x >> 5];
+    EePairs<kEeRing, kNear>& ring = ring_s[threadIdx.x >> 5];
+    EePairs<kNear ? 64 : 1, true>& near = near_s[threadIdx.x >> 5];
     const int item = v.lo + warp_global_id() * per_warp + lane;
     long long st = 0;
     int lim = 0;
@@ -1947,14 +1993,14 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
     const int total = __shfl_sync(0xffffffffu, incl, 31);
     const int excl = incl - lim;
     unsigned takes = 0, pushes = 0, gathers = 0;
-    int head = 0, tail = 0;  // warp-uniform ring positions
-    auto drain = [&](int n) {
-        const int2 e = lane < n ? ring[(head + lane) & (kEeRing - 1)] : make_int2(0, -1);
+    int head = 0, tail = 0, near_head = 0, near_tail = 0;  // warp-uniform ring positions
+    const unsigned lower = (1u << lane) - 1u;
+    auto evaluate = [&](bool run, int2 e) {
         const int o_item = __shfl_sync(0xffffffffu, item, e.x);
         const float o_target = __shfl_sync(0xffffffffu, target, e.x), o_onset = __shfl_sync(0xffffffffu, onset, e.x);
         SoftPush sp;
         sp.apply = false;
-        const bool accepted = lane < n && ee_eval(v, o_item, e.y, o_target, o_onset, &sp);
+        const bool accepted = run && ee_eval<kNear>(v, o_item, e.y, o_target, o_onset, &sp);
         const bool push = accepted && sp.apply;
         takes += __popc(__ballot_sync(0xffffffffu, accepted));
         pushes += __popc(__ballot_sync(0xffffffffu, push));
@@ -1964,10 +2010,29 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
                 if ((k > 1 ? -wk : wk) > 0.0f) accumulate(v, sp.idx[k], sp.delta * wk);
             }
         }
-        head += n;
+    };
+    auto evaluate_near = [&](int n) {
+        evaluate(lane < n, near.take(near_head, lane, n));
+        near_head += n;
         __syncwarp();
     };
-    const unsigned lower = (1u << lane) - 1u;
+    auto drain = [&](int n) {
+        const int2 e = ring.take(head, lane, n);
+        head += n;
+        if (!kNear) {
+            evaluate(lane < n, e);
+            __syncwarp();
+            return;
+        }
+        const int o_item = __shfl_sync(0xffffffffu, item, e.x);
+        const float o_onset = __shfl_sync(0xffffffffu, onset, e.x);
+        const bool possible = lane < n && ee_possible(v, o_item, e.y, o_onset);
+        const unsigned m = __ballot_sync(0xffffffffu, possible);
+        if (possible) near.put(near_tail + __popc(m & lower), e.x, e.y);
+        near_tail += __popc(m);
+        __syncwarp();
+        if (near_tail - near_head >= 32) evaluate_near(32);
+    };
     // Two rounds of 32 slot ids per step, both loads issued before either
     // is used; the ring holds what two rounds add to fewer than 32 waiting.
     for (int base = 0; base < total; base += 64) {
@@ -1988,7 +2053,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
         for (int r = 0; r < 2; ++r) {
             const bool keep = base + 32 * r + lane < total && other[r] > owner[r];
             const unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (keep) ring[(tail + __popc(m & lower)) & (kEeRing - 1)] = make_int2(jr[r], other[r]);
+            if (keep) ring.put(tail + __popc(m & lower), jr[r], other[r]);
             tail += __popc(m);
             gathers += __popc(m);
         }
@@ -1996,6 +2061,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
         while (tail - head >= 32) drain(32);
     }
     if (tail > head) drain(tail - head);
+    if (near_tail > near_head) evaluate_near(near_tail - near_head);
     const unsigned items = __popc(__ballot_sync(0xffffffffu, counted));
     if (lane == 0) {
         count_add(v.counts, kCntSelfCandidates, takes);
@@ -2793,7 +2859,7 @@ void self_set_carveout() {
                  k_edge_insert<16>, k_edge_ovf_offsets, k_edge_ovf_fill<1>, k_edge_ovf_fill<2>,
                  k_edge_ovf_fill<4>, k_edge_ovf_fill<8>, k_edge_ovf_fill<16>, k_edge_trim, k_bucket_sort,
                  k_bucket_trim, k_neighbors_brute, k_vv, k_vv_warp, k_vt_hash, k_vt_brute, k_ee_brute, k_vt_warp<4>, k_vt_warp<8>,
-                 k_vt_warp<16>, k_ee_warp<4>, k_ee_warp<8>, k_ee_warp<16>, k_flat_vt, k_flat_ee, k_ee_fast_flat, k_ee_fast,
+                 k_vt_warp<16>, k_ee_warp<4>, k_ee_warp<8>, k_ee_warp<16>, k_flat_vt, k_flat_ee<true>, k_flat_ee<false>, k_ee_fast_flat, k_ee_fast,
                  k_island<kIslandLanes>, k_self_apply, k_neighbors<true, 1>, k_neighbors<true, 2>,
                  k_neighbors<true, 4>, k_neighbors<true, 8>, k_neighbors<true, 16>, k_neighbors<true, 32>,
                  k_neighbors<false, 1>, k_neighbors<false, 2>, k_neighbors<false, 4>, k_neighbors<false, 8>,
@@ -2891,8 +2957,10 @@ void self_vt(const View& v, const SelfVariants& sv, cudaStream_t s) {
 void self_ee(const View& v, const SelfVariants& sv, cudaStream_t s) {
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     const int gb = tune_of(v.tune, kTuneGroupBlock);
-    if (sv.hashed_e && sv.strict_wide && sv.e_strict.size() > 0)
-        flat_launch(k_flat_ee, v, sv.e_strict, wb, flat_items(sv.e_strict.size(), 64 << 10, 300 << 10), s);
+    if (sv.hashed_e && sv.strict_wide && sv.e_strict.size() > 0) {
+        const int n = flat_items(sv.e_strict.size(), 64 << 10, 300 << 10);
+        flat_launch(n > 8 ? k_flat_ee<true> : k_flat_ee<false>, v, sv.e_strict, wb, n, s);
+    }
     if (sv.hashed_e && sv.strict_narrow && sv.e_strict.size() > 0) group_queries_lanes(v, sv, s, true);
     if (sv.hashed_e && sv.fast && sv.e_fast.size() > 0) {
         if (tune_of(v.tune, kTuneFastEeForm) == 32) {
