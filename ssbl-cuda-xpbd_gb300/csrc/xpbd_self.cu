@@ -2074,28 +2074,15 @@ __global__ void __launch_bounds__(kThreads, 6) k_flat_ee(View v, int per_warp) {
     }
 }
 
-// Fast-mode edge-edge pair as ee_pair walks it (rest test first, then the
-// current distance), without the cluster filter.  Returns 0 (no pair),
-// 1 (rejected by the rest pose), 2 (beyond the onset distance) or 3 (a
-// candidate: *key is its cluster key, *out its push).
-// kPush = false stops at the class and key (the push is left unset).
-template <bool kPush = true>
-__device__ int ee_fast_classify(const View& v, int ia, int ib, float target, float onset, int ieee, SoftPush* out,
-                                unsigned* key) {
-    if (ib <= ia || ia < 0 || ib < 0 || ia >= v.nE || ib >= v.nE || target <= 0.0f || onset <= target) return 0;
+// Push of a fast-mode edge-edge pair whose closest points lie at s and t.
+__device__ void ee_fast_push(const View& v, int ia, int ib, float s, float t, float target, float onset, SoftPush* out) {
     const int2 ea = __ldg(&v.edges[ia]), eb = __ldg(&v.edges[ib]);
-    if (!edge_valid(v.nV, ea) || !edge_valid(v.nV, eb)) return 0;
-    if (rest_ee_neighbor(v, ea, eb, target, onset)) return 1;
     const F3 a0 = f3(v.pos[ea.x]), a1 = f3(v.pos[ea.y]), b0 = f3(v.pos[eb.x]), b1 = f3(v.pos[eb.y]);
-    if (segments_far(a0, a1, b0, b1, onset)) return 2;
-    float s, t;
-    segment_params(a0, a1, b0, b1, &s, &t);
     const F3 pa = a0 + (a1 - a0) * s;
     const F3 pb = b0 + (b1 - b0) * t;
     const F3 d = pa - pb;
     const float dsq = dot3(d, d);
     float dist = sqrtf(fmaxf(dsq, kEps));
-    if (dist >= onset) return 2;
     F3 nrm{0.0f, 0.0f, 1.0f};
     if (dsq > kEps) {
         nrm = d * (1.0f / dist);
@@ -2115,8 +2102,6 @@ __device__ int ee_fast_classify(const View& v, int ia, int ib, float target, flo
         }
         dist = 0.0f;
     }
-    *key = cluster_key(2, (pa + pb) * 0.5f, F3{0.0f, 0.0f, 0.0f}, fmaxf(onset * 12.0f, 1.0e-3f), ieee);
-    if (!kPush) return 3;
     const float pen = target - dist;
     float push;
     if (pen > 0.0f) {
@@ -2141,7 +2126,79 @@ __device__ int ee_fast_classify(const View& v, int ia, int ib, float target, flo
         out->w[2] = -(mb0 * wt0);
         out->w[3] = -(mb1 * wt1);
     }
-    return 3;
+}
+
+// Fast-mode edge-edge pairs of a warp, one per lane with `live`, as ee_pair
+// walks each (rest test first, then the current distance), without the cluster
+// filter: 0 (no pair), 1 (rejected by the rest pose), 2 (beyond the onset
+// distance) or 3 (a candidate: *key is its cluster key, *ps and *pt its closest
+// points).  A pair that neither a common vertex nor its boxes settle needs the
+// closest points of its segments, in the rest pose or, once that is known to
+// be far, where they are: the lanes that need the one and those that need the
+// other go through the same arithmetic together, so a round runs it once (and
+// again only for a pair near by its boxes in both poses), not once per pose.
+// `lanes`: who calls.
+__device__ __forceinline__ int ee_fast_classify(const View& v, unsigned lanes, bool live, int ia, int ib, float target, float onset, int ieee,
+                                                unsigned* key, float* ps, float* pt) {
+    const float skip = fmaxf(onset * 1.25f, target * 2.5f);
+    int cls = 0;
+    bool need = false, in_rest = false;
+    int2 ea = make_int2(0, 0), eb = ea;
+    F3 a0{0.0f, 0.0f, 0.0f}, a1 = a0, b0 = a0, b1 = a0;
+    auto ends = [&](const float4* at) {
+        a0 = f3(at[ea.x]);
+        a1 = f3(at[ea.y]);
+        b0 = f3(at[eb.x]);
+        b1 = f3(at[eb.y]);
+    };
+    auto here = [&] {  // the current positions, unless their boxes settle it
+        ends(v.pos);
+        need = !segments_far(a0, a1, b0, b1, onset);
+        if (!need) cls = 2;
+    };
+    if (live && ib > ia && ia >= 0 && ib >= 0 && ia < v.nE && ib < v.nE && target > 0.0f && onset > target) {
+        ea = __ldg(&v.edges[ia]);
+        eb = __ldg(&v.edges[ib]);
+        if (edge_valid(v.nV, ea) && edge_valid(v.nV, eb)) {
+            if (ea.x == eb.x || ea.x == eb.y || ea.y == eb.x || ea.y == eb.y) {
+                cls = 1;
+            } else {
+                ends(v.rest);
+                if (segments_far(a0, a1, b0, b1, skip))
+                    here();
+                else
+                    need = in_rest = true;
+            }
+        }
+    }
+    while (__any_sync(lanes, need)) {
+        if (!need) continue;
+        float s, t;
+        segment_params(a0, a1, b0, b1, &s, &t);
+        const F3 pa = a0 + (a1 - a0) * s;
+        const F3 pb = b0 + (b1 - b0) * t;
+        const F3 d = pa - pb;
+        const float dsq = dot3(d, d);
+        if (in_rest) {
+            in_rest = false;
+            if (dsq < skip * skip) {
+                cls = 1;
+                need = false;
+            } else {
+                here();
+            }
+        } else {
+            need = false;
+            cls = 2;
+            if (!(sqrtf(fmaxf(dsq, kEps)) >= onset)) {
+                cls = 3;
+                *key = cluster_key(2, (pa + pb) * 0.5f, F3{0.0f, 0.0f, 0.0f}, fmaxf(onset * 12.0f, 1.0e-3f), ieee);
+                *ps = s;
+                *pt = t;
+            }
+        }
+    }
+    return cls;
 }
 
 __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
@@ -2230,15 +2287,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v, int per_wa
         const float o_target = __shfl_sync(0xffffffffu, target, j), o_onset = __shfl_sync(0xffffffffu, onset, j);
         const int o_ieee = __shfl_sync(0xffffffffu, run ? P->key_ieee : 0, j);
         const bool live = w < total;
-        int cls = 0, id = -1;
+        const int id = live ? v.eb_slot[o_st + slot] : -1;
+        const bool again = live && slot > 0 && id == v.eb_slot[o_st + slot - 1];
         unsigned key = 0u;
-        if (live) {
-            id = v.eb_slot[o_st + slot];
-            SoftPush sp;
-            cls = slot > 0 && id == v.eb_slot[o_st + slot - 1]
-                      ? 4
-                      : ee_fast_classify<false>(v, o_item, id, o_target, o_onset, o_ieee, &sp, &key);
-        }
+        float s = 0.0f, t = 0.0f;
+        int cls = ee_fast_classify(v, 0xffffffffu, live && !again, o_item, id, o_target, o_onset, o_ieee, &key, &s, &t);
+        if (again) cls = 4;
         const unsigned item = __match_any_sync(0xffffffffu, live ? j : -1);
         const bool carried = live && j == open_j;
         const unsigned passing = __ballot_sync(0xffffffffu, cls == 3);
@@ -2265,8 +2319,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_ee_fast_flat(View v, int per_wa
             SoftPush sp;
             sp.apply = false;
             if (take) {
-                unsigned same_key;
-                ee_fast_classify(v, o_item, id, o_target, o_onset, o_ieee, &sp, &same_key);
+                ee_fast_push(v, o_item, id, s, t, o_target, o_onset, &sp);
                 if (sp.apply) {
                     for (int k = 0; k < 4; ++k) {
                         const float wk = sp.w[k];
@@ -2387,7 +2440,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_ee_fast(View v) {
             SoftPush sp;
             sp.apply = false;
             unsigned key = 0u;
-            const int cls = (valid && !dup) ? ee_fast_classify(v, e, id, target, onset, P->key_ieee, &sp, &key) : 0;
+            float s = 0.0f, t = 0.0f;
+            const int cls = ee_fast_classify(v, gm, valid && !dup, e, id, target, onset, P->key_ieee, &key, &s, &t);
             const unsigned pass_mask = (__ballot_sync(gm, cls == 3) >> gbase) & 0xffu;
             const int remaining = budget - accepted;
             const int cut = __popc(pass_mask) >= remaining ? nth_set_bit(pass_mask, remaining - 1) : kQueryLanes;
@@ -2421,6 +2475,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_ee_fast(View v) {
             c_own += (cand && !take) ? 1 : 0;
             if (take) {
                 c_acc += 1;
+                ee_fast_push(v, e, id, s, t, target, onset, &sp);
                 if (sp.apply) {
                     c_contact += 1;
                     for (int k = 0; k < 4; ++k) {
