@@ -2860,7 +2860,7 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
               cudaStream_t s) {
     if (items.size() == 0) return;
     const View iv = ranged(v, items);
-    const int b = tune_of(v.tune, kTuneHashBlock), lanes = tune_of(v.tune, kTuneTriLanes);
+    const int b = hash_block(v.tune, v.nE), lanes = tune_of(v.tune, kTuneTriLanes);
     tri_pass_lanes(iv, items.size(), lanes, b, false, s);
     scan_counts(v.tb_count, v.tb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s, v.trim_list,
                 v.trim_count);
@@ -2932,7 +2932,7 @@ void self_build_vertex_hash(const View& v, const SelfVariants& sv, int nb, cudaS
     const ItemRange& r = sv.v_all;
     if (r.size() == 0) return;
     const View iv = ranged(v, r);
-    const int b = tune_of(v.tune, kTuneHashBlock);
+    const int b = hash_block(v.tune, v.nE);
     k_vhash_count<<<grid(r.size(), 1, b), b, 0, s>>>(iv);
     scan_counts(v.vb_count, v.vb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s);
     k_vhash_scatter<<<grid(r.size(), 1, b), b, 0, s>>>(iv);
@@ -2950,7 +2950,7 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     const ItemRange& items = sv.e_all;
     if (items.size() == 0) return;
     const View iv = ranged(v, items);
-    const int b = tune_of(v.tune, kTuneHashBlock), lanes = tune_of(v.tune, kTunePrimLanes);
+    const int b = hash_block(v.tune, v.nE), lanes = tune_of(v.tune, kTunePrimLanes);
     const long long n = items.size();
     switch (lanes) {
         case 1: k_edge_insert<1><<<grid(n, 1, b), b, 0, s>>>(iv); break;
@@ -2969,6 +2969,10 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     }
     k_edge_trim<<<kTrimBlocks, kThreads, 0, s>>>(v);
     if (order != 0) bucket_order(v, order == 3 ? sv.eb : sv.eb_ord, nullptr, v.eb_slot, nb, 2, 3, s);
+}
+
+int hash_block(const LaunchTune& t, int edges) {
+    return t.v[kTuneHashBlock] > 0 ? t.v[kTuneHashBlock] : (edges < (300 << 10) ? 128 : 256);
 }
 
 int neighbor_lanes(const LaunchTune& t, int vertices) {
