@@ -1841,6 +1841,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
     unsigned pending = 0;
     int pending_last = 0;  // last_it of the iteration that queued `pending`
     int gather = 0;        // 0 none, 1 stretch, 2 tethers, 3 bends without colours
+    bool chain = false;    // a pass, a prediction or a bend colour was the last launch
     auto timed = [&](int kind, int launches, auto&& fn) {
         cudaEvent_t a = nullptr, b = nullptr;
         if (prof) {
@@ -1849,6 +1850,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
             cudaEventRecord(a, S->stream);
         }
         fn();
+        chain = false;
         if (prof) {
             cudaEventRecord(b, S->stream);
             prof->marks.push_back({kind, {a, b}});
@@ -1862,10 +1864,13 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
         v.pos_in = S->pos[cur];
         const unsigned gflag = gather == 1 ? kPassSpring : (gather == 2 ? kPassTether : (gather == 3 ? kPassBend : 0u));
         v.pos = gather ? S->pos[cur ^ 1] : S->pos[cur];
-        if (S->rec)
+        if (S->rec) {
             S->rec->push_back(FrameOp{1, gflag | pending, buf_index(S, v.pos_in), buf_index(S, v.pos), v.substep, v.last_it, 0});
-        else
-            timed(gather == 1 ? kKStretchPass : kKVertexPass, 1, [&] { launch_vertex_pass(v, nV, gflag | pending, S->stream); });
+        } else {
+            timed(gather == 1 ? kKStretchPass : kKVertexPass, 1,
+                  [&] { launch_vertex_pass(v, nV, gflag | pending, S->stream, chain && !prof); });
+            chain = true;
+        }
         if (gather) cur ^= 1;
         pending = 0;
         gather = 0;
@@ -1920,8 +1925,10 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
         if (normals) pv.pos = S->pos[cur ^ 1];  // vertex normals read the snapshot
         if (S->rec)
             S->rec->push_back(FrameOp{0, 0u, buf_index(S, pv.pos_in), buf_index(S, pv.pos), s, 0, 0});
-        else if (!ride || s == 0)
+        else if (!ride || s == 0) {
             timed(kKPredict, 1, [&] { launch_predict(pv, nV, S->stream); });
+            chain = true;
+        }
         if (normals) cur ^= 1;
         for (int it = 0; it < iterations; ++it) {
             const bool last_it = it == iterations - 1;
@@ -1963,8 +1970,10 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
                     const int start = S->bend_colors[k], n = S->bend_colors[k + 1] - start;
                     if (n > 0 && S->rec)
                         S->rec->push_back(FrameOp{2, 0u, buf_index(S, bv.pos_in), buf_index(S, bv.pos), s, 1, (int)k});
-                    else if (n > 0)
-                        timed(kKBendColor, 1, [&] { launch_bend_color(bv, start, n, S->stream); });
+                    else if (n > 0) {
+                        timed(kKBendColor, 1, [&] { launch_bend_color(bv, start, n, S->stream, chain && !prof); });
+                        chain = true;
+                    }
                 }
             }
             if (final_c && S->jacobi_bends) {

@@ -439,7 +439,9 @@ enum PassFlags : unsigned {
     kPassPredict = 256u,  // the next substep's prediction after the velocity stage (no vertex normals)
     kPassApply = 512u,    // the last self-collision pass's pushes before the other stages
 };
-void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s);
+// chained: a pass, a prediction or a bend colour came just before on the
+// stream, and nothing else of the frame runs: the launch may start as that ends
+void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s, bool chained = false);
 
 // One operation of a recorded frame (the launches of the normal schedule):
 // kind 0 prediction, 1 vertex pass (flags), 2 bends of colour `color`,
@@ -479,7 +481,7 @@ bool frame_fits(const FramePlan& f);
 // Runs operations [first, last) of the recorded frame from buffer 0 to buffer 0.
 cudaError_t launch_frame_edges(const View& v, const FramePlan& f, const FrameOp* ops, int first, int last, float4* buf0,
                                const int2* bend_ranges, int K, cudaStream_t s);
-void launch_bend_color(const View& v, int start, int count, cudaStream_t s);
+void launch_bend_color(const View& v, int start, int count, cudaStream_t s, bool chained = false);
 void launch_copy_pos(float4* dst, const float4* src, int V, cudaStream_t s);
 void launch_pin_scatter(const int* idx, const float4* target, const float* weight, const float* relax, int n,
                         float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s);

@@ -522,20 +522,41 @@ __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned 
 // vertex_pass_item.  A thread per vertex walks its six or so entries one after
 // another, each a load and a chain of a root and two quotients, while a cloth
 // of a few ten thousand vertices leaves most of the chip's warps unused.
+// A launch that was allowed to start before the one before it on the stream
+// ended (launch_chained) waits here until that one has ended and its writes are
+// visible; any other launch passes at once.  Every thread of such a kernel
+// calls it, so that no launch ends before those ahead of it have.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <int L>
 __global__ void __launch_bounds__(kThreads) k_vertex_pass_lanes(View v, unsigned flags) {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(g / L), sub = (int)(g % L);
     bool work = i < v.nV;
+    // before the wait: what no kernel of the frame writes, parameters and
+    // constraints
     const Params* P = nullptr;
-    float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    int k = 0, end = 0;
-    VState s{F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, 0.0f};
+    int k = 0, end = 0, active = 0;
     float dt = 0.0f, alpha = 0.0f;
     if (work) {
         P = &params_v(v, i);
+        active = P->active;
+        dt = P->sub_dt;
+        alpha = stretch_alpha(P->stretch_compliance, dt);
+        if (active && !P->pcg_on) {
+            k = __ldg(&v.sp_off[i]);
+            end = __ldg(&v.sp_off[i + 1]);
+        }
+    }
+    const int rounds = (__reduce_max_sync(0xffffffffu, end - k) + L - 1) / L;
+    k += sub;
+    int2 next = k < end ? __ldg(&v.sp_ent[k]) : make_int2(0, 0);
+    wait_for_previous();
+    float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    VState s{F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, F3{0.0f, 0.0f, 0.0f}, 0.0f};
+    if (work) {
         p4 = v.pos_in[i];
-        if (!P->active) {
+        if (!active) {
             if (sub == 0 && v.pos != v.pos_in) v.pos[i] = p4;  // keep the ping-pong buffers in step
             work = false;
         }
@@ -547,20 +568,13 @@ __global__ void __launch_bounds__(kThreads) k_vertex_pass_lanes(View v, unsigned
             s.prev = f3(v.prev[i]);
             s.vel = f3(v.vel[i]);
         }
-        dt = P->sub_dt;
-        alpha = stretch_alpha(P->stretch_compliance, dt);
-        if (!P->pcg_on) {
-            k = __ldg(&v.sp_off[i]);
-            end = __ldg(&v.sp_off[i + 1]);
-        }
     }
-    const int rounds = (__reduce_max_sync(0xffffffffu, end - k) + L - 1) / L;
-    k += sub;
     for (int n = 0; n < rounds; ++n, k += L) {
         F3 d{0.0f, 0.0f, 0.0f};
         int use = 0;  // bit 0 a correction, bit 1 a stretched edge
+        const int2 e = next;
+        if (k + L < end) next = __ldg(&v.sp_ent[k + L]);
         if (k < end) {
-            const int2 e = __ldg(&v.sp_ent[k]);
             const bool self_is_j = (e.x & kSideBit) != 0;
             const float4 q4 = v.pos_in[e.x & 0x7fffffff];
             F3 corr;
@@ -595,12 +609,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_vertex_pass(View v, unsigned fl
 
 // Bend constraints of one colour, applied in place: no two bends of a colour
 // share a vertex (abi41.cu:2886-2970).
-__device__ __forceinline__ void bend_item(const View& v, int b) {
-    if (b < 0 || b >= v.nB) {
-        count1(v.counts, kCntBendingGuards);
-        return;
-    }
-    const int2 pr = __ldg(&v.bends[b]);
+__device__ __forceinline__ void bend_pair(const View& v, int2 pr, float rest) {
     const int i = pr.x, j = pr.y;
     if (i < 0 || j < 0 || i >= v.nV || j >= v.nV || i == j) {
         count1(v.counts, kCntBendingGuards);
@@ -612,7 +621,7 @@ __device__ __forceinline__ void bend_item(const View& v, int b) {
     const float4 pi4 = v.pos[i], pj4 = v.pos[j];
     F3 corr;
     bool guard;
-    const bool applied = bend_correction(P, dt, pi4, pj4, __ldg(&v.bend_rest[b]), &corr, &guard);
+    const bool applied = bend_correction(P, dt, pi4, pj4, rest, &corr, &guard);
     if (guard) count1(v.counts, kCntBendingGuards);
     if (!applied) return;
     if (pi4.w > 0.0f) {
@@ -628,9 +637,21 @@ __device__ __forceinline__ void bend_item(const View& v, int b) {
     count1(v.counts, kCntBendingWings);
 }
 
+__device__ __forceinline__ void bend_item(const View& v, int b) {
+    if (b < 0 || b >= v.nB) {
+        count1(v.counts, kCntBendingGuards);
+        return;
+    }
+    bend_pair(v, __ldg(&v.bends[b]), __ldg(&v.bend_rest[b]));
+}
+
 __global__ void __launch_bounds__(kThreads) k_bend_color(View v, int start, int count) {
-    const int local = blockIdx.x * blockDim.x + threadIdx.x;
-    if (local < count) bend_item(v, start + local);
+    const int local = blockIdx.x * blockDim.x + threadIdx.x, b = start + local;
+    const bool listed = local < count && b >= 0 && b < v.nB;
+    const int2 pr = listed ? __ldg(&v.bends[b]) : make_int2(-1, -1);
+    const float rest = listed ? __ldg(&v.bend_rest[b]) : 0.0f;
+    wait_for_previous();
+    if (local < count) bend_pair(v, pr, rest);
 }
 
 __global__ void k_copy_pos(float4* dst, const float4* src, int n) {
@@ -1158,23 +1179,48 @@ void launch_predict(const View& v, int V, cudaStream_t s) {
 // 410; 90,000 457, 430, 479, 578; 202,500 733, 732, 866, 1,076.
 constexpr int kPassLanes8 = 16 << 10, kPassLanes4 = 32 << 10, kPassLanes2 = 128 << 10;
 
-void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s) {
+// A kernel that waits by itself (wait_for_previous) may start while the one
+// before it drains: its launch and its first loads, of constraints and
+// parameters, then overlap that one's last blocks.  Us per frame without and
+// with it: 112 x 112 vertices 117 and 111, 140 x 140 125 and 117, 180 x 180 137
+// and 133, 240 x 240 140 and 134, 300 x 300 198 and 188.  Not earlier still: a
+// kernel that lets the next one start beside all of its blocks shares the SMs
+// with them (240 x 240 153).
+template <class... A>
+static void launch_chained(void (*kernel)(A...), unsigned blocks, int b, cudaStream_t s, bool chained, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks, 1, 1);
+    cfg.blockDim = dim3((unsigned)b, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+void launch_bend_color(const View& v, int start, int count, cudaStream_t s, bool chained) {
+    const int b = tune_of(v.tune, kTuneVertexBlock);
+    if (count > 0) launch_chained<View, int, int>(k_bend_color, grid_for(count, b), b, s, chained, v, start, count);
+}
+
+void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s, bool chained) {
     const int b = tune_of(v.tune, kTuneVertexBlock);
     if (V <= 0) return;
+    auto lanes = [&](void (*kernel)(View, unsigned), int n) {
+        launch_chained<View, unsigned>(kernel, grid_for((long long)n * V, b), b, s, chained, v, flags);
+    };
     if ((flags & kPassSpring) && V <= kPassLanes8)
-        k_vertex_pass_lanes<8><<<grid_for(8ll * V, b), b, 0, s>>>(v, flags);
+        lanes(k_vertex_pass_lanes<8>, 8);
     else if ((flags & kPassSpring) && V <= kPassLanes4)
-        k_vertex_pass_lanes<4><<<grid_for(4ll * V, b), b, 0, s>>>(v, flags);
+        lanes(k_vertex_pass_lanes<4>, 4);
     else if ((flags & kPassSpring) && V <= kPassLanes2)
-        k_vertex_pass_lanes<2><<<grid_for(2ll * V, b), b, 0, s>>>(v, flags);
+        lanes(k_vertex_pass_lanes<2>, 2);
     else
         k_vertex_pass<<<grid_for(V, b), b, 0, s>>>(v, flags);
 }
 
-void launch_bend_color(const View& v, int start, int count, cudaStream_t s) {
-    const int b = tune_of(v.tune, kTuneVertexBlock);
-    if (count > 0) k_bend_color<<<grid_for(count, b), b, 0, s>>>(v, start, count);
-}
 
 void launch_pin_scatter(const int* idx, const float4* target, const float* weight, const float* relax, int n,
                         float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s) {
