@@ -275,6 +275,7 @@ struct Solver {
     unsigned* max_delta_bits = nullptr;
     float* pack = nullptr;
     float* io = nullptr;         // page-locked host memory of small transfers (kSmallTransfer bytes), from the first one on
+    size_t io_used = 0;          // bytes of it that uploads not waited for may still be read from
 
     std::vector<float> h_w;      // effective inverse mass per vertex
     std::vector<float> h_inv;    // inverse mass as given

@@ -81,3 +81,20 @@ def test_pin_updates(pins, gpu_lib, oracle_lib):
             s.update_pin_targets(new, to, w)
             s.step(4, 2)
         assert np.array_equal(gpu.download_positions(), ora.download_positions()), f
+
+
+@pytest.mark.parametrize("sizes", [[1365] * 9, [5461, 40, 5461], [300] * 40])
+def test_uploads_one_after_another(sizes, gpu_lib):
+    """More small uploads than the page-locked memory holds at once, each from
+    a buffer that is overwritten as soon as the call returns."""
+    batch = NativeXpbdBatch([_strip(v) for v in sizes])
+    rng = np.random.default_rng(len(sizes))
+    at = np.concatenate([[0], np.cumsum(sizes)])
+    for _ in range(3):
+        want = rng.normal(0.0, 1.0, (at[-1], 3)).astype(np.float32)
+        for k in range(len(sizes)):
+            p = want[at[k]:at[k + 1]].copy()
+            batch.update_cloth_positions(k, p)
+            p[:] = np.nan
+        assert np.array_equal(batch.download_positions(), want)
+        assert np.array_equal(_rows(batch, 1, at[-1])[:, :3], want)
