@@ -2822,9 +2822,20 @@ inline int grid(long long items, int per_item, int b) { return grid_for(items * 
 
 constexpr int kTrimBlocks = 152 * 4;  // fixed grid of the trim pass (4 blocks per SM)
 
+// Dynamic shared memory that the hash build kernels ask for and do not use.
+// A launch without any runs in another configuration of the SM than the share
+// that the frame's kernels ask for (kCarveout) names, and the edge insertion is
+// half as fast again in the one that it gets with a few bytes: alone 2,383 ->
+// 1,596 us per build of 256 uneven cloths, 454 -> 350 of a 450 x 450 cloth; in
+// the frame, beside other branches, 1,874 -> 1,745 us at 200 x 200, 884 -> 839 at
+// 100 x 100, 604 -> 589 at 64 x 64, and the largest unchanged.  The queries are
+// slower so (their branches stop overlapping: 100 x 100 1,084 us) and ask for
+// none.
+constexpr size_t kBuildShared = 1000;
+
 template <int L>
 void tri_pass(const View& iv, int blocks, int b, bool scatter, cudaStream_t s) {
-    k_tri_hash<L><<<blocks, b, 0, s>>>(iv, scatter);
+    k_tri_hash<L><<<blocks, b, kBuildShared, s>>>(iv, scatter);
 }
 
 void tri_pass_lanes(const View& iv, long long items, int lanes, int b, bool scatter, cudaStream_t s) {
@@ -2849,11 +2860,11 @@ void bucket_order(const View& v, const ItemRange& buckets, const int* start, int
                   cudaStream_t s) {
     if (buckets.size() == 0) return;
     const int b = tune_of(v.tune, kTuneWarpBlock);
-    k_bucket_sort<<<grid((buckets.size() + 31) / 32, 32, b), b, 0, s>>>(ranged(v, buckets), start, ent, nb, kind, mode);
+    k_bucket_sort<<<grid((buckets.size() + 31) / 32, 32, b), b, kBuildShared, s>>>(ranged(v, buckets), start, ent, nb, kind, mode);
 }
 
 void bucket_trim(const View& v, const int* start, int* ent, cudaStream_t s) {
-    k_bucket_trim<<<kTrimBlocks, kThreads, 0, s>>>(start, ent, v.trim_list, v.trim_count);
+    k_bucket_trim<<<kTrimBlocks, kThreads, kBuildShared, s>>>(start, ent, v.trim_list, v.trim_count);
 }
 
 void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, const ItemRange& ordered, int nb, int order,
@@ -2933,9 +2944,9 @@ void self_build_vertex_hash(const View& v, const SelfVariants& sv, int nb, cudaS
     if (r.size() == 0) return;
     const View iv = ranged(v, r);
     const int b = hash_block(v.tune, v.nE);
-    k_vhash_count<<<grid(r.size(), 1, b), b, 0, s>>>(iv);
+    k_vhash_count<<<grid(r.size(), 1, b), b, kBuildShared, s>>>(iv);
     scan_counts(v.vb_count, v.vb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s);
-    k_vhash_scatter<<<grid(r.size(), 1, b), b, 0, s>>>(iv);
+    k_vhash_scatter<<<grid(r.size(), 1, b), b, kBuildShared, s>>>(iv);
     bucket_order(v, sv.vb, v.vb_start, v.vb_ent, nb, 0, 1, s);
 }
 void self_build_triangle_hash(const View& v, const SelfVariants& sv, int nb, int order, cudaStream_t s) {
@@ -2953,21 +2964,21 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     const int b = hash_block(v.tune, v.nE), lanes = tune_of(v.tune, kTunePrimLanes);
     const long long n = items.size();
     switch (lanes) {
-        case 1: k_edge_insert<1><<<grid(n, 1, b), b, 0, s>>>(iv); break;
-        case 2: k_edge_insert<2><<<grid(n, 2, b), b, 0, s>>>(iv); break;
-        case 4: k_edge_insert<4><<<grid(n, 4, b), b, 0, s>>>(iv); break;
-        case 16: k_edge_insert<16><<<grid(n, 16, b), b, 0, s>>>(iv); break;
-        default: k_edge_insert<8><<<grid(n, 8, b), b, 0, s>>>(iv); break;
+        case 1: k_edge_insert<1><<<grid(n, 1, b), b, kBuildShared, s>>>(iv); break;
+        case 2: k_edge_insert<2><<<grid(n, 2, b), b, kBuildShared, s>>>(iv); break;
+        case 4: k_edge_insert<4><<<grid(n, 4, b), b, kBuildShared, s>>>(iv); break;
+        case 16: k_edge_insert<16><<<grid(n, 16, b), b, kBuildShared, s>>>(iv); break;
+        default: k_edge_insert<8><<<grid(n, 8, b), b, kBuildShared, s>>>(iv); break;
     }
     k_edge_ovf_offsets<<<1, 1024, 0, s>>>(v);
     switch (lanes) {
-        case 1: k_edge_ovf_fill<1><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        case 2: k_edge_ovf_fill<2><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        case 4: k_edge_ovf_fill<4><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        case 16: k_edge_ovf_fill<16><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
-        default: k_edge_ovf_fill<8><<<kTrimBlocks, kThreads, 0, s>>>(iv); break;
+        case 1: k_edge_ovf_fill<1><<<kTrimBlocks, kThreads, kBuildShared, s>>>(iv); break;
+        case 2: k_edge_ovf_fill<2><<<kTrimBlocks, kThreads, kBuildShared, s>>>(iv); break;
+        case 4: k_edge_ovf_fill<4><<<kTrimBlocks, kThreads, kBuildShared, s>>>(iv); break;
+        case 16: k_edge_ovf_fill<16><<<kTrimBlocks, kThreads, kBuildShared, s>>>(iv); break;
+        default: k_edge_ovf_fill<8><<<kTrimBlocks, kThreads, kBuildShared, s>>>(iv); break;
     }
-    k_edge_trim<<<kTrimBlocks, kThreads, 0, s>>>(v);
+    k_edge_trim<<<kTrimBlocks, kThreads, kBuildShared, s>>>(v);
     if (order != 0) bucket_order(v, order == 3 ? sv.eb : sv.eb_ord, nullptr, v.eb_slot, nb, 2, 3, s);
 }
 
