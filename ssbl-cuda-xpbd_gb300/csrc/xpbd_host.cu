@@ -2423,7 +2423,6 @@ bool tune_value_ok(int slot, int v) {
 
 int effective_tune(const Solver* S, int slot) {
     if (slot == kTuneFusedFrame) return fused_mode(S);
-    if (slot == kTuneHashBlock) return hash_block(S->tune, S->nE);
     if (slot == kTuneNeighborLanes) {
         int n = 0;
         for (int k = 0; k < S->K; ++k) n += S->cl[k].self_enabled && !S->cl[k].fast ? S->hp[k].V : 0;

@@ -485,8 +485,8 @@ __device__ __forceinline__ void edge_cells_walk4(const View& v, int k, int r0, b
 // edges come sorted by colour, so in that order every bucket is visited once
 // per colour, each time long enough after the last for its sector of slots to
 // have left L2: 860 MB of DRAM traffic for the 16 M insertions of a
-// 450 x 450 cloth, 630 us per build, 500 us in this order (256 uneven
-// cloths 2.54 -> 2.39 ms, 100 x 100 50 -> 46 us).
+// 450 x 450 cloth, 553 us per build, 354 us in this order (256 uneven
+// cloths 1.63 -> 1.60 ms, 100 x 100 40 -> 38 us).
 template <int L>
 __global__ void __launch_bounds__(kThreads) k_edge_insert(View v) {
     __shared__ unsigned guard_s;  // the block's guard events: one global atomic per block
@@ -2871,7 +2871,7 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
               cudaStream_t s) {
     if (items.size() == 0) return;
     const View iv = ranged(v, items);
-    const int b = hash_block(v.tune, v.nE), lanes = tune_of(v.tune, kTuneTriLanes);
+    const int b = tune_of(v.tune, kTuneHashBlock), lanes = tune_of(v.tune, kTuneTriLanes);
     tri_pass_lanes(iv, items.size(), lanes, b, false, s);
     scan_counts(v.tb_count, v.tb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s, v.trim_list,
                 v.trim_count);
@@ -2943,7 +2943,7 @@ void self_build_vertex_hash(const View& v, const SelfVariants& sv, int nb, cudaS
     const ItemRange& r = sv.v_all;
     if (r.size() == 0) return;
     const View iv = ranged(v, r);
-    const int b = hash_block(v.tune, v.nE);
+    const int b = tune_of(v.tune, kTuneHashBlock);
     k_vhash_count<<<grid(r.size(), 1, b), b, kBuildShared, s>>>(iv);
     scan_counts(v.vb_count, v.vb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s);
     k_vhash_scatter<<<grid(r.size(), 1, b), b, kBuildShared, s>>>(iv);
@@ -2961,7 +2961,7 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     const ItemRange& items = sv.e_all;
     if (items.size() == 0) return;
     const View iv = ranged(v, items);
-    const int b = hash_block(v.tune, v.nE), lanes = tune_of(v.tune, kTunePrimLanes);
+    const int b = tune_of(v.tune, kTuneHashBlock), lanes = tune_of(v.tune, kTunePrimLanes);
     const long long n = items.size();
     switch (lanes) {
         case 1: k_edge_insert<1><<<grid(n, 1, b), b, kBuildShared, s>>>(iv); break;
@@ -2980,10 +2980,6 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     }
     k_edge_trim<<<kTrimBlocks, kThreads, kBuildShared, s>>>(v);
     if (order != 0) bucket_order(v, order == 3 ? sv.eb : sv.eb_ord, nullptr, v.eb_slot, nb, 2, 3, s);
-}
-
-int hash_block(const LaunchTune& t, int edges) {
-    return t.v[kTuneHashBlock] > 0 ? t.v[kTuneHashBlock] : (edges < (300 << 10) ? 128 : 256);
 }
 
 int neighbor_lanes(const LaunchTune& t, int vertices) {

@@ -243,7 +243,7 @@ struct HardPlan {
 // same for any block size, lanes per primitive or lanes per query item.
 enum TuneSlot {
     kTuneVertexBlock = 0,  // per-vertex constraint passes and prediction (default 128)
-    kTuneHashBlock,        // hash count / scatter kernels (by size, hash_block)
+    kTuneHashBlock,        // hash count / scatter kernels (256)
     kTunePrimLanes,        // lanes per primitive of the edge hash: 1, 2, 4, 8, 16 (8)
     kTuneWarpBlock,        // warp-per-item kernels: neighbour table, strict VV, flat queries, bucket order (256)
     kTuneQueryBlock,       // thread-per-item queries: fast VV / VT, brute queries, islands, apply (256)
@@ -263,13 +263,6 @@ struct LaunchTune {
 constexpr short kTuneDefault[kTuneSlots] = {128, 256, 8, 256, 256, 8, 256, 128, 32, 0, 1, 2};
 constexpr int kMaxBlock = 256;  // the kernels' launch bounds
 inline int tune_of(const LaunchTune& t, int slot) { return t.v[slot] > 0 ? t.v[slot] : kTuneDefault[slot]; }
-// Threads per block of the hash builds of a solver with so many edges: a block
-// waits for its slowest insertion, which smaller blocks wait less for; where
-// the grid has several waves of blocks larger ones are as good or better.  Us
-// per frame with 128 and 256: 37 x 37 strict 516 and 520, 64 x 64 612 and 617,
-// folded 160 x 160 (76,000 edges) 3,819 and 3,929; 450 x 450 (606,000) 7,045 and
-// 7,008, 256 uneven cloths 44,369 and 44,075.
-int hash_block(const LaunchTune& t, int edges);
 // Lanes per vertex of the neighbour table over so many vertices: fewer lanes
 // give a warp more vertices and so fuller rounds, more lanes more warps while
 // the chip has room for them.  Us per frame with 8, 4, 2 and 1 lanes: 4,096

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 # vertices 6,084 / 6,241 (neighbour lanes 8 / 4), 20,449 / 20,736 (4 / 2),
 # 48,841 / 49,284 (2 / 1); edges 64,237 / 65,121 (8 / 16 items per warp),
-# 305,921 / 307,840 (16 / 32; hash blocks of 128 / 256 threads); 32,761 / 33,124 vertices (8 / 32)
+# 305,921 / 307,840 (16 / 32); 32,761 / 33,124 vertices (8 / 32)
 @pytest.mark.parametrize("n", [63, 64, 78, 79, 143, 144, 147, 148, 156, 157, 181, 182, 221, 222, 253, 256, 320, 321])
 @pytest.mark.parametrize("mode", [2, 1], ids=["strict", "fast"])
 def test_folded(n, mode, gpu_lib, oracle_lib):
