@@ -106,10 +106,11 @@ __attribute__((visibility("default"))) long long xpbd_gb300_pc2_close(void* writ
  * queries (4, 8 or 16; default 8), block size of the group queries (256), of
  * the dynamic-collider pass (128), the form of the fast-mode edge-edge query
  * (8: groups of 8 lanes, 32: flattened warps; default 32), and whether
- * solvers whose cloths all fit one block (at most 1024 vertices, no self
- * collision, hard stretch or dynamic colliders) run each frame as one fused
- * launch, a block per cloth (1, default) or an 8-CTA thread-block cluster per
- * cloth exchanging through distributed shared memory (8), or as launched
+ * solvers without self collision, hard stretch or dynamic colliders run each
+ * frame as one or two fused launches where their cloths fit: a thread-block
+ * cluster per cloth with an edge per thread, or a block per cloth where vertex
+ * normals are gathered (1, default), an 8-CTA cluster per cloth whose CTAs all
+ * hold the full state and exchange it (8; at most 1024 vertices), or launched
  * kernels (2), lanes per primitive of the triangle hash (1, 2, 4, 8 or 16;
  * default 1), and lanes per vertex of the neighbour table and strict VV
  * responses (1, 2, 4, 8, 16 or 32; default by the number of vertices).  Block sizes

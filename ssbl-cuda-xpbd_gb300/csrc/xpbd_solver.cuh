@@ -251,8 +251,8 @@ enum TuneSlot {
     kTuneGroupBlock,       // group query kernels (256)
     kTuneDynamicBlock,     // dynamic colliders (128)
     kTuneFastEeForm,       // fast-mode EE query: 8 = groups of 8 lanes, 32 = one warp per 32 items, flattened (32)
-    kTuneFusedFrame,       // small cloths: 1 = whole frame in one block per cloth, 8 = in an 8-CTA cluster per cloth,
-                           // 2 = launched kernels (1)
+    kTuneFusedFrame,       // small cloths: 1 = whole frame in a cluster per cloth, an edge per thread (in a block where
+                           // vertex normals are gathered), 8 = in 8 CTAs with the full state each, 2 = launched kernels (1)
     kTuneTriLanes,         // lanes per primitive of the triangle hash: 1, 2, 4, 8, 16 (1)
     kTuneNeighborLanes,    // lanes per vertex of the neighbour table (+ strict VV): 1, 2, 4, 8, 16, 32 (by size, neighbor_lanes)
     kTuneSlots

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 # 16,129 / 16,641 vertices (8 / 4 lanes), 32,761 / 33,124 (4 / 2), 131,044 / 131,769 (2 / 1)
 @pytest.mark.parametrize("n", [112, 127, 129, 181, 182, 362, 363])
-@pytest.mark.parametrize("kind", ["plain", "uncoloured", "pressure"])
+@pytest.mark.parametrize("kind", ["plain", "uncoloured", "pressure", "no graph"])
 def test_frames_equal_profiled_frames(n, kind, gpu_lib):
     sc = scene.plain_grid_scene(n, 3)
     if kind == "uncoloured":
@@ -24,6 +24,8 @@ def test_frames_equal_profiled_frames(n, kind, gpu_lib):
         sc.options.use_volume_pressure, sc.options.pressure_strength = True, 2.0
     sc.options.use_sphere, sc.options.sphere_center, sc.options.sphere_radius = True, (0.1, 0.0, -0.29), 0.3
     a, b = (NativeXpbdSolver(sc.cloth, sc.options, sc.static_triangles) for _ in range(2))
+    if kind == "no graph":
+        a.set_graph_capture(False)
     for substeps, iterations in ((10, 2), (3, 1), (1, 3)):
         a.step(substeps, iterations, diagnostics=True)
         b.profile_frame(substeps, iterations)
