@@ -531,7 +531,7 @@ def run_prep(args, world, rank, local):
         "config": {"workload": DESCRIPTIONS["prep"], "vertices": V, "triangles": len(tris), "parallelism": f"replicas x{world}"},
         "device_step": {"ms": 1000.0 * dev, "replaces_numpy_ms": 1000.0 * ref_steps,
                         "what": "edges + bend pairs + rest lengths + inverse masses (host arrays in and out)"},
-        "gpu_launches": 15 * args.steps,  # kernels of one xpbd_gb300_prepare_cloth_device call
+        "gpu_launches": 12 * args.steps,  # kernels of one xpbd_gb300_prepare_cloth_device call
         "cpu_baseline": {"value": V / ref_full, "unit": "vertices/s", "cores": 1, "kind": "port",
                          "sample": "one numpy build of the same cloth"},
         "e2e": {"value": value, "unit": "vertices/s", "h2d_bytes_per_step": int(pos.nbytes + tris.nbytes + V),
