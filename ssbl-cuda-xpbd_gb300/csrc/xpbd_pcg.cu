@@ -729,8 +729,11 @@ __global__ void __launch_bounds__(kThreads) k_cap_store(View v, const float4* po
 // A warp's partial of a dot product covers the same 32 vertices as in the
 // launched form and goes to the same place of the same sum, into the shared
 // memory of every CTA, so each warp computes the total itself in the launched
-// form's order.  Two sets of partials alternate: a set is written again only
-// after the barrier of the sum between.
+// form's order.  Two sets of partials alternate.  Every warp that waits for a
+// sum also sends to it, zeros where it has no vertex: so a set is written
+// again only when every warp that reads it has sent its partial of the sum
+// between, and no warp falls a phase behind the counter it waits on.  Warps
+// past the CTA's share (a smaller cloth of a batch) take no part.
 //
 // The direction update is folded into the next product: a neighbour's
 // d = z + beta d_old is formed where it is read (the same fused step), and
@@ -778,7 +781,8 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
     static_assert(sizeof(Params) % 4 == 0, "copied as words");
     for (int k = threadIdx.x; k < (int)(sizeof(Params) / 4); k += S)
         reinterpret_cast<unsigned*>(&sP)[k] = reinterpret_cast<const unsigned*>(&v.P[cloth])[k];
-    // partials of the launched grid's warps past the cluster's stay zero
+    // partials of the launched grid's warps past the cluster's stay zero (those
+    // of the cluster's past the grid's are not read)
     for (int k = threadIdx.x; k < 2 * kHardMaxVertices / 32; k += S) (&part[0][0])[k] = 0.0f;
     if (threadIdx.x == 0) {
         ClusterBarrier::init(&s_counter, C);
@@ -810,7 +814,7 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
         }
     }
     barrier();
-    if (!final_caps) {
+    if (!final_caps && (kOne || (int)threadIdx.x < kChunk)) {
         const int nw = P.pcg_nblocks * (kThreads / 32);  // warps of the launched grid, those past V included
         Sym diag[N], pinv[N];
         F3 r[N], q[N];
@@ -821,13 +825,13 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
             float* mine = part[sums & 1];
             if (!kOne && threadIdx.x == 0)
                 asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&s_sum[sums & 1])),
-                             "r"(4 * min(nw, C * kChunk / 32))
+                             "r"(4 * (C * kChunk / 32))
                              : "memory");
 #pragma unroll
             for (int n = 0; n < N; ++n) {
                 const int gw = (first + n * S) >> 5;
                 const float t = __shfl_sync(0xffffffffu, warp_tree(val[n]), 0);
-                const bool mine_too = (int)threadIdx.x + n * S < kChunk && gw < nw;
+                const bool mine_too = (int)threadIdx.x + n * S < kChunk;
                 if (kOne) {
                     if (mine_too && lane == 0) mine[gw] = t;
                 } else {
@@ -964,8 +968,8 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
             R[kRedRZNext] = rz_next;
             R[kRedStatus] = bar.lost ? kStatusBadAlpha : status;
         }
-        if (P.pcg_hard) barrier();  // the polish reads every vertex
     }
+    if (!final_caps && P.pcg_hard) barrier();  // the polish reads every vertex
     if (P.pcg_hard) {
         int epoch = 0;
         // Whether some edge of the cloth may be longer than `ratio` rest
