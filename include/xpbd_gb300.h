@@ -264,6 +264,12 @@ __attribute__((visibility("default"))) int xpbd_gb300_prepare_cloth_device(const
 /* Wait for the solver's stream. */
 __attribute__((visibility("default"))) int xpbd_gb300_synchronize(void* handle);
 
+/* Host word that a frame sets when a wait between the thread blocks of one of
+ * its cluster kernels ran out (null: the solver runs no such kernel).  While
+ * it is set, steps, downloads, buffer reads, cache samples and
+ * xpbd_gb300_synchronize fail; a reset of the whole solver clears it. */
+__attribute__((visibility("default"))) int* xpbd_gb300_barrier_word(void* handle);
+
 #ifdef __cplusplus
 }
 #endif

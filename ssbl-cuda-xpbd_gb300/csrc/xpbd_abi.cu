@@ -447,7 +447,7 @@ XG_EXPORT long long xpbd_gb300_read_buffer(void* handle, int id, void* out, long
         fail("output buffer too small");
         return -1;
     }
-    if (!cuda_ok(cudaStreamSynchronize(S->stream), "read buffer") ||
+    if (!cuda_ok(cudaStreamSynchronize(S->stream), "read buffer") || frame_lost(S) ||
         (bytes > 0 && !cuda_ok(cudaMemcpy(out, src, (size_t)bytes, cudaMemcpyDeviceToHost), "read buffer")))
         return -1;
     return bytes;
@@ -621,5 +621,10 @@ XG_EXPORT int xpbd_gb300_synchronize(void* handle) {
     g_error.clear();
     Solver* S = as_solver(handle);
     if (!S) return fail("invalid solver handle") ? 1 : 0;
-    return cuda_ok(cudaStreamSynchronize(S->stream), "synchronize") ? 1 : 0;
+    return cuda_ok(cudaStreamSynchronize(S->stream), "synchronize") && !frame_lost(S) ? 1 : 0;
+}
+
+XG_EXPORT int* xpbd_gb300_barrier_word(void* handle) {
+    Solver* S = as_solver(handle);
+    return S ? S->lost : nullptr;
 }

@@ -59,8 +59,8 @@ struct ClusterMap {
 // Barrier of a cluster: one thread per CTA arrives at every CTA's counter
 // after its own CTA's barrier; every thread then waits on its own counter
 // (initialised for `ctas` arrivals).  The waits are bounded: when one runs
-// out the barrier gives up for good (`lost`), so the kernel ends and can
-// report it.
+// out the thread waits no more (`lost`), so the kernel ends, and end() tells
+// every thread of the cluster, which then writes no result but reports it.
 struct ClusterBarrier {
     unsigned counter, parity;
     int ctas;
@@ -99,14 +99,31 @@ struct ClusterBarrier {
     // sync that also tells every CTA whether `mark` (of the own CTA, written
     // before) holds `epoch` in some CTA; `any` is the cluster's answer, in one
     // of two places by turns: the next answer may be written while a slower
-    // CTA still reads this one.
+    // CTA still reads this one.  The CTA's threads agree on it, also where a
+    // wait gave up: what they do next has block barriers.
     __device__ __forceinline__ bool sync_any(const volatile int* mark, volatile int* any, int epoch) {
         if (ctas == 1) return __syncthreads_or(*mark == epoch);
         __syncthreads();
         if ((int)threadIdx.x < ctas && *mark == epoch)
             asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(map_rank(smem_addr((const void*)any), threadIdx.x)), "r"(epoch) : "memory");
         sync();
-        return *any == epoch;
+        return __syncthreads_or(*any == epoch);
+    }
+    // The last barrier of a kernel: afterwards no CTA addresses another's
+    // shared memory.  The hardware's, which waits for every thread of the
+    // cluster (all come here, since every wait before is bounded).  Returns
+    // whether a wait of some thread of the cluster gave up; `mark` is a word
+    // of each CTA, zero since before the first arrival.
+    __device__ __forceinline__ bool end(volatile int* mark) {
+        if (lost)
+            for (int r = 0; r < ctas; ++r)
+                asm volatile("st.shared::cluster.s32 [%0], 1;" ::"r"(map_rank(smem_addr((const void*)mark), r)) : "memory");
+        __syncwarp();
+        if (ctas > 1)
+            cooperative_groups::this_cluster().sync();
+        else
+            __syncthreads();
+        return *mark != 0;
     }
 };
 

@@ -677,11 +677,13 @@ template <int T, bool kOne, bool kBack>
 __global__ void __launch_bounds__(T, 1) k_d_cluster(DView d, DiffCluster a) {
     extern __shared__ float4 sm[];
     __shared__ unsigned long long s_counter;
+    __shared__ int s_lost;
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int rank = kOne ? 0 : (int)cluster.block_rank();
     if (threadIdx.x == 0) {
         ClusterBarrier::init(&s_counter, a.ctas);
         ClusterBarrier::init_fence();
+        s_lost = 0;
     }
     __syncthreads();
     if (!kOne) cluster.sync();  // every CTA's counter is set before the first arrival
@@ -756,8 +758,7 @@ __global__ void __launch_bounds__(T, 1) k_d_cluster(DView d, DiffCluster a) {
         for (int e = threadIdx.x; e < edges; e += blockDim.x)
             if (edge[e].x & kEdgeMine) a.grad_stretch[a.cta_edge[edge0 + e]] = gk[e];
     }
-    if (bar.lost) *a.lost = 1;
-    bar.sync();  // no CTA leaves while another still reads its shared memory
+    if (bar.end(&s_lost) && threadIdx.x == 0) *a.lost = 1;
 }
 
 // ---------------------------------------------------------------- host --

@@ -475,6 +475,7 @@ View Solver::view() const {
     v.scan_tmp = scan_tmp;
     v.acc = acc;
     v.max_delta_bits = max_delta_bits;
+    v.lost = lost;
     return v;
 }
 
@@ -960,17 +961,22 @@ bool upload_fields(Solver* S, int cloth, const SsblXpbdForceField* fields, int c
 // moves 400 KB in 3 us.
 constexpr size_t kSmallTransfer = 64 << 10;
 
+// Behind it lies the word of frame_lost.
+bool small_memory(Solver* S) {
+    if (!S->io && cudaHostAlloc(reinterpret_cast<void**>(&S->io), kSmallTransfer + sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();  // none to be had
+        S->io = nullptr;
+    }
+    return S->io != nullptr;
+}
+
 // Uploads take their places in it one after another and are only waited for
 // when it is full, so the cloths of a batch, placed one by one, cost a launch
 // each (180 cloths of 6 x 6 to 40 x 40 vertices: 13 -> 5 us a call).  A download
 // ends in a wait and leaves it empty.
 float* small_transfer(Solver* S, size_t bytes, bool upload) {
     if (bytes > kSmallTransfer) return nullptr;
-    if (!S->io && cudaHostAlloc(reinterpret_cast<void**>(&S->io), kSmallTransfer, cudaHostAllocMapped) != cudaSuccess) {
-        cudaGetLastError();  // none to be had: copy
-        S->io = nullptr;
-    }
-    if (!S->io || !upload) return S->io;
+    if (!small_memory(S) || !upload) return S->io;
     if (S->io_used + bytes > kSmallTransfer) {
         if (!cuda_ok(cudaStreamSynchronize(S->stream), "upload positions")) return nullptr;
         S->io_used = 0;
@@ -1014,6 +1020,7 @@ bool download_positions(Solver* S, int cloth, float* out, int max_floats) {
         !cuda_ok(cudaStreamSynchronize(S->stream), "download ABI41 positions"))
         return false;
     S->io_used = 0;
+    if (frame_lost(S)) return false;
     if (small) std::memcpy(out, small, bytes);
     return true;
 }
@@ -1023,8 +1030,15 @@ bool reset_cloths(Solver* S, int cloth) {
     const Range r = cloth_range(S, cloth);
     launch_reset_state(S->pos[0] + r.lo, S->prev + r.lo, S->vel + r.lo, S->rest + r.lo, r.hi - r.lo, S->counts, S->stream);
     if (!cuda_ok(cudaGetLastError(), "reset solver") || !cuda_ok(cudaStreamSynchronize(S->stream), "reset solver")) return false;
+    if (S->lost && r.hi - r.lo == S->nV) *S->lost = 0;
     S->diag = SsblXpbdDiagnostics{};
     S->diag.finite_flag = 1;
+    return true;
+}
+
+bool frame_lost(const Solver* S) {
+    if (!S->lost || *reinterpret_cast<const volatile int*>(S->lost) == 0) return false;
+    fail("a thread-block cluster's barrier timed out: the solver's state is undefined until a reset");
     return true;
 }
 
@@ -1598,6 +1612,15 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
                 S->frame.edge = S->frame_tables + t.off.size();
                 S->frame.ent = S->frame.edge + t.edge.size();
             }
+        }
+    }
+    // the cluster forms report through host memory; without any, the launched forms run
+    if (ok && (S->frame.ctas > 0 || S->hard.cluster > 0)) {
+        if (small_memory(S)) {
+            S->lost = reinterpret_cast<int*>(S->io + kSmallTransfer / sizeof(float));
+            *S->lost = 0;
+        } else {
+            S->frame.ctas = S->hard.cluster = 0;
         }
     }
     if (!ok) return bail(0, "");
@@ -2337,6 +2360,7 @@ bool prepare_step(Solver* S, int substeps, int iterations) {
 
 bool step(Solver* S, int substeps, int iterations, int fetch_diagnostics, int force_sync) {
     const auto t0 = std::chrono::high_resolution_clock::now();
+    if (frame_lost(S)) return false;
     int ff = 0, uff = 0;
     for (const Cloth& C : S->cl) {
         ff += C.force_field_count;
@@ -2372,7 +2396,7 @@ bool step(Solver* S, int substeps, int iterations, int fetch_diagnostics, int fo
     S->pcg_iterations = st.pcg_solves * 8;
     if (force_sync || fetch_diagnostics) {
         const auto ts = std::chrono::high_resolution_clock::now();
-        if (!cuda_ok(cudaStreamSynchronize(S->stream), "ABI41 solver step")) return false;
+        if (!cuda_ok(cudaStreamSynchronize(S->stream), "ABI41 solver step") || frame_lost(S)) return false;
         S->diag.sync_ms = (float)ms_since(ts);
     }
     if (fetch_diagnostics && !fetch_counts(S, st)) return false;
@@ -2395,7 +2419,8 @@ bool profile_frame(Solver* S, int substeps, int iterations, float* kernel_ms, lo
     FrameStats st;
     Profile prof;
     enqueue_frame(S, substeps, iterations, &st, &prof);
-    const bool ok = cuda_ok(cudaGetLastError(), "profile frame") && cuda_ok(cudaStreamSynchronize(S->stream), "profile frame");
+    const bool ok = cuda_ok(cudaGetLastError(), "profile frame") && cuda_ok(cudaStreamSynchronize(S->stream), "profile frame") &&
+                    !frame_lost(S);
     for (auto& m : prof.marks) {
         float ms = 0.0f;
         if (ok) cudaEventElapsedTime(&ms, m.second.first, m.second.second);

@@ -275,6 +275,7 @@ struct Solver {
     unsigned* max_delta_bits = nullptr;
     float* pack = nullptr;
     float* io = nullptr;         // page-locked host memory of small transfers (kSmallTransfer bytes), from the first one on
+    int* lost = nullptr;         // behind it: set by a frame whose cluster barrier gave up (solvers with a cluster form)
     size_t io_used = 0;          // bytes of it that uploads not waited for may still be read from
 
     std::vector<float> h_w;      // effective inverse mass per vertex
@@ -391,6 +392,10 @@ bool scene_update(GlobalScene* G, const SsblXpbdGlobalDynamicSceneInputs* in);
 bool scene_attach(Solver* S, int cloth, GlobalScene* G, int source_id, int layer, int mode);
 void scene_detach(Solver* S, int cloth);
 void sdf_diagnostics(Solver* S);
+// Whether a frame's cluster barrier gave up: the state is undefined from then
+// on, and calls that hand it out or go on from it fail until a reset of the
+// whole solver.  A read of host memory: call it after a wait.
+bool frame_lost(const Solver* S);
 
 // Tables of a cluster form that computes each edge once per CTA: the CTAs of a
 // cloth own `chunk` consecutive vertices each.

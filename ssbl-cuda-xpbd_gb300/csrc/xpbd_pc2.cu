@@ -152,6 +152,7 @@ void* pc2_open(Solver* S, int cloth, const char* path, int start_frame) {
 bool pc2_write(Solver* S, void* writer, const float* matrix16) {
     Pc2Writer* W = reinterpret_cast<Pc2Writer*>(writer);
     if (!S || !W) return fail("invalid PC2 writer request");
+    if (frame_lost(S)) return false;
     float m[12] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0};
     if (matrix16) std::memcpy(m, matrix16, sizeof(m));
     const int s = W->slot;

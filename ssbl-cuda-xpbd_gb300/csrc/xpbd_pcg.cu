@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
     __shared__ float part[2][kHardMaxVertices / 32];
     __shared__ Params sP;
     __shared__ unsigned long long s_counter, s_sum[2];  // barrier; arrivals of the two sets of partials
-    __shared__ int s_mark, s_any[2];
+    __shared__ int s_mark, s_any[2], s_lost;
     __shared__ int s_color[kHardColors + 1];  // first kept cap edge of each colour
     const cgx::cluster_group cluster = cgx::this_cluster();
     const int C = kOne ? 1 : (int)cluster.num_blocks(), rank = kOne ? 0 : (int)cluster.block_rank();
@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
         ClusterBarrier::init(&s_counter, C);
         for (int k = 0; k < 2; ++k) ClusterBarrier::init(&s_sum[k], 1);
         ClusterBarrier::init_fence();
-        s_mark = s_any[0] = s_any[1] = 0;
+        s_mark = s_any[0] = s_any[1] = s_lost = 0;
     }
     __syncthreads();
     const Params& P = sP;
@@ -966,7 +966,7 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
             R[kRedIterations] = iterations;
             R[kRedDAD] = dad;
             R[kRedRZNext] = rz_next;
-            R[kRedStatus] = bar.lost ? kStatusBadAlpha : status;
+            R[kRedStatus] = status;
         }
     }
     if (!final_caps && P.pcg_hard) barrier();  // the polish reads every vertex
@@ -1087,7 +1087,10 @@ __global__ void __launch_bounds__(T) k_hard_cluster(View v, PcgView g, HardPlan 
             }
         }
     }
-    barrier();  // no CTA leaves while another still reads or writes its shared memory
+    if (bar.end(&s_lost)) {  // positions stay as they were
+        if (threadIdx.x == 0) *v.lost = 1;
+        return;
+    }
 #pragma unroll
     for (int n = 0; n < N; ++n) {
         const int t = (int)threadIdx.x + n * S, l = rank * kChunk + t;

@@ -342,6 +342,7 @@ struct View {
     int* nb_idx;            // [nV * 32]
     Acc4* acc;              // fixed-point delta xyz + contact weight
     unsigned* max_delta_bits;
+    int* lost;              // host word, set when a wait in a cluster form ran out (null: no cluster form)
     // work counters of a profiled frame (null otherwise): query items and
     // bucket slots evaluated by the EE and VT queries
     unsigned long long* perf;

@@ -891,6 +891,7 @@ __global__ void __launch_bounds__(T, 1) k_frame_edges(View v, FramePlan f, const
                                                       const int2* bend_ranges, int K) {
     extern __shared__ float4 sm[];
     __shared__ unsigned long long s_counter;
+    __shared__ int s_lost;
     __shared__ Params sP;
     const cgx::cluster_group cluster = cgx::this_cluster();
     const int C = kOne ? 1 : (int)cluster.num_blocks(), rank = kOne ? 0 : (int)cluster.block_rank();
@@ -900,6 +901,7 @@ __global__ void __launch_bounds__(T, 1) k_frame_edges(View v, FramePlan f, const
     if (threadIdx.x == 0) {
         ClusterBarrier::init(&s_counter, C);
         ClusterBarrier::init_fence();
+        s_lost = 0;
     }
     __syncthreads();
     const Params& P = sP;
@@ -1073,12 +1075,15 @@ __global__ void __launch_bounds__(T, 1) k_frame_edges(View v, FramePlan f, const
         count_add(v.counts, kCntBendingWings, wings);
         count_add(v.counts, kCntBendingGuards, guards);
     }
+    if (bar.end(&s_lost)) {  // the state stays as it was
+        if (t == 0) *v.lost = 1;
+        return;
+    }
     if (mine) {
         buf0[i] = f4(s.p, s.w);
         v.prev[i] = f4(s.prev, 0.0f);
         v.vel[i] = f4(s.vel, 0.0f);
     }
-    bar.sync();  // no CTA leaves while another still reads its shared memory
 }
 
 namespace {

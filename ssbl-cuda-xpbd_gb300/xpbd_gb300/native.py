@@ -223,6 +223,7 @@ def _load_library(path: str | None = None):
         "xpbd_gb300_set_default_key_division": (ctypes.c_int, [ctypes.c_int]),
         "xpbd_gb300_last_step_launches": (ctypes.c_longlong, [vp]),
         "xpbd_gb300_synchronize": (ctypes.c_int, [vp]),
+        "xpbd_gb300_barrier_word": (_PI, [vp]),
         "xpbd_gb300_stream": (vp, [vp]),
         "xpbd_gb300_profile_frame": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int, _PF,
                                                     ctypes.POINTER(ctypes.c_longlong), ctypes.c_int]),
