@@ -690,12 +690,20 @@ struct DynCtx {
     float margin;
     float thickness;
     int key_ieee;  // cell-key division of the hashes built
+    Solver* S;     // null for a shared scene
 };
 
 DynCtx cloth_ctx(Solver* S, int k) {
     const SsblXpbdConfig& c = S->cl[k].cfg;
     return DynCtx{S->stream, &S->device_bytes, std::max(c.collision_margin, 0.0f), std::max(c.cloth_thickness, 0.0f),
-                  S->key_ieee};
+                  S->key_ieee, S};
+}
+
+// Copies from memory that is the caller's, or gone when the call returns.
+template <class T>
+bool put(const DynCtx& c, DynHost& D, T* dst, const T* src, size_t n, const char* what) {
+    if (c.S) return staged_upload(c.S, dst, src, sizeof(T) * n, &D.direct, what);
+    return dupload(dst, src, n, c.st, what);  // a shared scene's update waits for all of them
 }
 
 // (Re)allocate a device array of at least n elements; the old contents are
@@ -832,7 +840,7 @@ bool put_rows(const DynCtx& c, DynHost& D, const float* tris, int count) {
     }
     std::vector<float4> rows((size_t)count * 3);
     for (int q = 0; q < count * 3; ++q) rows[q] = make_float4(tris[3 * q], tris[3 * q + 1], tris[3 * q + 2], 0.0f);
-    return dupload(D.tris, rows.data(), rows.size(), c.st, "dynamic triangle upload");
+    return put(c, D, D.tris, rows.data(), rows.size(), "dynamic triangle upload");
 }
 
 void clear_triangles(DynHost& D) {
@@ -890,13 +898,13 @@ bool put_particles(const DynCtx& c, DynHost& D, const float* pos, const float* p
     if (prev) {
         q4.resize(count);
         for (int q = 0; q < count; ++q) q4[q] = make_float4(prev[3 * q], prev[3 * q + 1], prev[3 * q + 2], 0.0f);
-        if (!dupload(D.pprev, q4.data(), (size_t)count, st, "dynamic particle previous upload")) return false;
+        if (!put(c, D, D.pprev, q4.data(), (size_t)count, "dynamic particle previous upload")) return false;
     } else if (motion && !cuda_ok(cudaMemcpyAsync(D.pprev, D.ppos, sizeof(float4) * count, cudaMemcpyDeviceToDevice, st),
                                   "keep dynamic particle positions")) {
         return false;
     }
-    if (!dupload(D.ppos, p4.data(), (size_t)count, st, "dynamic particle upload") ||
-        !dupload(D.prad, radii, (size_t)count, st, "dynamic particle radius upload"))
+    if (!put(c, D, D.ppos, p4.data(), (size_t)count, "dynamic particle upload") ||
+        !put(c, D, D.prad, radii, (size_t)count, "dynamic particle radius upload"))
         return false;
     if (!prev && !motion &&
         !cuda_ok(cudaMemcpyAsync(D.pprev, D.ppos, sizeof(float4) * count, cudaMemcpyDeviceToDevice, st), "init dynamic particle positions"))
@@ -941,7 +949,7 @@ bool put_particles(const DynCtx& c, DynHost& D, const float* pos, const float* p
 // Copy the descriptor to the device (allocated on first use).
 bool put_set(const DynCtx& c, DynHost& D) {
     if (!D.dev && !dalloc(&D.dev, 1, "dynamic collider descriptor")) return false;
-    return dupload(D.dev, &D.h, 1, c.st, "dynamic collider descriptor");
+    return put(c, D, D.dev, &D.h, 1, "dynamic collider descriptor");
 }
 
 // The same for a shared scene, whose readers run on streams of their own.
@@ -950,10 +958,13 @@ bool publish_set(const DynCtx& c, DynHost& D) {
 }
 
 // Point the cloth's parameters at its descriptor (null when it has no
-// dynamic collider).  Frames follow on the upload's own stream.
+// dynamic collider).  Frames follow on the upload's own stream, so the only
+// wait is for copies that read the caller's arrays.
 bool publish(Solver* S, int k) {
     DynHost& D = S->cl[k].dyn;
     if (!put_set(cloth_ctx(S, k), D)) return false;
+    if (D.direct && !cuda_ok(cudaStreamSynchronize(S->stream), "dynamic collider upload")) return false;
+    D.direct = false;
     const bool any = D.h.tri_count > 0 || D.h.par_count > 0;
     S->hp[k].dyn = any ? D.dev : nullptr;
     S->params_dirty = true;
@@ -1032,13 +1043,13 @@ bool upload_dynamic_indexed(Solver* S, int cloth, const float* verts, int vcount
             if (!realloc_dev(cx, &D.verts, (size_t)D.verts_cap, (size_t)vcount, "dynamic triangle vertex upload")) return false;
             D.verts_cap = vcount;
         }
-        if (!dupload(D.verts, v4.data(), (size_t)vcount, S->stream, "dynamic triangle vertex upload")) return false;
+        if (!put(cx, D, D.verts, v4.data(), (size_t)vcount, "dynamic triangle vertex upload")) return false;
         if (topology_changed || count != D.topology_count || count > D.idx_cap) {
             if (count > D.idx_cap) {
                 if (!realloc_dev(cx, &D.idx, (size_t)D.idx_cap * 3, (size_t)count * 3, "dynamic triangle index upload")) return false;
                 D.idx_cap = count;
             }
-            if (!dupload(D.idx, idx, (size_t)3 * count, S->stream, "dynamic triangle index upload")) return false;
+            if (!put(cx, D, D.idx, idx, (size_t)3 * count, "dynamic triangle index upload")) return false;
             D.topology_count = count;
         }
         if (count > D.tris_cap) {
@@ -1114,7 +1125,7 @@ bool scene_update(GlobalScene* G, const SsblXpbdGlobalDynamicSceneInputs* in) {
     G->thickness = std::max(in->cloth_thickness, 0.0f);
     G->hash_overflow = 0;
     AllocAccount account(&G->device_bytes);
-    const DynCtx c{G->stream, &G->device_bytes, G->margin, G->thickness, G->key_ieee};
+    const DynCtx c{G->stream, &G->device_bytes, G->margin, G->thickness, G->key_ieee, nullptr};
     DynHost& D = G->dyn;
     if (!G->overflow && !dalloc(&G->overflow, 1, "global dynamic scene counters")) return false;
     if (!cuda_ok(cudaMemsetAsync(G->overflow, 0, sizeof(unsigned long long), c.st), "global dynamic scene counters")) return false;
@@ -1174,7 +1185,7 @@ bool scene_attach(Solver* S, int cloth, GlobalScene* G, int source_id, int layer
         if (C.gscene && C.gscene != G) C.gscene->attached.erase({S, k});
         if (!G->dyn.dev) {
             AllocAccount account(&G->device_bytes);
-            if (!publish_set(DynCtx{G->stream, &G->device_bytes, G->margin, G->thickness, G->key_ieee}, G->dyn)) return false;
+            if (!publish_set(DynCtx{G->stream, &G->device_bytes, G->margin, G->thickness, G->key_ieee, nullptr}, G->dyn)) return false;
         }
         C.gscene = G;
         G->attached.insert({S, k});

@@ -986,6 +986,22 @@ float* small_transfer(Solver* S, size_t bytes, bool upload) {
     return at;
 }
 
+bool staged_upload(Solver* S, void* dst, const void* src, size_t bytes, bool* direct, const char* what) {
+    if (bytes == 0) return true;
+    if (bytes > kSmallTransfer) {
+        *direct = true;
+    } else {
+        S->staged.resize(kSmallTransfer);
+        if (S->staged_used + bytes > kSmallTransfer) {
+            if (!cuda_ok(cudaStreamSynchronize(S->stream), what)) return false;
+            S->staged_used = 0;
+        }
+        src = std::memcpy(S->staged.data() + S->staged_used, src, bytes);
+        S->staged_used += (bytes + 15) & ~(size_t)15;
+    }
+    return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, S->stream), what);
+}
+
 bool upload_positions(Solver* S, int cloth, const float* positions, int max_floats) {
     if (!valid_cloth(S, cloth) || !positions) return fail("invalid position upload");
     const Range r = cloth_range(S, cloth);
@@ -1019,7 +1035,7 @@ bool download_positions(Solver* S, int cloth, float* out, int max_floats) {
         (!small && !cuda_ok(cudaMemcpyAsync(out, dst, bytes, cudaMemcpyDeviceToHost, S->stream), "download ABI41 positions")) ||
         !cuda_ok(cudaStreamSynchronize(S->stream), "download ABI41 positions"))
         return false;
-    S->io_used = 0;
+    S->io_used = S->staged_used = 0;
     if (frame_lost(S)) return false;
     if (small) std::memcpy(out, small, bytes);
     return true;

@@ -171,6 +171,7 @@ struct DynHost {
     int topology_count = -1;      // triangles of the uploaded index buffer
     int par_upload_count = 0;
     unsigned long long radius_signature = 0;
+    bool direct = false;          // an upload reads memory that the caller gets back: the call ends in a wait
     int large_count = 0;          // triangles spanning more than 64 cells
     int max_occupancy = 0;        // largest bucket of the triangle hash
 };
@@ -275,7 +276,9 @@ struct Solver {
     unsigned* max_delta_bits = nullptr;
     float* pack = nullptr;
     float* io = nullptr;         // page-locked host memory of small transfers (kSmallTransfer bytes), from the first one on
-    int* lost = nullptr;         // behind it: set by a frame whose cluster barrier gave up (solvers with a cluster form)
+    std::vector<char> staged;    // what staged_upload's copies read, from the first one on
+    size_t staged_used = 0;      // bytes of it that copies not waited for may still read
+    int* lost = nullptr;         // behind `io`: set by a frame whose cluster barrier gave up (solvers with a cluster form)
     size_t io_used = 0;          // bytes of it that uploads not waited for may still be read from
 
     std::vector<float> h_w;      // effective inverse mass per vertex
@@ -392,6 +395,14 @@ bool scene_update(GlobalScene* G, const SsblXpbdGlobalDynamicSceneInputs* in);
 bool scene_attach(Solver* S, int cloth, GlobalScene* G, int source_id, int layer, int mode);
 void scene_detach(Solver* S, int cloth);
 void sdf_diagnostics(Solver* S);
+// A copy to the device on the solver's stream.  Up to kSmallTransfer bytes are
+// copied from memory of the solver that is used again only after a wait; more
+// are read from `src` itself, which `direct` tells: the caller waits for the
+// stream before `src` changes.  (cudaMemcpyAsync may return before it has read
+// page-locked memory, and need not have read any other.  The solver's is
+// pageable: copies of 10 KB from page-locked memory cost a frame with two
+// uploads 27 us more, kernels that read it 12 us.)
+bool staged_upload(Solver* S, void* dst, const void* src, size_t bytes, bool* direct, const char* what);
 // Whether a frame's cluster barrier gave up: the state is undefined from then
 // on, and calls that hand it out or go on from it fail until a reset of the
 // whole solver.  A read of host memory: call it after a wait.
