@@ -476,6 +476,7 @@ View Solver::view() const {
     v.acc = acc;
     v.max_delta_bits = max_delta_bits;
     v.lost = lost;
+    v.carve = self_any ? kCarveout : -1;
     return v;
 }
 
@@ -1446,7 +1447,6 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
     }
     if (ok && S->self_any) {
         self_set_carveout();
-        step_set_carveout();
         cudaFuncSetAttribute(k_zero_spans, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
         cudaGetLastError();
         ok = dalloc(&S->nb_count, nV, "self collision count allocation") &&
@@ -2157,7 +2157,7 @@ void enqueue_frame(Solver* S, int substeps, int iterations, FrameStats* st, Prof
     if (cur != 0 && S->rec)
         S->rec->push_back(FrameOp{3, 0u, 1, 0, 0, 0, 0});
     else if (cur != 0)
-        timed(kKCopy, 1, [&] { launch_copy_pos(S->pos[0], S->pos[1], nV, S->stream); });
+        timed(kKCopy, 1, [&] { launch_copy_pos(base, S->pos[0], S->pos[1], nV, S->stream); });
 }
 
 namespace {

@@ -410,17 +410,17 @@ __global__ void __launch_bounds__(1024) k_scan_down(int* counts, int* start, int
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) start[n] = run;
 }
 
-void scan_counts(int* counts, int* start, int n, int* block_sums, unsigned long long* overflow, cudaStream_t s,
+void scan_counts(int* counts, int* start, int n, int* block_sums, unsigned long long* overflow, int carve, cudaStream_t s,
                  int* trim = nullptr, int* trim_count = nullptr) {
     if (n <= kScanTile) {
-        k_scan_one<<<1, 1024, 0, s>>>(counts, start, n, overflow, trim, trim_count);
+        launch_carved(k_scan_one, 1, 1024, s, carve, false, counts, start, n, overflow, trim, trim_count);
         return;
     }
     const int blocks = (n + kScanTile - 1) / kScanTile;
     const bool sums = blocks > kScanSums;
-    k_scan_reduce<<<blocks, 1024, 0, s>>>(counts, n, block_sums, overflow, trim, trim_count);
-    if (sums) k_scan_sums<<<1, 1024, 0, s>>>(block_sums, blocks);
-    k_scan_down<<<blocks, 1024, 0, s>>>(counts, start, n, block_sums, sums);
+    launch_carved(k_scan_reduce, blocks, 1024, s, carve, false, counts, n, block_sums, overflow, trim, trim_count);
+    if (sums) launch_carved(k_scan_sums, 1, 1024, s, carve, false, block_sums, blocks);
+    launch_carved(k_scan_down, blocks, 1024, s, carve, false, counts, start, n, block_sums, sums);
 }
 
 __device__ __forceinline__ int warp_global_id() { return (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); }
@@ -2873,7 +2873,7 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
     const View iv = ranged(v, items);
     const int b = tune_of(v.tune, kTuneHashBlock), lanes = tune_of(v.tune, kTuneTriLanes);
     tri_pass_lanes(iv, items.size(), lanes, b, false, s);
-    scan_counts(v.tb_count, v.tb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s, v.trim_list,
+    scan_counts(v.tb_count, v.tb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, kCarveout, s, v.trim_list,
                 v.trim_count);
     tri_pass_lanes(iv, items.size(), lanes, b, true, s);
     if (v.trim_list) {
@@ -2921,7 +2921,7 @@ void set_carveout(K... kernels) {
 
 void self_set_carveout() {
     set_carveout(k_vhash_count, k_vhash_scatter, k_tri_hash<1>, k_tri_hash<2>, k_tri_hash<4>, k_tri_hash<8>, k_tri_hash<16>,
-                 k_scan_one, k_scan_reduce, k_scan_sums, k_scan_down, k_edge_insert<1>, k_edge_insert<2>, k_edge_insert<4>, k_edge_insert<8>,
+                 k_edge_insert<1>, k_edge_insert<2>, k_edge_insert<4>, k_edge_insert<8>,
                  k_edge_insert<16>, k_edge_ovf_offsets, k_edge_ovf_fill<1>, k_edge_ovf_fill<2>,
                  k_edge_ovf_fill<4>, k_edge_ovf_fill<8>, k_edge_ovf_fill<16>, k_edge_trim, k_bucket_sort,
                  k_bucket_trim, k_neighbors_brute, k_vv, k_vv_warp, k_vt_hash, k_vt_brute, k_ee_brute, k_vt_warp<4>, k_vt_warp<8>,
@@ -2936,7 +2936,7 @@ void self_set_carveout() {
 int scan_launches(int n) { return n <= kScanTile ? 1 : (n <= kScanSums * kScanTile ? 2 : 3); }
 
 void scan_bucket_counts(int* counts, int* start, int n, int* block_sums, cudaStream_t s) {
-    if (n > 0) scan_counts(counts, start, n, block_sums, nullptr, s);
+    if (n > 0) scan_counts(counts, start, n, block_sums, nullptr, -1, s);
 }
 
 void self_build_vertex_hash(const View& v, const SelfVariants& sv, int nb, cudaStream_t s) {
@@ -2945,7 +2945,7 @@ void self_build_vertex_hash(const View& v, const SelfVariants& sv, int nb, cudaS
     const View iv = ranged(v, r);
     const int b = tune_of(v.tune, kTuneHashBlock);
     k_vhash_count<<<grid(r.size(), 1, b), b, kBuildShared, s>>>(iv);
-    scan_counts(v.vb_count, v.vb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, s);
+    scan_counts(v.vb_count, v.vb_start, nb, v.scan_tmp, v.counts ? v.counts + kCntSelfOverflow : nullptr, kCarveout, s);
     k_vhash_scatter<<<grid(r.size(), 1, b), b, kBuildShared, s>>>(iv);
     bucket_order(v, sv.vb, v.vb_start, v.vb_ent, nb, 0, 1, s);
 }

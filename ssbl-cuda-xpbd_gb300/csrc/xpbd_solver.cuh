@@ -342,6 +342,7 @@ struct View {
     int* nb_idx;            // [nV * 32]
     Acc4* acc;              // fixed-point delta xyz + contact weight
     unsigned* max_delta_bits;
+    int carve;              // launch_carved's share for the kernels that all frames use
     int* lost;              // host word, set when a wait in a cluster form ran out (null: no cluster form)
     // work counters of a profiled frame (null otherwise): query items and
     // bucket slots evaluated by the EE and VT queries
@@ -476,7 +477,7 @@ bool frame_fits(const FramePlan& f);
 cudaError_t launch_frame_edges(const View& v, const FramePlan& f, const FrameOp* ops, int first, int last, float4* buf0,
                                const int2* bend_ranges, int K, cudaStream_t s);
 void launch_bend_color(const View& v, int start, int count, cudaStream_t s, bool chained = false);
-void launch_copy_pos(float4* dst, const float4* src, int V, cudaStream_t s);
+void launch_copy_pos(const View& v, float4* dst, const float4* src, int V, cudaStream_t s);
 void launch_pin_scatter(const int* idx, const float4* target, const float* weight, const float* relax, int n,
                         float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s);
 // Positions of vertices [lo, lo + n) as rows of three floats, and back into
@@ -565,8 +566,32 @@ void self_apply(const View& v, const SelfVariants& sv, cudaStream_t s);
 // neighbour table (none) and the edge-edge query (64 KB) took turns, and a
 // faster neighbour table made the frame slower (100 x 100 drop 1.49 -> 2.08 ms;
 // with one share 1.18).
+// The self-collision kernels have it as a property of their own
+// (self_set_carveout).  Kernels that other frames launch too are asked for it
+// launch by launch (launch_carved): a solver's speed does not depend on which
+// others the process has made.
 constexpr int kCarveout = 28;
 void self_set_carveout();
-void step_set_carveout();
+
+// carve: percent, or below zero for the kernel's own preference; chained: see
+// launch_vertex_pass.
+template <class... A, class... B>
+cudaError_t launch_carved(void (*kernel)(A...), unsigned blocks, int threads, cudaStream_t s, int carve, bool chained, B&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks, 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (carve >= 0) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[cfg.numAttrs++].val.sharedMemCarveout = (unsigned)carve;
+    }
+    if (chained) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<A>(args)...);
+}
 
 }  // namespace xg

@@ -14,6 +14,7 @@
 // deterministic.
 #include "xpbd_constraint.cuh"
 #include <algorithm>
+#include <initializer_list>
 
 #include "xpbd_cluster.cuh"
 #include "xpbd_contact.cuh"
@@ -523,7 +524,7 @@ __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned 
 // another, each a load and a chain of a root and two quotients, while a cloth
 // of a few ten thousand vertices leaves most of the chip's warps unused.
 // A launch that was allowed to start before the one before it on the stream
-// ended (launch_chained) waits here until that one has ended and its writes are
+// ended (launch_carved, chained) waits here until that one has ended and its writes are
 // visible; any other launch passes at once.  Every thread of such a kernel
 // calls it, so that no launch ends before those ahead of it have.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -1162,20 +1163,22 @@ void launch_frame_fused(const View& v, const FrameOp* ops, int nops, float4* buf
     if (K > 0) k_frame_fused<<<K, block, smem, s>>>(v, ops, nops, buf0, bend_ranges, K);
 }
 
-void step_set_carveout() {
-    cudaFuncSetAttribute(k_predict, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaFuncSetAttribute(k_vertex_pass, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaFuncSetAttribute(k_vertex_pass_lanes<2>, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaFuncSetAttribute(k_vertex_pass_lanes<4>, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaFuncSetAttribute(k_vertex_pass_lanes<8>, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaFuncSetAttribute(k_bend_color, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaFuncSetAttribute(k_copy_pos, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
-    cudaGetLastError();  // a preference: the kernels run without it
+// The share of L1 that the launched passes prefer as a kernel property (-1: the
+// driver's choice): no solver changes it.
+extern "C" __attribute__((visibility("default"))) int xpbd_gb300_pass_carveout(void) {
+    int share = -2;
+    for (const void* k : {(const void*)k_predict, (const void*)k_vertex_pass, (const void*)k_vertex_pass_lanes<2>,
+                          (const void*)k_bend_color, (const void*)k_copy_pos}) {
+        cudaFuncAttributes a;
+        if (cudaFuncGetAttributes(&a, k) != cudaSuccess || (share != -2 && a.preferredShmemCarveout != share)) return -2;
+        share = a.preferredShmemCarveout;
+    }
+    return share;
 }
 
 void launch_predict(const View& v, int V, cudaStream_t s) {
     const int b = tune_of(v.tune, kTuneVertexBlock);
-    if (V > 0) k_predict<<<grid_for(V, b), b, 0, s>>>(v);
+    if (V > 0) launch_carved(k_predict, grid_for(V, b), b, s, v.carve, false, v);
 }
 
 // Lanes per vertex of a stretch pass over V vertices.  Us per frame of a plain
@@ -1191,30 +1194,16 @@ constexpr int kPassLanes8 = 16 << 10, kPassLanes4 = 32 << 10, kPassLanes2 = 128 
 // and 133, 240 x 240 140 and 134, 300 x 300 198 and 188.  Not earlier still: a
 // kernel that lets the next one start beside all of its blocks shares the SMs
 // with them (240 x 240 153).
-template <class... A>
-static void launch_chained(void (*kernel)(A...), unsigned blocks, int b, cudaStream_t s, bool chained, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks, 1, 1);
-    cfg.blockDim = dim3((unsigned)b, 1, 1);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 void launch_bend_color(const View& v, int start, int count, cudaStream_t s, bool chained) {
     const int b = tune_of(v.tune, kTuneVertexBlock);
-    if (count > 0) launch_chained<View, int, int>(k_bend_color, grid_for(count, b), b, s, chained, v, start, count);
+    if (count > 0) launch_carved(k_bend_color, grid_for(count, b), b, s, v.carve, chained, v, start, count);
 }
 
 void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s, bool chained) {
     const int b = tune_of(v.tune, kTuneVertexBlock);
     if (V <= 0) return;
     auto lanes = [&](void (*kernel)(View, unsigned), int n) {
-        launch_chained<View, unsigned>(kernel, grid_for((long long)n * V, b), b, s, chained, v, flags);
+        launch_carved(kernel, grid_for((long long)n * V, b), b, s, v.carve, chained, v, flags);
     };
     if ((flags & kPassSpring) && V <= kPassLanes8)
         lanes(k_vertex_pass_lanes<8>, 8);
@@ -1223,7 +1212,7 @@ void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s, bo
     else if ((flags & kPassSpring) && V <= kPassLanes2)
         lanes(k_vertex_pass_lanes<2>, 2);
     else
-        k_vertex_pass<<<grid_for(V, b), b, 0, s>>>(v, flags);
+        launch_carved(k_vertex_pass, grid_for(V, b), b, s, v.carve, false, v, flags);
 }
 
 
@@ -1232,8 +1221,8 @@ void launch_pin_scatter(const int* idx, const float4* target, const float* weigh
     if (n > 0) k_pin_scatter<<<blocks_for(n), kThreads, 0, s>>>(idx, target, weight, relax, n, pin_target, pin_weight, pin_relax, nV);
 }
 
-void launch_copy_pos(float4* dst, const float4* src, int V, cudaStream_t s) {
-    if (V > 0) k_copy_pos<<<blocks_for(V), kThreads, 0, s>>>(dst, src, V);
+void launch_copy_pos(const View& v, float4* dst, const float4* src, int V, cudaStream_t s) {
+    if (V > 0) launch_carved(k_copy_pos, blocks_for(V), kThreads, s, v.carve, false, dst, src, V);
 }
 
 void launch_pin_batch(const PinBatch& b, int n, float4* pin_target, float* pin_weight, float* pin_relax, int nV, cudaStream_t s) {
