@@ -2465,9 +2465,16 @@ bool tune_value_ok(int slot, int v) {
 int effective_tune(const Solver* S, int slot) {
     if (slot == kTuneFusedFrame) return fused_mode(S);
     if (slot == kTuneNeighborLanes) {
-        int n = 0;
-        for (int k = 0; k < S->K; ++k) n += S->cl[k].self_enabled && !S->cl[k].fast ? S->hp[k].V : 0;
-        return neighbor_lanes(S->tune, n);
+        if (S->tune.v[slot] > 0) return S->tune.v[slot];
+        // by size, of the fast cloths and of the strict ones each; 0 where the two differ
+        int lanes[2] = {0, 0};
+        for (const bool fast : {false, true}) {
+            int n = 0;
+            for (int k = 0; k < S->K; ++k) n += S->cl[k].self_enabled && S->cl[k].fast == fast ? S->hp[k].V : 0;
+            if (n > 0) lanes[fast] = neighbor_lanes(S->tune, n);
+        }
+        if (lanes[0] == 0 || lanes[1] == 0) return lanes[0] + lanes[1];
+        return lanes[0] == lanes[1] ? lanes[0] : 0;
     }
     return tune_of(S->tune, slot);
 }
@@ -2538,12 +2545,13 @@ bool autotune(Solver* S, int substeps, int iterations, int rounds, float* ms_out
         {64, 128, 256},   // dynamic colliders
         {8, 32},          // fast EE: groups of 8 lanes or flattened warps
         {1, 2, 8},        // small cloths: fused frame (block or cluster per cloth) or launched kernels
-        {1, 2, 4, 16},    // lanes per triangle of the triangle hash
+        {1, 2, 4, 8, 16}, // lanes per triangle of the triangle hash
         {1, 2, 4, 8},     // lanes per vertex of the neighbour table
     };
     const LaunchTune start = S->tune;
     LaunchTune best = start;
-    for (int k = 0; k < kTuneSlots; ++k) best.v[k] = (short)effective_tune(S, k);
+    for (int k = 0; k < kTuneSlots; ++k)
+        if (k != kTuneNeighborLanes) best.v[k] = (short)effective_tune(S, k);  // those stay by size until one value is faster
     S->tune = best;
     S->drop_graphs();
     float best_ms = 0.0f, default_ms = 0.0f;
