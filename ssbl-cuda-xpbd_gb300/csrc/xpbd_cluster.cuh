@@ -128,9 +128,10 @@ struct ClusterBarrier {
 };
 
 // Clusters of c CTAs of `threads` threads with `smem` bytes of dynamic shared
-// memory that fit this GPU at once (0: the shape cannot run).
+// memory that fit this GPU at once (0: the shape cannot run).  `limit` is the
+// most that any launch of the kernel asks for: one value for every call.
 template <class K>
-int cluster_fit(K kernel, int c, int threads, size_t smem) {
+int cluster_fit(K kernel, int c, int threads, size_t smem, size_t limit) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)c, 1, 1);
     cfg.blockDim = dim3((unsigned)threads, 1, 1);
@@ -143,7 +144,7 @@ int cluster_fit(K kernel, int c, int threads, size_t smem) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int fit = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();

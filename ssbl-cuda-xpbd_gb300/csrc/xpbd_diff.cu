@@ -981,8 +981,8 @@ bool plan_cluster(DiffSolver* D, const std::vector<int>& off, const std::vector<
     D->chunk = chunk;
     D->edge_rows = t.edge_rows;
     D->ent_rows = t.ent_rows;
-    if (diff_smem(D, true) > (size_t)kDiffSmem || cluster_fit(diff_kernel<false>(c, chunk), c, diff_threads(chunk), kDiffSmem) < 1 ||
-        cluster_fit(diff_kernel<true>(c, chunk), c, diff_threads(chunk), kDiffSmem) < 1) {
+    if (diff_smem(D, true) > (size_t)kDiffSmem || cluster_fit(diff_kernel<false>(c, chunk), c, diff_threads(chunk), kDiffSmem, kDiffSmem) < 1 ||
+        cluster_fit(diff_kernel<true>(c, chunk), c, diff_threads(chunk), kDiffSmem, kDiffSmem) < 1) {
         D->ctas = 0;
         return true;
     }

@@ -1617,7 +1617,7 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
                 cluster_tables(P.vstart, P.V, P.estart, P.E, S->frame.chunk, S->frame.ctas, sp_off.data(), ids.data(), &t);
             S->frame.edge_rows = t.edge_rows;
             S->frame.ent_rows = t.ent_rows;
-            if (!frame_fits(S->frame)) {
+            if (!frame_fits(K, &S->frame)) {
                 S->frame.ctas = 0;
             } else {
                 frame_tables = t.off;

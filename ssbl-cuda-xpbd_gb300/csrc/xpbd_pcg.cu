@@ -1125,7 +1125,7 @@ namespace {
 
 template <int T, int N, bool kOne>
 int hard_fit(int c) {
-    return cluster_fit(k_hard_cluster<T, N, kOne>, c, T, kHardSmem);
+    return cluster_fit(k_hard_cluster<T, N, kOne>, c, T, kHardSmem, kHardSmem);
 }
 
 template <int T, int N, bool kOne>

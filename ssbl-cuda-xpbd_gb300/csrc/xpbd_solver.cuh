@@ -462,17 +462,19 @@ void launch_frame_fused(const View& v, const FrameOp* ops, int nops, float4* buf
 void launch_frame_cluster(const View& v, const FrameOp* ops, int nops, float4* buf0, const int2* bend_ranges, int K, int cap,
                           int cluster, int block, cudaStream_t s);
 // The fused frame with an edge per thread: a cluster of `ctas` CTAs per cloth,
-// `chunk` vertices per CTA of the largest cloth; tables as ClusterTables.
+// `chunk` vertices per CTA of the largest cloth, `threads` threads per CTA;
+// tables as ClusterTables.
 struct FramePlan {
-    int ctas, chunk, edge_rows, ent_rows;
+    int ctas, chunk, threads, edge_rows, ent_rows;
     const int* off;
     const int* edge;
     const int* ent;
 };
 // Shape for K cloths of at most max_v vertices; false where the form is not
-// used.  Then, with the rows known, whether it fits the GPU.
+// used.  Then, with the rows known, the threads of a CTA; false where it does
+// not fit the GPU.
 bool frame_shape(int K, int max_v, FramePlan* f);
-bool frame_fits(const FramePlan& f);
+bool frame_fits(int K, FramePlan* f);
 // Runs operations [first, last) of the recorded frame from buffer 0 to buffer 0.
 cudaError_t launch_frame_edges(const View& v, const FramePlan& f, const FrameOp* ops, int first, int last, float4* buf0,
                                const int2* bend_ranges, int K, cudaStream_t s);

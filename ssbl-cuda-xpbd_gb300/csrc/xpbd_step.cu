@@ -1106,26 +1106,59 @@ constexpr int kFrameSmem = 220 * 1024;
 bool frame_shape(int K, int max_v, FramePlan* f) {
     f->ctas = 0;
     if (K < 1 || max_v < 1) return false;
-    // as many CTAs per cloth as keep every cloth resident at once, with at
-    // least 128 vertices each; past 768 vertices per CTA the launched passes
-    // are no slower (30 cloths of up to 64 x 64: 235 us launched, 232 here)
+    // as many CTAs per cloth as keep every cloth resident at once (of 16-CTA
+    // clusters, one per processing cluster), with at least 128 vertices each;
+    // past 768 vertices per CTA the launched passes are no slower (30 cloths
+    // of up to 64 x 64: 235 us launched, 232 here)
+    auto shape = [&](int c) {
+        f->ctas = c;
+        f->chunk = std::max((max_v + 32 * c - 1) / (32 * c), 1) * 32;
+    };
     int c = 1;
-    while (c < 16 && c * 128 < max_v && 2 * c * (long long)K <= 152) c *= 2;
-    f->chunk = std::max((max_v + 32 * c - 1) / (32 * c), 1) * 32;
-    if (f->chunk > (c == 1 ? 1024 : 768)) return false;
-    f->ctas = c;
-    return true;
+    while (c < 16 && c * 128 < max_v && 2 * c * (long long)K <= 152) {
+        shape(2 * c);
+        if (f->chunk <= 768 && cluster_fit(frame_kernel(*f).run, f->ctas, frame_kernel(*f).threads, kFrameSmem, kFrameSmem) < K) break;
+        c *= 2;
+    }
+    shape(c);
+    if (f->chunk > (c == 1 ? 1024 : 768)) f->ctas = 0;
+    return f->ctas > 0;
 }
 
-bool frame_fits(const FramePlan& f) {
-    const FrameShape k = frame_kernel(f);
-    return frame_smem(f) <= (size_t)kFrameSmem && cluster_fit(k.run, f.ctas, k.threads, kFrameSmem) >= 1;
+bool frame_fits(int K, FramePlan* f) {
+    const FrameShape k = frame_kernel(*f);
+    const size_t smem = frame_smem(*f);
+    if (smem > (size_t)kFrameSmem || cluster_fit(k.run, f->ctas, k.threads, kFrameSmem, kFrameSmem) < 1) return false;
+    auto warps = [](int n) { return (n + 31) / 32 * 32; };
+    f->threads = std::min(k.threads, warps(std::max(f->chunk, f->edge_rows)));
+    // More cloths than SMs: the shape with the fewest waves of resident
+    // clusters, from an edge per thread down to a thread per vertex with more
+    // rounds over the edges; of equal ones the most threads.  Us per frame
+    // with 512 threads for each cloth, k_frame_fused and so: 1,000 cloths of
+    // 8 x 8 294, 153, 74; 600 of 16 x 16 231, 194, 142; 160 of 8 x 8 87, 123,
+    // 48.
+    auto waves = [&](int threads) {
+        const int fit = std::max(cluster_fit(k.run, f->ctas, threads, smem, kFrameSmem), 1);
+        return (K + fit - 1) / fit;
+    };
+    if ((long long)K * f->ctas > 152) {
+        int best = waves(f->threads);
+        for (int rounds = 2, t = f->threads; best > 1 && t > f->chunk; ++rounds) {
+            t = std::max(f->chunk, warps((f->edge_rows + rounds - 1) / rounds));
+            const int w = waves(t);
+            if (w < best) {
+                best = w;
+                f->threads = t;
+            }
+        }
+    }
+    return true;
 }
 
 cudaError_t launch_frame_edges(const View& v, const FramePlan& f, const FrameOp* ops, int first, int last, float4* buf0,
                                const int2* bend_ranges, int K, cudaStream_t s) {
     const FrameShape k = frame_kernel(f);
-    return cluster_launch(k.run, K, f.ctas, k.threads, frame_smem(f), s, v, f, ops, first, last, buf0, bend_ranges, K);
+    return cluster_launch(k.run, K, f.ctas, f.threads, frame_smem(f), s, v, f, ops, first, last, buf0, bend_ranges, K);
 }
 
 // cluster > 1: one cluster of that many CTAs per cloth (block threads each)
