@@ -101,7 +101,7 @@ __attribute__((visibility("default"))) long long xpbd_gb300_pc2_close(void* writ
 /* Launch configuration (no counterpart in the reference): 12 slots, in order
  * block size of the per-vertex passes (default 128), of the hash count /
  * scatter kernels (256), lanes per primitive of the edge hash (1, 2, 4, 8
- * or 16; default 8), block size of the warp-per-item kernels (256), of
+ * or 16; default 4 up to 307,200 edges, then 8), block size of the warp-per-item kernels (256), of
  * the thread-per-item queries (256), lanes per item of the strict group
  * queries (4, 8 or 16; default 8), block size of the group queries (256), of
  * the dynamic-collider pass (128), the form of the fast-mode edge-edge query
@@ -113,8 +113,8 @@ __attribute__((visibility("default"))) long long xpbd_gb300_pc2_close(void* writ
  * hold the full state and exchange it (8; at most 1024 vertices), or launched
  * kernels (2), lanes per primitive of the triangle hash (1, 2, 4, 8 or 16;
  * default 1), and lanes per vertex of the neighbour table and strict VV
- * responses (1, 2, 4, 8, 16 or 32; default by the number of vertices of the fast and of the strict
- * cloths; reported as 0 where the two differ).  Block sizes
+ * responses (1, 2, 4, 8, 16 or 32; default by the number of vertices of the
+ * fast and of the strict cloths; reported as 0 where the two differ).  Block sizes
  * are multiples of 32 up to 256; 0 selects the default.  No value changes a
  * result.  Setting drops the captured frame graphs. */
 __attribute__((visibility("default"))) int xpbd_gb300_set_launch_config(void* handle, const int* values, int count);

@@ -2464,6 +2464,11 @@ bool tune_value_ok(int slot, int v) {
 
 int effective_tune(const Solver* S, int slot) {
     if (slot == kTuneFusedFrame) return fused_mode(S);
+    if (slot == kTunePrimLanes) {
+        long long n = 0;
+        for (int k = 0; k < S->K; ++k) n += S->cl[k].self_enabled ? S->hp[k].E : 0;
+        return edge_lanes(S->tune, n);
+    }
     if (slot == kTuneNeighborLanes) {
         if (S->tune.v[slot] > 0) return S->tune.v[slot];
         // by size, of the fast cloths and of the strict ones each; 0 where the two differ

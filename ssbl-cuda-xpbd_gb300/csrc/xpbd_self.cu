@@ -2886,9 +2886,21 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
     }
 }
 
-// Items per warp of a flattened query over n items: 8 up to `few`, 16 up to
-// `some`, then 32.  The warps' rounds are a chain of dependent loads, so while
-// the chip has room for more warps fewer items each are faster.
+// Vertices per warp of the flattened VT query.  Up to some 16,000 vertices
+// another branch of the frame is the longest whatever it takes, so it packs its
+// warps full and leaves the GPU to that branch and to other solvers; then it is
+// the longest itself, and fewer vertices per warp shorten its chain of
+// dependent rounds, until the chip has more warps than it can hold either way.
+// Us per strict frame with 8, 16 and 32: 100 x 100 1,005, 999, 999; 140 x 140
+// 1,818, 1,821, 1,840; 160 x 160 2,485, 2,626, 2,808; 200 x 200 4,896, 5,195,
+// 6,034; 300 x 300 17,645, 17,844, 18,648; 400 x 400 34,260, 35,417, 36,316;
+// 450 x 450 38,441, 38,354, 38,655.  16 handles of 100 x 100 at once 6,669,
+// 6,466, 6,345.
+int vt_items(int n) { return n > (16 << 10) && n <= (192 << 10) ? 8 : 32; }
+
+// Items per warp of a flattened edge-edge query over n items: 8 up to `few`, 16
+// up to `some`, then 32.  The warps' rounds are a chain of dependent loads, so
+// while the chip has room for more warps fewer items each are faster.
 int flat_items(int n, int few, int some) { return n < few ? 8 : (n < some ? 16 : 32); }
 
 void flat_launch(void (*kernel)(View, int), const View& v, const ItemRange& r, int b, int per_warp, cudaStream_t s) {
@@ -2961,8 +2973,8 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
     const ItemRange& items = sv.e_all;
     if (items.size() == 0) return;
     const View iv = ranged(v, items);
-    const int b = tune_of(v.tune, kTuneHashBlock), lanes = tune_of(v.tune, kTunePrimLanes);
     const long long n = items.size();
+    const int b = tune_of(v.tune, kTuneHashBlock), lanes = edge_lanes(v.tune, n);
     switch (lanes) {
         case 1: k_edge_insert<1><<<grid(n, 1, b), b, kBuildShared, s>>>(iv); break;
         case 2: k_edge_insert<2><<<grid(n, 2, b), b, kBuildShared, s>>>(iv); break;
@@ -2985,6 +2997,11 @@ void self_build_edge_hash(const View& v, const SelfVariants& sv, int nb, int ord
 int neighbor_lanes(const LaunchTune& t, int vertices) {
     if (t.v[kTuneNeighborLanes] > 0) return t.v[kTuneNeighborLanes];
     return vertices < (6 << 10) ? 8 : (vertices < (20 << 10) ? 4 : (vertices < (48 << 10) ? 2 : 1));
+}
+
+int edge_lanes(const LaunchTune& t, long long edges) {
+    if (t.v[kTunePrimLanes] > 0) return t.v[kTunePrimLanes];
+    return edges <= (300 << 10) ? 4 : 8;
 }
 
 void self_neighbors(const View& v, int mode, const SelfVariants& sv, cudaStream_t s) {
@@ -3014,7 +3031,7 @@ void self_vv(const View& v, const SelfVariants& sv, cudaStream_t s) {
 void self_vt(const View& v, const SelfVariants& sv, cudaStream_t s) {
     const int wb = tune_of(v.tune, kTuneWarpBlock), qb = tune_of(v.tune, kTuneQueryBlock);
     if (sv.hashed_t && sv.strict_wide && sv.v_strict.size() > 0)
-        flat_launch(k_flat_vt, v, sv.v_strict, wb, flat_items(sv.v_strict.size(), 32 << 10, 32 << 10), s);
+        flat_launch(k_flat_vt, v, sv.v_strict, wb, vt_items(sv.v_strict.size()), s);
     if (sv.hashed_t && sv.strict_narrow && sv.v_strict.size() > 0) group_queries_lanes(v, sv, s, false);
     if (sv.hashed_t && sv.fast && sv.v_fast.size() > 0)
         k_vt_hash<<<grid(sv.v_fast.size(), 1, qb), qb, 0, s>>>(ranged(v, sv.v_fast));

@@ -244,7 +244,7 @@ struct HardPlan {
 enum TuneSlot {
     kTuneVertexBlock = 0,  // per-vertex constraint passes and prediction (default 128)
     kTuneHashBlock,        // hash count / scatter kernels (256)
-    kTunePrimLanes,        // lanes per primitive of the edge hash: 1, 2, 4, 8, 16 (8)
+    kTunePrimLanes,        // lanes per primitive of the edge hash: 1, 2, 4, 8, 16 (by size, edge_lanes)
     kTuneWarpBlock,        // warp-per-item kernels: neighbour table, strict VV, flat queries, bucket order (256)
     kTuneQueryBlock,       // thread-per-item queries: fast VV / VT, brute queries, islands, apply (256)
     kTuneGroupLanes,       // lanes per item of the strict group queries: 4, 8, 16 (8)
@@ -269,6 +269,14 @@ inline int tune_of(const LaunchTune& t, int slot) { return t.v[slot] > 0 ? t.v[s
 // vertices 616, 629, 739, 766; 10,000 901, 888, 923, 960; 40,000 1,961, 1,876,
 // 1,877, 1,885; 202,500 7,601, 7,262, 7,109, 7,023.
 int neighbor_lanes(const LaunchTune& t, int vertices);
+// Lanes per edge of the edge hash over so many edges.  An edge of a cloth spans
+// a few cells, so 8 lanes are half idle, and a GPU shared with other solvers
+// feels it; over many edges, whose insertions wait for memory, they keep more
+// of those in flight.  Us per frame with 8 and 4: strict 64 x 64 595, 608; 100 x
+// 100 814, 812; 200 x 200 4,581, 4,390; 450 x 450 of 1 cm edges 14,572, 14,776
+// (two frames); fast 100 x 100 940, 936; 300 x 300 15,294, 14,558; 256 handles
+// of 16 x 16 to 128 x 128 stepped at once 64,356, 61,515.
+int edge_lanes(const LaunchTune& t, long long edges);
 inline int grid_for(long long threads, int block) { return (int)((threads + block - 1) / block); }
 
 // Device pointers of one solver, passed by value to each kernel, plus the

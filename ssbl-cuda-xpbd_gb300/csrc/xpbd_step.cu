@@ -591,8 +591,11 @@ __global__ void __launch_bounds__(kThreads) k_vertex_pass_lanes(View v, unsigned
         }
 #pragma unroll
         for (int u = 0; u < L; ++u) {
-            const F3 du{__shfl_sync(0xffffffffu, d.x, u, L), __shfl_sync(0xffffffffu, d.y, u, L), __shfl_sync(0xffffffffu, d.z, u, L)};
-            const int uu = __shfl_sync(0xffffffffu, use, u, L);
+            // (only the first lane's sums count: its own correction needs no exchange)
+            const F3 du = u == 0 ? d
+                                 : F3{__shfl_down_sync(0xffffffffu, d.x, u, L), __shfl_down_sync(0xffffffffu, d.y, u, L),
+                                      __shfl_down_sync(0xffffffffu, d.z, u, L)};
+            const int uu = u == 0 ? use : __shfl_down_sync(0xffffffffu, use, u, L);
             if (uu & 1) s.p = s.p + du;
             if (uu & 2) s.prev = s.prev + du * 0.08f;
         }
@@ -888,7 +891,7 @@ __global__ void __launch_bounds__(256) k_frame_cluster(View base, const FrameOp*
 constexpr unsigned kEdgeFixed = 1u, kEdgeMine = 2u, kEdgeAddr = ~7u;
 
 template <int T, bool kOne>
-__global__ void __launch_bounds__(T, 1) k_frame_edges(View v, FramePlan f, const FrameOp* ops, int first, int last, float4* buf0,
+__global__ void __launch_bounds__(T, T == 384 ? 2 : 1) k_frame_edges(View v, FramePlan f, const FrameOp* ops, int first, int last, float4* buf0,
                                                       const int2* bend_ranges, int K) {
     extern __shared__ float4 sm[];
     __shared__ unsigned long long s_counter;
@@ -1096,6 +1099,13 @@ struct FrameShape {
 };
 FrameShape frame_kernel(const FramePlan& f) {
     if (f.ctas == 1) return f.chunk <= 512 ? FrameShape{k_frame_edges<512, true>, 512} : FrameShape{k_frame_edges<1024, true>, 1024};
+    // 129 to 288 vertices per CTA: two rounds over the edges by 512 threads or
+    // three by 384, of which an SM holds two blocks.  Us per frame of one cloth
+    // and of 64 handles stepped at once: 48 x 48 100 and 850, 98 and 475; 64 x
+    // 64 99 and 847, 100 and 502.  Up to 128 one round of 512 counts for more
+    // (40 x 40 76 and 655, 94 and 466), and so do two of 512 above (72 x 72
+    // 104 and 905, 123 and 629).
+    if (f.chunk > 128 && f.chunk <= 288) return FrameShape{k_frame_edges<384, false>, 384};
     return f.chunk <= 512 ? FrameShape{k_frame_edges<512, false>, 512} : FrameShape{k_frame_edges<768, false>, 768};
 }
 size_t frame_smem(const FramePlan& f) { return 3 * 16 * (size_t)f.chunk + 32 * (size_t)f.edge_rows + 4 * (size_t)f.ent_rows; }
@@ -1107,9 +1117,9 @@ bool frame_shape(int K, int max_v, FramePlan* f) {
     f->ctas = 0;
     if (K < 1 || max_v < 1) return false;
     // as many CTAs per cloth as keep every cloth resident at once (of 16-CTA
-    // clusters, one per processing cluster), with at least 128 vertices each;
-    // past 768 vertices per CTA the launched passes are no slower (30 cloths
-    // of up to 64 x 64: 235 us launched, 232 here)
+    // clusters, one per processing cluster), with at least 128 vertices each.
+    // Past 768 vertices per CTA the launched passes are no slower (30 cloths
+    // of up to 64 x 64: 235 us launched, 232 here).
     auto shape = [&](int c) {
         f->ctas = c;
         f->chunk = std::max((max_v + 32 * c - 1) / (32 * c), 1) * 32;
@@ -1214,11 +1224,18 @@ void launch_predict(const View& v, int V, cudaStream_t s) {
     if (V > 0) launch_carved(k_predict, grid_for(V, b), b, s, v.carve, false, v);
 }
 
-// Lanes per vertex of a stretch pass over V vertices.  Us per frame of a plain
-// cloth (with the host calls) with 1, 2, 4, 8 lanes: 10,000 vertices in a drop
-// 1,165, 1,103, 1,103, 1,099; 32,400 291, 241, 241, 276; 57,600 374, 319, 359,
-// 410; 90,000 457, 430, 479, 578; 202,500 733, 732, 866, 1,076.
-constexpr int kPassLanes8 = 16 << 10, kPassLanes4 = 32 << 10, kPassLanes2 = 128 << 10;
+// Lanes per vertex of a stretch pass over V vertices: more shorten the pass,
+// but a vertex's remaining stages take a warp's slot for each, which a GPU
+// shared with other solvers feels.  Us per frame of a plain cloth (launched
+// passes, with the host calls) with 1, 2, 4, 8 lanes: 1,600 vertices 214, 135,
+// 125, 118; 4,096 210, 136, 127, 120; 8,100 223, 147, 137, 132; 12,544 233, 150,
+// 138, 139; 32,400 235, 154, 167, 208.  Of handles stepped at once, 64 of 4,096
+// vertices 462, 445, 685, 1,069; 32 of 8,100 395, 399, 633, 994; 16 of 12,544
+// 340, 301, 477, 738; 16 of 32,400 609, 719, 1,168, 1,819; 4 of 202,500 872,
+// 1,138, 1,887, 3,023.  Small cloths in launched passes mostly have other,
+// longer, stages (self collision, dynamic colliders), whose chain the passes
+// lengthen: they keep their lanes.
+constexpr int kPassLanes8 = 2 << 10, kPassLanes4 = 12 << 10, kPassLanes2 = 128 << 10;
 
 // A kernel that waits by itself (wait_for_previous) may start while the one
 // before it drains: its launch and its first loads, of constraints and
