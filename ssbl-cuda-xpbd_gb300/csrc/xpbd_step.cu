@@ -1117,7 +1117,11 @@ bool frame_shape(int K, int max_v, FramePlan* f) {
     f->ctas = 0;
     if (K < 1 || max_v < 1) return false;
     // as many CTAs per cloth as keep every cloth resident at once (of 16-CTA
-    // clusters, one per processing cluster), with at least 128 vertices each.
+    // clusters, one per processing cluster), with at least 128 vertices each,
+    // past 256 vertices: the barriers between CTAs cost a small cloth more than
+    // they save.  Us per frame with the host calls at 64, 128 and 256 vertices
+    // per CTA: 144 vertices 81, 80, 65; 256 85, 84, 76; 576 84, 83, 96; 1,024
+    // 86, 86, 100.
     // Past 768 vertices per CTA the launched passes are no slower (30 cloths
     // of up to 64 x 64: 235 us launched, 232 here).
     auto shape = [&](int c) {
@@ -1125,7 +1129,7 @@ bool frame_shape(int K, int max_v, FramePlan* f) {
         f->chunk = std::max((max_v + 32 * c - 1) / (32 * c), 1) * 32;
     };
     int c = 1;
-    while (c < 16 && c * 128 < max_v && 2 * c * (long long)K <= 152) {
+    while (c < 16 && max_v > 256 && c * 128 < max_v && 2 * c * (long long)K <= 152) {
         shape(2 * c);
         if (f->chunk <= 768 && cluster_fit(frame_kernel(*f).run, f->ctas, frame_kernel(*f).threads, kFrameSmem, kFrameSmem) < K) break;
         c *= 2;

@@ -12,7 +12,8 @@ from xpbd_gb300.native import NativeXpbdSolver
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [44, 47, 67, 68])
+# 256 and 289 vertices: one CTA, four
+@pytest.mark.parametrize("n", [16, 17, 44, 47, 67, 68])
 @pytest.mark.parametrize("extras", [False, True])
 def test_fused_frame_threads(n, extras, gpu_lib, oracle_lib):
     frames.test_single(n, extras, gpu_lib, oracle_lib)
