@@ -397,7 +397,7 @@ struct DiffCluster {
     int frames, substeps, iterations;
     int colours;             // bend colours: order[colour[c] .. colour[c + 1])
     const int* cta_off;      // CTA's edges: cta_edge[cta_off[r] .. cta_off[r + 1])
-    const int* cta_edge;     // edge ids, increasing
+    const int* cta_edge;     // edge ids, those to other CTAs first
     const int2* ends;        // edge -> endpoints
     const int* cta_ent;      // per constraint entry: its edge's place among the CTA's | side bit
     const int* colour;
@@ -967,8 +967,8 @@ auto diff_kernel(int ctas, int chunk) -> void (*)(DView, DiffCluster) {
 }
 int diff_threads(int chunk) { return chunk <= 512 ? 512 : 768; }
 
-// Each CTA's edges (every edge of its vertices, increasing) and the place of
-// an entry's edge among them; uploads them.
+// Each CTA's edges (every edge of its vertices, those to other CTAs first) and
+// the place of an entry's edge among them; uploads them.
 bool plan_cluster(DiffSolver* D, const std::vector<int>& off, const std::vector<int2>& ent, const std::vector<int2>& ends) {
     const int V = D->V;
     int c = 1;

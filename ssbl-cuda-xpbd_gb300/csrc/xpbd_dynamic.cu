@@ -591,7 +591,7 @@ __device__ void dyn_particles(const View& v, const Params& P, const DynSet& D, i
 // bounds, corners), which a thread per vertex paid up to 343 cells in a row
 // for: 4,096 vertices on a 1,280-triangle mesh with 500 particles took 298 us
 // per launch, 16 launches per frame, 5.0 ms per frame with the uploads; spread
-// over a warp the rounds are independent, 0.70 ms per frame (11 launches).
+// over a warp the rounds are independent, 0.54 ms per frame (11 launches).
 __global__ void __launch_bounds__(kMaxBlock) k_dynamic(View v, int which, int per_warp) {
     __shared__ unsigned counts[kDCounts];
     if (threadIdx.x < kDCounts) counts[threadIdx.x] = 0u;

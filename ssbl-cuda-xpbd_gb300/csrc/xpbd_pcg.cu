@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(kThreads) k_cap_store(View v, const float4* po
 // thread.  The launched form is bound by its launches: 23 per solve and one
 // per cap colour and sweep (144 per substep on a 32 x 32 cloth), 2-3 us each
 // for work of well under 1 us.  Per frame, launched and cluster form: 32 x 32
-// with caps 4.4 -> 0.69 ms, 100 x 100 without 1.56 -> 0.71 ms.
+// with caps 4.4 -> 0.65 ms, 100 x 100 without 1.56 -> 0.66 ms.
 //
 // With the launches gone the steps are bound by load latency (600-800 cycles
 // to L2 for every dependent gather), so the cluster's shared memory holds

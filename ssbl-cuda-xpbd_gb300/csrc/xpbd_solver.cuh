@@ -232,7 +232,6 @@ struct HardPlan {
     int rows;            // matrix entries per CTA kept in shared memory
     const int2* edges;
     const float* rest;
-    int count;
     const int2* ranges;  // [colours x K]: first cap edge, count
     int colors;
 };
@@ -260,7 +259,7 @@ enum TuneSlot {
 struct LaunchTune {
     short v[kTuneSlots];
 };
-constexpr short kTuneDefault[kTuneSlots] = {128, 256, 8, 256, 256, 8, 256, 128, 32, 0, 1, 0};
+constexpr short kTuneDefault[kTuneSlots] = {128, 256, 0, 256, 256, 8, 256, 128, 32, 0, 1, 0};  // 0: rules of their own
 constexpr int kMaxBlock = 256;  // the kernels' launch bounds
 inline int tune_of(const LaunchTune& t, int slot) { return t.v[slot] > 0 ? t.v[slot] : kTuneDefault[slot]; }
 // Lanes per vertex of the neighbour table over so many vertices: fewer lanes

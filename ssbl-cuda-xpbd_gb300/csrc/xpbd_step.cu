@@ -517,18 +517,20 @@ __device__ __forceinline__ void vertex_pass_item(const View& v, int i, unsigned 
     finish_vertex(v, P, i, flags, inv_mass, dt, &s);
 }
 
+// A launch that was allowed to start before the one before it on the stream
+// ended (launch_carved, chained) waits here until that one has ended and its
+// writes are visible; any other launch passes at once.  Every thread of such a
+// kernel calls it, so that no launch ends before those ahead of it have.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The same pass with L lanes per vertex (32 / L vertices per warp) for the
 // stretch gather: lane u takes entries u, u + L, ... and the vertex's first
 // lane adds the corrections in entry order, so the sums are those of
 // vertex_pass_item.  A thread per vertex walks its six or so entries one after
 // another, each a load and a chain of a root and two quotients, while a cloth
-// of a few ten thousand vertices leaves most of the chip's warps unused.
-// A launch that was allowed to start before the one before it on the stream
-// ended (launch_carved, chained) waits here until that one has ended and its writes are
-// visible; any other launch passes at once.  Every thread of such a kernel
-// calls it, so that no launch ends before those ahead of it have.
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
+// of a few ten thousand vertices leaves most of the chip's warps unused (180 x
+// 180, launched, with the host calls: 235 us per frame with one lane, 154 with
+// two).
 template <int L>
 __global__ void __launch_bounds__(kThreads) k_vertex_pass_lanes(View v, unsigned flags) {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -885,9 +887,8 @@ __global__ void __launch_bounds__(256) k_frame_cluster(View base, const FrameOp*
 // are published by turns in two buffers, so an operation costs one cluster
 // barrier.  Counters are kept per thread and added at the end: a barrier would
 // wait for atomics in flight.  Per frame with the host calls, k_frame_fused or
-// launched kernels -> this form: 8 x 8 148 -> 84 us, 32 x 32 198 -> 119,
-// 64 x 64 246 -> 145, 110 x 110 263 -> 201; 150 cloths of 8 x 8 to 32 x 32
-// 177 -> 103.
+// launched kernels -> this form: 8 x 8 144 -> 61 us, 32 x 32 216 -> 86,
+// 64 x 64 248 -> 119, 110 x 110 258 -> 174; 150 cloths of 20 x 20 156 -> 72.
 constexpr unsigned kEdgeFixed = 1u, kEdgeMine = 2u, kEdgeAddr = ~7u;
 
 template <int T, bool kOne>
