@@ -2890,13 +2890,14 @@ void tri_hash(const View& v, const ItemRange& items, const ItemRange& buckets, c
 // another branch of the frame is the longest whatever it takes, so it packs its
 // warps full and leaves the GPU to that branch and to other solvers; then it is
 // the longest itself, and fewer vertices per warp shorten its chain of
-// dependent rounds, until the chip has more warps than it can hold either way.
-// Us per strict frame with 8, 16 and 32: 100 x 100 1,005, 999, 999; 140 x 140
-// 1,818, 1,821, 1,840; 160 x 160 2,485, 2,626, 2,808; 200 x 200 4,896, 5,195,
-// 6,034; 300 x 300 17,645, 17,844, 18,648; 400 x 400 34,260, 35,417, 36,316;
-// 450 x 450 38,441, 38,354, 38,655.  16 handles of 100 x 100 at once 6,669,
-// 6,466, 6,345.
-int vt_items(int n) { return n > (16 << 10) && n <= (192 << 10) ? 8 : 32; }
+// dependent rounds.  Past 32,768 a frame fills much of the GPU: fewer would
+// still gain alone, and lose where several solvers run.  Us per strict frame
+// with 8, 16 and 32: 100 x 100 1,005, 999, 999; 140 x 140 1,818, 1,821, 1,840;
+// 160 x 160 2,485, 2,626, 2,808; 200 x 200 4,896, 5,195, 6,034; 300 x 300 17,645,
+// 17,844, 18,648; 450 x 450 38,441, 38,354, 38,655.  16 handles of 100 x 100 at
+// once 6,669, 6,466, 6,345; the serving workload (1k to 250k vertices) with 8
+// or 16 from 32,768 on, and with 32: 280, 286 and 290 M vertex-substeps/s.
+int vt_items(int n) { return n > (16 << 10) && n <= (32 << 10) ? 8 : 32; }
 
 // Items per warp of a flattened edge-edge query over n items: 8 up to `few`, 16
 // up to `some`, then 32.  The warps' rounds are a chain of dependent loads, so

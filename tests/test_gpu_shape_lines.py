@@ -1,6 +1,6 @@
 """Both sides of the lines where a launch changes its shape by size: threads of
 the fused frame (128 and 288 vertices per CTA), vertices per warp of the flat
-VT query (16,384), lanes per edge of the edge hash (307,200 edges).  Handles
+VT query (16,384 and 32,768), lanes per edge of the edge hash (307,200 edges).  Handles
 stepped at once give what each gives alone."""
 import numpy as np
 import pytest
@@ -30,7 +30,7 @@ def _folded(n, mode):
     return sc, np.ascontiguousarray(p, np.float32)
 
 
-@pytest.mark.parametrize("n", [128, 129])
+@pytest.mark.parametrize("n", [128, 129, 181, 182])
 def test_flat_vt_items(n, gpu_lib, oracle_lib):
     sc, p = _folded(n, 2)
     gpu = NativeXpbdSolver(sc.cloth, sc.options, sc.static_triangles)
