@@ -158,11 +158,11 @@ def full_gather_bytes(kind: str, counters: dict) -> float | None:
 # launch of one profiled frame of the 64-cloth batch under ncu (cold caches:
 # ncu flushes them before each launch), divided by the slots that frame
 # evaluated (`--profile-frame`); scaled by the slots of the measured workload.
-EE_DRAM_BYTES_PER_SLOT = 14.4
+EE_DRAM_BYTES_PER_SLOT = 14.3
 # ... and per insertion of an edge-hash build (slot insertion, overflow
 # kernels, trim and bucket ordering) from the same capture: the frame's last
 # build over its insertions.
-EDGE_HASH_DRAM_BYTES_PER_ENTRY = 20.2
+EDGE_HASH_DRAM_BYTES_PER_ENTRY = 18.5
 
 
 def measured_traffic(kind: str, counters: dict, launches: int) -> float | None:
