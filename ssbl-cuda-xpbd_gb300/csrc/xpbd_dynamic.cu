@@ -799,6 +799,7 @@ bool finish_triangles(const DynCtx& c, DynHost& D, int T, bool signed_mode, bool
         if (!cuda_ok(cudaMemcpyAsync(got, D.small, sizeof(got), cudaMemcpyDeviceToHost, st), "dynamic triangle hash") ||
             !cuda_ok(cudaStreamSynchronize(st), "dynamic triangle hash"))
             return false;
+        if (c.S) stream_waited(c.S);
         const int occupancy = got[0], entries = got[1], large = got[2];
         scan_bucket_counts(D.tcount, D.tstart, nb, D.scan_tmp, st);
         if (entries > D.tent_cap) {

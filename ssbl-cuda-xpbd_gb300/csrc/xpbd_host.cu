@@ -1036,7 +1036,7 @@ bool download_positions(Solver* S, int cloth, float* out, int max_floats) {
         (!small && !cuda_ok(cudaMemcpyAsync(out, dst, bytes, cudaMemcpyDeviceToHost, S->stream), "download ABI41 positions")) ||
         !cuda_ok(cudaStreamSynchronize(S->stream), "download ABI41 positions"))
         return false;
-    S->io_used = S->staged_used = 0;
+    stream_waited(S);
     if (frame_lost(S)) return false;
     if (small) std::memcpy(out, small, bytes);
     return true;
@@ -2412,6 +2412,7 @@ bool step(Solver* S, int substeps, int iterations, int fetch_diagnostics, int fo
     if (force_sync || fetch_diagnostics) {
         const auto ts = std::chrono::high_resolution_clock::now();
         if (!cuda_ok(cudaStreamSynchronize(S->stream), "ABI41 solver step") || frame_lost(S)) return false;
+        stream_waited(S);
         S->diag.sync_ms = (float)ms_since(ts);
     }
     if (fetch_diagnostics && !fetch_counts(S, st)) return false;

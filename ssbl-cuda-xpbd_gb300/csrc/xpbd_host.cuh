@@ -403,6 +403,8 @@ void sdf_diagnostics(Solver* S);
 // pageable: copies of 10 KB from page-locked memory cost a frame with two
 // uploads 27 us more, kernels that read it 12 us.)
 bool staged_upload(Solver* S, void* dst, const void* src, size_t bytes, bool* direct, const char* what);
+// After a wait for the solver's stream: its copies' memory is free again.
+inline void stream_waited(Solver* S) { S->io_used = S->staged_used = 0; }
 // Whether a frame's cluster barrier gave up: the state is undefined from then
 // on, and calls that hand it out or go on from it fail until a reset of the
 // whole solver.  A read of host memory: call it after a wait.
