@@ -574,6 +574,7 @@ void free_solver(Solver* S) {
     dfree(S->cap_rest);
     dfree(S->stage);
     if (S->io) cudaFreeHost(S->io);
+    if (S->lost && S->lost != &S->lost_word) cudaFreeHost(S->lost);
     for (int k = 0; k < 3; ++k) {
         if (S->aux[k]) cudaStreamDestroy(S->aux[k]);
         if (S->ev_join[k]) cudaEventDestroy(S->ev_join[k]);
@@ -962,22 +963,17 @@ bool upload_fields(Solver* S, int cloth, const SsblXpbdForceField* fields, int c
 // moves 400 KB in 3 us.
 constexpr size_t kSmallTransfer = 64 << 10;
 
-// Behind it lies the word of frame_lost.
-bool small_memory(Solver* S) {
-    if (!S->io && cudaHostAlloc(reinterpret_cast<void**>(&S->io), kSmallTransfer + sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
-        cudaGetLastError();  // none to be had
-        S->io = nullptr;
-    }
-    return S->io != nullptr;
-}
-
 // Uploads take their places in it one after another and are only waited for
 // when it is full, so the cloths of a batch, placed one by one, cost a launch
 // each (180 cloths of 6 x 6 to 40 x 40 vertices: 13 -> 5 us a call).  A download
 // ends in a wait and leaves it empty.
 float* small_transfer(Solver* S, size_t bytes, bool upload) {
     if (bytes > kSmallTransfer) return nullptr;
-    if (!small_memory(S) || !upload) return S->io;
+    if (!S->io && cudaHostAlloc(reinterpret_cast<void**>(&S->io), kSmallTransfer, cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();  // none to be had: copy
+        S->io = nullptr;
+    }
+    if (!S->io || !upload) return S->io;
     if (S->io_used + bytes > kSmallTransfer) {
         if (!cuda_ok(cudaStreamSynchronize(S->stream), "upload positions")) return nullptr;
         S->io_used = 0;
@@ -1629,14 +1625,21 @@ Solver* create_solver(const SsblXpbdConfig* in_configs, const SsblXpbdMesh* in_m
             }
         }
     }
-    // the cluster forms report through host memory; without any, the launched forms run
+    // The cluster forms report through host memory: a word of the solver's own
+    // where the GPU reaches any (page-locked memory costs 0.3 ms per solver),
+    // else a page-locked one; without either, the launched forms run.
     if (ok && (S->frame.ctas > 0 || S->hard.cluster > 0)) {
-        if (small_memory(S)) {
-            S->lost = reinterpret_cast<int*>(S->io + kSmallTransfer / sizeof(float));
+        int device = 0, reaches = 0;
+        if (cudaGetDevice(&device) == cudaSuccess &&
+            cudaDeviceGetAttribute(&reaches, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess && reaches)
+            S->lost = &S->lost_word;
+        else if (cudaHostAlloc(reinterpret_cast<void**>(&S->lost), sizeof(int), cudaHostAllocMapped) != cudaSuccess)
+            S->lost = nullptr;
+        cudaGetLastError();
+        if (S->lost)
             *S->lost = 0;
-        } else {
+        else
             S->frame.ctas = S->hard.cluster = 0;
-        }
     }
     if (!ok) return bail(0, "");
     cudaStream_t st = S->stream;

@@ -278,7 +278,8 @@ struct Solver {
     float* io = nullptr;         // page-locked host memory of small transfers (kSmallTransfer bytes), from the first one on
     std::vector<char> staged;    // what staged_upload's copies read, from the first one on
     size_t staged_used = 0;      // bytes of it that copies not waited for may still read
-    int* lost = nullptr;         // behind `io`: set by a frame whose cluster barrier gave up (solvers with a cluster form)
+    int* lost = nullptr;         // set by a frame whose cluster barrier gave up (solvers with a cluster form)
+    int lost_word = 0;
     size_t io_used = 0;          // bytes of it that uploads not waited for may still be read from
 
     std::vector<float> h_w;      // effective inverse mass per vertex
