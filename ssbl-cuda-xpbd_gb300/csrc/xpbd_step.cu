@@ -1237,10 +1237,13 @@ void launch_predict(const View& v, int V, cudaStream_t s) {
 // 138, 139; 32,400 235, 154, 167, 208.  Of handles stepped at once, 64 of 4,096
 // vertices 462, 445, 685, 1,069; 32 of 8,100 395, 399, 633, 994; 16 of 12,544
 // 340, 301, 477, 738; 16 of 32,400 609, 719, 1,168, 1,819; 4 of 202,500 872,
-// 1,138, 1,887, 3,023.  Small cloths in launched passes mostly have other,
-// longer, stages (self collision, dynamic colliders), whose chain the passes
-// lengthen: they keep their lanes.
-constexpr int kPassLanes8 = 2 << 10, kPassLanes4 = 12 << 10, kPassLanes2 = 128 << 10;
+// 1,138, 1,887, 3,023.  With volume pressure 10,000 vertices take 193 us with 4
+// lanes and 195 with 2, 24 handles of them 621 and 429.  Frames with self
+// collision spend little of a shared GPU on their passes and wait for them
+// between longer stages, so they keep 4 lanes for longer (three fast frames of
+// a folded 100 x 100 cloth with 8 lanes and with 2: 2,819 and 2,860 us; with 8
+// and with 4: 2,799 and 2,813).
+constexpr int kPassLanes8 = 2 << 10, kPassLanes4 = 4608, kPassLanes4Self = 12 << 10, kPassLanes2 = 128 << 10;
 
 // A kernel that waits by itself (wait_for_previous) may start while the one
 // before it drains: its launch and its first loads, of constraints and
@@ -1262,7 +1265,7 @@ void launch_vertex_pass(const View& v, int V, unsigned flags, cudaStream_t s, bo
     };
     if ((flags & kPassSpring) && V <= kPassLanes8)
         lanes(k_vertex_pass_lanes<8>, 8);
-    else if ((flags & kPassSpring) && V <= kPassLanes4)
+    else if ((flags & kPassSpring) && V <= (v.carve >= 0 ? kPassLanes4Self : kPassLanes4))
         lanes(k_vertex_pass_lanes<4>, 4);
     else if ((flags & kPassSpring) && V <= kPassLanes2)
         lanes(k_vertex_pass_lanes<2>, 2);
