@@ -983,13 +983,15 @@ float* small_transfer(Solver* S, size_t bytes, bool upload) {
     return at;
 }
 
+constexpr size_t kStagedBytes = 1 << 20;
+
 bool staged_upload(Solver* S, void* dst, const void* src, size_t bytes, bool* direct, const char* what) {
     if (bytes == 0) return true;
-    if (bytes > kSmallTransfer) {
+    if (bytes > kStagedBytes) {
         *direct = true;
     } else {
-        S->staged.resize(kSmallTransfer);
-        if (S->staged_used + bytes > kSmallTransfer) {
+        S->staged.resize(kStagedBytes);
+        if (S->staged_used + bytes > kStagedBytes) {
             if (!cuda_ok(cudaStreamSynchronize(S->stream), what)) return false;
             S->staged_used = 0;
         }

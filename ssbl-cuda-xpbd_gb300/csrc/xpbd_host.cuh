@@ -396,13 +396,14 @@ bool scene_update(GlobalScene* G, const SsblXpbdGlobalDynamicSceneInputs* in);
 bool scene_attach(Solver* S, int cloth, GlobalScene* G, int source_id, int layer, int mode);
 void scene_detach(Solver* S, int cloth);
 void sdf_diagnostics(Solver* S);
-// A copy to the device on the solver's stream.  Up to kSmallTransfer bytes are
+// A copy to the device on the solver's stream.  Up to kStagedBytes are
 // copied from memory of the solver that is used again only after a wait; more
 // are read from `src` itself, which `direct` tells: the caller waits for the
 // stream before `src` changes.  (cudaMemcpyAsync may return before it has read
 // page-locked memory, and need not have read any other.  The solver's is
 // pageable: copies of 10 KB from page-locked memory cost a frame with two
-// uploads 27 us more, kernels that read it 12 us.)
+// uploads 27 us more, kernels that read it 12 us.  An upload of 6,000
+// triangles takes 111 us without a wait and 170 with one.)
 bool staged_upload(Solver* S, void* dst, const void* src, size_t bytes, bool* direct, const char* what);
 // After a wait for the solver's stream: its copies' memory is free again.
 inline void stream_waited(Solver* S) { S->io_used = S->staged_used = 0; }
